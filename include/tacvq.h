@@ -201,6 +201,28 @@ TACVQ_API int tacvq_decode_step(const uint16_t *q_f16, const void *k_rows, const
                                 int D, int G, int S, int K, int T_new, int64_t T_cap, tacvq_stream_t stream);
 
 /*
+ * The same step with everything that stays the same from token to token in one record (plain data, host memory, read
+ * during the call only).  With rope_table_f16 not NULL the codes are of PRE-rotary keys and attention rotates them as
+ * tacvq_attn_decode_rotary does (evaluate_mistral_longbench.py:113-118); the query is then the one already rotated
+ * at its own position.
+ * Argument errors are found before anything is launched.
+ */
+typedef struct tacvq_step_plan {
+    const uint16_t *ktab_f16, *vtab_f16;
+    const uint16_t *rope_table_f16;
+    uint8_t *kcodes, *vcodes;
+    int32_t *seq_start, *seq_end;
+    void *workspace;
+    size_t workspace_bytes;
+    int64_t window, T_cap;
+    int B, Hq, Hkv, D, G, S, K;
+} tacvq_step_plan;
+
+TACVQ_API int tacvq_decode_step_planned(const tacvq_step_plan *plan, const uint16_t *q_f16, const void *k_rows, const void *v_rows,
+                                        int rows_dtype, int T_new, int64_t length, uint16_t *out_f16, float *state_out,
+                                        tacvq_stream_t stream);
+
+/*
  * tacvq_decode_step for a host that holds the new token's rows and wants the result in HOST memory: one call
  * enqueues the host-to-device copy of the rows, the decode step and the device-to-host copy of the result,
  * and optionally waits for the stream.  It covers one iteration of the reference's generation loop around

@@ -30,6 +30,7 @@ _SIGNATURES = {
     "tacvq_attn_decode": (c_int, [c_void_p] * 8 + [c_size_t, c_void_p, c_void_p] + [c_int] * 7 + [c_int64, c_void_p]),
     "tacvq_decode_step": (c_int, [c_void_p, c_void_p, c_void_p, c_int] + [c_void_p] * 6 + [c_int64, c_int64, c_void_p, c_size_t,
                                   c_void_p, c_void_p] + [c_int] * 8 + [c_int64, c_void_p]),
+    "tacvq_decode_step_planned": (c_int, [c_void_p] * 4 + [c_int, c_int, c_int64, c_void_p, c_void_p, c_void_p]),
     "tacvq_decode_step_host": (c_int, [c_void_p, c_void_p, c_int] + [c_void_p] * 6 + [c_int64, c_int64, c_void_p, c_size_t,
                                        c_void_p, c_void_p] + [c_int] * 8 + [c_int64, c_int, c_void_p]),
     "tacvq_set_ranges": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
@@ -41,6 +42,16 @@ _SIGNATURES = {
 }
 
 EXPORTS = tuple(_SIGNATURES)
+
+
+class StepPlan(ctypes.Structure):
+    """``tacvq_step_plan``: what stays the same from token to token of a decoding loop."""
+
+    _fields_ = (
+        [(name, c_void_p) for name in ("ktab", "vtab", "rope", "kcodes", "vcodes", "seq_start", "seq_end", "workspace")]
+        + [("workspace_bytes", c_size_t), ("window", c_int64), ("t_cap", c_int64)]
+        + [(name, c_int) for name in ("b", "hq", "hkv", "d", "g", "s", "k")]
+    )
 
 
 class TacvqError(RuntimeError):

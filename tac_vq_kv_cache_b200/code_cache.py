@@ -19,6 +19,8 @@ kernel (keys are stored as encoded).
 
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import ops
@@ -70,7 +72,7 @@ class VQCodeCache:
         self._range = torch.zeros(2, batch, dtype=torch.int32, device=self.device)  # [start; end) per row
         self._range_is = (0, 0)
         self._workspace: torch.Tensor | None = None
-        self._step_key, self._step_args = None, None  # decode_step's checked and marshalled arguments
+        self._plans: dict[int, tuple] = {}  # query heads -> (record of everything that decode_step passes every time, its workspace)
         self._host_key, self._host_call = None, None  # decode_step_host's
         self.rope = None if rope_theta is None else ops.rope_table(self.max_tokens, self.dim, float(rope_theta), self.device)
 
@@ -111,74 +113,72 @@ class VQCodeCache:
         if (start, end) != self._range_is:
             ops.set_ranges(self._range[0], self._range[1], start, end)
             self._range_is = (start, end)
-        if self._workspace is None:
-            need = ops.attn_workspace_bytes(self.batch, int(query.shape[1]), self.heads, self.dim, self.groups, self.stages)
-            if need == 0:
-                raise ValueError("attention geometry not supported")
-            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
         out, state = ops.attn_decode(
             query, self.key, self.value, self.key_tables, self.value_tables, self._range[0], self._range[1],
-            workspace=self._workspace, want_state=want_state, rope=self.rope,
+            workspace=self._scratch(int(query.shape[1])), want_state=want_state, rope=self.rope,
         )
         return (out, state) if want_state else out
 
     def decode_step(self, query: torch.Tensor, raw_key: torch.Tensor, raw_value: torch.Tensor, out: torch.Tensor | None = None):
         """Append the new token rows and attend, in one library call (``append`` + ``attend`` fused).
 
-        ``query [B,Hq,D]`` fp16 scaled, ``raw_key`` / ``raw_value`` ``[B,H,T_new,D]`` contiguous fp16 or fp32.
+        ``query [B,Hq,D]`` fp16 scaled (and rotated, for a cache of pre-rotary keys), ``raw_key`` / ``raw_value``
+        ``[B,H,T_new,D]`` contiguous fp16 or fp32.
         """
-        from . import _lib
-
-        if self.rope is not None:  # the fused call has no rotary step: append, then attend
-            self.append(raw_key, raw_value)
-            result = self.attend(query)
-            if out is not None:
-                out.copy_(result)
-                return out
-            return result
-        # A decoding loop calls this with the same buffers every step: the argument checks and the
-        # marshalling of everything but `length` are done once per set of buffers.
+        shape, q_shape = raw_key.shape, query.shape
+        if len(shape) != 4 or shape != raw_value.shape or shape[0] != self.batch or shape[1] != self.heads or shape[3] != self.dim:
+            raise ValueError("rows must be [B,H,T,D] matching the cache geometry")
+        if len(q_shape) != 3 or q_shape[0] != self.batch or q_shape[2] != self.dim or query.dtype != torch.float16:
+            raise ValueError("query must be fp16 [B,Hq,D]")
+        if raw_key.dtype != raw_value.dtype or raw_key.dtype not in ops._DTYPE_TAG:
+            raise ValueError("rows must be of one dtype, fp16 or fp32")
         if not (raw_key.is_contiguous() and raw_value.is_contiguous() and query.is_contiguous()):
             raise ValueError("query and rows must be contiguous")
-        key = (query.data_ptr(), raw_key.data_ptr(), raw_value.data_ptr(), 0 if out is None else out.data_ptr(),
-               raw_key.dtype, raw_value.dtype, query.dtype, tuple(raw_key.shape), tuple(raw_value.shape), tuple(query.shape))
-        if key != self._step_key:
-            tokens = int(raw_key.shape[2])
-            if raw_key.shape != raw_value.shape or tuple(raw_key.shape[:2]) != (self.batch, self.heads) or raw_key.shape[3] != self.dim:
-                raise ValueError("rows must be [B,H,T,D] matching the cache geometry")
-            if raw_key.dtype != raw_value.dtype:
-                raise ValueError("rows must be of one dtype")
-            ops._require_cuda(query, raw_key, raw_value, out)
-            hq = int(query.shape[1])
-            if tuple(query.shape) != (self.batch, hq, self.dim) or query.dtype != torch.float16:
-                raise ValueError("query must be fp16 [B,Hq,D]")
-            if out is not None and (tuple(out.shape) != (self.batch, hq, self.dim) or out.dtype != torch.float16 or not out.is_contiguous()):
-                raise ValueError("out must be contiguous fp16 [B,Hq,D]")
-            if self._workspace is None:
-                need = ops.attn_workspace_bytes(self.batch, hq, self.heads, self.dim, self.groups, self.stages)
-                if need == 0:
-                    raise ValueError("attention geometry not supported")
-                self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
-            head = (query.data_ptr(), raw_key.data_ptr(), raw_value.data_ptr(), ops._DTYPE_TAG[raw_key.dtype],
-                    self.key_tables.data_ptr(), self.value_tables.data_ptr(), self.key.data_ptr(), self.value.data_ptr(),
-                    self._range[0].data_ptr(), self._range[1].data_ptr())
-            tail = (self.batch, hq, self.heads, self.dim, self.groups, self.stages, int(self.key_tables.shape[-2]), tokens,
-                    self.max_tokens)
-            self._step_key, self._step_args = (key if out is not None else None), (head, tail, tokens, hq)
-        head, tail, tokens, hq = self._step_args
+        device = self.key.device
+        if query.device != device or raw_key.device != device or raw_value.device != device:
+            ops._require_cuda(self.key, query, raw_key, raw_value)
+        if out is None:
+            out = torch.empty(q_shape, dtype=torch.float16, device=device)
+        elif out.shape != q_shape or out.dtype != torch.float16 or not out.is_contiguous() or out.device != device:
+            raise ValueError("out must be contiguous fp16 [B,Hq,D] on the cache's device")
+        tokens = shape[2]
         if self.length + tokens > self.max_tokens:
             raise ValueError("code cache is full")
-        if out is None:
-            out = torch.empty(self.batch, hq, self.dim, dtype=torch.float16, device=self.device)
-        with ops._on(self.device):
-            status = _lib.load().tacvq_decode_step(
-                *head, self.length, 0 if self.window is None else self.window, self._workspace.data_ptr(),
-                self._workspace.numel(), out.data_ptr(), 0, *tail, ops._stream(self.device),
-            )
-        _lib.check("tacvq_decode_step", status)
+        plan = self._plans.get(q_shape[1]) or self._plan(int(q_shape[1]))
+        with ops._on(device):
+            status = plan[0](plan[1], query.data_ptr(), raw_key.data_ptr(), raw_value.data_ptr(), ops._DTYPE_TAG[raw_key.dtype], tokens,
+                             self.length, out.data_ptr(), None, _raw_stream(device.index))
+        if status:
+            from . import _lib
+
+            _lib.check("tacvq_decode_step_planned", status)
         self.length += tokens
         self._range_is = self.visible()
         return out
+
+    def _plan(self, q_heads: int) -> tuple:
+        """The library's step call and the record it reads, for steps with ``q_heads`` query heads."""
+        from . import _lib
+
+        ops._require_cuda(self.key)
+        workspace = self._scratch(q_heads)
+        record = _lib.StepPlan(
+            ktab=self.key_tables.data_ptr(), vtab=self.value_tables.data_ptr(), rope=ops._ptr(self.rope), kcodes=self.key.data_ptr(), vcodes=self.value.data_ptr(),
+            seq_start=self._range[0].data_ptr(), seq_end=self._range[1].data_ptr(), workspace=workspace.data_ptr(),
+            workspace_bytes=workspace.numel(), window=self.window or 0, t_cap=self.max_tokens, b=self.batch, hq=q_heads, hkv=self.heads,
+            d=self.dim, g=self.groups, s=self.stages, k=int(self.key_tables.shape[-2]),
+        )
+        self._plans[q_heads] = (_lib.load().tacvq_decode_step_planned, ctypes.byref(record), record, workspace)
+        return self._plans[q_heads]
+
+    def _scratch(self, q_heads: int) -> torch.Tensor:
+        """The attention workspace, large enough for ``q_heads`` query heads (kept; only ever replaced by a larger one)."""
+        need = ops.attn_workspace_bytes(self.batch, q_heads, self.heads, self.dim, self.groups, self.stages)
+        if need == 0:
+            raise ValueError("attention geometry not supported")
+        if self._workspace is None or self._workspace.numel() < need:
+            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
+        return self._workspace
 
     def decode_step_host(self, host_rows: torch.Tensor, host_out: torch.Tensor, q_heads: int, *, tokens: int = 1,
                          synchronize: bool = True, direct: bool | str = False) -> torch.Tensor:
@@ -231,18 +231,14 @@ class VQCodeCache:
             raise ValueError("host buffers must be fp16")
         if host_rows.numel() != nq + 2 * nkv or host_out.numel() != nq or not (host_rows.is_contiguous() and host_out.is_contiguous()):
             raise ValueError("host_rows must hold q, K rows and V rows back to back; host_out must be [B,Hq,D]")
-        if self._workspace is None:
-            need = ops.attn_workspace_bytes(self.batch, q_heads, self.heads, self.dim, self.groups, self.stages)
-            if need == 0:
-                raise ValueError("attention geometry not supported")
-            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
+        workspace = self._scratch(q_heads)
         dev_rows = None if direct == "rows" else torch.empty(nq + 2 * nkv, dtype=torch.float16, device=self.device)
         dev_out = None if direct else torch.empty(nq, dtype=torch.float16, device=self.device)
         args = [host_rows.data_ptr(), ops._ptr(dev_rows), ops._DTYPE_TAG[torch.float16], self.key_tables.data_ptr(),
                 self.value_tables.data_ptr(), self.key.data_ptr(), self.value.data_ptr(), self._range[0].data_ptr(),
-                self._range[1].data_ptr(), 0, 0 if self.window is None else self.window, self._workspace.data_ptr(),
-                self._workspace.numel(), ops._ptr(dev_out), host_out.data_ptr(), self.batch, q_heads, self.heads, self.dim,
+                self._range[1].data_ptr(), 0, 0 if self.window is None else self.window, workspace.data_ptr(),
+                workspace.numel(), ops._ptr(dev_out), host_out.data_ptr(), self.batch, q_heads, self.heads, self.dim,
                 self.groups, self.stages, int(self.key_tables.shape[-2]), tokens, self.max_tokens, 1, 0]
         index = self.device.index if self.device.index is not None else torch.cuda.current_device()
-        self._host_buffers = (dev_rows, dev_out)  # keep the landing buffers alive
+        self._host_buffers = (dev_rows, dev_out, workspace)  # keep what the call points at alive
         self._host_call = (args, _lib.load().tacvq_decode_step_host, index)

@@ -36,9 +36,9 @@ int attn_gsrq_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vc
                        __half *out, float *state_out, int B, int Hq, int Hkv, int64_t T_cap, int sms,
                        cudaStream_t stream, const GsrqNewToken *fresh = nullptr);
 int decode_prologue_dispatch(const void *k_rows, const void *v_rows, int rows_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
-                             const __half *ktab, const __half *vtab, uint8_t *kcodes, uint8_t *vcodes, int32_t *seq_start,
-                             int32_t *seq_end, int start, int end, int B, int H, int T, int D, int G, int S, int K, int64_t t0,
-                             int64_t T_cap, cudaStream_t stream);
+                             const __half *ktab, const __half *vtab, uint8_t *kcodes,
+                             uint8_t *vcodes, int32_t *seq_start, int32_t *seq_end, int start, int end, int B, int H, int T, int D,
+                             int G, int S, int K, int64_t t0, int64_t T_cap, cudaStream_t stream);
 
 int attn_rotary_splits(int B, int Hkv, int64_t T_cap, int sms);
 bool attn_rotary_staged_supported(int Hq, int Hkv, int D, int G, int S, int K);
@@ -329,65 +329,73 @@ int tacvq_set_ranges(int32_t *seq_start, int32_t *seq_end, int B, int start, int
     return launch_status();
 }
 
+// One decode step: the new rows of both sides encoded into the code buffers, the visible ranges set, attention.
+static int decode_step(const tacvq_step_plan &p, const uint16_t *q_f16, const void *k_rows, const void *v_rows, int rows_dtype,
+                       int T_new, int64_t length, uint16_t *out_f16, float *state_out, tacvq_stream_t stream) {
+    if (!k_rows || !v_rows || !p.seq_start || !p.seq_end) return TACVQ_ERR_NULL;
+    if (length < 0 || p.window < 0 || T_new <= 0 || length + T_new > p.T_cap) return TACVQ_ERR_RANGE;
+    if (!q_f16 || !p.ktab_f16 || !p.vtab_f16 || !p.kcodes || !p.vcodes || (!out_f16 && !state_out)) return TACVQ_ERR_NULL;
+    if (!dtype_ok(rows_dtype)) return TACVQ_ERR_DTYPE;
+    int st = check_code_geometry(p.B, p.Hkv, T_new, p.D, p.G, p.S, p.K, length, p.T_cap);
+    if (st == TACVQ_OK) st = check_attn_geometry(p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K);
+    if (st != TACVQ_OK) return st;
+    if (p.rope_table_f16 && p.D < 64) return TACVQ_ERR_UNSUPPORTED;
+    if (p.T_cap > 0x7fffffff) return TACVQ_ERR_RANGE;
+    if (!p.workspace || ((uintptr_t)p.workspace & 255) != 0 ||
+        p.workspace_bytes < tacvq_attn_workspace_bytes(p.B, p.Hq, p.Hkv, p.D, p.G, p.S))
+        return TACVQ_ERR_WORKSPACE;
+    if (((((uintptr_t)p.kcodes | (uintptr_t)p.vcodes) & 15) != 0 && !p.rope_table_f16) || ((uintptr_t)p.rope_table_f16 & 3) != 0)
+        return TACVQ_ERR_ALIGN;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int end = (int)(length + T_new), start = p.window > 0 && end > p.window ? (int)(end - p.window) : 0;
+    const __half *ktab = (const __half *)p.ktab_f16, *vtab = (const __half *)p.vtab_f16;
+    if (!p.rope_table_f16 && T_new == 1 && ((((uintptr_t)k_rows | (uintptr_t)v_rows) & 15) == 0) &&
+        attn_gsrq_supported(p.Hq, p.Hkv, p.D, p.G, p.S, p.K) && gsrq_batch_ok(p.B, p.Hkv) && gsrq_aligned(q_f16, ktab, vtab)) {
+        // benchmark geometry, one new token: the table preparation encodes the token and sets the ranges
+        // itself, so the whole step is two launches
+        const GsrqNewToken token = {k_rows, v_rows, rows_dtype == TACVQ_F32 ? 1 : 0, p.kcodes, p.vcodes, p.seq_start, p.seq_end,
+                                    start, end, (long long)length, (long long)p.T_cap};
+        const int fast = attn_gsrq_dispatch((const __half *)q_f16, p.kcodes, p.vcodes, ktab, vtab, p.seq_start, p.seq_end,
+                                            p.workspace, (__half *)out_f16, state_out, p.B, p.Hq, p.Hkv, p.T_cap, sm_count(), s,
+                                            &token);
+        if (fast != TACVQ_ERR_UNSUPPORTED) return fast;
+    }
+    // one launch for a handful of rows, otherwise three
+    const int64_t row = (int64_t)T_new * p.D;
+    st = decode_prologue_dispatch(k_rows, v_rows, rows_dtype, (int64_t)p.Hkv * row, row, p.D, ktab, vtab,
+                                   p.kcodes, p.vcodes, p.seq_start, p.seq_end, start, end, p.B, p.Hkv, T_new, p.D,
+                                  p.G, p.S, p.K, length, p.T_cap, s);
+    if (st == TACVQ_ERR_UNSUPPORTED) {
+        st = tacvq_encode(k_rows, rows_dtype, (int64_t)p.Hkv * row, row, p.D, p.ktab_f16, nullptr, p.kcodes, nullptr, TACVQ_F16,
+                          p.B, p.Hkv, T_new, p.D, p.G, p.S, p.K, length, p.T_cap, stream);
+        if (st == TACVQ_OK)
+            st = tacvq_encode(v_rows, rows_dtype, (int64_t)p.Hkv * row, row, p.D, p.vtab_f16, nullptr, p.vcodes, nullptr,
+                              TACVQ_F16, p.B, p.Hkv, T_new, p.D, p.G, p.S, p.K, length, p.T_cap, stream);
+        if (st == TACVQ_OK) st = tacvq_set_ranges(p.seq_start, p.seq_end, p.B, start, end, stream);
+    }
+    if (st != TACVQ_OK) return st;
+    if (p.rope_table_f16)
+        return tacvq_attn_decode_rotary(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.rope_table_f16, p.seq_start, p.seq_end,
+                                        p.workspace, p.workspace_bytes, out_f16, state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K,
+                                        p.T_cap, stream);
+    return tacvq_attn_decode(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.seq_start, p.seq_end, p.workspace,
+                             p.workspace_bytes, out_f16, state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K, p.T_cap, stream);
+}
+
+int tacvq_decode_step_planned(const tacvq_step_plan *plan, const uint16_t *q_f16, const void *k_rows, const void *v_rows,
+                              int rows_dtype, int T_new, int64_t length, uint16_t *out_f16, float *state_out, tacvq_stream_t stream) {
+    if (!plan) return TACVQ_ERR_NULL;
+    return decode_step(*plan, q_f16, k_rows, v_rows, rows_dtype, T_new, length, out_f16, state_out, stream);
+}
+
 int tacvq_decode_step(const uint16_t *q_f16, const void *k_rows, const void *v_rows, int rows_dtype,
                       const uint16_t *ktab_f16, const uint16_t *vtab_f16, uint8_t *kcodes, uint8_t *vcodes,
                       int32_t *seq_start, int32_t *seq_end, int64_t length, int64_t window, void *workspace,
                       size_t workspace_bytes, uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv, int D, int G,
                       int S, int K, int T_new, int64_t T_cap, tacvq_stream_t stream) {
-    if (!k_rows || !v_rows || !seq_start || !seq_end) return TACVQ_ERR_NULL;
-    if (length < 0 || window < 0 || T_new <= 0 || length + T_new > T_cap) return TACVQ_ERR_RANGE;
-    const int64_t row = (int64_t)T_new * D;
-    {
-        // Fast path: one launch encodes both sides and sets the ranges, and the attention kernels that do
-        // not read its results start while it runs.  Every argument check of the separate calls is made first.
-        const int64_t new_end = length + T_new;
-        const int64_t new_start = (window > 0 && new_end > window) ? new_end - window : 0;
-        const bool plain = dtype_ok(rows_dtype) && q_f16 && ktab_f16 && vtab_f16 && kcodes && vcodes && (out_f16 || state_out) &&
-                           check_code_geometry(B, Hkv, T_new, D, G, S, K, length, T_cap) == TACVQ_OK &&
-                           check_attn_geometry(B, Hq, Hkv, D, G, S, K) == TACVQ_OK && T_cap <= 0x7fffffff && workspace &&
-                           ((uintptr_t)workspace & 255) == 0 && workspace_bytes >= tacvq_attn_workspace_bytes(B, Hq, Hkv, D, G, S) &&
-                           (((uintptr_t)kcodes | (uintptr_t)vcodes) & 15) == 0;
-        if (plain) {
-            cudaStream_t s = (cudaStream_t)stream;
-            const bool gsrq = attn_gsrq_supported(Hq, Hkv, D, G, S, K) && gsrq_batch_ok(B, Hkv) && gsrq_aligned(q_f16, ktab_f16, vtab_f16);
-            if (gsrq && T_new == 1 && ((((uintptr_t)k_rows | (uintptr_t)v_rows) & 15) == 0)) {
-                // benchmark geometry, one new token: the table preparation encodes the token and sets the ranges
-                // itself, so the whole step is two launches
-                const GsrqNewToken token = {k_rows, v_rows, rows_dtype == TACVQ_F32 ? 1 : 0, kcodes, vcodes, seq_start, seq_end,
-                                            (int)new_start, (int)new_end, (long long)length, (long long)T_cap};
-                const int fast = attn_gsrq_dispatch((const __half *)q_f16, kcodes, vcodes, (const __half *)ktab_f16,
-                                                    (const __half *)vtab_f16, seq_start, seq_end, workspace, (__half *)out_f16,
-                                                    state_out, B, Hq, Hkv, T_cap, sm_count(), s, &token);
-                if (fast != TACVQ_ERR_UNSUPPORTED) return fast;
-            }
-            const int pro = decode_prologue_dispatch(k_rows, v_rows, rows_dtype, (int64_t)Hkv * row, row, D, (const __half *)ktab_f16,
-                                                     (const __half *)vtab_f16, kcodes, vcodes, seq_start, seq_end, (int)new_start,
-                                                     (int)new_end, B, Hkv, T_new, D, G, S, K, length, T_cap, s);
-            if (pro == TACVQ_OK) {
-                if (gsrq) {
-                    const int fast = attn_gsrq_dispatch((const __half *)q_f16, kcodes, vcodes, (const __half *)ktab_f16,
-                                                        (const __half *)vtab_f16, seq_start, seq_end, workspace,
-                                                        (__half *)out_f16, state_out, B, Hq, Hkv, T_cap, sm_count(), s);
-                    if (fast != TACVQ_ERR_UNSUPPORTED) return fast;
-                }
-                return tacvq_attn_decode(q_f16, kcodes, vcodes, ktab_f16, vtab_f16, seq_start, seq_end, workspace,
-                                         workspace_bytes, out_f16, state_out, B, Hq, Hkv, D, G, S, K, T_cap, stream);
-            }
-            if (pro != TACVQ_ERR_UNSUPPORTED) return pro;
-        }
-    }
-    int st = tacvq_encode(k_rows, rows_dtype, (int64_t)Hkv * row, row, D, ktab_f16, nullptr, kcodes, nullptr, TACVQ_F16, B,
-                          Hkv, T_new, D, G, S, K, length, T_cap, stream);
-    if (st != TACVQ_OK) return st;
-    st = tacvq_encode(v_rows, rows_dtype, (int64_t)Hkv * row, row, D, vtab_f16, nullptr, vcodes, nullptr, TACVQ_F16, B, Hkv,
-                      T_new, D, G, S, K, length, T_cap, stream);
-    if (st != TACVQ_OK) return st;
-    const int64_t end = length + T_new;
-    const int64_t start = (window > 0 && end > window) ? end - window : 0;
-    st = tacvq_set_ranges(seq_start, seq_end, B, (int)start, (int)end, stream);
-    if (st != TACVQ_OK) return st;
-    return tacvq_attn_decode(q_f16, kcodes, vcodes, ktab_f16, vtab_f16, seq_start, seq_end, workspace, workspace_bytes,
-                             out_f16, state_out, B, Hq, Hkv, D, G, S, K, T_cap, stream);
+    const tacvq_step_plan plan = {ktab_f16, vtab_f16, nullptr, kcodes, vcodes, seq_start, seq_end, workspace,
+                                  workspace_bytes, window, T_cap, B, Hq, Hkv, D, G, S, K};
+    return decode_step(plan, q_f16, k_rows, v_rows, rows_dtype, T_new, length, out_f16, state_out, stream);
 }
 
 // The device address of a host buffer that kernels may dereference in place (pinned or registered memory), or

@@ -23,6 +23,11 @@ namespace tacvq {
 
 int encode_tc8_launch(const EncodeArgs &a);
 int encode_tc_large_launch(const EncodeArgs &a);
+int encode_few_wide_launch(const EncodeArgs &a);
+int decode_prologue_wide_launch(const void *k_rows, const void *v_rows, int rows_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
+                                const __half *ktab, const __half *vtab, uint8_t *kcodes,
+                                uint8_t *vcodes, int32_t *seq_start, int32_t *seq_end, int start, int end, int B, int H, int T, int D,
+                                int G, int S, int K, int64_t t0, int64_t T_cap, cudaStream_t stream);
 
 // ------------------------------------------------------------------------------------------------
 // d <= 16
@@ -461,6 +466,11 @@ static int launch_large(const EncodeArgs &a) {
 
 constexpr int kFewRows = 32;  // at or below this many rows a warp per (row, head, group) wins
 
+// 32-, 64- and 128-wide groups: a block per (head, group) and four rows while that is at most two blocks per SM.
+// Measured, 8 heads, against a launch of 128-row tiles: 128 rows of 16 x 128 (256 blocks) 76 us against 102 us, 2 x 128
+// 15.5 against 18.1; 192 rows (384 blocks) 108 against 103 and 19.0 against 17.8.
+static bool few_wide_rows(int64_t rows, int64_t units) { return (rows + 3) / 4 * units <= 2 * 148; }
+
 template <typename XT, typename TT>
 static int dispatch_d(const EncodeArgs &a) {
     if constexpr (sizeof(TT) == 2) {
@@ -474,6 +484,10 @@ static int dispatch_d(const EncodeArgs &a) {
         }
         if (TACVQ_ENCODE_TC && (a.D / a.G == 8 || a.D / a.G == 4)) {
             const int st = encode_tc8_launch(a);
+            if (st != TACVQ_ERR_UNSUPPORTED) return st;
+        }
+        if (a.D / a.G >= 32 && few_wide_rows((int64_t)a.B * a.T, (int64_t)a.H * a.G)) {
+            const int st = encode_few_wide_launch(a);
             if (st != TACVQ_ERR_UNSUPPORTED) return st;
         }
         if (TACVQ_ENCODE_TC && a.D / a.G >= 32) {
@@ -498,12 +512,12 @@ static int dispatch_d(const EncodeArgs &a) {
     }
 }
 
-// Returns TACVQ_ERR_UNSUPPORTED when the step is not a handful of rows of narrow groups; the caller then
-// makes the three separate launches.
+// Returns TACVQ_ERR_UNSUPPORTED when the step is not a handful of rows, or of a group width without a kernel for
+// few rows; the caller then makes the three separate launches.
 int decode_prologue_dispatch(const void *k_rows, const void *v_rows, int rows_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
-                             const __half *ktab, const __half *vtab, uint8_t *kcodes, uint8_t *vcodes, int32_t *seq_start,
-                             int32_t *seq_end, int start, int end, int B, int H, int T, int D, int G, int S, int K, int64_t t0,
-                             int64_t T_cap, cudaStream_t stream) {
+                             const __half *ktab, const __half *vtab, uint8_t *kcodes,
+                             uint8_t *vcodes, int32_t *seq_start, int32_t *seq_end, int start, int end, int B, int H, int T, int D,
+                             int G, int S, int K, int64_t t0, int64_t T_cap, cudaStream_t stream) {
     if ((int64_t)B * T > kFewRows) return TACVQ_ERR_UNSUPPORTED;
 #define TACVQ_CASE(N)                                                                                                          \
     case N:                                                                                                                    \
@@ -516,7 +530,9 @@ int decode_prologue_dispatch(const void *k_rows, const void *v_rows, int rows_dt
         TACVQ_CASE(4)
         TACVQ_CASE(8)
         TACVQ_CASE(16)
-        default: return TACVQ_ERR_UNSUPPORTED;
+        default:
+            return decode_prologue_wide_launch(k_rows, v_rows, rows_dtype, sxb, sxh, sxt, ktab, vtab, kcodes, vcodes,
+                                               seq_start, seq_end, start, end, B, H, T, D, G, S, K, t0, T_cap, stream);
     }
 #undef TACVQ_CASE
 }

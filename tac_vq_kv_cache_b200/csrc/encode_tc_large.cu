@@ -28,11 +28,9 @@
 // Reference statements: src/jointkv/closed_loop_vq.py:52-76 (search), :343-395 (stage recursion).
 
 #include <atomic>
-#include <cstring>
-
-#include <cuda.h>  // CUtensorMap and the driver's encoder signature; the entry point is looked up at run time
 
 #include "common.cuh"
+#include "table_map.cuh"
 
 namespace tacvq {
 
@@ -1110,41 +1108,9 @@ encode_tm_large_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64
 #define TACVQ_ENCODE_TENSOR_MEMORY 2  // 2: residual tile in tensor memory; 1: scores only; 0: mma.sync from registers
 #endif
 
-// cuTensorMapEncodeTiled, looked up through the runtime so that the library does not link against the driver
-typedef CUresult (*TensorMapEncoder)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                     const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static TensorMapEncoder tensor_map_encoder() {
-    static const TensorMapEncoder found = [] {
-        void *entry = nullptr;
-        cudaDriverEntryPointQueryResult status;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &entry, cudaEnableDefault, &status) != cudaSuccess ||
-            status != cudaDriverEntryPointSuccess)
-            entry = nullptr;
-        return reinterpret_cast<TensorMapEncoder>(entry);
-    }();
-    return found;
-}
-
 // Launches whose tables had at least 256 words but got no tensor map (no encoder in the driver, or it refused):
 // added to the count that tacvq_encode_tensor_memory_timeouts reports, so a silent cp.async-only run shows up.
 static std::atomic<unsigned int> g_table_map_failures{0};
-
-// The fp16 tables as a 2-D tensor [all words][d] read in boxes of 256 words x 64 elements with the 128-byte swizzle.
-// Returns 0 when no map could be made (the kernel then copies tables with cp.async).
-static int make_table_map(CUtensorMap *map, const void *tables, int64_t words, int d) {
-    memset(map, 0, sizeof(*map));
-    const TensorMapEncoder encode = tensor_map_encoder();
-    if (encode == nullptr || words < kMaxWords) return 0;
-    const cuuint64_t dims[2] = {(cuuint64_t)d, (cuuint64_t)words};
-    const cuuint64_t strides[1] = {(cuuint64_t)d * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)kMaxWords};
-    const cuuint32_t steps[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(tables), dims, strides, box, steps,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 1 : 0;
-}
 
 template <int DSUB>
 static int launch_tc_large(const EncodeArgs &a) {
