@@ -123,6 +123,18 @@ TACVQ_API int tacvq_encode_whitened(const void *x, int x_dtype, int64_t sxb, int
                           int G, int S, int K, int64_t t0, int64_t T_cap, tacvq_stream_t stream);
 
 /*
+ * The same with room for what the tensor-core search of 64- and 128-wide groups filters with (the fp16 rounding of the
+ * transformed words and their norms): `filter` holds at least tacvq_encode_whitened_filter_bytes bytes, 256-byte
+ * aligned.  That is 0 for other widths, and `filter` may be NULL: the search is then the plain fp32 one.  Same codes.
+ */
+TACVQ_API size_t tacvq_encode_whitened_filter_bytes(int H, int D, int G, int S, int K);
+TACVQ_API int tacvq_encode_whitened_filtered(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
+                          const uint16_t *tables_f16, const float *whitener, float *search_tables,
+                          float *search_rows, void *filter, size_t filter_bytes, uint8_t *codes, void *recon,
+                          int recon_dtype, int B, int H, int T, int D, int G, int S, int K, int64_t t0, int64_t T_cap,
+                          tacvq_stream_t stream);
+
+/*
  * Decode: rebuild rows t0 .. t0+T-1 from stored codes using the first S_use stages.
  * Replaces _gather_words + the fp32 stage sum (closed_loop_vq.py:127-139, 376-381, 398-403),
  * _gather_group_words (cq_tac.py:21-30) and frozen_assignment_u16_reconstruction

@@ -14,6 +14,7 @@ int codeword_grad_dispatch(const uint8_t *codes, const float *grad_out, float *g
                            int G, int S, int S_use, int K, int64_t t0, int64_t T_cap, cudaStream_t stream);
 int table_sqnorm_dispatch(const __half *tables, float *out, int64_t words, int d, cudaStream_t stream);
 int tensor_memory_timeouts(unsigned int *out);
+int round_words_dispatch(const float *words32, __half *words16, float *norms, int64_t words, int d, cudaStream_t stream);
 int whiten_dispatch(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt, const __half *tables,
                     const float *whitener, float *search_tables, float *search_rows, int B, int H, int T, int D, int G,
                     int S, int K, cudaStream_t stream);
@@ -169,10 +170,19 @@ int tacvq_encode(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t s
     return encode_dispatch(a);
 }
 
-int tacvq_encode_whitened(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
-                          const uint16_t *tables_f16, const float *whitener, float *search_tables,
-                          float *search_rows, uint8_t *codes, void *recon, int recon_dtype, int B, int H, int T, int D,
-                          int G, int S, int K, int64_t t0, int64_t T_cap, tacvq_stream_t stream) {
+size_t tacvq_encode_whitened_filter_bytes(int H, int D, int G, int S, int K) {
+    if (H <= 0 || D <= 0 || G <= 0 || S <= 0 || K <= 0 || K > kMaxWords || D % G != 0) return 0;
+    const int d = D / G;
+    if (d != 64 && d != 128) return 0;  // the widths with a kernel that filters
+    const size_t words = (size_t)H * S * G * K;
+    return ((words * d * sizeof(__half) + 255) & ~(size_t)255) + words * sizeof(float);
+}
+
+int tacvq_encode_whitened_filtered(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
+                                   const uint16_t *tables_f16, const float *whitener, float *search_tables,
+                                   float *search_rows, void *filter, size_t filter_bytes, uint8_t *codes, void *recon,
+                                   int recon_dtype, int B, int H, int T, int D, int G, int S, int K, int64_t t0, int64_t T_cap,
+                                   tacvq_stream_t stream) {
     if (!dtype_ok(x_dtype) || (recon && !dtype_ok(recon_dtype))) return TACVQ_ERR_DTYPE;
     const int g = check_code_geometry(B, H, T, D, G, S, K, t0, T_cap);
     if (g != TACVQ_OK) return g;
@@ -180,13 +190,31 @@ int tacvq_encode_whitened(const void *x, int x_dtype, int64_t sxb, int64_t sxh, 
     if ((int64_t)B * T == 0) return TACVQ_OK;
     if (!x || !tables_f16 || !codes || !whitener || !search_tables || !search_rows) return TACVQ_ERR_NULL;
     if (sxb < 0 || sxh < 0 || sxt < D) return TACVQ_ERR_GEOMETRY;
+    const size_t need = filter ? tacvq_encode_whitened_filter_bytes(H, D, G, S, K) : 0;
+    if (need > 0 && (((uintptr_t)filter & 255) != 0 || filter_bytes < need)) return TACVQ_ERR_WORKSPACE;
     int st = whiten_dispatch(x, x_dtype, sxb, sxh, sxt, (const __half *)tables_f16, whitener, search_tables,
                              search_rows, B, H, T, D, G, S, K, (cudaStream_t)stream);
     if (st != TACVQ_OK) return st;
     EncodeArgs a{search_rows, TACVQ_F32, (int64_t)H * T * D, (int64_t)T * D, (int64_t)D, search_tables, true, nullptr,
                  codes, recon, recon_dtype, (const __half *)tables_f16, B, H, T, D, G, S, K, t0, T_cap,
                  (cudaStream_t)stream};
+    if (need > 0) {
+        const int64_t words = (int64_t)H * S * G * K;
+        float *norms = (float *)((unsigned char *)filter + need - words * sizeof(float));
+        st = round_words_dispatch(search_tables, (__half *)filter, norms, words, D / G, (cudaStream_t)stream);
+        if (st != TACVQ_OK) return st;
+        a.filter_tables = (const __half *)filter;
+        a.sqnorm = norms;
+    }
     return encode_dispatch(a);
+}
+
+int tacvq_encode_whitened(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
+                          const uint16_t *tables_f16, const float *whitener, float *search_tables,
+                          float *search_rows, uint8_t *codes, void *recon, int recon_dtype, int B, int H, int T, int D,
+                          int G, int S, int K, int64_t t0, int64_t T_cap, tacvq_stream_t stream) {
+    return tacvq_encode_whitened_filtered(x, x_dtype, sxb, sxh, sxt, tables_f16, whitener, search_tables, search_rows, nullptr, 0,
+                                          codes, recon, recon_dtype, B, H, T, D, G, S, K, t0, T_cap, stream);
 }
 
 int tacvq_decode(const uint8_t *codes, const uint16_t *tables_f16, void *out, int out_dtype, int B, int H, int T,

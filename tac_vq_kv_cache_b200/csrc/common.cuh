@@ -128,6 +128,7 @@ struct EncodeArgs {
     int B, H, T, D, G, S, K;
     int64_t t0, T_cap;
     cudaStream_t stream;
+    const __half *filter_tables = nullptr;  // fp16 rounding of fp32 search tables, for kernels that filter on the tensor core
 };
 
 // The new token of a decode step, handed to the benchmark-geometry attention when its table preparation

@@ -23,6 +23,7 @@ namespace tacvq {
 
 int encode_tc8_launch(const EncodeArgs &a);
 int encode_tc_large_launch(const EncodeArgs &a);
+int encode_wide_launch(const EncodeArgs &a);
 int encode_few_wide_launch(const EncodeArgs &a);
 int decode_prologue_wide_launch(const void *k_rows, const void *v_rows, int rows_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
                                 const __half *ktab, const __half *vtab, uint8_t *kcodes,
@@ -490,10 +491,14 @@ static int dispatch_d(const EncodeArgs &a) {
             const int st = encode_few_wide_launch(a);
             if (st != TACVQ_ERR_UNSUPPORTED) return st;
         }
-        if (TACVQ_ENCODE_TC && a.D / a.G >= 32) {
+        if (TACVQ_ENCODE_TC && a.D / a.G == 32) {
             const int st = encode_tc_large_launch(a);
             if (st != TACVQ_ERR_UNSUPPORTED) return st;
         }
+    }
+    if (TACVQ_ENCODE_TC && a.D / a.G >= 64) {
+        const int st = encode_wide_launch(a);
+        if (st != TACVQ_ERR_UNSUPPORTED) return st;
     }
     switch (a.D / a.G) {
         case 1: return launch_small<1, 4, XT, TT>(a);

@@ -206,4 +206,34 @@ int whiten_dispatch(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_
     return launch_status();
 }
 
+// Transformed words (d a multiple of 32) for a search that filters on the tensor core: their fp16 rounding, and |word|^2 in
+// the library's order, eight neighbouring lanes per word (lane j owns running sum j of each of the four sets).
+__global__ void __launch_bounds__(256)
+round_words_kernel(const float *__restrict__ words32, __half *__restrict__ words16, float *__restrict__ norms, int64_t words, int d) {
+    const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, j = lane & 7;
+    const int64_t word = slot >> 3;
+    const int64_t at = (word < words ? word : words - 1) * d;  // spare lanes redo the last word
+    float set[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int i = 0; i < d; i += 32) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float v = words32[at + i + 8 * u + j];
+            if (word < words) words16[at + i + 8 * u + j] = __float2half_rn(v);
+            set[u] = __fadd_rn(set[u], __fmul_rn(v, v));
+        }
+    }
+    const float mine = __fadd_rn(__fadd_rn(__fadd_rn(set[0], set[1]), set[2]), set[3]);
+    const int first = lane & 24;
+    float total = __shfl_sync(0xffffffffu, mine, first);
+#pragma unroll
+    for (int k = 1; k < 8; ++k) total = __fadd_rn(total, __shfl_sync(0xffffffffu, mine, first + k));
+    if (j == 0 && word < words) norms[word] = total;
+}
+
+int round_words_dispatch(const float *words32, __half *words16, float *norms, int64_t words, int d, cudaStream_t stream) {
+    round_words_kernel<<<(unsigned)((words * 8 + 255) / 256), 256, 0, stream>>>(words32, words16, norms, words, d);
+    return launch_status();
+}
+
 }  // namespace tacvq

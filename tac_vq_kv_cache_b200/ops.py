@@ -139,12 +139,14 @@ def encode(
                 raise ValueError("whitener must be [H,G,d,d]")
             search_tables = torch.empty(tables_f16.shape, dtype=torch.float32, device=device)
             search_rows = torch.empty(b, h, t, dim, dtype=torch.float32, device=device)
-            status = lib.tacvq_encode_whitened(
+            need = lib.tacvq_encode_whitened_filter_bytes(h, dim, g, s, k)
+            scratch = torch.empty(need, dtype=torch.uint8, device=device) if need else None
+            status = lib.tacvq_encode_whitened_filtered(
                 _ptr(x), _DTYPE_TAG[x.dtype], x.stride(0), x.stride(1), x.stride(2), _ptr(tables_f16), _ptr(w),
-                _ptr(search_tables), _ptr(search_rows), _ptr(codes), _ptr(recon), _DTYPE_TAG[states.dtype], b, h, t, dim,
-                g, s, k, t0, codes.shape[2], _stream(device),
+                _ptr(search_tables), _ptr(search_rows), _ptr(scratch), need, _ptr(codes), _ptr(recon), _DTYPE_TAG[states.dtype],
+                b, h, t, dim, g, s, k, t0, codes.shape[2], _stream(device),
             )
-            _lib.check("tacvq_encode_whitened", status)
+            _lib.check("tacvq_encode_whitened_filtered", status)
     return codes, recon
 
 

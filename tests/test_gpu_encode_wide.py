@@ -1,0 +1,68 @@
+"""GPU parity of the tensor-core encode of 64- and 128-wide groups, plain and whitened.
+
+Row counts around the tile of 128, one and two tiles a block, blocks that walk over several tiles with resident tables
+(up to two stages) and with the ring (an odd and an even number of stages), small codebooks, ties, and rows that are near
+several words at once.  Codes and rows are bit-exact with the C oracle.
+"""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import c_oracle as C
+from tests.util import make_states, make_tables
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize(
+    "batch,heads,tokens,sub,groups,stages,words,dtype,whitened",
+    [
+        (1, 2, 257, 128, 1, 2, 256, torch.float16, False),
+        (1, 2, 385, 128, 1, 1, 256, torch.float32, False),
+        (2, 2, 191, 64, 2, 3, 100, torch.float16, False),
+        (1, 40, 1025, 128, 1, 2, 256, torch.float16, False),   # 360 tiles: two a block, several trips, resident tables
+        (1, 80, 641, 64, 2, 3, 256, torch.float16, False),     # the same through the ring of tables
+        (3, 100, 299, 128, 1, 4, 33, torch.float32, False),
+        (1, 2, 1, 128, 1, 16, 256, torch.float16, True),
+        (1, 2, 129, 64, 2, 2, 77, torch.float16, True),
+        (1, 90, 513, 128, 1, 3, 256, torch.float32, True),
+    ],
+)
+def test_wide_encode_is_bit_exact(device, batch, heads, tokens, sub, groups, stages, words, dtype, whitened):
+    from tac_vq_kv_cache_b200 import ops
+
+    gen = torch.Generator().manual_seed(sub + tokens)
+    tables = make_tables(gen, heads, stages, groups, sub, [0.1 * 0.9**s for s in range(stages)])[:, :, :, :words].contiguous()
+    if words > 8:
+        tables[:, :, :, 5] = tables[:, :, :, 3]  # a tie: the lower index wins
+    states = make_states(gen, (batch, heads, tokens, sub * groups), dtype, 4)
+    cache = torch.full((batch, heads, tokens + 3, stages, groups), 0xEE, dtype=torch.uint8, device=device)
+    if whitened:
+        w = torch.eye(sub).expand(heads, groups, sub, sub) + 0.3 * torch.randn(heads, groups, sub, sub, generator=gen) / sub**0.5
+        want, want_recon = C.encode_whitened(states, tables, w)
+        codes, recon = ops.encode(states.to(device), tables.to(device), codes=cache, t0=2, whitener=w.to(device))
+    else:
+        want, want_recon = C.encode(states, tables)
+        codes, recon = ops.encode(states.to(device), tables.to(device), codes=cache, t0=2)
+    assert torch.equal(codes[:, :, 2 : 2 + tokens].cpu(), want)
+    assert torch.equal(recon.cpu(), want_recon)
+    assert bool((codes[:, :, :2] == 0xEE).all()) and bool((codes[:, :, 2 + tokens :] == 0xEE).all())
+    assert ops.encode_tensor_memory_timeouts(device) == 0
+
+
+def test_rows_between_words_take_the_exact_chains(device):
+    """Every row lies on a bisector of two words, or at a word that occurs three times: nothing but the exact order decides."""
+    from tac_vq_kv_cache_b200 import ops
+
+    gen = torch.Generator().manual_seed(3)
+    tables = make_tables(gen, 2, 2, 1, 128, [0.1, 0.1])
+    tables[:, :, :, 200] = tables[:, :, :, 100] = tables[:, :, :, 7]
+    pick = torch.randint(0, 256, (2, 2, 260), generator=gen)
+    rows = torch.stack([(tables[h, 0, 0][pick[h, 0]].float() + tables[h, 0, 0][pick[h, 1]].float()) / 2 for h in range(2)])
+    rows[:, ::9] = tables[:, 0, 0, 7, None].float()
+    states = rows[None]
+    want, want_recon = C.encode(states, tables)
+    codes, recon = ops.encode(states.to(device), tables.to(device))
+    assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
