@@ -22,6 +22,7 @@
 namespace tacvq {
 
 int encode_tc8_launch(const EncodeArgs &a);
+int encode_narrow_launch(const EncodeArgs &a);
 int encode_tc_large_launch(const EncodeArgs &a);
 int encode_wide_launch(const EncodeArgs &a);
 int encode_few_wide_launch(const EncodeArgs &a);
@@ -467,6 +468,11 @@ static int launch_large(const EncodeArgs &a) {
 
 constexpr int kFewRows = 32;  // at or below this many rows a warp per (row, head, group) wins
 
+// From this many rows on, 8- and 4-wide groups go to the tcgen05 kernel (up to its 12 stages).  Measured with 8 heads, fp16, call
+// included: 512 rows of 16 x 8 at two stages 39 us against 44 us for the mma.sync kernel, 32768 rows 460 against 600;
+// 256 rows 46 against 39.
+constexpr int kNarrowRows = 512;
+
 // 32-, 64- and 128-wide groups: a block per (head, group) and four rows while that is at most two blocks per SM.
 // Measured, 8 heads, against a launch of 128-row tiles: 128 rows of 16 x 128 (256 blocks) 76 us against 102 us, 2 x 128
 // 15.5 against 18.1; 192 rows (384 blocks) 108 against 103 and 19.0 against 17.8.
@@ -484,6 +490,10 @@ static int dispatch_d(const EncodeArgs &a) {
             }
         }
         if (TACVQ_ENCODE_TC && (a.D / a.G == 8 || a.D / a.G == 4)) {
+            if ((int64_t)a.B * a.T >= kNarrowRows) {
+                const int st = encode_narrow_launch(a);
+                if (st != TACVQ_ERR_UNSUPPORTED) return st;
+            }
             const int st = encode_tc8_launch(a);
             if (st != TACVQ_ERR_UNSUPPORTED) return st;
         }

@@ -395,3 +395,30 @@ def test_decode_of_long_rows_matches_the_oracle(device, groups, stages, sub, dty
     if stages > 1:
         got = ops.decode(codes.to(device), tables.to(device), dtype, depth=1)
         assert torch.equal(got.cpu(), C.decode(codes, tables, dtype, depth=1))
+
+
+@pytest.mark.parametrize(
+    "batch,heads,tokens,sub,groups,stages,words,dtype",
+    [
+        (1, 2, 512, 8, 16, 2, 256, torch.float16),
+        (1, 3, 641, 8, 16, 1, 256, torch.float32),
+        (3, 2, 333, 4, 32, 1, 100, torch.float16),
+        (2, 1, 4161, 8, 4, 3, 256, torch.float16),   # two spans of 8192 rows, tables changed inside a block
+        (1, 1, 600, 4, 8, 12, 256, torch.float32),   # as many stages as fit
+        (1, 1, 600, 8, 4, 13, 256, torch.float16),   # and one more
+    ],
+)
+def test_narrow_groups_with_many_rows_are_bit_exact(device, batch, heads, tokens, sub, groups, stages, words, dtype):
+    """Tiles of 128 rows, fewer and more pairs of head and group than blocks, padding words, ties."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(tokens)
+    tables = make_tables(gen, heads, stages, groups, sub, [0.5 * 0.8**s for s in range(stages)])[:, :, :, :words].contiguous()
+    tables[:, :, :, 9] = tables[:, :, :, 2]
+    states = make_states(gen, (batch, heads, tokens, sub * groups), dtype)
+    cache = torch.full((batch, heads, tokens + 3, stages, groups), 0xEE, dtype=torch.uint8, device=device)
+    want, want_recon = C.encode(states, tables)
+    codes, recon = ops.encode(states.to(device), tables.to(device), codes=cache, t0=2)
+    assert torch.equal(codes[:, :, 2 : 2 + tokens].cpu(), want) and torch.equal(recon.cpu(), want_recon)
+    assert bool((codes[:, :, :2] == 0xEE).all()) and bool((codes[:, :, 2 + tokens :] == 0xEE).all())
+    shifted = torch.empty(states.numel() + 1, dtype=dtype, device=device)[1:].view(states.shape).copy_(states)  # rows not 16-byte aligned
+    assert torch.equal(ops.encode(shifted, tables.to(device), want_recon=False)[0].cpu(), want)
