@@ -422,3 +422,24 @@ def test_narrow_groups_with_many_rows_are_bit_exact(device, batch, heads, tokens
     assert bool((codes[:, :, :2] == 0xEE).all()) and bool((codes[:, :, 2 + tokens :] == 0xEE).all())
     shifted = torch.empty(states.numel() + 1, dtype=dtype, device=device)[1:].view(states.shape).copy_(states)  # rows not 16-byte aligned
     assert torch.equal(ops.encode(shifted, tables.to(device), want_recon=False)[0].cpu(), want)
+
+
+@pytest.mark.parametrize(
+    "batch,tokens,sub,groups,stages,words,depth,dtype",
+    [
+        (1, 1025, 8, 16, 2, 256, None, torch.float16),
+        (3, 357, 8, 16, 2, 256, 1, torch.float32),
+        (2, 515, 4, 16, 2, 100, None, torch.float32),
+        (5, 301, 128, 1, 2, 256, None, torch.float32),
+        (2, 1111, 64, 1, 1, 96, None, torch.float16),
+        (1, 1500, 16, 12, 1, 32, None, torch.float16),
+    ],
+)
+def test_rows_of_one_or_two_stages_rebuild_exactly(device, batch, tokens, sub, groups, stages, words, depth, dtype):
+    """Row counts that leave ragged last trips, several sequences per block, a depth below the stored one, odd codebooks."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(tokens)
+    tables = make_tables(gen, 3, stages, groups, sub)[:, :, :, :words].contiguous()
+    codes = torch.randint(0, words, (batch, 3, tokens + 2, stages, groups), generator=gen, dtype=torch.uint8)
+    got = ops.decode(codes.to(device), tables.to(device), dtype, depth=depth, t0=1, tokens=tokens)
+    assert torch.equal(got.cpu(), C.decode(codes, tables, dtype, depth=depth, t0=1, tokens=tokens))
