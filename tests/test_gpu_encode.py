@@ -443,3 +443,21 @@ def test_rows_of_one_or_two_stages_rebuild_exactly(device, batch, tokens, sub, g
     codes = torch.randint(0, words, (batch, 3, tokens + 2, stages, groups), generator=gen, dtype=torch.uint8)
     got = ops.decode(codes.to(device), tables.to(device), dtype, depth=depth, t0=1, tokens=tokens)
     assert torch.equal(got.cpu(), C.decode(codes, tables, dtype, depth=depth, t0=1, tokens=tokens))
+
+
+@pytest.mark.parametrize("sub,groups,stages,depth", [(128, 1, 16, 16), (4, 32, 1, 1), (8, 16, 2, 1), (2, 16, 2, 2)])
+def test_codeword_gradient_sums_the_rows_that_chose_a_word(device, sub, groups, stages, depth):
+    """Against float64 index_add: at most 2^-23 times the number of addends relative to the sum of their magnitudes."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(sub)
+    codes = torch.randint(0, 256, (2, 3, 301, stages, groups), generator=gen, dtype=torch.uint8)
+    grad = torch.randn(2, 3, 301, groups * sub, generator=gen)
+    got = ops.codeword_grad(codes.to(device), grad.to(device), (3, stages, groups, 256, sub), depth=depth).cpu()
+    want, size = torch.zeros(got.shape, dtype=torch.float64), torch.zeros(got.shape, dtype=torch.float64)
+    for h in range(3):
+        for s in range(depth):
+            for g in range(groups):
+                rows = grad[:, h, :, g * sub : (g + 1) * sub].reshape(-1, sub).double()
+                want[h, s, g].index_add_(0, codes[:, h, :, s, g].reshape(-1).long(), rows)
+                size[h, s, g].index_add_(0, codes[:, h, :, s, g].reshape(-1).long(), rows.abs())
+    assert bool(((got.double() - want).abs() <= 602 * 2.0**-23 * size).all())
