@@ -97,7 +97,7 @@ template <int DSUB, typename XT, typename Rows>
 __global__ void __launch_bounds__(kWideThreads)
 whiten_wide_kernel(const XT *__restrict__ x, const float *__restrict__ whitener, float *__restrict__ out, Rows map_proto,
                    int64_t rows, int G, int64_t in_group_stride, int64_t out_group_stride, int64_t in_head_stride,
-                   int64_t out_head_stride) {
+                   int64_t out_head_stride, int vec_ok) {
     using L = WideLayout<DSUB>;
     extern __shared__ __align__(16) float wsm[];
     float *wt = wsm;                                  // [j][i] : W transposed
@@ -108,15 +108,41 @@ whiten_wide_kernel(const XT *__restrict__ x, const float *__restrict__ whitener,
     const int64_t in_off = (int64_t)h * in_head_stride + (int64_t)g * in_group_stride;
     const int64_t out_off = (int64_t)h * out_head_stride + (int64_t)g * out_group_stride;
     const float *w = whitener + (int64_t)hg * DSUB * DSUB;
-    for (int e = tid; e < DSUB * DSUB; e += kWideThreads) {  // coalesced read of W[i][j], transposed store
-        const int i = e / DSUB, j = e % DSUB;
-        wt[j * L::kWStride + i] = w[e];
+    // four columns of a row of W per thread, neighbouring threads in neighbouring rows: the transposed stores miss each
+    // other's banks
+    for (int e = tid; e < DSUB * DSUB / 4; e += kWideThreads) {
+        const int i = e % DSUB, j = (e / DSUB) * 4;
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(w + i * DSUB + j));
+        wt[j * L::kWStride + i] = v.x;
+        wt[(j + 1) * L::kWStride + i] = v.y;
+        wt[(j + 2) * L::kWStride + i] = v.z;
+        wt[(j + 3) * L::kWStride + i] = v.w;
     }
     const int64_t row0 = (int64_t)blockIdx.x * kWideRows;
-    for (int e = tid; e < kWideRows * DSUB; e += kWideThreads) {
-        const int r = e / DSUB, j = e % DSUB;
+    for (int e = tid; e < kWideRows * DSUB / 8; e += kWideThreads) {
+        const int r = e / (DSUB / 8), j = (e % (DSUB / 8)) * 8;
         const int64_t row = row0 + r;
-        xs[e] = row < rows ? to_float<XT>(x[in_off + map.in(row) + j]) : 0.0f;
+        float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (row < rows) {
+            const XT *src = x + in_off + map.in(row) + j;
+            if (!vec_ok) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = to_float<XT>(src[i]);
+            } else if constexpr (sizeof(XT) == 2) {
+                const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(src));
+                const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f = __half22float2(h2[i]);
+                    v[2 * i] = f.x, v[2 * i + 1] = f.y;
+                }
+            } else {
+                *reinterpret_cast<float4 *>(v) = __ldg(reinterpret_cast<const float4 *>(src));
+                *reinterpret_cast<float4 *>(v + 4) = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+            }
+        }
+        *reinterpret_cast<float4 *>(xs + r * DSUB + j) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4 *>(xs + r * DSUB + j + 4) = make_float4(v[4], v[5], v[6], v[7]);
     }
     __syncthreads();
     const int i0 = (tid % L::kOutPerRow) * 4, rg = tid / L::kOutPerRow;
@@ -154,14 +180,14 @@ whiten_wide_kernel(const XT *__restrict__ x, const float *__restrict__ whitener,
 template <int DSUB, typename XT, typename Rows>
 static int launch_wide(const XT *x, const float *whitener, float *out, const Rows &map, int64_t rows, int H, int G,
                        int64_t in_group_stride, int64_t out_group_stride, int64_t in_head_stride, int64_t out_head_stride,
-                       cudaStream_t stream) {
+                       int vec_ok, cudaStream_t stream) {
     using L = WideLayout<DSUB>;
     auto kernel = whiten_wide_kernel<DSUB, XT, Rows>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kBytes);
     if (e != cudaSuccess) return (int)e;
     dim3 grid((unsigned)((rows + kWideRows - 1) / kWideRows), (unsigned)(H * G));
     kernel<<<grid, kWideThreads, L::kBytes, stream>>>(x, whitener, out, map, rows, G, in_group_stride, out_group_stride,
-                                                      in_head_stride, out_head_stride);
+                                                      in_head_stride, out_head_stride, vec_ok);
     return launch_status();
 }
 
@@ -171,14 +197,17 @@ static int whiten_wide(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int
                        int S, int K, cudaStream_t stream) {
     TableRows tr{0, (int64_t)G * K * DSUB, K, DSUB};
     int st = launch_wide<DSUB, __half, TableRows>(tables, whitener, search_tables, tr, (int64_t)S * K, H, G, (int64_t)K * DSUB,
-                                                  (int64_t)K * DSUB, (int64_t)S * G * K * DSUB, (int64_t)S * G * K * DSUB, stream);
+                                                  (int64_t)K * DSUB, (int64_t)S * G * K * DSUB, (int64_t)S * G * K * DSUB,
+                                                  (reinterpret_cast<uintptr_t>(tables) & 15u) == 0, stream);
     if (st != TACVQ_OK) return st;
     StateRows sr{sxb, sxt, 0, 0, T, D, (int64_t)H * T};
+    const int per_vec = x_dtype == TACVQ_F16 ? 8 : 4;
+    const int vec_ok = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && sxb % per_vec == 0 && sxh % per_vec == 0 && sxt % per_vec == 0;
     if (x_dtype == TACVQ_F16)
         return launch_wide<DSUB, __half, StateRows>((const __half *)x, whitener, search_rows, sr, (int64_t)B * T, H, G, DSUB, DSUB,
-                                                    sxh, (int64_t)T * D, stream);
+                                                    sxh, (int64_t)T * D, vec_ok, stream);
     return launch_wide<DSUB, float, StateRows>((const float *)x, whitener, search_rows, sr, (int64_t)B * T, H, G, DSUB, DSUB, sxh,
-                                               (int64_t)T * D, stream);
+                                               (int64_t)T * D, vec_ok, stream);
 }
 
 int whiten_dispatch(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt, const __half *tables,
@@ -186,7 +215,7 @@ int whiten_dispatch(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_
                     int S, int K, cudaStream_t stream) {
     const int d = D / G;
     // the tiled kernels read rows and matrices in 16-byte pieces
-    const bool aligned = (((uintptr_t)search_rows | (uintptr_t)search_tables) & 15) == 0;
+    const bool aligned = (((uintptr_t)search_rows | (uintptr_t)search_tables | (uintptr_t)whitener) & 15) == 0;
     if (aligned && d == 128) return whiten_wide<128>(x, x_dtype, sxb, sxh, sxt, tables, whitener, search_tables, search_rows, B, H, T, D, G, S, K, stream);
     if (aligned && d == 64) return whiten_wide<64>(x, x_dtype, sxb, sxh, sxt, tables, whitener, search_tables, search_rows, B, H, T, D, G, S, K, stream);
     if (aligned && d == 32) return whiten_wide<32>(x, x_dtype, sxb, sxh, sxt, tables, whitener, search_tables, search_rows, B, H, T, D, G, S, K, stream);
