@@ -12,7 +12,7 @@
 //      there are more, the row goes to shared memory and the library's exact chains decide,
 //   4. subtracts the chosen word and writes the new fp16 row.
 // The two groups share the word tables: resident for the block's life up to two stages, otherwise a ring of two
-// that the group which leaves a stage last refills by TMA.  While one group waits for its product the other one reads
+// that the group which leaves a stage last refills (words by TMA, norms by four of its warps).  While one group waits for its product the other one reads
 // scores, which keeps the tensor core and the schedulers busy in turn.
 //
 // Margin (encode_tc.cu has the argument that twice the error bound E of a score keeps the exact argmin and its ties on
@@ -196,9 +196,9 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     float *nrms = reinterpret_cast<float *>(smem + L::kNrm);
     const uint32_t misc = smem_u32(smem + L::kMisc);
     const uint32_t full_bar = misc, mma_bar = misc + 16;  // [2] each
-    unsigned int *left = reinterpret_cast<unsigned int *>(smem + L::kMisc + 32);  // [2]: groups that left a stage of this buffer, all uses together
+    unsigned int *left = reinterpret_cast<unsigned int *>(smem + L::kMisc + 64);  // [2][4]: groups that left a stage of this buffer, all uses together, per quarter
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::kMisc + 48);
-    float *cc_tops = reinterpret_cast<float *>(smem + L::kMisc + 56);            // [2]
+    float *cc_tops = reinterpret_cast<float *>(smem + L::kMisc + 128);            // [2][4]: largest norm of a quarter
 
     const int hg = blockIdx.y, h = hg / a.G, g = hg % a.G;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -214,10 +214,10 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     }
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full_bar + 8 * i) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(full_bar + 8 * i) : "memory");  // a warp per quarter of the words
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mma_bar + 8 * i) : "memory");
         }
-        left[0] = left[1] = 0u;
+        for (int i = 0; i < 8; ++i) left[i] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < kRows * 2; i += blockDim.x) {  // 16-byte piece c of row r sits at piece c ^ ((r >> 2) & 1)
@@ -246,13 +246,13 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             *reinterpret_cast<uint4 *>(tab + L::template at<kMaxWords>(k, p * 8)) = v;
         }
     };
-    auto copy_norms = [&](int buf, int64_t first) {
+    auto copy_norms = [&](int buf, int64_t first, int k_begin, int k_end) {
         if (a.sqnorm != nullptr) {
 #pragma unroll 1
-            for (int k = lane; k < kMaxWords; k += 32) nrms[buf * kMaxWords + k] = k < K ? a.sqnorm[first + k] : inf;
+            for (int k = k_begin + lane; k < k_end; k += 32) nrms[buf * kMaxWords + k] = k < K ? __ldg(a.sqnorm + first + k) : inf;
         } else {
 #pragma unroll 1
-            for (int k0 = 0; k0 < kMaxWords; k0 += 4) {
+            for (int k0 = k_begin; k0 < k_end; k0 += 4) {
                 const int k = k0 + (lane >> 3);
                 const float v = word_norm_by_eight<DSUB>(a.tables + (first + min(k, K - 1)) * DSUB, lane);
                 if ((lane & 7) == 0) nrms[buf * kMaxWords + k] = k < K ? v : inf;
@@ -260,11 +260,13 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         }
         __syncwarp();
     };
-    // one warp: the words of use u by TMA (or plain copies without a tensor map), their norms and seeds
-    auto load_table = [&](uint32_t u) {
+    // four warps, a quarter each: the norms and seeds of use u; the first one also fetches the words by TMA (or plain copies
+    // without a tensor map)
+    auto load_table = [&](uint32_t u, int quarter) {
         const int s = (int)(u % (uint32_t)S), buf = (int)(u & 1u);
         const int64_t first = head_words + s * stage_words;
-        if (a.use_map) {
+        if (quarter != 0) {
+        } else if (a.use_map) {
             if (lane == 0) {
                 asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(full_bar + 8 * buf), "r"((uint32_t)L::kTabBytes) : "memory");
 #pragma unroll
@@ -276,11 +278,11 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         } else {
             copy_table(buf, first);
         }
-        copy_norms(buf, first);
+        copy_norms(buf, first, quarter * 64, quarter * 64 + 64);
         float top = 0.0f;
         unsigned char *seed = smem + L::kSeed + buf * kSeedBytes;
 #pragma unroll 1
-        for (int k = lane; k < kMaxWords; k += 32) {
+        for (int k = quarter * 64 + lane; k < quarter * 64 + 64; k += 32) {
             const float v = nrms[buf * kMaxWords + k];
             if (k < K && v == v) top = fmaxf(top, v);
             const float t = -0.5f * v;  // padding words: -inf, never within the margin
@@ -296,12 +298,12 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         }
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-        if (lane == 0) cc_tops[buf] = top;
+        if (lane == 0) cc_tops[buf * 4 + quarter] = top;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full_bar + 8 * buf) : "memory");
     };
-    if (warp < 2 && (uint32_t)warp < uses) load_table((uint32_t)warp);
+    if (warp < 8 && (uint32_t)(warp >> 2) < uses) load_table((uint32_t)(warp >> 2), warp & 3);
 
     const int grp = warp >> 4, part = warp & 3, q = (warp >> 2) & 3;
     const int row = part * 32 + lane;                     // of the group's tile
@@ -405,7 +407,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             fail = __any_sync(0xffffffffu, fail);
             if (fail) {  // never seen: the warp brings the words itself (the same bytes) and lists them all
                 copy_table(buf, first);
-                copy_norms(buf, first);
+                copy_norms(buf, first, 0, kMaxWords);
             }
             if ((warp & 15) == 0) {
                 if (lane == 0 && !fail) {
@@ -419,17 +421,18 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(my_mma) : "memory");
                 }
                 __syncwarp();
-                // use u - 1 is left: the last group to leave it refills its buffer
-                if (!resident && u >= 1 && u + 1 < uses) {
-                    unsigned int n = 0u;
-                    __threadfence_block();
-                    if (lane == 0) n = atomicAdd(left + ((u - 1) & 1u), 1u) + 1u;
-                    __threadfence_block();
-                    n = __shfl_sync(0xffffffffu, n, 0);
-                    if (n % (unsigned int)groups == 0u) load_table(u + 1);
-                }
             }
-            const float xx = (xxs[0] + xxs[kRows]) + (xxs[2 * kRows] + xxs[3 * kRows]), cc_top = cc_tops[buf];
+            // use u - 1 is left: the last group to leave it refills its buffer, a quarter per warp of q = 0
+            if (q == 0 && !resident && u >= 1 && u + 1 < uses) {
+                unsigned int n = 0u;
+                __threadfence_block();
+                if (lane == 0) n = atomicAdd(left + ((u - 1) & 1u) * 4 + part, 1u) + 1u;
+                __threadfence_block();
+                n = __shfl_sync(0xffffffffu, n, 0);
+                if (n % (unsigned int)groups == 0u) load_table(u + 1, part);
+            }
+            const float xx = (xxs[0] + xxs[kRows]) + (xxs[2 * kRows] + xxs[3 * kRows]);
+            const float cc_top = fmaxf(fmaxf(cc_tops[buf * 4], cc_tops[buf * 4 + 1]), fmaxf(cc_tops[buf * 4 + 2], cc_tops[buf * 4 + 3]));
             const float u_top = rough_sqrt(xx * cc_top);
             const float margin = (sizeof(XT) == 2 && s == 0 ? 1.220703125e-04f : EXACT32 ? 2.01416015625e-03f : 1.03759765625e-03f) * u_top +
                                  9.5367431640625e-07f * xx + 3.0517578125e-05f * cc_top + 3.814697265625e-06f * rough_sqrt(cc_top) +
