@@ -182,12 +182,13 @@ struct Args {
     const float *sqnorm;     // |word|^2 of the deciding words; may be null for fp16 words
     uint8_t *codes;
     void *recon;
-    int recon_dtype, B, H, T, G, S, K, groups, vec_ok, use_map;
+    int recon_dtype, B, H, T, G, S, K, vec_ok, use_map;
     int64_t t0, T_cap;
 };
 
-template <int DSUB, typename XT, bool EXACT32>
-__global__ void __launch_bounds__(kMaxGroups * kGroupThreads, 1)
+// GROUPS = 1: one tile a block, for launches that leave no tile waiting; twice the registers per thread.
+template <int DSUB, typename XT, bool EXACT32, int GROUPS>
+__global__ void __launch_bounds__(GROUPS * kGroupThreads, 1)
 encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) {
     using L = Layout<DSUB>;
     constexpr int kPieces = DSUB / 8, kOwn = kPieces / kShare;
@@ -202,7 +203,8 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
 
     const int hg = blockIdx.y, h = hg / a.G, g = hg % a.G;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int S = a.S, K = a.K, groups = a.groups;
+    const int S = a.S, K = a.K;
+    constexpr int groups = GROUPS;
     const uint32_t rows = (uint32_t)a.B * (uint32_t)a.T;  // the launcher keeps B*T below 2^31
     const uint32_t tiles = (rows + kRows - 1) / kRows;
     const float inf = __int_as_float(0x7f800000);
@@ -738,8 +740,8 @@ static int launch(const EncodeArgs &e, const __half *scored) {
     const int64_t most = units < 148 ? 148 / units : 1;
     if (blocks > most) blocks = most;
     const Args a{e.x, e.sxb, e.sxh, e.sxt, scored, EXACT32 ? (const float *)e.tables : nullptr, e.recon_tables, e.sqnorm, e.codes, e.recon,
-                 e.recon_dtype, e.B, e.H, e.T, e.G, e.S, e.K, groups, vec_ok, use_map, e.t0, e.T_cap};
-    auto kernel = encode_wide_kernel<DSUB, XT, EXACT32>;
+                 e.recon_dtype, e.B, e.H, e.T, e.G, e.S, e.K, vec_ok, use_map, e.t0, e.T_cap};
+    auto kernel = groups == 1 ? encode_wide_kernel<DSUB, XT, EXACT32, 1> : encode_wide_kernel<DSUB, XT, EXACT32, kMaxGroups>;
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
     kernel<<<dim3((unsigned)blocks, (unsigned)units), groups * kGroupThreads, smem, e.stream>>>(a, map);
