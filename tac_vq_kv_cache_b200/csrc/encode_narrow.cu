@@ -14,7 +14,8 @@
 // Blocks split the tiles of all (head, group) pairs evenly, span by span of 8192 rows, and bring a pair's tables in when they
 // enter it, so the chip stays full whatever the number of pairs; a table costs about one tile's time.
 //
-// Bound by instruction issue (about 450 per row, stage and 256 words).
+// Bound by latency between the phases of a stage at 16 warps an SM (issue 52 % busy).  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
+// stages, rows wanted: 460 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.
 //
 // Reference statements: src/jointkv/closed_loop_vq.py:52-76 (search), :343-395 (stage recursion),
 // src/jointkv/cq_tac.py:86-105.

@@ -93,6 +93,11 @@ def encode_tensor_memory_timeouts(device=None) -> int:
 _word_norms = table_sqnorm  # encode() has a keyword argument of the same name
 
 
+@functools.lru_cache(maxsize=256)
+def _whitened_filter_bytes(h: int, dim: int, g: int, s: int, k: int) -> int:
+    return int(_lib.load().tacvq_encode_whitened_filter_bytes(h, dim, g, s, k))
+
+
 def encode(
     states: torch.Tensor,
     tables_f16: torch.Tensor,
@@ -139,7 +144,7 @@ def encode(
                 raise ValueError("whitener must be [H,G,d,d]")
             search_tables = torch.empty(tables_f16.shape, dtype=torch.float32, device=device)
             search_rows = torch.empty(b, h, t, dim, dtype=torch.float32, device=device)
-            need = lib.tacvq_encode_whitened_filter_bytes(h, dim, g, s, k)
+            need = _whitened_filter_bytes(h, dim, g, s, k)
             scratch = torch.empty(need, dtype=torch.uint8, device=device) if need else None
             status = lib.tacvq_encode_whitened_filtered(
                 _ptr(x), _DTYPE_TAG[x.dtype], x.stride(0), x.stride(1), x.stride(2), _ptr(tables_f16), _ptr(w),
