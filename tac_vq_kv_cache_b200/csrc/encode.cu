@@ -468,10 +468,10 @@ static int launch_large(const EncodeArgs &a) {
 
 constexpr int kFewRows = 32;  // at or below this many rows a warp per (row, head, group) wins
 
-// From this many rows on, 8- and 4-wide groups go to the tcgen05 kernel (up to its 12 stages).  Measured with 8 heads, fp16, call
-// included: 512 rows of 16 x 8 at two stages 39 us against 44 us for the mma.sync kernel, 32768 rows 460 against 600;
-// 256 rows 46 against 39.
-constexpr int kNarrowRows = 512;
+// From this many rows on, 8- and 4-wide groups go to the tcgen05 kernel (up to its 12 stages).  Measured with 8 heads, fp16 rows
+// wanted, against the mma.sync kernel: 512 rows of 16 x 8 at two stages 24.7 us against 24.9 and of 32 x 4 24.6 against 22.8;
+// 700 rows 24.7 against 25.1 and 24.9 against 29.0; 4096 rows 66 against 88 and 75 against 94.
+constexpr int kNarrowRows = 640;
 
 // 32-, 64- and 128-wide groups: a block per (head, group) and four rows while that is at most two blocks per SM.
 // Measured, 8 heads, against a launch of 128-row tiles: 128 rows of 16 x 128 (256 blocks) 76 us against 102 us, 2 x 128

@@ -400,12 +400,12 @@ def test_decode_of_long_rows_matches_the_oracle(device, groups, stages, sub, dty
 @pytest.mark.parametrize(
     "batch,heads,tokens,sub,groups,stages,words,dtype",
     [
-        (1, 2, 512, 8, 16, 2, 256, torch.float16),
+        (1, 2, 640, 8, 16, 2, 256, torch.float16),
         (1, 3, 641, 8, 16, 1, 256, torch.float32),
         (3, 2, 333, 4, 32, 1, 100, torch.float16),
         (2, 1, 4161, 8, 4, 3, 256, torch.float16),   # two spans of 8192 rows, tables changed inside a block
-        (1, 1, 600, 4, 8, 12, 256, torch.float32),   # as many stages as fit
-        (1, 1, 600, 8, 4, 13, 256, torch.float16),   # and one more
+        (1, 1, 650, 4, 8, 12, 256, torch.float32),   # as many stages as fit
+        (1, 1, 650, 8, 4, 13, 256, torch.float16),   # and one more
     ],
 )
 def test_narrow_groups_with_many_rows_are_bit_exact(device, batch, heads, tokens, sub, groups, stages, words, dtype):
