@@ -7,6 +7,7 @@ is not a B200-class GPU the calls raise - there is no CPU or PyTorch fallback.
 from __future__ import annotations
 
 import ctypes
+import struct
 from ctypes import c_char_p, c_double, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
@@ -47,14 +48,9 @@ _SIGNATURES = {
 EXPORTS = tuple(_SIGNATURES)
 
 
-class StepPlan(ctypes.Structure):
-    """``tacvq_step_plan``: what stays the same from token to token of a decoding loop."""
-
-    _fields_ = (
-        [(name, c_void_p) for name in ("ktab", "vtab", "rope", "kcodes", "vcodes", "seq_start", "seq_end", "workspace")]
-        + [("workspace_bytes", c_size_t), ("window", c_int64), ("t_cap", c_int64)]
-        + [(name, c_int) for name in ("b", "hq", "hkv", "d", "g", "s", "k")]
-    )
+# ``tacvq_step_plan``: addresses of the K and V tables, rope table, K and V codes, range starts and ends, workspace; its bytes;
+# window, T_cap; B, Hq, Hkv, D, G, S, K
+STEP_PLAN = struct.Struct("@8PN2q7i0q")
 
 
 class TacvqError(RuntimeError):

@@ -19,11 +19,9 @@ kernel (keys are stored as encoded).
 
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
-from . import ops
+from . import _lib, ops
 
 
 
@@ -71,9 +69,8 @@ class VQCodeCache:
         self.length = 0
         self._range = torch.zeros(2, batch, dtype=torch.int32, device=self.device)  # [start; end) per row
         self._range_is = (0, 0)
-        self._workspace: torch.Tensor | None = None
-        self._plans: dict[int, tuple] = {}  # query heads -> (record of everything that decode_step passes every time, its workspace)
-        self._host_key, self._host_call = None, None  # decode_step_host's
+        self._workspaces: list[torch.Tensor] = []
+        self._host_key, self._host_call, self._host_buffers = None, None, None  # decode_step_host's
         self.rope = None if rope_theta is None else ops.rope_table(self.max_tokens, self.dim, float(rope_theta), self.device)
 
     def reset(self) -> None:
@@ -123,62 +120,90 @@ class VQCodeCache:
         """Append the new token rows and attend, in one library call (``append`` + ``attend`` fused).
 
         ``query [B,Hq,D]`` fp16 scaled (and rotated, for a cache of pre-rotary keys), ``raw_key`` / ``raw_value``
-        ``[B,H,T_new,D]`` contiguous fp16 or fp32.
+        ``[B,H,T_new,D]`` contiguous fp16 or fp32.  The buffers, tables and window are the cache's at this call.
         """
-        shape, q_shape = raw_key.shape, query.shape
-        if len(shape) != 4 or shape != raw_value.shape or shape[0] != self.batch or shape[1] != self.heads or shape[3] != self.dim:
+        batch, heads, dim = self.batch, self.heads, self.dim
+        shape, q_shape, dtype = raw_key.shape, query.shape, raw_key.dtype
+        if len(shape) != 4 or shape != raw_value.shape or shape[0] != batch or shape[1] != heads or shape[3] != dim:
             raise ValueError("rows must be [B,H,T,D] matching the cache geometry")
-        if len(q_shape) != 3 or q_shape[0] != self.batch or q_shape[2] != self.dim or query.dtype != torch.float16:
+        if len(q_shape) != 3 or q_shape[0] != batch or q_shape[2] != dim or query.dtype != torch.float16:
             raise ValueError("query must be fp16 [B,Hq,D]")
-        if raw_key.dtype != raw_value.dtype or raw_key.dtype not in ops._DTYPE_TAG:
+        if dtype != raw_value.dtype or dtype not in ops._DTYPE_TAG:
             raise ValueError("rows must be of one dtype, fp16 or fp32")
         if not (raw_key.is_contiguous() and raw_value.is_contiguous() and query.is_contiguous()):
             raise ValueError("query and rows must be contiguous")
-        device = self.key.device
-        if query.device != device or raw_key.device != device or raw_value.device != device:
+        ktab, vtab, rope, key, value, start, end, words, index = self._addresses()
+        if not (index == query.get_device() == raw_key.get_device() == raw_value.get_device()):
             ops._require_cuda(self.key, query, raw_key, raw_value)
         if out is None:
-            out = torch.empty(q_shape, dtype=torch.float16, device=device)
-        elif out.shape != q_shape or out.dtype != torch.float16 or not out.is_contiguous() or out.device != device:
+            out = torch.empty_like(query)
+        elif out.shape != q_shape or out.dtype != torch.float16 or not out.is_contiguous() or out.get_device() != index:
             raise ValueError("out must be contiguous fp16 [B,Hq,D] on the cache's device")
-        tokens = shape[2]
+        tokens, q_heads = shape[2], q_shape[1]
         if self.length + tokens > self.max_tokens:
             raise ValueError("code cache is full")
-        plan = self._plans.get(q_shape[1]) or self._plan(int(q_shape[1]))
-        with ops._on(device):
-            status = plan[0](plan[1], query.data_ptr(), raw_key.data_ptr(), raw_value.data_ptr(), ops._DTYPE_TAG[raw_key.dtype], tokens,
-                             self.length, out.data_ptr(), None, _raw_stream(device.index))
+        workspace = self._scratch(q_heads)
+        # read by the library during the call only
+        record = _lib.STEP_PLAN.pack(
+            ktab, vtab, rope, key, value, start, end, workspace.data_ptr(), workspace.numel(), self.window or 0, self.max_tokens, batch, q_heads,
+            heads, dim, self.groups, self.stages, words,
+        )
+        args = (record, query.data_ptr(), raw_key.data_ptr(), raw_value.data_ptr(), ops._DTYPE_TAG[dtype], tokens, self.length, out.data_ptr(),
+                None, _raw_stream(index))
+        if index == torch.cuda.current_device():
+            status = _lib.load().tacvq_decode_step_planned(*args)
+        else:
+            with torch.cuda.device(index):
+                status = _lib.load().tacvq_decode_step_planned(*args)
         if status:
-            from . import _lib
-
             _lib.check("tacvq_decode_step_planned", status)
         self.length += tokens
         self._range_is = self.visible()
         return out
 
-    def _plan(self, q_heads: int) -> tuple:
-        """The library's step call and the record it reads, for steps with ``q_heads`` query heads."""
-        from . import _lib
+    def _addresses(self) -> tuple[int, ...]:
+        """Where the K and V tables, the rotary table, the K and V codes and the range's two ends are; words a table, device.
 
-        ops._require_cuda(self.key)
-        workspace = self._scratch(q_heads)
-        record = _lib.StepPlan(
-            ktab=self.key_tables.data_ptr(), vtab=self.value_tables.data_ptr(), rope=ops._ptr(self.rope), kcodes=self.key.data_ptr(), vcodes=self.value.data_ptr(),
-            seq_start=self._range[0].data_ptr(), seq_end=self._range[1].data_ptr(), workspace=workspace.data_ptr(),
-            workspace_bytes=workspace.numel(), window=self.window or 0, t_cap=self.max_tokens, b=self.batch, hq=q_heads, hkv=self.heads,
-            d=self.dim, g=self.groups, s=self.stages, k=int(self.key_tables.shape[-2]),
-        )
-        self._plans[q_heads] = (_lib.load().tacvq_decode_step_planned, ctypes.byref(record), record, workspace)
-        return self._plans[q_heads]
+        Asked for at every step, because a caller may put other tensors in their place; what the library would misread is refused.
+        """
+        ktab, vtab, rope, key, value = self.key_tables, self.value_tables, self.rope, self.key, self.value
+        tokens, shape = self.max_tokens, ktab.shape
+        code_shape = (self.batch, self.heads, tokens, self.stages, self.groups)
+        if key.shape != code_shape or value.shape != code_shape or key.dtype != torch.uint8 or value.dtype != torch.uint8:
+            raise ValueError("codes must be uint8 [B,H,T_max,S,G]")
+        if len(shape) != 5 or shape != vtab.shape or ktab.dtype != torch.float16 or vtab.dtype != torch.float16:
+            raise ValueError("tables must be fp16 [H,S,G,K,d]")
+        heads, stages, groups, words, sub = shape
+        if heads != self.heads or stages != self.stages or groups != self.groups or groups * sub != self.dim:
+            raise ValueError("table and cache geometry differs")
+        if not (key.is_contiguous() and value.is_contiguous() and ktab.is_contiguous() and vtab.is_contiguous()):
+            raise ValueError("codes and tables must be contiguous")
+        index = key.get_device()
+        if not (index == value.get_device() == ktab.get_device() == vtab.get_device() >= 0) or ops._capability_major(index) != 10:
+            ops._require_cuda(key, value, ktab, vtab)
+        rope_at = 0
+        if rope is not None:
+            if rope.shape != (tokens, 2, self.dim // 2) or rope.dtype != torch.float16 or not rope.is_contiguous() or rope.get_device() != index:
+                raise ValueError("rope must be contiguous fp16 [T_max, 2, D/2] on the cache's device")
+            rope_at = rope.data_ptr()
+        ranges = self._range.data_ptr()
+        return ktab.data_ptr(), vtab.data_ptr(), rope_at, key.data_ptr(), value.data_ptr(), ranges, ranges + 4 * self.batch, words, index
+
+    def __getstate__(self) -> dict:
+        """For copies and pickles: scratch and marshalled calls stay with the cache they were made for."""
+        return {**self.__dict__, "_range": self._range.clone(), "_workspaces": [], "_host_key": None, "_host_call": None, "_host_buffers": None}
 
     def _scratch(self, q_heads: int) -> torch.Tensor:
-        """The attention workspace, large enough for ``q_heads`` query heads (kept; only ever replaced by a larger one)."""
+        """The attention workspace, large enough for ``q_heads`` query heads.
+
+        Smaller ones are kept beside it: a captured graph goes on using the one that it was captured with.
+        """
         need = ops.attn_workspace_bytes(self.batch, q_heads, self.heads, self.dim, self.groups, self.stages)
         if need == 0:
             raise ValueError("attention geometry not supported")
-        if self._workspace is None or self._workspace.numel() < need:
-            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
-        return self._workspace
+        if not self._workspaces or self._workspaces[-1].numel() < need:
+            self._workspaces.append(torch.empty(need, dtype=torch.uint8, device=self.device))
+        return self._workspaces[-1]
 
     def decode_step_host(self, host_rows: torch.Tensor, host_out: torch.Tensor, q_heads: int, *, tokens: int = 1,
                          synchronize: bool = True, direct: bool | str = False) -> torch.Tensor:
@@ -211,8 +236,6 @@ class VQCodeCache:
             with torch.cuda.device(self.device):
                 status = call(*args)
         if status:
-            from . import _lib
-
             _lib.check("tacvq_decode_step_host", status)
         self.length += tokens
         self._range_is = self.visible()
@@ -220,8 +243,6 @@ class VQCodeCache:
 
     def _prepare_host_call(self, host_rows: torch.Tensor, host_out: torch.Tensor, q_heads: int, tokens: int, direct: bool | str) -> None:
         """Checks and argument marshalling of :meth:`decode_step_host`, done once per pair of host buffers."""
-        from . import _lib
-
         if self.rope is not None:
             raise ValueError("the single-call host path has no rotary step; use append() + attend()")
         nq, nkv = self.batch * q_heads * self.dim, self.batch * self.heads * tokens * self.dim

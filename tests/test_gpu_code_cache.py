@@ -82,3 +82,82 @@ def test_single_call_host_step_equals_the_device_step(device, direct):
     assert a.length == b.length == 90 and torch.equal(a.key, b.key) and torch.equal(a.value, b.value)
     with pytest.raises(ValueError):
         a.decode_step_host(host_rows[:-1], host_out, q_heads, direct=direct)
+
+
+def _decoding_pair(gen, device, groups, stages, sub, rope, batch=2, heads=2, prompt=50):
+    """A cache that is stepped and one that appends and attends, after the same prompt, and a source of step inputs."""
+    from tac_vq_kv_cache_b200.code_cache import VQCodeCache
+
+    tables = [make_tables(gen, heads, stages, groups, sub, [0.1 * 0.9**s for s in range(stages)]) for _ in range(2)]
+    pair = [VQCodeCache(*tables, batch=batch, max_tokens=80, window=32, device=device, rope_theta=rope) for _ in range(2)]
+    rows = [make_states(gen, (batch, heads, prompt, groups * sub)).to(device) for _ in range(2)]
+    for cache in pair:
+        cache.append(*rows)
+
+    def inputs():
+        query = (torch.randn(batch, 8, groups * sub, generator=gen) / (groups * sub) ** 0.5).half().to(device)
+        return query, *(make_states(gen, (batch, heads, 1, groups * sub)).to(device) for _ in range(2))
+
+    return (*pair, inputs)
+
+
+def _step_equals_append_and_attend(stepped, plain, query, key, value):
+    out = stepped.decode_step(query, key, value)
+    plain.append(key, value)
+    want = plain.attend(query)
+    assert rel_l2(out, want) <= 1e-3
+    assert torch.equal(stepped.key, plain.key) and torch.equal(stepped.value, plain.value)
+    assert rel_l2(stepped.attend(query), want) <= 1e-3  # and the range left on the device is the one that was seen
+
+
+@pytest.mark.parametrize("rope", [None, 1e6])
+@pytest.mark.parametrize("groups,stages,sub", [(16, 2, 8), (1, 2, 128)])
+def test_a_step_uses_the_buffers_tables_and_window_that_the_cache_has_now(device, groups, stages, sub, rope):
+    gen = torch.Generator().manual_seed(8611)
+    stepped, plain, inputs = _decoding_pair(gen, device, groups, stages, sub, rope)
+    _step_equals_append_and_attend(stepped, plain, *inputs())
+    for cache in (stepped, plain):
+        cache.window = 8
+    _step_equals_append_and_attend(stepped, plain, *inputs())
+    for cache in (stepped, plain):
+        cache.window = None
+    left = stepped.key
+    before = left.clone()
+    for cache in (stepped, plain):  # sequences change places, as in a beam search
+        cache.key, cache.value = cache.key.flip(0).contiguous(), cache.value.flip(0).contiguous()
+    _step_equals_append_and_attend(stepped, plain, *inputs())
+    assert torch.equal(left, before)
+    tables = [make_tables(gen, 2, stages, groups, sub, [0.2 * 0.9**s for s in range(stages)]).to(device) for _ in range(2)]
+    for cache in (stepped, plain):  # tables after a training step
+        cache.key_tables, cache.value_tables = tables[0].clone(), tables[1].clone()
+    _step_equals_append_and_attend(stepped, plain, *inputs())
+    length = stepped.length
+    for name, wrong in (("key", stepped.key[:, :, :-1]), ("value", stepped.value.to(torch.int16)), ("key_tables", stepped.key_tables[:, :, :, :, : sub // 2]),
+                        ("value_tables", stepped.value_tables.float())):
+        kept = getattr(stepped, name)
+        setattr(stepped, name, wrong)
+        with pytest.raises(ValueError):
+            stepped.decode_step(*inputs())
+        setattr(stepped, name, kept)
+    assert stepped.length == length
+
+
+@pytest.mark.parametrize("duplicate", ["copy", "deepcopy", "pickle"])
+@pytest.mark.parametrize("groups,stages,sub", [(16, 2, 8), (1, 2, 128)])
+def test_a_copied_cache_steps_on_its_own_buffers(device, groups, stages, sub, duplicate):
+    import copy
+    import pickle
+
+    gen = torch.Generator().manual_seed(8612)
+    stepped, plain, inputs = _decoding_pair(gen, device, groups, stages, sub, None)
+    _step_equals_append_and_attend(stepped, plain, *inputs())
+    fork = {"copy": copy.copy, "deepcopy": copy.deepcopy, "pickle": lambda cache: pickle.loads(pickle.dumps(cache))}[duplicate](stepped)
+    other = copy.deepcopy(plain)
+    if duplicate == "copy":
+        fork.key, fork.value = fork.key.clone(), fork.value.clone()
+    for _ in range(2):  # the fork runs ahead; the original goes on from where it was
+        _step_equals_append_and_attend(fork, other, *inputs())
+    assert torch.equal(stepped.key, plain.key) and torch.equal(stepped.value, plain.value)
+    query, _, _ = inputs()
+    assert rel_l2(stepped.attend(query), plain.attend(query)) <= 1e-3
+    _step_equals_append_and_attend(stepped, plain, *inputs())
