@@ -120,7 +120,9 @@ class VQCodeCache:
         """Append the new token rows and attend, in one library call (``append`` + ``attend`` fused).
 
         ``query [B,Hq,D]`` fp16 scaled (and rotated, for a cache of pre-rotary keys), ``raw_key`` / ``raw_value``
-        ``[B,H,T_new,D]`` contiguous fp16 or fp32.  The buffers, tables and window are the cache's at this call.
+        ``[B,H,T_new,D]`` contiguous fp16 or fp32.  The buffers, tables and window are the cache's at this call.  A cache of
+        pre-rotary keys also takes what ``append`` and ``attend`` take (strided rows and queries, K and V of different
+        types, no new token, strided tables) and any ``out`` that the result can be copied to: these steps are the separate calls.
         """
         batch, heads, dim = self.batch, self.heads, self.dim
         shape, q_shape, dtype = raw_key.shape, query.shape, raw_key.dtype
@@ -128,9 +130,15 @@ class VQCodeCache:
             raise ValueError("rows must be [B,H,T,D] matching the cache geometry")
         if len(q_shape) != 3 or q_shape[0] != batch or q_shape[2] != dim or query.dtype != torch.float16:
             raise ValueError("query must be fp16 [B,Hq,D]")
+        packed = raw_key.is_contiguous() and raw_value.is_contiguous() and query.is_contiguous()
+        if self.rope is not None and not (packed and dtype == raw_value.dtype and shape[2] and (out is None or self._result_fits(out, query))
+                                          and self.key_tables.is_contiguous() and self.value_tables.is_contiguous()):
+            self.append(raw_key, raw_value)
+            result = self.attend(query)
+            return result if out is None else out.copy_(result)
         if dtype != raw_value.dtype or dtype not in ops._DTYPE_TAG:
             raise ValueError("rows must be of one dtype, fp16 or fp32")
-        if not (raw_key.is_contiguous() and raw_value.is_contiguous() and query.is_contiguous()):
+        if not packed:
             raise ValueError("query and rows must be contiguous")
         ktab, vtab, rope, key, value, start, end, words, index = self._addresses()
         if not (index == query.get_device() == raw_key.get_device() == raw_value.get_device()):
@@ -160,6 +168,17 @@ class VQCodeCache:
         self.length += tokens
         self._range_is = self.visible()
         return out
+
+    def _result_fits(self, out: torch.Tensor, query: torch.Tensor) -> bool:
+        """Whether attention may write its result to ``out`` while it reads ``query``."""
+        apart = out.data_ptr() + 2 * out.numel() <= query.data_ptr() or query.data_ptr() + 2 * query.numel() <= out.data_ptr()
+        return apart and out.shape == query.shape and out.dtype == torch.float16 and out.is_contiguous() and out.device == query.device
+
+    @staticmethod
+    def _result_fits(out: torch.Tensor, query: torch.Tensor) -> bool:
+        """Whether attention may write its result to ``out`` while it reads ``query``."""
+        apart = out.data_ptr() + 2 * out.numel() <= query.data_ptr() or query.data_ptr() + 2 * query.numel() <= out.data_ptr()
+        return apart and out.shape == query.shape and out.dtype == torch.float16 and out.is_contiguous() and out.device == query.device
 
     def _addresses(self) -> tuple[int, ...]:
         """Where the K and V tables, the rotary table, the K and V codes and the range's two ends are; words a table, device.

@@ -161,3 +161,36 @@ def test_a_copied_cache_steps_on_its_own_buffers(device, groups, stages, sub, du
     query, _, _ = inputs()
     assert rel_l2(stepped.attend(query), plain.attend(query)) <= 1e-3
     _step_equals_append_and_attend(stepped, plain, *inputs())
+
+
+def test_a_rotary_cache_takes_the_rows_that_append_takes(device):
+    """Rows of a [B,T,H,D] projection seen as [B,H,T,D], rows and queries cut out of one fused buffer, K and V of different
+    types, rows at odd addresses, no new token; results copied to another type, to strided memory and over the query."""
+    gen = torch.Generator().manual_seed(8613)
+    stepped, plain, inputs = _decoding_pair(gen, device, 1, 3, 128, 1e6)
+
+    def projected(tokens):
+        return make_states(gen, (2, tokens, 2, 128)).to(device).transpose(1, 2)
+
+    fused = make_states(gen, (2, 1, 8 + 2 + 2, 128)).to(device) / 4  # heads of q, k, v side by side
+    query, key, value = inputs()
+    shifted = torch.empty(key.numel() + 1, dtype=key.dtype, device=device)[1:].view(key.shape).copy_(key)
+    for case in (
+        (query, projected(3), projected(3)),
+        (fused[:, 0, :8], fused[:, :, 8:10].transpose(1, 2), fused[:, :, 10:].transpose(1, 2)),
+        (query, key, value.float()),
+        (query, shifted, shifted),
+        (query, key[:, :, :0], value[:, :, :0]),
+    ):
+        _step_equals_append_and_attend(stepped, plain, *case)
+    for cache in (stepped, plain):
+        cache.key_tables = cache.key_tables.transpose(3, 4).contiguous().transpose(3, 4)
+    _step_equals_append_and_attend(stepped, plain, query, key, value)
+    wide = torch.zeros(2, 8, 256, dtype=torch.float16, device=device)
+    for out in (torch.empty(2, 8, 128, device=device), wide[:, :, ::2], torch.empty_like(query), query.clone()):
+        case = (out if out.dtype == torch.float16 and torch.equal(out, query) else query, key, value)
+        before = case[0].clone()
+        got = stepped.decode_step(*case, out=out)
+        plain.append(key, value)
+        assert got is out and torch.equal(got.half(), plain.attend(before))
+    assert torch.equal(stepped.key, plain.key) and bool((wide[:, :, 1::2] == 0).all())
