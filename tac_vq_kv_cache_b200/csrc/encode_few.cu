@@ -164,7 +164,6 @@ encode_few_wide_kernel(FewSide first, FewSide second, int64_t sxb, int64_t sxh, 
     const uint32_t tab0 = (uint32_t)__cvta_generic_to_shared(tab);
     constexpr int PS = DSUB + 8;  // halves per column of `parts`: padded so that a fragment's columns differ in bank
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int h = blockIdx.y / G, g = blockIdx.y % G;
     const bool is_second = blockIdx.z != 0;
     const FewSide side = is_second ? second : first;

@@ -88,3 +88,25 @@ def test_ties_and_extreme_scales_are_left_to_the_exact_chain(device, rows, sub, 
     want, want_recon = C.encode(states, tables)
     codes, recon = ops.encode(states.to(device), tables.to(device))
     assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
+
+
+def test_rows_of_a_wide_cache_feed_the_next_step_of_a_narrow_one(device):
+    """The quantised rows of a few-row encode are a later launch's input on the same stream: all of them are there when it reads them."""
+    from tac_vq_kv_cache_b200.code_cache import VQCodeCache
+
+    gen = torch.Generator().manual_seed(5)
+    wide_tables = [make_tables(gen, 8, 16, 1, 128, [0.1 * 0.9**s for s in range(16)]) for _ in range(2)]
+    narrow_tables = [make_tables(gen, 8, 2, 16, 8) for _ in range(2)]
+    wide = VQCodeCache(*wide_tables, batch=1, max_tokens=12, device=device)
+    narrow = VQCodeCache(*narrow_tables, batch=1, max_tokens=12, device=device)
+    query = (torch.randn(1, 32, 128, generator=gen) / 128**0.5).half().to(device)
+    states = [[make_states(gen, (1, 8, 1, 128)).to(device) for _ in range(2)] for _ in range(12)]
+    rows = []
+    for key, value in states:
+        rows.append(wide.append(key, value, want_recon=True))
+        narrow.decode_step(query, *rows[-1])
+    for t, (key, value) in enumerate(states):
+        for got, codes, table, deep, x in zip(rows[t], (narrow.key, narrow.value), narrow_tables, wide_tables, (key, value)):
+            want_row = C.encode(x.cpu(), deep)[1]
+            assert torch.equal(got.cpu(), want_row)
+            assert torch.equal(codes[:, :, t : t + 1].cpu(), C.encode(want_row, table, want_recon=False)[0])
