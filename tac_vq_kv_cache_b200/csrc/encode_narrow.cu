@@ -332,7 +332,7 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
 
                 // ---- exact re-evaluation.  A lane starts at word lane % 4 of its four and reads copy (lane / 4) % 2 of the words, so that
                 // eight neighbouring lanes meet eight different 16-byte banks whatever their fours are ----
-                float best = inf;
+                float best = 3.402823466e38f;  // an infinite or NaN distance never wins, as in a scan for '<' from +inf
                 int arg = 0x7fffffff;
                 while ((low | high) != 0u) {
                     const int p = low != 0u ? __ffs((int)low) - 1 : 31 + __ffs((int)high);
@@ -351,7 +351,7 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                     }
                 }
                 __syncwarp();
-                if (arg >= K) arg = 0;  // every distance was +inf or NaN
+                if (arg >= K) arg = 0;  // no distance was finite
                 float sel[8];
                 unpack8(*reinterpret_cast<const uint4 *>(stage + arg * 32 + copy), sel);
 #pragma unroll

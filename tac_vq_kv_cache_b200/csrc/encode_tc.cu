@@ -280,7 +280,8 @@ encode_tc8_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t sx
             // Exact re-evaluation, shared by the quad: every lane holds both rows, so the four words of a
             // candidate pair (two tiles x two columns of the owning lane) go one to each lane.  Usually
             // one trip handles the single candidate of row a and of row b together.
-            float best_a = inf, best_b = inf;
+            // (from the largest finite value: an infinite or NaN distance never wins, as in a scan for '<' from +inf)
+            float best_a = 3.402823466e38f, best_b = 3.402823466e38f;
             int arg_a = 0x7fffffff, arg_b = 0x7fffffff;
             const int quad = lane & 28;
             while (true) {
@@ -313,7 +314,7 @@ encode_tc8_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t sx
                 const int ib = __shfl_xor_sync(0xffffffffu, arg_b, off);
                 if (ob < best_b || (ob == best_b && ib < arg_b)) best_b = ob, arg_b = ib;
             }
-            if (arg_a >= K) arg_a = 0;  // every distance was +inf or NaN
+            if (arg_a >= K) arg_a = 0;  // no distance was finite
             if (arg_b >= K) arg_b = 0;
 
             const float2 sel_a = *reinterpret_cast<const float2 *>(wordf + arg_a * 8 + 2 * q);

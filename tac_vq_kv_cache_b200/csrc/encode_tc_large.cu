@@ -395,7 +395,7 @@ encode_tc_large_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64
                     dot = __fmaf_rn(r1.w, c.y, dot);
                 }
                 const float dist = distance_expr(xxs[r], nrm[k], dot);
-                if (dist == dist) {  // a NaN distance never wins, as in a strict '<' scan
+                if (dist < inf) {  // an infinite or NaN distance never wins, as in a strict '<' scan
                     const unsigned long long key = ((unsigned long long)ordered_bits(dist) << 32) | (unsigned)k;
                     atomicMin(best + r, key);
                 }

@@ -461,3 +461,30 @@ def test_codeword_gradient_sums_the_rows_that_chose_a_word(device, sub, groups, 
                 want[h, s, g].index_add_(0, codes[:, h, :, s, g].reshape(-1).long(), rows)
                 size[h, s, g].index_add_(0, codes[:, h, :, s, g].reshape(-1).long(), rows.abs())
     assert bool(((got.double() - want).abs() <= 602 * 2.0**-23 * size).all())
+
+
+@pytest.mark.parametrize(
+    "tokens,sub,groups,stages,dtype,whitened",
+    [(tokens, sub, groups, stages, dtype, False)
+     for sub, groups, stages in ((4, 32, 1), (8, 16, 2), (16, 4, 2), (32, 4, 2), (64, 2, 2), (128, 1, 3))
+     for tokens, dtype in ((5, torch.float16), (150, torch.float16), (1300, torch.float16), (1300, torch.float32))]
+    + [(150, 128, 1, 2, torch.float32, True), (150, 4, 32, 1, torch.float16, True)],
+)
+def test_rows_with_infinities_and_nan_take_word_zero_and_leave_their_neighbours_alone(device, tokens, sub, groups, stages, dtype, whitened):
+    """The oracle's scan keeps word 0 where no distance is finite, for however many rows travel together."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(tokens + sub)
+    tables = make_tables(gen, 4, stages, groups, sub, [0.3 * 0.8**s for s in range(stages)])
+    states = make_states(gen, (1, 4, tokens, sub * groups), dtype)
+    big = 3e30 if dtype == torch.float32 else 65504.0
+    for i, value in enumerate((float("inf"), -float("inf"), float("nan"), big)):
+        states[0, i % 4, i :: 5, i * 3 % sub :: sub] = value  # an element in every group
+    states[0, 0, ::7, : sub] = float("inf")
+    if whitened:
+        w = torch.eye(sub).expand(4, groups, sub, sub) + 0.3 * torch.randn(4, groups, sub, sub, generator=gen) / sub**0.5
+        want, want_recon = C.encode_whitened(states, tables, w)
+        codes, recon = ops.encode(states.to(device), tables.to(device), whitener=w.to(device))
+    else:
+        want, want_recon = C.encode(states, tables)
+        codes, recon = ops.encode(states.to(device), tables.to(device))
+    assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
