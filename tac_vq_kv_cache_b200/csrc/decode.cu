@@ -95,6 +95,11 @@ constexpr int kStagedThreads = 1024;
 constexpr int kStagedMaxBytes = 160 * 1024;
 constexpr int kBulkPiece = 16 * 1024;
 
+// A row of one or two fp16 words, asked for in fp16, is their packed fp16 sum: the fp32 sum rounded to fp16 is the same value,
+// because a format of 24 bits holds twice 11 bits and two more, so that rounding twice changes nothing.  A sum that starts at
+// +0, as the library's does, is never -0, hence the last step.
+__device__ __forceinline__ __half2 plus_zero(__half2 v) { return __hadd2(v, __half2half2(__ushort_as_half(0))); }
+
 template <typename OT>
 __global__ void __launch_bounds__(kStagedThreads)
 decode_staged_kernel(const uint8_t *__restrict__ codes, const __half *__restrict__ tables, OT *__restrict__ out, int B,
@@ -212,16 +217,18 @@ decode_staged_kernel(const uint8_t *__restrict__ codes, const __half *__restrict
             continue;
         }
         if (S_use <= 2 && sizeof(OT) == 2) {
-            // one or two fp16 words: their fp32 sum is exact, so its single rounding to fp16 is a packed fp16 add
+            // one or two fp16 words: packed fp16 adds (see plus_zero)
             uint4 packed = make_uint4(0u, 0u, 0u, 0u);
             if (S_use >= 1) packed = *reinterpret_cast<const uint4 *>(tab_g + c_first * d);
+            __half2 *pv = reinterpret_cast<__half2 *>(&packed);
             if (S_use == 2) {
                 const uint4 second = *reinterpret_cast<const uint4 *>(tab_g + stage_stride + c_second * d);
-                __half2 *pv = reinterpret_cast<__half2 *>(&packed);
                 const __half2 *sv = reinterpret_cast<const __half2 *>(&second);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) pv[i] = __hadd2(pv[i], sv[i]);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) pv[i] = plus_zero(pv[i]);
             *reinterpret_cast<uint4 *>(dst) = packed;
             continue;
         }
@@ -403,14 +410,15 @@ decode_rows_kernel(const uint8_t *__restrict__ codes, const __half *__restrict__
             if (sizeof(OT) == 2 && !there) continue;
             OT *dst = out + (there ? to[i] : 0);
             if constexpr (sizeof(OT) == 2) {
-                // the fp32 sum of one or two fp16 words is exact, so its single rounding to fp16 is a packed fp16 add
                 uint4 sum = w[0];
+                __half2 *pv = reinterpret_cast<__half2 *>(&sum);
                 if constexpr (STAGES == 2) {
-                    __half2 *pv = reinterpret_cast<__half2 *>(&sum);
                     const __half2 *sv = reinterpret_cast<const __half2 *>(&w[STAGES - 1]);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) pv[j] = __hadd2(pv[j], sv[j]);
                 }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) pv[j] = plus_zero(pv[j]);
                 __stcs(reinterpret_cast<uint4 *>(dst), sum);
             } else {
                 float sum[8];

@@ -488,3 +488,18 @@ def test_rows_with_infinities_and_nan_take_word_zero_and_leave_their_neighbours_
         want, want_recon = C.encode(states, tables)
         codes, recon = ops.encode(states.to(device), tables.to(device))
     assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
+
+
+@pytest.mark.parametrize("sub,groups,stages,words,depth", [(4, 32, 1, 256, 1), (4, 32, 2, 256, 2), (8, 16, 2, 256, 1), (8, 16, 2, 256, 2), (8, 16, 2, 99, 2), (128, 1, 1, 256, 1)])
+@pytest.mark.parametrize("tokens", [100, 1100])
+def test_rebuilt_fp16_rows_equal_the_oracle_bit_for_bit(device, sub, groups, stages, words, depth, tokens):
+    """Signs of zero included (words that are -0 give +0, as a sum from +0 does), and sums that fp32 does not hold exactly."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(words)
+    tables = make_tables(gen, 3, stages, groups, sub)[:, :, :, :words].contiguous()
+    tables[torch.rand(tables.shape, generator=gen) < 0.3] = -0.0
+    tables[torch.rand(tables.shape, generator=gen) < 0.2] *= 2.0**-18
+    tables[torch.rand(tables.shape, generator=gen) < 0.2] *= 2.0**14
+    codes = torch.randint(0, words, (1, 3, tokens, stages, groups), generator=gen, dtype=torch.uint8)
+    got = ops.decode(codes.to(device), tables.to(device), depth=depth).cpu()
+    assert torch.equal(got.view(torch.int16), C.decode(codes, tables, torch.float16, depth=depth).view(torch.int16))
