@@ -231,13 +231,17 @@ class VQCodeCache:
         ``host_rows``: pinned CPU fp16 tensor holding, back to back, the scaled query ``[B,Hq,D]``, the new K
         rows ``[B,H,tokens,D]`` and the new V rows; ``host_out``: pinned CPU fp16 ``[B,Hq,D]`` that receives the
         result.  The call enqueues the copy to the device, the encode + append + attention of
-        :meth:`decode_step` and the copy back, and by default waits for them.  A decoding loop passes the same
-        buffers every step: checks and argument marshalling happen once per pair of buffers.
+        :meth:`decode_step` and the copy back, and by default waits for them.  A decoding loop passes the same host
+        buffers every step: they are checked once per pair; the cache's buffers, tables and window are those at the call.
         ``direct=True`` enqueues no copy back: the attention kernel stores the result straight into the pinned
         ``host_out`` (the rows still arrive by an enqueued copy, which was measured faster than reading them in
         place).  ``direct="rows"`` enqueues no copy at all: the kernels also read the pinned rows in place.
         """
-        key = (host_rows.data_ptr(), host_out.data_ptr(), host_rows.numel(), host_out.numel(), q_heads, tokens, direct)
+        codes_k, codes_v, ktab, vtab = self.key, self.value, self.key_tables, self.value_tables
+        # what the checked call rests on; the cache's tensors may have changed place, but not size, layout or device
+        key = (host_rows.data_ptr(), host_out.data_ptr(), host_rows.nbytes, host_out.nbytes, host_rows.dtype, host_out.dtype, q_heads, tokens, direct,
+               codes_k.nbytes, codes_v.nbytes, ktab.nbytes, vtab.nbytes, codes_k.get_device(), codes_v.get_device(), ktab.get_device(), vtab.get_device(),
+               codes_k.is_contiguous() and codes_v.is_contiguous() and ktab.is_contiguous() and vtab.is_contiguous())
         if key != self._host_key:
             if direct not in (False, True, "rows"):
                 raise ValueError('direct must be False, True or "rows"')
@@ -246,7 +250,8 @@ class VQCodeCache:
         args, call, index = self._host_call
         if self.length + tokens > self.max_tokens:
             raise ValueError("code cache is full")
-        args[9] = self.length
+        args[3:7] = ktab.data_ptr(), vtab.data_ptr(), codes_k.data_ptr(), codes_v.data_ptr()
+        args[9], args[10] = self.length, self.window or 0
         args[24] = 1 if synchronize else 0
         args[25] = _raw_stream(index)
         if index == torch.cuda.current_device():
@@ -274,11 +279,10 @@ class VQCodeCache:
         workspace = self._scratch(q_heads)
         dev_rows = None if direct == "rows" else torch.empty(nq + 2 * nkv, dtype=torch.float16, device=self.device)
         dev_out = None if direct else torch.empty(nq, dtype=torch.float16, device=self.device)
-        args = [host_rows.data_ptr(), ops._ptr(dev_rows), ops._DTYPE_TAG[torch.float16], self.key_tables.data_ptr(),
-                self.value_tables.data_ptr(), self.key.data_ptr(), self.value.data_ptr(), self._range[0].data_ptr(),
-                self._range[1].data_ptr(), 0, 0 if self.window is None else self.window, workspace.data_ptr(),
+        _, _, _, _, _, start, end, words, index = self._addresses()
+        # tables, codes, length and window are filled in at every call
+        args = [host_rows.data_ptr(), ops._ptr(dev_rows), ops._DTYPE_TAG[torch.float16], 0, 0, 0, 0, start, end, 0, 0, workspace.data_ptr(),
                 workspace.numel(), ops._ptr(dev_out), host_out.data_ptr(), self.batch, q_heads, self.heads, self.dim,
-                self.groups, self.stages, int(self.key_tables.shape[-2]), tokens, self.max_tokens, 1, 0]
-        index = self.device.index if self.device.index is not None else torch.cuda.current_device()
-        self._host_buffers = (dev_rows, dev_out, workspace)  # keep what the call points at alive
+                self.groups, self.stages, words, tokens, self.max_tokens, 1, 0]
+        self._host_buffers = (dev_rows, dev_out, workspace, self._range)  # keep what the call points at alive
         self._host_call = (args, _lib.load().tacvq_decode_step_host, index)

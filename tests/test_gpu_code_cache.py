@@ -194,3 +194,35 @@ def test_a_rotary_cache_takes_the_rows_that_append_takes(device):
         plain.append(key, value)
         assert got is out and torch.equal(got.half(), plain.attend(before))
     assert torch.equal(stepped.key, plain.key) and bool((wide[:, :, 1::2] == 0).all())
+
+
+def test_a_host_step_uses_the_buffers_tables_and_window_that_the_cache_has_now(device):
+    gen = torch.Generator().manual_seed(8614)
+    stepped, plain, inputs = _decoding_pair(gen, device, 16, 2, 8, None)
+    host_rows = torch.empty(2 * 8 * 128 + 2 * 2 * 2 * 128, dtype=torch.float16).pin_memory()
+    host_out = torch.empty(2, 8, 128, dtype=torch.float16).pin_memory()
+
+    def step():
+        query, key, value = inputs()
+        host_rows.copy_(torch.cat([query.flatten(), key.flatten(), value.flatten()]))
+        torch.cuda.synchronize()
+        stepped.decode_step_host(host_rows, host_out, 8)
+        plain.append(key, value)
+        want = plain.attend(query)
+        assert rel_l2(host_out, want) <= 1e-3 and rel_l2(stepped.attend(query), want) <= 1e-3
+        assert torch.equal(stepped.key, plain.key) and torch.equal(stepped.value, plain.value)
+
+    step()
+    for cache in (stepped, plain):
+        cache.window = 8
+    step()
+    left, before = stepped.key, stepped.key.clone()
+    for cache in (stepped, plain):
+        cache.window = None
+        cache.key, cache.value = cache.key.flip(0).contiguous(), cache.value.flip(0).contiguous()
+    step()
+    assert torch.equal(left, before)
+    tables = [make_tables(gen, 2, 2, 16, 8, [0.2, 0.1]).to(device) for _ in range(2)]
+    for cache in (stepped, plain):
+        cache.key_tables, cache.value_tables = tables[0].clone(), tables[1].clone()
+    step()
