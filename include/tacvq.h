@@ -72,12 +72,11 @@ TACVQ_API const char *tacvq_status_string(int status);
 TACVQ_API int tacvq_table_sqnorm(const uint16_t *tables_f16, float *out, int64_t words, int d, tacvq_stream_t stream);
 
 /*
- * Diagnostic of the wide-group encode (d = 64, 128), whose approximate scores are tensor-core products
- * (tcgen05) kept in tensor memory: *count = how many times, on the current device since the library was
- * loaded, a block stopped waiting for those products and re-evaluated every pair of the stage instead,
- * or stopped waiting for a table copy of the copy engine (TMA) and copied the table itself, plus the number
- * of launches that could not get a tensor map for their tables at all (codes stay exact either way).  Synchronises the device.  Expected value: 0.  No counterpart in the
- * reference.
+ * Diagnostic of the encode kernels that wait for tensor-core products (tcgen05) or for table copies of the copy engine
+ * (TMA): groups 32, 64 and 128 wide, and many rows of groups 4 and 8 wide.  *count = in how many blocks, on the current
+ * device since the library was loaded, a wait was given up - the rows concerned are then searched word by word, from
+ * tables in global memory - plus the number of launches that could not get a tensor map for their tables at all (codes
+ * stay exact either way).  Synchronises the device.  Expected value: 0.  No counterpart in the reference.
  */
 TACVQ_API int tacvq_encode_tensor_memory_timeouts(unsigned int *count);
 
@@ -133,6 +132,16 @@ TACVQ_API int tacvq_encode_whitened_filtered(const void *x, int x_dtype, int64_t
                           float *search_rows, void *filter, size_t filter_bytes, uint8_t *codes, void *recon,
                           int recon_dtype, int B, int H, int T, int D, int G, int S, int K, int64_t t0, int64_t T_cap,
                           tacvq_stream_t stream);
+
+/*
+ * tacvq_encode (whitener NULL) or tacvq_encode_whitened_filtered with every wait inside the kernels given up after
+ * `wait_spins` >= 0 polls (0: at once), for checking the route that a late product or table takes.  Same codes.
+ */
+TACVQ_API int tacvq_encode_wait_limited(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
+                          const uint16_t *tables_f16, const float *table_sqnorm, const float *whitener,
+                          float *search_tables, float *search_rows, void *filter, size_t filter_bytes, uint8_t *codes,
+                          void *recon, int recon_dtype, int B, int H, int T, int D, int G, int S, int K, int64_t t0,
+                          int64_t T_cap, int wait_spins, tacvq_stream_t stream);
 
 /*
  * Decode: rebuild rows t0 .. t0+T-1 from stored codes using the first S_use stages.

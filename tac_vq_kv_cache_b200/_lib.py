@@ -28,6 +28,8 @@ _SIGNATURES = {
     "tacvq_encode_whitened_filter_bytes": (c_size_t, [c_int] * 5),
     "tacvq_encode_whitened_filtered": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int64] + [c_void_p] * 5 + [c_size_t, c_void_p, c_void_p,
                                                c_int] + [c_int] * 7 + [c_int64, c_int64, c_void_p]),
+    "tacvq_encode_wait_limited": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int64] + [c_void_p] * 6 + [c_size_t, c_void_p, c_void_p, c_int]
+                                  + [c_int] * 7 + [c_int64, c_int64, c_int, c_void_p]),
     "tacvq_decode": (c_int, [c_void_p, c_void_p, c_void_p, c_int] + [c_int] * 8 + [c_int64, c_int64, c_void_p]),
     "tacvq_codeword_grad": (c_int, [c_void_p, c_void_p, c_void_p] + [c_int] * 8 + [c_int64, c_int64, c_void_p]),
     "tacvq_attn_workspace_bytes": (c_size_t, [c_int] * 6),

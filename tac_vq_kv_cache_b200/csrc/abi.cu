@@ -155,9 +155,9 @@ int tacvq_encode_tensor_memory_timeouts(unsigned int *count) {
     return tensor_memory_timeouts(count);
 }
 
-int tacvq_encode(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt, const uint16_t *tables_f16,
-                 const float *table_sqnorm, uint8_t *codes, void *recon, int recon_dtype, int B, int H, int T, int D,
-                 int G, int S, int K, int64_t t0, int64_t T_cap, tacvq_stream_t stream) {
+static int encode_plain(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt, const uint16_t *tables_f16,
+                        const float *table_sqnorm, uint8_t *codes, void *recon, int recon_dtype, int B, int H, int T, int D,
+                        int G, int S, int K, int64_t t0, int64_t T_cap, int wait_spins, tacvq_stream_t stream) {
     if (!dtype_ok(x_dtype) || (recon && !dtype_ok(recon_dtype))) return TACVQ_ERR_DTYPE;
     const int g = check_code_geometry(B, H, T, D, G, S, K, t0, T_cap);
     if (g != TACVQ_OK) return g;
@@ -167,7 +167,15 @@ int tacvq_encode(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t s
     if (sxb < 0 || sxh < 0 || sxt < D) return TACVQ_ERR_GEOMETRY;
     EncodeArgs a{x, x_dtype, sxb, sxh, sxt, tables_f16, false, table_sqnorm, codes, recon, recon_dtype,
                  (const __half *)tables_f16, B, H, T, D, G, S, K, t0, T_cap, (cudaStream_t)stream};
+    a.wait_spins = wait_spins;
     return encode_dispatch(a);
+}
+
+int tacvq_encode(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt, const uint16_t *tables_f16,
+                 const float *table_sqnorm, uint8_t *codes, void *recon, int recon_dtype, int B, int H, int T, int D,
+                 int G, int S, int K, int64_t t0, int64_t T_cap, tacvq_stream_t stream) {
+    return encode_plain(x, x_dtype, sxb, sxh, sxt, tables_f16, table_sqnorm, codes, recon, recon_dtype, B, H, T, D, G, S, K, t0,
+                        T_cap, -1, stream);
 }
 
 size_t tacvq_encode_whitened_filter_bytes(int H, int D, int G, int S, int K) {
@@ -178,11 +186,11 @@ size_t tacvq_encode_whitened_filter_bytes(int H, int D, int G, int S, int K) {
     return ((words * d * sizeof(__half) + 255) & ~(size_t)255) + words * sizeof(float);
 }
 
-int tacvq_encode_whitened_filtered(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
-                                   const uint16_t *tables_f16, const float *whitener, float *search_tables,
-                                   float *search_rows, void *filter, size_t filter_bytes, uint8_t *codes, void *recon,
-                                   int recon_dtype, int B, int H, int T, int D, int G, int S, int K, int64_t t0, int64_t T_cap,
-                                   tacvq_stream_t stream) {
+static int encode_whitened(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
+                           const uint16_t *tables_f16, const float *whitener, float *search_tables,
+                           float *search_rows, void *filter, size_t filter_bytes, uint8_t *codes, void *recon,
+                           int recon_dtype, int B, int H, int T, int D, int G, int S, int K, int64_t t0, int64_t T_cap,
+                           int wait_spins, tacvq_stream_t stream) {
     if (!dtype_ok(x_dtype) || (recon && !dtype_ok(recon_dtype))) return TACVQ_ERR_DTYPE;
     const int g = check_code_geometry(B, H, T, D, G, S, K, t0, T_cap);
     if (g != TACVQ_OK) return g;
@@ -198,6 +206,7 @@ int tacvq_encode_whitened_filtered(const void *x, int x_dtype, int64_t sxb, int6
     EncodeArgs a{search_rows, TACVQ_F32, (int64_t)H * T * D, (int64_t)T * D, (int64_t)D, search_tables, true, nullptr,
                  codes, recon, recon_dtype, (const __half *)tables_f16, B, H, T, D, G, S, K, t0, T_cap,
                  (cudaStream_t)stream};
+    a.wait_spins = wait_spins;
     if (need > 0) {
         const int64_t words = (int64_t)H * S * G * K;
         float *norms = (float *)((unsigned char *)filter + need - words * sizeof(float));
@@ -209,12 +218,34 @@ int tacvq_encode_whitened_filtered(const void *x, int x_dtype, int64_t sxb, int6
     return encode_dispatch(a);
 }
 
+int tacvq_encode_whitened_filtered(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
+                                   const uint16_t *tables_f16, const float *whitener, float *search_tables,
+                                   float *search_rows, void *filter, size_t filter_bytes, uint8_t *codes, void *recon,
+                                   int recon_dtype, int B, int H, int T, int D, int G, int S, int K, int64_t t0, int64_t T_cap,
+                                   tacvq_stream_t stream) {
+    return encode_whitened(x, x_dtype, sxb, sxh, sxt, tables_f16, whitener, search_tables, search_rows, filter, filter_bytes,
+                           codes, recon, recon_dtype, B, H, T, D, G, S, K, t0, T_cap, -1, stream);
+}
+
+int tacvq_encode_wait_limited(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt, const uint16_t *tables_f16,
+                              const float *table_sqnorm, const float *whitener, float *search_tables, float *search_rows,
+                              void *filter, size_t filter_bytes, uint8_t *codes, void *recon, int recon_dtype, int B, int H,
+                              int T, int D, int G, int S, int K, int64_t t0, int64_t T_cap, int wait_spins,
+                              tacvq_stream_t stream) {
+    if (wait_spins < 0) return TACVQ_ERR_RANGE;
+    if (whitener)
+        return encode_whitened(x, x_dtype, sxb, sxh, sxt, tables_f16, whitener, search_tables, search_rows, filter, filter_bytes,
+                               codes, recon, recon_dtype, B, H, T, D, G, S, K, t0, T_cap, wait_spins, stream);
+    return encode_plain(x, x_dtype, sxb, sxh, sxt, tables_f16, table_sqnorm, codes, recon, recon_dtype, B, H, T, D, G, S, K, t0,
+                        T_cap, wait_spins, stream);
+}
+
 int tacvq_encode_whitened(const void *x, int x_dtype, int64_t sxb, int64_t sxh, int64_t sxt,
                           const uint16_t *tables_f16, const float *whitener, float *search_tables,
                           float *search_rows, uint8_t *codes, void *recon, int recon_dtype, int B, int H, int T, int D,
                           int G, int S, int K, int64_t t0, int64_t T_cap, tacvq_stream_t stream) {
-    return tacvq_encode_whitened_filtered(x, x_dtype, sxb, sxh, sxt, tables_f16, whitener, search_tables, search_rows, nullptr, 0,
-                                          codes, recon, recon_dtype, B, H, T, D, G, S, K, t0, T_cap, stream);
+    return encode_whitened(x, x_dtype, sxb, sxh, sxt, tables_f16, whitener, search_tables, search_rows, nullptr, 0,
+                           codes, recon, recon_dtype, B, H, T, D, G, S, K, t0, T_cap, -1, stream);
 }
 
 int tacvq_decode(const uint8_t *codes, const uint16_t *tables_f16, void *out, int out_dtype, int B, int H, int T,

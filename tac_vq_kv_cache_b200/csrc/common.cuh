@@ -128,6 +128,7 @@ struct EncodeArgs {
     int B, H, T, D, G, S, K;
     int64_t t0, T_cap;
     cudaStream_t stream;
+    int wait_spins = -1;                    // polls of a wait inside a kernel before it is given up; -1: the kernel's own bound
     const __half *filter_tables = nullptr;  // fp16 rounding of fp32 search tables, for kernels that filter on the tensor core
 };
 

@@ -37,6 +37,10 @@ namespace {
 constexpr int kThreads = kMaxWords;  // a thread per word; as many threads again compute |c|^2 one stage ahead
 constexpr int kWarps = kThreads / 32;
 constexpr int kRing = 3;             // stages of tables in shared memory
+constexpr int kSpins = 1 << 20;
+
+// blocks in which a wait was given up; expected to stay 0
+__device__ unsigned int g_timeouts = 0;
 
 struct FewSide {
     const void *x;
@@ -148,7 +152,7 @@ template <int DSUB, typename XT, int R>
 __global__ void __launch_bounds__(2 * kThreads, 1)
 encode_few_wide_kernel(FewSide first, FewSide second, int64_t sxb, int64_t sxh, int64_t sxt, int recon_dtype, int ring,
                        int32_t *__restrict__ seq_start, int32_t *__restrict__ seq_end, int start, int end, int B, int H, int T,
-                       int G, int S, int K, int64_t t0, int64_t T_cap, const __grid_constant__ CUtensorMap first_map,
+                       int G, int S, int K, int64_t t0, int64_t T_cap, int spins, const __grid_constant__ CUtensorMap first_map,
                        const __grid_constant__ CUtensorMap second_map) {
     using L = FewLayout<DSUB, R>;
     extern __shared__ __align__(128) unsigned char smem_dyn[];
@@ -184,9 +188,9 @@ encode_few_wide_kernel(FewSide first, FewSide second, int64_t sxb, int64_t sxh, 
                          "l"(is_second ? &second_map : &first_map), "r"(panel * 64), "r"(first_word), "r"(bar)
                          : "memory");
     };
-    auto arrived = [&](int slot, int phase) {
+    auto arrived = [&](int slot, int phase, int polls) {
         int ok = 0;
-        for (int spin = 0; spin < (1 << 20) && !ok; ++spin)  // bounded: on running out the stage reads global memory
+        for (int spin = 0; spin < polls && !ok; ++spin)  // bounded: on running out the stage reads global memory
             asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.s32 %0, 1, 0, p;\n}"
                          : "=r"(ok) : "r"(bar0 + slot * 8), "r"((uint32_t)phase) : "memory");
         return ok != 0;
@@ -238,24 +242,25 @@ encode_few_wide_kernel(FewSide first, FewSide second, int64_t sxb, int64_t sxh, 
         }
         nrm[(s & 1) * kMaxWords + word] = v;
     };
-    if (!searcher) norm_stage(0, 0, __all_sync(0xffffffffu, arrived(0, 0)));
+    if (!searcher) norm_stage(0, 0, __all_sync(0xffffffffu, arrived(0, 0, spins)));
 
-    bool missed = false;
+    int requested = S < 2 ? S : 2;
     int slot = 0, phase = 0, next = ring > 2 ? 2 : 0;  // slot of stage s with its phase, slot of stage s + 2
     for (int s = 0; s < S; ++s) {
-        const bool staged = __syncthreads_and(arrived(slot, phase));  // also: norms of stage s and the previous update have settled
-        missed |= !staged;
+        const bool staged = __syncthreads_and(arrived(slot, phase, spins));  // also: norms of stage s and the previous update have settled
+        if (!staged) spins = 0;  // a table did not arrive in time: no further one is asked for or waited for
         const int slot_now = slot;
         slot = slot + 1 == ring ? (phase ^= 1, 0) : slot + 1;
         if (!searcher) {
-            if (s + 1 < S) norm_stage(s + 1, slot, __all_sync(0xffffffffu, arrived(slot, phase)));
+            if (s + 1 < S) norm_stage(s + 1, slot, __all_sync(0xffffffffu, arrived(slot, phase, spins)));
             continue;
         }
         const unsigned char *stage = tab + (size_t)slot_now * L::kSlot;
         const __half *plain = words + s * stage_halves;
-        if (tid == 0 && s + 2 < S) {  // its slot was last read by the previous stage's update
+        if (tid == 0 && s + 2 < S && spins != 0) {  // its slot was last read by the previous stage's update
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             request(s + 2, next);
+            ++requested;
         }
         next = next + 1 == ring ? 0 : next + 1;
         auto piece_of = [&](int k, int e) {  // eight elements of word k
@@ -390,8 +395,10 @@ encode_few_wide_kernel(FewSide first, FewSide second, int64_t sxb, int64_t sxh, 
             if (code_at != nullptr) code_at[(int64_t)s * G] = (uint8_t)k;
         }
     }
-    if (missed && tid == 0)  // never seen: one more bounded wait, so that no copy outlives the block
-        for (int i = 0; i < ring; ++i) arrived(i, ((S - i + ring - 1) / ring - 1) & 1);
+    if (spins == 0 && tid == 0) {  // never seen: one more bounded wait, so that no copy outlives the block
+        atomicAdd(&g_timeouts, 1u);
+        for (int i = 0; i < ring && i < requested; ++i) arrived(i, ((requested - i + ring - 1) / ring - 1) & 1, kSpins);
+    }
     if (side.recon != nullptr) {
         for (int i = tid; searcher && i < R * DSUB; i += kThreads) {  // each thread's own elements
             const int row = row0 + i / DSUB;
@@ -407,7 +414,7 @@ encode_few_wide_kernel(FewSide first, FewSide second, int64_t sxb, int64_t sxh, 
 template <int DSUB, typename XT>
 static int launch_few(const FewSide &first, const FewSide &second, int sides, int64_t sxb, int64_t sxh, int64_t sxt, int recon_dtype,
                       int32_t *seq_start, int32_t *seq_end, int start, int end, int B, int H, int T, int G, int S, int K,
-                      int64_t t0, int64_t T_cap, cudaStream_t stream) {
+                      int64_t t0, int64_t T_cap, int spins, cudaStream_t stream) {
     const int64_t rows = (int64_t)B * T;
     const int ring = S < kRing ? S : kRing;
     CUtensorMap first_map, second_map;
@@ -419,7 +426,7 @@ static int launch_few(const FewSide &first, const FewSide &second, int sides, in
         if (e != cudaSuccess) return (int)e;
         dim3 grid((unsigned)((rows + per_block - 1) / per_block), (unsigned)(H * G), (unsigned)sides);
         kernel<<<grid, 2 * kThreads, smem, stream>>>(first, second, sxb, sxh, sxt, recon_dtype, ring, seq_start, seq_end, start, end, B,
-                                                 H, T, G, S, K, t0, T_cap, first_map, second_map);
+                                                 H, T, G, S, K, t0, T_cap, spins < 0 ? kSpins : spins, first_map, second_map);
         return launch_status();
     };
     // the fewest rows per block that keep the launch to about one block per SM
@@ -437,12 +444,12 @@ static bool few_wide_ok(const void *x, const void *tables, int x_dtype, int64_t 
 template <typename XT>
 static int dispatch_few(int d, const FewSide &first, const FewSide &second, int sides, int64_t sxb, int64_t sxh, int64_t sxt,
                         int recon_dtype, int32_t *seq_start, int32_t *seq_end, int start, int end, int B, int H, int T, int G,
-                        int S, int K, int64_t t0, int64_t T_cap, cudaStream_t stream) {
+                        int S, int K, int64_t t0, int64_t T_cap, int spins, cudaStream_t stream) {
     switch (d) {
 #define TACVQ_CASE(N)                                                                                                             \
     case N:                                                                                                                       \
         return launch_few<N, XT>(first, second, sides, sxb, sxh, sxt, recon_dtype, seq_start, seq_end, start, end, B, H, T, G, S, \
-                                 K, t0, T_cap, stream);
+                                 K, t0, T_cap, spins, stream);
         TACVQ_CASE(32)
         TACVQ_CASE(64)
         TACVQ_CASE(128)
@@ -458,7 +465,7 @@ int encode_few_wide_launch(const EncodeArgs &a) {
     auto go = [&](auto *tag) {
         using XT = typename std::remove_pointer<decltype(tag)>::type;
         return dispatch_few<XT>(a.D / a.G, side, side, 1, a.sxb, a.sxh, a.sxt, a.recon_dtype, nullptr, nullptr, 0, 0, a.B, a.H, a.T,
-                                a.G, a.S, a.K, a.t0, a.T_cap, a.stream);
+                                a.G, a.S, a.K, a.t0, a.T_cap, a.wait_spins, a.stream);
     };
     return a.x_dtype == TACVQ_F16 ? go((__half *)nullptr) : go((float *)nullptr);
 }
@@ -472,9 +479,11 @@ int decode_prologue_wide_launch(const void *k_rows, const void *v_rows, int rows
     const FewSide first = {k_rows, ktab, nullptr, kcodes, nullptr}, second = {v_rows, vtab, nullptr, vcodes, nullptr};
     return rows_dtype == TACVQ_F16
                ? dispatch_few<__half>(D / G, first, second, 2, sxb, sxh, sxt, TACVQ_F16, seq_start, seq_end, start, end, B, H, T, G, S, K,
-                                      t0, T_cap, stream)
+                                      t0, T_cap, -1, stream)
                : dispatch_few<float>(D / G, first, second, 2, sxb, sxh, sxt, TACVQ_F16, seq_start, seq_end, start, end, B, H, T, G, S, K,
-                                     t0, T_cap, stream);
+                                     t0, T_cap, -1, stream);
 }
+
+int few_timeouts(unsigned int *out) { return (int)cudaMemcpyFromSymbol(out, g_timeouts, sizeof(unsigned int)); }
 
 }  // namespace tacvq

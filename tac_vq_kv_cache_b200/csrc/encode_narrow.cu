@@ -36,10 +36,14 @@ constexpr int kMaxStages = 12;                                        // and the
 static_assert(kMaxStages * (kStageBytes + 4) + kFixedBytes <= 227 * 1024, "one block's tables");
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity) {
+// blocks in which a wait was given up; expected to stay 0
+__device__ unsigned int g_timeouts = 0;
+
+constexpr int kSpins = 1 << 17;
+__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, int spins) {
     int done = 0;
 #pragma unroll 1
-    for (int spin = 0; spin < (1 << 17) && !done; ++spin)
+    for (int spin = 0; spin < spins && !done; ++spin)
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.s32 %0, 1, 0, p;\n}"
                      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
@@ -105,10 +109,11 @@ template <int DSUB, typename XT>
 __global__ void __launch_bounds__(kThreads, 1)
 encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t sxt, const __half *__restrict__ tables,
                      const float *__restrict__ sqnorm_in, uint8_t *__restrict__ codes, void *__restrict__ recon, int recon_dtype,
-                     int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap, int vec_ok) {
+                     int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap, int vec_ok, int spins) {
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *ones = smem + (size_t)S * kStageBytes, *misc = ones + (1 + kGroups) * kABytes;
     const uint32_t bars = smem_u32(misc);                               // [kGroups]
+    uint32_t *in_flight = reinterpret_cast<uint32_t *>(misc + 32);      // [kGroups] phase of the last product asked for; 2: none
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(misc + 64);
     int *cc_tops = reinterpret_cast<int *>(misc + 128);                 // [S] largest |word|^2 as bits (they order like ints)
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -120,7 +125,10 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int i = 0; i < kGroups; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * i) : "memory");
+        for (int i = 0; i < kGroups; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * i) : "memory");
+            in_flight[i] = 2u;
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (tid < kRows * 2) {
@@ -148,6 +156,7 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
             mma(tmem, descriptor(smem_u32(ones)), descriptor(words_a + (uint32_t)kWordBytes), 0u);
             mma(tmem, descriptor(smem_u32(A)), descriptor(words_a), 1u);
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+            in_flight[grp] = phase;
         }
         __syncwarp();
     };
@@ -290,7 +299,7 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                 for (int half = 0; half < 2; ++half) {
                     float top4[32];
                     if (half == 0) issue(stage, 0);
-                    if (!fail && !bounded_wait(bar, phase)) fail = true;
+                    if (!fail && !bounded_wait(bar, phase, spins)) fail = true;
                     phase ^= 1u;
                     fail = __any_sync(0xffffffffu, fail);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -385,7 +394,10 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
         at += tile1 - tile0;
     }
     }
-    if (fail) bounded_wait(bar, phase ^ 1u);  // what is still in flight gets one more bounded wait
+    if (__syncthreads_or(fail)) {  // each group's last product ends before the block's memory goes
+        if (row == 0 && in_flight[grp] < 2u) bounded_wait(bar, in_flight[grp], kSpins);
+        if (tid == 0) atomicAdd(&g_timeouts, 1u);
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
@@ -416,7 +428,8 @@ int encode_narrow_launch(const EncodeArgs &a) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         kernel<<<(unsigned)blocks, kThreads, smem, a.stream>>>(xp, a.sxb, a.sxh, a.sxt, (const __half *)a.tables, a.sqnorm, a.codes, a.recon,
-                                                               a.recon_dtype, a.B, a.H, a.T, a.G, a.S, a.K, a.t0, a.T_cap, vec_ok);
+                                                               a.recon_dtype, a.B, a.H, a.T, a.G, a.S, a.K, a.t0, a.T_cap, vec_ok,
+                                                               a.wait_spins < 0 ? kSpins : a.wait_spins);
         return launch_status();
     };
     if (sub == 8) {
@@ -426,5 +439,7 @@ int encode_narrow_launch(const EncodeArgs &a) {
     if (a.x_dtype == TACVQ_F16) return launch(encode_narrow_kernel<4, __half>, (const __half *)a.x);
     return launch(encode_narrow_kernel<4, float>, (const float *)a.x);
 }
+
+int narrow_timeouts(unsigned int *out) { return (int)cudaMemcpyFromSymbol(out, narrow::g_timeouts, sizeof(unsigned int)); }
 
 }  // namespace tacvq

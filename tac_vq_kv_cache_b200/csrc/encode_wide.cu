@@ -48,14 +48,15 @@ constexpr int kMaxGroups = 2;       // groups of threads per block
 constexpr int kSeedBytes = kMaxWords * 32;  // 16 halves a word
 constexpr int kOnesBytes = kRows * 32;
 
-// counts waits that were given up; read by tensor_memory_timeouts, expected to stay 0
+// blocks in which a wait was given up; read by tensor_memory_timeouts, expected to stay 0
 __device__ unsigned int g_timeouts = 0;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity) {
+constexpr int kSpins = 1 << 17;
+__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, int spins) {
     int done = 0;
 #pragma unroll 1
-    for (int spin = 0; spin < (1 << 17) && !done; ++spin)
+    for (int spin = 0; spin < spins && !done; ++spin)
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.s32 %0, 1, 0, p;\n}"
                      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
@@ -148,6 +149,35 @@ __device__ __forceinline__ float word_norm_by_eight(const __half *__restrict__ w
     return total;
 }
 
+// The same by one thread, with few registers: for words that did not arrive in time.
+template <int DSUB>
+__device__ __forceinline__ float word_norm_alone(const __half *__restrict__ word) {
+    float total = 0.0f;
+#pragma unroll 1
+    for (int j = 0; j < 8; ++j) {
+        float mine = 0.0f;
+#pragma unroll 1
+        for (int u = 0; u < 4; ++u) {
+            float set = 0.0f;
+#pragma unroll 1
+            for (int i = 8 * u + j; i < DSUB; i += 32) {
+                const float v = __half2float(word[i]);
+                set = __fadd_rn(set, __fmul_rn(v, v));
+            }
+            mine = u == 0 ? set : __fadd_rn(mine, set);
+        }
+        total = j == 0 ? mine : __fadd_rn(total, mine);
+    }
+    return total;
+}
+
+// A 16-byte load that is not moved ahead of others: for words that did not arrive in time, off the usual path.
+__device__ __forceinline__ uint4 load_in_place(const __half *from) {
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(from) : "memory");
+    return v;
+}
+
 // Which of a thread's 64 words a bit of its mask stands for: 16 columns take 16 bits, the even ones first.
 __device__ __forceinline__ int word_of_bit(int bit) { return (bit & 48) | ((bit & 7) << 1) | ((bit >> 3) & 1); }
 
@@ -182,7 +212,7 @@ struct Args {
     const float *sqnorm;     // |word|^2 of the deciding words; may be null for fp16 words
     uint8_t *codes;
     void *recon;
-    int recon_dtype, B, H, T, G, S, K, vec_ok, use_map;
+    int recon_dtype, B, H, T, G, S, K, vec_ok, use_map, spins;
     int64_t t0, T_cap;
 };
 
@@ -199,6 +229,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     const uint32_t full_bar = misc, mma_bar = misc + 16;  // [2] each
     unsigned int *left = reinterpret_cast<unsigned int *>(smem + L::kMisc + 64);  // [2][4]: groups that left a stage of this buffer, all uses together, per quarter
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::kMisc + 48);
+    uint32_t *in_flight = reinterpret_cast<uint32_t *>(smem + L::kMisc + 52);     // [2] phase of the last product asked for; 2: none
     float *cc_tops = reinterpret_cast<float *>(smem + L::kMisc + 128);            // [2][4]: largest norm of a quarter
 
     const int hg = blockIdx.y, h = hg / a.G, g = hg % a.G;
@@ -218,6 +249,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         for (int i = 0; i < 2; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(full_bar + 8 * i) : "memory");  // a warp per quarter of the words
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mma_bar + 8 * i) : "memory");
+            in_flight[i] = 2u;
         }
         for (int i = 0; i < 8; ++i) left[i] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -405,12 +437,11 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             sync_group();  // the group's rows are written, its scores read, the previous stage's words no longer used
-            if (!fail && !bounded_wait(full_bar + 8 * buf, (u >> 1) & 1u)) fail = true;
+            // A warp that gives up (never seen) lists every word from here on and takes words and norms from global memory.  It writes
+            // nothing to the ring and no longer counts as having left a stage: the other group may be working on the buffer's
+            // previous use, which is then not refilled either, so that all warps end up this way.
+            if (!fail && !bounded_wait(full_bar + 8 * buf, (u >> 1) & 1u, a.spins)) fail = true;
             fail = __any_sync(0xffffffffu, fail);
-            if (fail) {  // never seen: the warp brings the words itself (the same bytes) and lists them all
-                copy_table(buf, first);
-                copy_norms(buf, first, 0, kMaxWords);
-            }
             if ((warp & 15) == 0) {
                 if (lane == 0 && !fail) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -421,11 +452,12 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                         mma(d0, panel_descriptor(a0 + (ks >> 2) * (kRows * 128) + (ks & 3) * 32),
                             panel_descriptor(b0 + (ks >> 2) * (kMaxWords * 128) + (ks & 3) * 32), 1u);
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(my_mma) : "memory");
+                    in_flight[grp] = mma_phase;
                 }
                 __syncwarp();
             }
             // use u - 1 is left: the last group to leave it refills its buffer, a quarter per warp of q = 0
-            if (q == 0 && !resident && u >= 1 && u + 1 < uses) {
+            if (q == 0 && !resident && u >= 1 && u + 1 < uses && !fail) {
                 unsigned int n = 0u;
                 __threadfence_block();
                 if (lane == 0) n = atomicAdd(left + ((u - 1) & 1u) * 4 + part, 1u) + 1u;
@@ -439,7 +471,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             const float margin = (sizeof(XT) == 2 && s == 0 ? 1.220703125e-04f : EXACT32 ? 2.01416015625e-03f : 1.03759765625e-03f) * u_top +
                                  9.5367431640625e-07f * xx + 3.0517578125e-05f * cc_top + 3.814697265625e-06f * rough_sqrt(cc_top) +
                                  (EXACT32 ? 9.5367431640625e-07f * rough_sqrt(xx) : 0.0f) + 1.1920929e-07f;
-            if (!fail && !bounded_wait(my_mma, mma_phase)) fail = true;
+            if (!fail && !bounded_wait(my_mma, mma_phase, a.spins)) fail = true;
             mma_phase ^= 1u;
             fail = __any_sync(0xffffffffu, fail);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -458,7 +490,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                 }
                 top = fmaxf(m0, m1);
             }
-            tops[q * kRows] = top;
+            tops[q * kRows] = fail ? -inf : top;  // (what a warp that gave up has read says nothing, and must not raise the others' limit)
             sync_quad();
             top = fmaxf(fmaxf(tops[0], tops[kRows]), fmaxf(tops[2 * kRows], tops[3 * kRows]));
             // ---- the words close to it ----
@@ -580,22 +612,31 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                         const int k = q * 64 + word_of_bit(half * 32 + lane);
                         if ((((half ? listed[1] : listed[0]) >> lane) & 1u) != 0u && k < K) {
                             float dot = 0.0f;
+                            auto chain = [&](auto fetch) {
 #pragma unroll 2
-                            for (int p = 0; p < kPieces; ++p) {
-                                const float *from = piece_at(p & 3, p >> 2);
-                                float e[8], w[8];
-                                *reinterpret_cast<float4 *>(e) = *reinterpret_cast<const float4 *>(from);
-                                *reinterpret_cast<float4 *>(e + 4) = *reinterpret_cast<const float4 *>(from + 4);
-                                if constexpr (EXACT32) {
-                                    *reinterpret_cast<float4 *>(w) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + k) * DSUB + 8 * p));
-                                    *reinterpret_cast<float4 *>(w + 4) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + k) * DSUB + 8 * p + 4));
-                                } else {
-                                    unpack8(*reinterpret_cast<const uint4 *>(tab + L::template at<kMaxWords>(k, 8 * p)), w);
-                                }
+                                for (int p = 0; p < kPieces; ++p) {
+                                    const float *from = piece_at(p & 3, p >> 2);
+                                    float e[8], w[8];
+                                    *reinterpret_cast<float4 *>(e) = *reinterpret_cast<const float4 *>(from);
+                                    *reinterpret_cast<float4 *>(e + 4) = *reinterpret_cast<const float4 *>(from + 4);
+                                    fetch(8 * p, w);
 #pragma unroll
-                                for (int j = 0; j < 8; ++j) dot = __fmaf_rn(e[j], w[j], dot);
+                                    for (int j = 0; j < 8; ++j) dot = __fmaf_rn(e[j], w[j], dot);
+                                }
+                            };
+                            if constexpr (EXACT32) {
+                                chain([&](int e, float *w) {
+                                    *reinterpret_cast<float4 *>(w) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + k) * DSUB + e));
+                                    *reinterpret_cast<float4 *>(w + 4) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + k) * DSUB + e + 4));
+                                });
+                            } else if (!fail) {
+                                chain([&](int e, float *w) { unpack8(*reinterpret_cast<const uint4 *>(tab + L::template at<kMaxWords>(k, e)), w); });
+                            } else {
+                                chain([&](int e, float *w) { unpack8(load_in_place(a.tables + (first + k) * DSUB + e), w); });
                             }
-                            const float dist = distance_expr(exact, nrm[k], dot);
+                            float cc = nrm[k];
+                            if (fail) cc = a.sqnorm != nullptr ? __ldg(a.sqnorm + first + k) : word_norm_alone<DSUB>(a.tables + (first + k) * DSUB);
+                            const float dist = distance_expr(exact, cc, dot);
                             if (dist < best) best = dist, arg = k;  // a lane's two words ascend
                         }
                         __syncwarp();
@@ -623,19 +664,26 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
 
             // ---- update ----
             if (s + 1 < S) {
+                auto subtract = [&](auto fetch) {
 #pragma unroll
-                for (int m = 0; m < kOwn; ++m) {
-                    const int e = 8 * (4 * m + q);
-                    float c[8];
-                    if constexpr (EXACT32) {
+                    for (int m = 0; m < kOwn; ++m) {
+                        const int e = 8 * (4 * m + q);
+                        float c[8];
+                        fetch(e, c);
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2) sub2(r[8 * m + j], r[8 * m + j + 1], c[j], c[j + 1]);
+                        *reinterpret_cast<uint4 *>(A + L::template at<kRows>(row, e)) = pack8(r + 8 * m);
+                    }
+                };
+                if constexpr (EXACT32) {
+                    subtract([&](int e, float *c) {
                         *reinterpret_cast<float4 *>(c) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + pick) * DSUB + e));
                         *reinterpret_cast<float4 *>(c + 4) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + pick) * DSUB + e + 4));
-                    } else {
-                        unpack8(*reinterpret_cast<const uint4 *>(tab + L::template at<kMaxWords>(pick, e)), c);
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; j += 2) sub2(r[8 * m + j], r[8 * m + j + 1], c[j], c[j + 1]);
-                    *reinterpret_cast<uint4 *>(A + L::template at<kRows>(row, e)) = pack8(r + 8 * m);
+                    });
+                } else if (!fail) {
+                    subtract([&](int e, float *c) { unpack8(*reinterpret_cast<const uint4 *>(tab + L::template at<kMaxWords>(pick, e)), c); });
+                } else {
+                    subtract([&](int e, float *c) { unpack8(load_in_place(a.tables + (first + pick) * DSUB + e), c); });
                 }
             }
             if (live && q == 0) code_at[(int64_t)s * a.G] = (uint8_t)pick;
@@ -701,12 +749,20 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         }
         sync_quad();  // the rows' places in shared memory take the next tile
     }
-    if (fail) {
-        // give what is still in flight one more bounded wait before the block's memory goes
-        if ((tid & (kGroupThreads - 1)) == 0) atomicAdd(&g_timeouts, 1u);
-        bounded_wait(my_mma, mma_phase ^ 1u);
-        bounded_wait(full_bar, 0u);
-        if (S > 1) bounded_wait(full_bar + 8, 0u);
+    if (__syncthreads_or(fail)) {
+        // what is still in flight ends before the block's memory goes: each group's last product, each buffer's last copy (a
+        // warp that gave up since owes the barrier an arrival)
+        if ((tid & (kGroupThreads - 1)) == 0 && in_flight[grp] < 2u) bounded_wait(my_mma, in_flight[grp], kSpins);
+        if (tid == 0) {
+            atomicAdd(&g_timeouts, 1u);
+            for (uint32_t buf = 0; buf < 2 && buf < uses; ++buf) {
+                const unsigned int copies = left[buf * 4] / (unsigned int)groups;  // after the first one
+                for (int quarter = 1; quarter < 4; ++quarter)
+                    if (left[buf * 4 + quarter] / (unsigned int)groups < copies)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full_bar + 8 * buf) : "memory");
+                bounded_wait(full_bar + 8 * buf, copies & 1u, kSpins);
+            }
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -740,7 +796,7 @@ static int launch(const EncodeArgs &e, const __half *scored) {
     const int64_t most = units < 148 ? 148 / units : 1;
     if (blocks > most) blocks = most;
     const Args a{e.x, e.sxb, e.sxh, e.sxt, scored, EXACT32 ? (const float *)e.tables : nullptr, e.recon_tables, e.sqnorm, e.codes, e.recon,
-                 e.recon_dtype, e.B, e.H, e.T, e.G, e.S, e.K, vec_ok, use_map, e.t0, e.T_cap};
+                 e.recon_dtype, e.B, e.H, e.T, e.G, e.S, e.K, vec_ok, use_map, e.wait_spins < 0 ? kSpins : e.wait_spins, e.t0, e.T_cap};
     auto kernel = groups == 1 ? encode_wide_kernel<DSUB, XT, EXACT32, 1> : encode_wide_kernel<DSUB, XT, EXACT32, kMaxGroups>;
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
@@ -764,9 +820,16 @@ int encode_wide_launch(const EncodeArgs &e) {
     return d == 128 ? wide::launch<128, float, false>(e, tables) : wide::launch<64, float, false>(e, tables);
 }
 
+int narrow_timeouts(unsigned int *out);
+int few_timeouts(unsigned int *out);
+
+// of all encode kernels that wait for products or copies
 int tensor_memory_timeouts(unsigned int *out) {
-    const int st = (int)cudaMemcpyFromSymbol(out, wide::g_timeouts, sizeof(unsigned int));
-    if (st == 0) *out += wide::g_map_failures.load();
+    unsigned int narrow = 0, few = 0;
+    int st = (int)cudaMemcpyFromSymbol(out, wide::g_timeouts, sizeof(unsigned int));
+    if (st == 0) st = narrow_timeouts(&narrow);
+    if (st == 0) st = few_timeouts(&few);
+    if (st == 0) *out += wide::g_map_failures.load() + narrow + few;
     return st;
 }
 

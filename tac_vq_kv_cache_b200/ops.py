@@ -79,7 +79,7 @@ def table_sqnorm(tables_f16: torch.Tensor) -> torch.Tensor:
 
 
 def encode_tensor_memory_timeouts(device=None) -> int:
-    """How often a wide-group encode block gave up waiting for its tensor-core products (expected 0)."""
+    """In how many blocks an encode kernel gave up waiting for tensor-core products or table copies (expected 0)."""
     import ctypes
 
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)

@@ -422,6 +422,7 @@ def test_narrow_groups_with_many_rows_are_bit_exact(device, batch, heads, tokens
     assert bool((codes[:, :, :2] == 0xEE).all()) and bool((codes[:, :, 2 + tokens :] == 0xEE).all())
     shifted = torch.empty(states.numel() + 1, dtype=dtype, device=device)[1:].view(states.shape).copy_(states)  # rows not 16-byte aligned
     assert torch.equal(ops.encode(shifted, tables.to(device), want_recon=False)[0].cpu(), want)
+    assert ops.encode_tensor_memory_timeouts(device) == 0
 
 
 @pytest.mark.parametrize(

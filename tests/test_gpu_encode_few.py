@@ -44,6 +44,7 @@ def test_few_rows_of_wide_groups_are_bit_exact(device, batch, tokens, sub, group
     norms = ops.table_sqnorm(tables.to(device))
     again, _ = ops.encode(states.to(device), tables.to(device), table_sqnorm=norms, want_recon=False)
     assert torch.equal(again.cpu(), want)
+    assert ops.encode_tensor_memory_timeouts(device) == 0
 
 
 @pytest.mark.parametrize("rope", [None, 1e6])
