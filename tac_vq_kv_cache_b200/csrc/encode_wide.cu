@@ -531,7 +531,8 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                 if (n >= 2) wb = wa, wa = i * 64 + ((info >> 6) & 63);
             }
             int pick = wa;
-            bool undecided = n_words != 1;
+            // (rows past the end are all alike: one that is undecided would be 32 in a row)
+            bool undecided = live && n_words != 1;
             if (__any_sync(0xffffffffu, undecided)) {  // the same in the four warps
                 // Two words (nearly always all there are): their dot products once more in fp32, each thread over its part of the
                 // row.  E is then 2^-17 u for the chain that it stands for, 2^-18 u of its own and 2^-23 (|r|^2 + cc), which
