@@ -12,7 +12,7 @@
 //      there are more, the row goes to shared memory and the library's exact chains decide,
 //   4. subtracts the chosen word and writes the new fp16 row.
 // The two groups share the word tables: resident for the block's life up to two stages, otherwise a ring of two
-// that the group which leaves a stage last refills (words by TMA, norms by four of its warps).  While one group waits for its product the other one reads
+// that the group which leaves a stage last refills (words by TMA, norms by its warps).  While one group waits for its product the other one reads
 // scores, which keeps the tensor core and the schedulers busy in turn.
 //
 // Margin (encode_tc.cu has the argument that twice the error bound E of a score keeps the exact argmin and its ties on
@@ -130,22 +130,29 @@ __device__ __forceinline__ void unpack8(const uint4 raw, float *v) {
     }
 }
 
-// |word|^2 in the library's order, for callers that bring no norms: eight neighbouring lanes per word, lane j owns running
-// sum j of each of the four sets, and all eight return the total
+// |word|^2 in the library's order, for callers that bring no norms: lane u of four neighbouring ones owns the eight running
+// sums of set u, so that a word arrives in whole sectors, and all four return the total
 template <int DSUB>
-__device__ __forceinline__ float word_norm_by_eight(const __half *__restrict__ word, int lane) {
-    float set[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 1
-    for (int i = 0; i < DSUB; i += 32)
+__device__ __forceinline__ float word_norm_by_four(const __half *__restrict__ word, int lane) {
+    uint4 raw[DSUB / 32];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float v = __half2float(word[i + 8 * u + (lane & 7)]);
-            set[u] = __fadd_rn(set[u], __fmul_rn(v, v));
-        }
-    const float mine = __fadd_rn(__fadd_rn(__fadd_rn(set[0], set[1]), set[2]), set[3]);
-    float total = __shfl_sync(0xffffffffu, mine, lane & 24);
+    for (int i = 0; i < DSUB / 32; ++i) raw[i] = __ldg(reinterpret_cast<const uint4 *>(word) + 4 * i + (lane & 3));
+    float set[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int j = 1; j < 8; ++j) total = __fadd_rn(total, __shfl_sync(0xffffffffu, mine, (lane & 24) + j));
+    for (int i = 0; i < DSUB / 32; ++i) {
+        float v[8];
+        unpack8(raw[i], v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) set[j] = __fadd_rn(set[j], __fmul_rn(v[j], v[j]));
+    }
+    float total = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        float sum = __shfl_sync(0xffffffffu, set[j], lane & 28);
+#pragma unroll
+        for (int u = 1; u < 4; ++u) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, set[j], (lane & 28) + u));
+        total = j == 0 ? sum : __fadd_rn(total, sum);
+    }
     return total;
 }
 
@@ -227,10 +234,10 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     float *nrms = reinterpret_cast<float *>(smem + L::kNrm);
     const uint32_t misc = smem_u32(smem + L::kMisc);
     const uint32_t full_bar = misc, mma_bar = misc + 16;  // [2] each
-    unsigned int *left = reinterpret_cast<unsigned int *>(smem + L::kMisc + 64);  // [2][4]: groups that left a stage of this buffer, all uses together, per quarter
+    unsigned int *left = reinterpret_cast<unsigned int *>(smem + L::kMisc + 64);  // [2][16]: groups that left a stage of this buffer, all uses together, per share
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::kMisc + 48);
     uint32_t *in_flight = reinterpret_cast<uint32_t *>(smem + L::kMisc + 52);     // [2] phase of the last product asked for; 2: none
-    float *cc_tops = reinterpret_cast<float *>(smem + L::kMisc + 128);            // [2][4]: largest norm of a quarter
+    float *cc_tops = reinterpret_cast<float *>(smem + L::kMisc + 192);            // [2][16]: largest norm of a share
 
     const int hg = blockIdx.y, h = hg / a.G, g = hg % a.G;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -240,6 +247,10 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     const uint32_t tiles = (rows + kRows - 1) / kRows;
     const float inf = __int_as_float(0x7f800000);
     const bool resident = S <= 2;
+    // Warps that fill a stage's buffer, a share of the words each: four where the norms are there to be copied, all sixteen of a
+    // group where they are computed.  (Four warps, each 4 words at a time, took longer than the stage: 128 wide, 16 stages, 8 heads of 256 rows
+    // 294 us, 100 us so.)
+    const int shares = a.sqnorm != nullptr ? 4 : 16;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)(groups * kMaxWords)) : "memory");
@@ -247,11 +258,11 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     }
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(full_bar + 8 * i) : "memory");  // a warp per quarter of the words
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full_bar + 8 * i), "r"(shares) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mma_bar + 8 * i) : "memory");
             in_flight[i] = 2u;
         }
-        for (int i = 0; i < 8; ++i) left[i] = 0u;
+        for (int i = 0; i < 32; ++i) left[i] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < kRows * 2; i += blockDim.x) {  // 16-byte piece c of row r sits at piece c ^ ((r >> 2) & 1)
@@ -280,26 +291,12 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             *reinterpret_cast<uint4 *>(tab + L::template at<kMaxWords>(k, p * 8)) = v;
         }
     };
-    auto copy_norms = [&](int buf, int64_t first, int k_begin, int k_end) {
-        if (a.sqnorm != nullptr) {
-#pragma unroll 1
-            for (int k = k_begin + lane; k < k_end; k += 32) nrms[buf * kMaxWords + k] = k < K ? __ldg(a.sqnorm + first + k) : inf;
-        } else {
-#pragma unroll 1
-            for (int k0 = k_begin; k0 < k_end; k0 += 4) {
-                const int k = k0 + (lane >> 3);
-                const float v = word_norm_by_eight<DSUB>(a.tables + (first + min(k, K - 1)) * DSUB, lane);
-                if ((lane & 7) == 0) nrms[buf * kMaxWords + k] = k < K ? v : inf;
-            }
-        }
-        __syncwarp();
-    };
-    // four warps, a quarter each: the norms and seeds of use u; the first one also fetches the words by TMA (or plain copies
-    // without a tensor map)
-    auto load_table = [&](uint32_t u, int quarter) {
+    // the norms and seeds of a share of use u's words, by a warp; the first share's also fetches all the words by TMA (or plain
+    // copies without a tensor map)
+    auto load_table = [&](uint32_t u, int share) {
         const int s = (int)(u % (uint32_t)S), buf = (int)(u & 1u);
         const int64_t first = head_words + s * stage_words;
-        if (quarter != 0) {
+        if (share != 0) {
         } else if (a.use_map) {
             if (lane == 0) {
                 asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(full_bar + 8 * buf), "r"((uint32_t)L::kTabBytes) : "memory");
@@ -312,12 +309,25 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         } else {
             copy_table(buf, first);
         }
-        copy_norms(buf, first, quarter * 64, quarter * 64 + 64);
+        const int k_begin = share * (kMaxWords / shares), k_end = k_begin + kMaxWords / shares;
+        float *nrm = nrms + buf * kMaxWords;
+        if (a.sqnorm != nullptr) {
+#pragma unroll 1
+            for (int k = k_begin + lane; k < k_end; k += 32) nrm[k] = k < K ? __ldg(a.sqnorm + first + k) : inf;
+        } else {
+#pragma unroll 1
+            for (int k0 = k_begin; k0 < k_end; k0 += 8) {
+                const int k = k0 + (lane >> 2);
+                const float v = word_norm_by_four<DSUB>(a.tables + (first + min(k, K - 1)) * DSUB, lane);
+                if ((lane & 3) == 0) nrm[k] = k < K ? v : inf;
+            }
+        }
+        __syncwarp();
         float top = 0.0f;
         unsigned char *seed = smem + L::kSeed + buf * kSeedBytes;
 #pragma unroll 1
-        for (int k = quarter * 64 + lane; k < quarter * 64 + 64; k += 32) {
-            const float v = nrms[buf * kMaxWords + k];
+        for (int k = k_begin + lane; k < k_end; k += 32) {
+            const float v = nrm[k];
             if (k < K && v == v) top = fmaxf(top, v);
             const float t = -0.5f * v;  // padding words: -inf, never within the margin
             const __half p1 = __float2half_rn(t);
@@ -332,12 +342,14 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         }
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-        if (lane == 0) cc_tops[buf * 4 + quarter] = top;
+        if (lane == 0) cc_tops[buf * 16 + share] = top;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full_bar + 8 * buf) : "memory");
     };
-    if (warp < 8 && (uint32_t)(warp >> 2) < uses) load_table((uint32_t)(warp >> 2), warp & 3);
+#pragma unroll 1
+    for (int i = warp; i < 2 * shares; i += GROUPS * 16)
+        if ((uint32_t)(i / shares) < uses) load_table((uint32_t)(i / shares), i % shares);
 
     const int grp = warp >> 4, part = warp & 3, q = (warp >> 2) & 3;
     const int row = part * 32 + lane;                     // of the group's tile
@@ -456,17 +468,21 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                 }
                 __syncwarp();
             }
-            // use u - 1 is left: the last group to leave it refills its buffer, a quarter per warp of q = 0
-            if (q == 0 && !resident && u >= 1 && u + 1 < uses && !fail) {
+            // use u - 1 is left: the last group to leave it refills its buffer, a share per warp (where there are four, those of q = 0)
+            if (q * 4 < shares && !resident && u >= 1 && u + 1 < uses && !fail) {
                 unsigned int n = 0u;
                 __threadfence_block();
-                if (lane == 0) n = atomicAdd(left + ((u - 1) & 1u) * 4 + part, 1u) + 1u;
+                if (lane == 0) n = atomicAdd(left + ((u - 1) & 1u) * 16 + q * 4 + part, 1u) + 1u;
                 __threadfence_block();
                 n = __shfl_sync(0xffffffffu, n, 0);
-                if (n % (unsigned int)groups == 0u) load_table(u + 1, part);
+                if (n % (unsigned int)groups == 0u) load_table(u + 1, q * 4 + part);
             }
             const float xx = (xxs[0] + xxs[kRows]) + (xxs[2 * kRows] + xxs[3 * kRows]);
-            const float cc_top = fmaxf(fmaxf(cc_tops[buf * 4], cc_tops[buf * 4 + 1]), fmaxf(cc_tops[buf * 4 + 2], cc_tops[buf * 4 + 3]));
+            const float *share_tops = cc_tops + buf * 16;
+            float cc_top = fmaxf(fmaxf(share_tops[0], share_tops[1]), fmaxf(share_tops[2], share_tops[3]));
+            if (shares != 4)
+#pragma unroll 1
+                for (int i = 4; i < shares; ++i) cc_top = fmaxf(cc_top, share_tops[i]);
             const float u_top = rough_sqrt(xx * cc_top);
             const float margin = (sizeof(XT) == 2 && s == 0 ? 1.220703125e-04f : EXACT32 ? 2.01416015625e-03f : 1.03759765625e-03f) * u_top +
                                  9.5367431640625e-07f * xx + 3.0517578125e-05f * cc_top + 3.814697265625e-06f * rough_sqrt(cc_top) +
@@ -757,9 +773,9 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         if (tid == 0) {
             atomicAdd(&g_timeouts, 1u);
             for (uint32_t buf = 0; buf < 2 && buf < uses; ++buf) {
-                const unsigned int copies = left[buf * 4] / (unsigned int)groups;  // after the first one
-                for (int quarter = 1; quarter < 4; ++quarter)
-                    if (left[buf * 4 + quarter] / (unsigned int)groups < copies)
+                const unsigned int copies = left[buf * 16] / (unsigned int)groups;  // after the first one
+                for (int share = 1; share < shares; ++share)
+                    if (left[buf * 16 + share] / (unsigned int)groups < copies)
                         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full_bar + 8 * buf) : "memory");
                 bounded_wait(full_bar + 8 * buf, copies & 1u, kSpins);
             }
