@@ -707,7 +707,8 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         }
         if (a.recon != nullptr) {
             // a warp per row: the sum of the plain words in stage order, whole sectors in and out
-            constexpr int kEach = DSUB / 32, kTogether = 4;
+            // (all eight rows of a warp at once where a block has one tile and nothing hides the words' way from L2)
+            constexpr int kEach = DSUB / 32, kTogether = GROUPS == 1 ? 8 : 4;
             const int64_t o = (((int64_t)rb * a.H + h) * a.T + rt) * ((int64_t)a.G * DSUB) + (int64_t)g * DSUB;
             const long long mine = live ? o : -1ll;
             const unsigned long long codes_at = (unsigned long long)code_at;
