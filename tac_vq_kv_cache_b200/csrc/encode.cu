@@ -16,7 +16,7 @@
 #include "encode_rows.cuh"
 
 #ifndef TACVQ_ENCODE_TC
-#define TACVQ_ENCODE_TC 1  // 8-wide groups go to the tensor-core filtered kernel (encode_tc.cu)
+#define TACVQ_ENCODE_TC 1  // 0: the kernels of this file alone, without the tensor-core filtered ones
 #endif
 
 namespace tacvq {
@@ -468,15 +468,26 @@ static int launch_large(const EncodeArgs &a) {
 
 constexpr int kFewRows = 32;  // at or below this many rows a warp per (row, head, group) wins
 
-// From this many rows on, 8- and 4-wide groups go to the tcgen05 kernel (up to its 12 stages).  Measured with 8 heads, fp16 rows
-// wanted, against the mma.sync kernel: 512 rows of 16 x 8 at two stages 24.7 us against 24.9 and of 32 x 4 24.6 against 22.8;
-// 700 rows 24.7 against 25.1 and 24.9 against 29.0; 4096 rows 66 against 88 and 75 against 94.
-constexpr int kNarrowRows = 640;
+// Whether 8- and 4-wide groups go to the tcgen05 kernel, whose blocks of four tiles each stay a while, or to the mma.sync kernel of
+// many small blocks.  Measured with fp16 rows wanted, us of the mma.sync / tcgen05 kernel; T = tiles of 128 rows, all heads and groups:
+//   16 x 8, two stages  640 rows: T 80 7.5/17.4, 320 14.2/18.1, 640 22.0/19.7, 1280 37.3/32.2, 2560 58.4/58.9
+//                       T = 512: 17.1/14.0 (1024, 2048 or 4096 rows); T = 256: 9.9/13.5
+//   16 x 8, one stage   T = 512 11.8/10.6; 640 rows: T 640 15.0/14.7, 1280 25.2/23.2, 2560 36.9/41.3; 1024 rows: T 4096 52.9/49.3
+//   32 x 4, one stage   640 rows: T 640 15.0/14.0, 1280 25.4/22.4, 2560 37.0/38.8, 5120 63.7/67.1; 1024 rows: T 8192 92.7/85.2
+// From T of about 2048 on a block goes through whole (head, group) pairs, and five or six tiles of a pair leave its four groups of
+// threads half idle in the second round, which one stage does not make up for.
+static bool narrow_pays(int64_t rows, int64_t pairs, int stages) {
+    const int64_t tiles = (rows + 127) / 128 * pairs;
+    return rows >= 640 && tiles >= 512 && (tiles < 2048 || rows >= 1024 || stages >= 2);
+}
 
-// 32-, 64- and 128-wide groups: a block per (head, group) and four rows while that is at most two blocks per SM.
-// Measured, 8 heads, against a launch of 128-row tiles: 128 rows of 16 x 128 (256 blocks) 76 us against 102 us, 2 x 128
-// 15.5 against 18.1; 192 rows (384 blocks) 108 against 103 and 19.0 against 17.8.
-static bool few_wide_rows(int64_t rows, int64_t units) { return (rows + 3) / 4 * units <= 2 * 148; }
+// 32-, 64- and 128-wide groups: a block per (head, group) and four rows while that is at most two blocks per SM, or one and a half
+// for one stage of 32-wide words.  Measured against a launch of 128-row tiles: 256 blocks of 16 x 128 77 us against 107, of 2 x 128 16.5
+// against 19.8, of 2 x 64 12.7 against 14.0, of two stages of 32 11.2 against 12.8, of one 8.4 against 7.6 (192 blocks 7.4 against
+// 7.7); 384 blocks of 16 x 128 108 against 103, of 2 x 128 19.0 against 17.8.
+static bool few_wide_rows(int64_t rows, int64_t units, int d, int stages) {
+    return (rows + 3) / 4 * units <= (d == 32 && stages == 1 ? 222 : 2 * 148);
+}
 
 template <typename XT, typename TT>
 static int dispatch_d(const EncodeArgs &a) {
@@ -490,14 +501,14 @@ static int dispatch_d(const EncodeArgs &a) {
             }
         }
         if (TACVQ_ENCODE_TC && (a.D / a.G == 8 || a.D / a.G == 4)) {
-            if ((int64_t)a.B * a.T >= kNarrowRows) {
+            if (narrow_pays((int64_t)a.B * a.T, (int64_t)a.H * a.G, a.S)) {
                 const int st = encode_narrow_launch(a);
                 if (st != TACVQ_ERR_UNSUPPORTED) return st;
             }
             const int st = encode_tc8_launch(a);
             if (st != TACVQ_ERR_UNSUPPORTED) return st;
         }
-        if (a.D / a.G >= 32 && few_wide_rows((int64_t)a.B * a.T, (int64_t)a.H * a.G)) {
+        if (TACVQ_ENCODE_TC && a.D / a.G >= 32 && few_wide_rows((int64_t)a.B * a.T, (int64_t)a.H * a.G, a.D / a.G, a.S)) {
             const int st = encode_few_wide_launch(a);
             if (st != TACVQ_ERR_UNSUPPORTED) return st;
         }

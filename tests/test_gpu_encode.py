@@ -406,6 +406,13 @@ def test_decode_of_long_rows_matches_the_oracle(device, groups, stages, sub, dty
         (2, 1, 4161, 8, 4, 3, 256, torch.float16),   # two spans of 8192 rows, tables changed inside a block
         (1, 1, 650, 4, 8, 12, 256, torch.float32),   # as many stages as fit
         (1, 1, 650, 8, 4, 13, 256, torch.float16),   # and one more
+        # enough tiles of all heads and groups for the kernel of many rows (those above are for the one of fewer)
+        (1, 13, 640, 8, 8, 2, 256, torch.float16),
+        (1, 7, 641, 8, 16, 1, 256, torch.float32),
+        (3, 6, 333, 4, 32, 1, 100, torch.float16),
+        (2, 4, 4161, 8, 4, 3, 256, torch.float16),
+        (1, 11, 650, 4, 8, 12, 256, torch.float32),
+        (1, 16, 1024, 4, 32, 1, 256, torch.float16),  # whole pairs in a block
     ],
 )
 def test_narrow_groups_with_many_rows_are_bit_exact(device, batch, heads, tokens, sub, groups, stages, words, dtype):
