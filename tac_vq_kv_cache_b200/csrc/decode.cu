@@ -316,15 +316,18 @@ decode_rows_kernel(const uint8_t *__restrict__ codes, const __half *__restrict__
     extern __shared__ __align__(128) unsigned char staged[];
     const int h = blockIdx.y, tid = threadIdx.x;
     const int d = D / G, chunks = D / 8, slots = S * G;
-    {   // a warp copies, per trip, 4 neighbouring words of 8 neighbouring pieces: whole sectors in, few conflicts out
+    {   // A warp copies, per trip, 4 neighbouring words of 8 neighbouring pieces: whole sectors in, few conflicts out.  Its place advances
+        // by additions (divided out at every trip, the copy took longer than the rows of a short call).
         constexpr int kUnit = NARROW ? 8 : 16;                 // bytes
-        const int units = NARROW ? G : chunks, per_word = NARROW ? 1 : d / 8;
+        const int units = NARROW ? G : chunks, per_word = NARROW ? 1 : d / 8, blocks = units / 8, lane = tid & 31;
         const __half *src = tables + (size_t)h * S * G * K * d;
-        const int total = STAGES * K * units;
-        for (int i = tid; i < total; i += kRowsThreads) {
-            const int rest = i >> 5, unit = (rest % (units / 8)) * 8 + (i & 7), k4 = rest / (units / 8);
-            const int k = (k4 % (K / 4)) * 4 + ((i >> 3) & 3), s = k4 / (K / 4);
-            const __half *word = src + ((size_t)(s * G + unit / per_word) * K + k) * d + (unit % per_word) * 8;
+        // (pieces divide the block's threads, so that `blocks` divides its 32 warps and a warp keeps its pieces)
+        const int unit = (tid >> 5) % blocks * 8 + (lane & 7), from = (unit / per_word) * K * d + (unit % per_word) * 8;  // of word 0, stage 0
+        const int step = kRowsThreads / 32 / blocks;
+#pragma unroll(NARROW ? 2 : 4)
+        for (int k4 = (tid >> 5) / blocks; k4 < STAGES * (K / 4); k4 += step) {
+            const int s = STAGES == 2 && k4 >= K / 4 ? 1 : 0, k = (k4 - s * (K / 4)) * 4 + (lane >> 3);
+            const __half *word = src + (size_t)s * G * K * d + from + k * d;
             unsigned char *to = staged + ((size_t)(s * K + k) * units + unit) * kUnit;
             if constexpr (NARROW) *reinterpret_cast<uint2 *>(to) = __ldg(reinterpret_cast<const uint2 *>(word));
             else *reinterpret_cast<uint4 *>(to) = __ldg(reinterpret_cast<const uint4 *>(word));
