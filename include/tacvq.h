@@ -188,6 +188,8 @@ TACVQ_API size_t tacvq_attn_workspace_bytes(int B, int Hq, int Hkv, int D, int G
  *                      against: never above the maximum score and at most 8 ln 2 below it; m + ln l
  *                      (the log-sum-exp) and acc / l do not depend on it
  *   Hq % Hkv == 0, Hq/Hkv <= 8, K == 256, D % 32 == 0, D <= 256.
+ * On the two-stage layout of 16 x 8 the query (and the new rows of a decode step) are read before the attention launch
+ * that precedes on the stream has ended: they must not be its result buffers themselves.
  */
 TACVQ_API int tacvq_attn_decode(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
                       const uint16_t *vtab_f16, const int32_t *seq_start, const int32_t *seq_end, void *workspace,

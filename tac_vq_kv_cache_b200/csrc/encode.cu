@@ -1,13 +1,16 @@
 // Encode kernels: greedy residual nearest-codeword search with all stages fused.
 //
-// Two kernels cover the geometry family (G groups, S stages, d = D/G, K <= 256 codewords):
+// This file has the dispatch over all encode kernels and those without tensor cores:
 //   encode_small  d <= 16   one thread owns TPT rows of one (head, group); the stage tables of that
 //                           (head, group) live in shared memory as fp32 and are read as warp
 //                           broadcasts; residual, running minimum and reconstruction stay in registers.
+//   encode_rows   d <= 16   a handful of rows: a warp per (row, head, group).
 //   encode_large  d >= 32   a register-tiled fp32 GEMM per stage (4 rows x 16 codewords per thread),
 //                           residual tile and stage table in shared memory, the contraction index
 //                           outermost so every dot product is still one FMA chain from element 0.
-// Both are FFMA-bound by design: an exact fp32 distance is what decides a code.
+// These are FFMA-bound by design: an exact fp32 distance is what decides a code.  fp16 tables of 4-, 8-, 32-, 64- and
+// 128-wide groups (and whitened ones of 64 and 128) go to kernels that filter with tensor cores first: encode_narrow.cu,
+// encode_tc.cu, encode_tc_large.cu, encode_wide.cu, encode_few.cu.
 //
 // Reference statements: src/jointkv/closed_loop_vq.py:52-76 (search), :343-395 (stage recursion),
 // src/jointkv/cq_tac.py:86-105 (grouped one-stage form).

@@ -14,8 +14,8 @@
 // Blocks split the tiles of all (head, group) pairs evenly, span by span of 8192 rows, and bring a pair's tables in when they
 // enter it, so the chip stays full whatever the number of pairs; a table costs about one tile's time.
 //
-// Bound by latency between the phases of a stage at 16 warps an SM (issue 52 % busy).  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
-// stages, rows wanted: 460 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.
+// Bound by latency between the phases of a stage at 16 warps an SM (issue 48 % busy).  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
+// stages, rows wanted: 435 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.
 //
 // Reference statements: src/jointkv/closed_loop_vq.py:52-76 (search), :343-395 (stage recursion),
 // src/jointkv/cq_tac.py:86-105.
@@ -318,9 +318,9 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
 #pragma unroll
                     for (int p = 1; p < 15; p += 2) m0 = max3(m0, top4[p], top4[p + 1]), m1 = max3(m1, top4[16 + p], top4[17 + p]);
                     top = fmaxf(top, max3(fmaxf(m0, m1), top4[15], top4[31]));
-                    // Bits by saturating and doubling multiply-adds, 8 fours a chain.  A score less than 2^-60 above the limit may count in
-                    // part and disturb lower bits: it need not be listed (the margin exceeds the bound by more), and a four too many does
-                    // no harm.
+                    // Bits by saturating and doubling multiply-adds, 8 fours a chain.  No score lies less than 2^-60 above the limit, where it
+                    // would count in part and disturb the bits below: products of fp16 values and their sums are multiples of 2^-48, and so
+                    // is the limit, as the margin is at least 2^-23.
                     constexpr float kSteep = 1.152921504606846976e18f;  // 2^60
                     const float offset = (margin - top) * kSteep;
                     float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};

@@ -1,7 +1,7 @@
-"""GPU parity of the few-row encode of wide groups (decode steps): one cluster per (side, head, group).
+"""GPU parity of the few-row encode of wide groups (decode steps): a block per (side, head, group) and one, two or four rows.
 
-Row counts on both sides of every split (rows per warp, rows per cluster), table rings that are and are not
-recycled (more than 16 stages), codebooks that leave some or all of a block's 32 words empty, and the decode step that
+Row counts on both sides of every split (rows per block, the last block's missing rows), table rings that are and are not
+recycled (more than three stages), small codebooks, one so small that the kernel does not take it, and the decode step that
 encodes both sides at once.  Codes and rows are bit-exact with the C oracle.
 """
 
@@ -25,7 +25,8 @@ pytestmark = pytest.mark.gpu
         (1, 16, 128, 1, 18, 256, torch.float16),
         (17, 1, 64, 2, 2, 33, torch.float16),
         (4, 8, 32, 4, 2, 256, torch.float32),
-        (2, 5, 64, 2, 1, 7, torch.float16),
+        (2, 5, 64, 2, 1, 7, torch.float16),   # 28 words in all: not this kernel's
+        (2, 5, 64, 2, 16, 7, torch.float16),
         (1, 3, 32, 4, 33, 96, torch.float16),
     ],
 )
