@@ -48,6 +48,10 @@ int attn_rotary_staged_dispatch(const __half *q, const uint8_t *kcodes, const ui
                                 const __half *vtab, const __half *rope, const int32_t *seq_start, const int32_t *seq_end,
                                 float *part, int B, int Hq, int Hkv, int G, int S, int64_t T_cap, int splits,
                                 cudaStream_t stream);
+bool attn_rotary_mma_supported(int Hq, int Hkv, int D, int G, int S, int K);
+int attn_rotary_mma_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
+                             const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
+                             int Hkv, int64_t T_cap, int64_t visible, int sms, int *splits, cudaStream_t stream);
 int rope_table_dispatch(__half *table, int64_t tokens, int D, double theta, int64_t first, cudaStream_t stream);
 int attn_rotary_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab,
                          const __half *vtab, const __half *rope, const int32_t *seq_start, const int32_t *seq_end,
@@ -348,11 +352,11 @@ int tacvq_rope_table(uint16_t *table_f16, int64_t T, int D, double theta, int64_
     return rope_table_dispatch((__half *)table_f16, T, D, theta, first_position, (cudaStream_t)stream);
 }
 
-int tacvq_attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes,
-                             const uint16_t *ktab_f16, const uint16_t *vtab_f16, const uint16_t *rope_table,
-                             const int32_t *seq_start, const int32_t *seq_end, void *workspace, size_t workspace_bytes,
-                             uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv, int D, int G, int S, int K,
-                             int64_t T_cap, tacvq_stream_t stream) {
+// `visible`: positions between the first and the last that any row sees, as far as the host knows (T_cap otherwise).
+static int attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
+                              const uint16_t *vtab_f16, const uint16_t *rope_table, const int32_t *seq_start, const int32_t *seq_end,
+                              void *workspace, size_t workspace_bytes, uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv,
+                              int D, int G, int S, int K, int64_t T_cap, int64_t visible, tacvq_stream_t stream) {
     if (!q_f16 || !kcodes || !vcodes || !ktab_f16 || !vtab_f16 || !rope_table) return TACVQ_ERR_NULL;
     if (!out_f16 && !state_out) return TACVQ_ERR_NULL;
     const int g = check_attn_geometry(B, Hq, Hkv, D, G, S, K);
@@ -361,24 +365,37 @@ int tacvq_attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, const
     if (T_cap < 0 || T_cap > 0x7fffffff) return TACVQ_ERR_RANGE;
     if (!workspace || ((uintptr_t)workspace & 255) != 0 || workspace_bytes < tacvq_attn_workspace_bytes(B, Hq, Hkv, D, G, S))
         return TACVQ_ERR_WORKSPACE;
-    if (((uintptr_t)rope_table & 3) != 0) return TACVQ_ERR_ALIGN;  // the staged kernel wants 16 bytes and is skipped otherwise
+    if (((uintptr_t)rope_table & 3) != 0) return TACVQ_ERR_ALIGN;  // the kernels for head_dim 128 want 16 bytes and are skipped otherwise
     cudaStream_t s = (cudaStream_t)stream;
-    if (attn_rotary_staged_supported(Hq, Hkv, D, G, S, K) && (((uintptr_t)ktab_f16 | (uintptr_t)vtab_f16 | (uintptr_t)rope_table) & 15) == 0) {
-        const int staged = attn_rotary_staged_splits(B, Hkv, T_cap, sm_count());
-        if (staged > 0) {
-        int st = attn_rotary_staged_dispatch((const __half *)q_f16, kcodes, vcodes, (const __half *)ktab_f16,
-                                             (const __half *)vtab_f16, (const __half *)rope_table, seq_start, seq_end,
-                                             (float *)workspace, B, Hq, Hkv, G, S, T_cap, staged, s);
-        if (st != TACVQ_OK) return st;
-        return attn_combine_dispatch((const float *)workspace, staged, (__half *)out_f16, state_out, (int64_t)B * Hq, D, s);
+    const __half *q = (const __half *)q_f16, *ktab = (const __half *)ktab_f16, *vtab = (const __half *)vtab_f16, *rope = (const __half *)rope_table;
+    float *part = (float *)workspace;
+    int splits = 0, st = TACVQ_OK;
+    if ((((uintptr_t)ktab_f16 | (uintptr_t)vtab_f16 | (uintptr_t)rope_table) & 15) == 0) {
+        if (attn_rotary_mma_supported(Hq, Hkv, D, G, S, K) && (((uintptr_t)kcodes | (uintptr_t)vcodes | (uintptr_t)q_f16) & 15) == 0) {
+            st = attn_rotary_mma_dispatch(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, visible,
+                                          sm_count(), &splits, s);
+        } else if (attn_rotary_staged_supported(Hq, Hkv, D, G, S, K)) {
+            splits = attn_rotary_staged_splits(B, Hkv, T_cap, sm_count());
+            if (splits > 0)
+                st = attn_rotary_staged_dispatch(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, G, S, T_cap,
+                                                 splits, s);
         }
     }
-    const int splits = attn_rotary_splits(B, Hkv, T_cap, sm_count());
-    int st = attn_rotary_dispatch((const __half *)q_f16, kcodes, vcodes, (const __half *)ktab_f16, (const __half *)vtab_f16,
-                                  (const __half *)rope_table, seq_start, seq_end, (float *)workspace, B, Hq, Hkv, D, G, S, K,
-                                  T_cap, splits, s);
+    if (splits == 0) {
+        splits = attn_rotary_splits(B, Hkv, T_cap, sm_count());
+        st = attn_rotary_dispatch(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, D, G, S, K, T_cap, splits, s);
+    }
     if (st != TACVQ_OK) return st;
-    return attn_combine_dispatch((const float *)workspace, splits, (__half *)out_f16, state_out, (int64_t)B * Hq, D, s);
+    return attn_combine_dispatch(part, splits, (__half *)out_f16, state_out, (int64_t)B * Hq, D, s);
+}
+
+int tacvq_attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes,
+                             const uint16_t *ktab_f16, const uint16_t *vtab_f16, const uint16_t *rope_table,
+                             const int32_t *seq_start, const int32_t *seq_end, void *workspace, size_t workspace_bytes,
+                             uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv, int D, int G, int S, int K,
+                             int64_t T_cap, tacvq_stream_t stream) {
+    return attn_decode_rotary(q_f16, kcodes, vcodes, ktab_f16, vtab_f16, rope_table, seq_start, seq_end, workspace, workspace_bytes,
+                              out_f16, state_out, B, Hq, Hkv, D, G, S, K, T_cap, T_cap, stream);
 }
 
 int tacvq_set_ranges(int32_t *seq_start, int32_t *seq_end, int B, int start, int end, tacvq_stream_t stream) {
@@ -434,9 +451,9 @@ static int decode_step(const tacvq_step_plan &p, const uint16_t *q_f16, const vo
     }
     if (st != TACVQ_OK) return st;
     if (p.rope_table_f16)
-        return tacvq_attn_decode_rotary(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.rope_table_f16, p.seq_start, p.seq_end,
-                                        p.workspace, p.workspace_bytes, out_f16, state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K,
-                                        p.T_cap, stream);
+        return attn_decode_rotary(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.rope_table_f16, p.seq_start, p.seq_end,
+                                  p.workspace, p.workspace_bytes, out_f16, state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K, p.T_cap,
+                                  end - start, stream);
     return tacvq_attn_decode(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.seq_start, p.seq_end, p.workspace,
                              p.workspace_bytes, out_f16, state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K, p.T_cap, stream);
 }

@@ -156,31 +156,60 @@ attn_generic_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kc
     }
 }
 
-// Merge n_parts states laid out [n_parts][rows][2+D]; one block per row.
-__global__ void __launch_bounds__(128)
+// Merge n_parts states laid out [n_parts][rows][2+D]; one block per row.  What bounds it is the memory latency of a row's
+// n_parts states, so nothing walks them one after the other: the threads take a part's (m, l) each and reduce, then groups
+// of 128 threads (a thread per channel) take every groups-th part, up to eight loads in flight.
+constexpr int kCombineLanes = 128, kCombineGroups = 8;
+
+__global__ void __launch_bounds__(kCombineLanes * kCombineGroups)
 attn_combine_kernel(const float *__restrict__ states, int n_parts, int64_t rows, int D, __half *__restrict__ out,
                     float *__restrict__ merged) {
+    __shared__ float red[2 * kCombineLanes * kCombineGroups / 32];
+    __shared__ float sums[kCombineGroups * kCombineLanes];
     const int64_t row = blockIdx.x;
     const int W = D + 2;
+    const int64_t stride = rows * W;
+    const float *own = states + row * W;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
     float top = -INFINITY;
-    for (int p = 0; p < n_parts; ++p) top = fmaxf(top, states[((int64_t)p * rows + row) * W]);
+    for (int p = tid; p < n_parts; p += blockDim.x) top = fmaxf(top, own[p * stride]);
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+    if (lane == 0) red[warp] = top;
+    __syncthreads();
+    for (int w = 0; w < warps; ++w) top = fmaxf(top, red[w]);
     float l = 0.0f;
-    for (int p = 0; p < n_parts; ++p) {
-        const float *st = states + ((int64_t)p * rows + row) * W;
-        if (st[0] == -INFINITY) continue;
-        l += __expf(st[0] - top) * st[1];
+    for (int p = tid; p < n_parts; p += blockDim.x) {
+        const float m = own[p * stride];
+        if (m != -INFINITY) l += __expf(m - top) * own[p * stride + 1];
     }
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+    if (lane == 0) red[warps + warp] = l;
+    __syncthreads();
+    l = 0.0f;
+    for (int w = 0; w < warps; ++w) l += red[warps + w];
+    const int group = tid / kCombineLanes, groups = blockDim.x / kCombineLanes, at = tid % kCombineLanes;
+    for (int base = 0; base < D; base += kCombineLanes) {
+        const int i = base + at;
         float a = 0.0f;
-        for (int p = 0; p < n_parts; ++p) {
-            const float *st = states + ((int64_t)p * rows + row) * W;
-            if (st[0] == -INFINITY) continue;
-            a += __expf(st[0] - top) * st[2 + i];
+        if (i < D) {
+#pragma unroll 8
+            for (int p = group; p < n_parts; p += groups) {
+                const float m = own[p * stride], v = own[p * stride + 2 + i];
+                if (m != -INFINITY) a += __expf(m - top) * v;
+            }
         }
-        if (merged) merged[row * W + 2 + i] = a;
-        if (out) out[row * D + i] = __float2half_rn(l > 0.0f ? a / l : 0.0f);
+        sums[group * kCombineLanes + at] = a;
+        __syncthreads();
+        if (group == 0 && i < D) {
+            for (int g = 1; g < groups; ++g) a += sums[g * kCombineLanes + at];
+            if (merged) merged[row * W + 2 + i] = a;
+            if (out) out[row * D + i] = __float2half_rn(l > 0.0f ? a / l : 0.0f);
+        }
+        __syncthreads();
     }
-    if (merged && threadIdx.x == 0) {
+    if (merged && tid == 0) {
         merged[row * W] = top;
         merged[row * W + 1] = l;
     }
@@ -189,7 +218,9 @@ attn_combine_kernel(const float *__restrict__ states, int n_parts, int64_t rows,
 int attn_combine_dispatch(const float *states, int n_parts, __half *out, float *merged, int64_t rows, int D,
                           cudaStream_t stream) {
     if (rows == 0) return TACVQ_OK;
-    attn_combine_kernel<<<(unsigned)rows, 128, 0, stream>>>(states, n_parts, rows, D, out, merged);
+    // a group for every eight parts: more would have less than one round of loads each
+    const int groups = n_parts > 8 * kCombineGroups ? kCombineGroups : n_parts > 8 ? (n_parts + 7) / 8 : 1;
+    attn_combine_kernel<<<(unsigned)rows, kCombineLanes * groups, 0, stream>>>(states, n_parts, rows, D, out, merged);
     return launch_status();
 }
 

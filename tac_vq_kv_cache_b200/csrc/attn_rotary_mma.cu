@@ -1,20 +1,23 @@
 // Attention over codes of PRE-rotary keys for the benchmark geometry (head_dim 128 = 16 groups x 8,
 // two residual stages, 256 words), with both contractions on the tensor cores (mma.sync).
 //
-// A block serves one (batch row, KV head, sequence split) of at most 4096 tokens in two passes:
-//   pass K   key tables (128 KB) in shared memory.  Four lanes share a token; lane j of them rebuilds the
-//            channels 16j..16j+15 and 64+16j..64+16j+15 (groups 2j, 2j+1, 2j+8, 2j+9) as fp16 (packed add
-//            of the two stages = the reference's fp16 window), which are exactly the rotary partners
-//            c, c+64, rotates them with the cos/sin of the token's position, and the warp multiplies
+// A block serves one KV head, up to R batch rows and one range of positions, at most 6144 tokens in all, in two passes:
+//   pass K   key tables (128 KB) in shared memory.  Four lanes share a token; lane j of them rebuilds groups j, j+4, j+8
+//            and j+12 as fp16 (packed add of the two stages = the reference's fp16 window), which are exactly the
+//            rotary partners c, c+64, rotates them with the cos/sin of the token's position, and the warp multiplies
 //            8 tokens x 128 channels with the 4 query heads by four m16n8k16 products: rows 0-7 of the A
 //            operand carry the lower 64 channels of the 8 tokens, rows 8-15 the upper 64, and the 8 columns
 //            of the B operand are (4 heads) x (lower | upper query channels); the two halves of a score
 //            meet through one shuffle.  fp32 scores go to shared memory.
-//   softmax  block maximum, p = exp(score - max) as fp16 [head][token] over the score area.
+//   softmax  maximum of every row and head, p = exp(score - max) as fp16 [row][head][token] over the score area.
 //   pass V   value tables loaded over the key tables (the copy overlaps the softmax step); P.V with
 //            m16n8k8 products exactly as in the kernel without rotary step (attn_gsrq.cu): rows =
 //            channels, columns = 4 heads x 2 visiting orders, contraction = tokens; value codes land by
 //            cp.async and are handed out by ldmatrix.trans.
+// All rows of a batch stand at the same positions, so the rows of a block share their cos/sin (256 bytes a position, eight
+// times a token's codes): a warp keeps those of its 8 positions in registers and goes through the block's rows.  A chunk is as
+// long as the score area allows, because each one copies both tables (2 x 128 KB).
+//
 // Every shared-memory gather is conflict-free for arbitrary codes: a code's 32 codewords lie in one
 // 512-byte row, the position of (stage, group) inside the row decides the bank, and the lanes that are
 // served together read different positions (the two tokens of a quarter warp take the stages in opposite
@@ -33,14 +36,18 @@ namespace rotmma {
 
 constexpr int kThreads = 512, kWarps = kThreads / 32;
 constexpr int kDim = 128, kWords = 256, kRowBytes = 512;   // a code's 32 codewords
-constexpr int kChunk = 4096;                               // tokens per block at most
+constexpr int kChunk = 6144;                               // tokens per block at most, over all its rows
 constexpr int kTabBytes = kWords * kRowBytes;              // 131072
 constexpr int kScoreBytes = kChunk * 4 * 4;                // fp32 [token][4 heads]
-constexpr int kProbStride = kChunk * 2 + 16;               // bytes per head of the fp16 probabilities
+template <int R>
+constexpr int kPositions = kChunk / R;                     // positions per block at most
+template <int R>
+constexpr int kProbStride = kPositions<R> * 2 + 16;        // bytes per row and head of the fp16 probabilities
 constexpr int kVStagePerWarp = 1024;                       // one 32-token tile of value codes
 constexpr int kRedFloats = kWarps * 4;
-constexpr int kSmemBytes = kTabBytes + kScoreBytes + 2 * kRedFloats * 4;
-static_assert(4 * kProbStride + kWarps * kVStagePerWarp <= kScoreBytes, "probabilities and code staging reuse the score area");
+constexpr int kSmemBytes = kTabBytes + kScoreBytes + 2 * kRedFloats * 4 + 4 * 16;
+static_assert(16 * kProbStride<4> + kWarps * kVStagePerWarp <= kScoreBytes, "probabilities and code staging reuse the score area");
+static_assert(kSmemBytes <= 227 * 1024, "");
 static_assert(kWarps * 32 * 32 * 4 <= kTabBytes, "merge scratch reuses the table area");
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -82,6 +89,7 @@ __device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
 }
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -96,155 +104,181 @@ __device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1,
         : "r"(a0), "r"(a1), "r"(b0));
 }
 
-// position of the codeword (stage s, group g) inside a code's 512-byte row
-//   key tables:   the bank (position mod 8) is s*4 + (g/2)%4: in pass K lane j reads groups 2j + {0,1,8,9}
-//   value tables: the bank is s*4 + g%4 (as in attn_gsrq.cu)
-__device__ __forceinline__ int key_pos(int s, int g) { return (((g >> 3) << 1) | (g & 1)) * 8 + s * 4 + ((g >> 1) & 3); }
-__device__ __forceinline__ int value_pos(int s, int g) { return (g >> 2) * 8 + s * 4 + (g & 3); }
+// position of the codeword (stage s, group g) inside a code's 512-byte row; the bank is s*4 + g%4 (as in attn_gsrq.cu)
+__device__ __forceinline__ int word_pos(int s, int g) { return (g >> 2) * 8 + s * 4 + (g & 3); }
 
 // A head's tables [stage][group][word][8] -> shared memory rows [word][position]; a warp copies, per trip,
 // 4 neighbouring words of 8 positions with different banks: full 32-byte sectors in, no conflicts out.
-template <bool KEYS>
 __device__ __forceinline__ void copy_tables(uint32_t tab_u32, const __half *__restrict__ src, int tid) {
     for (int idx = tid; idx < kWords * 32; idx += kThreads) {
         const int pos = ((idx >> 5) & 3) * 8 + (idx & 7);
         const int word = ((idx >> 7) << 2) | ((idx >> 3) & 3);
-        int s, g;
-        if (KEYS) {
-            s = (pos >> 2) & 1;
-            g = ((pos >> 4) << 3) | ((pos & 3) << 1) | ((pos >> 3) & 1);
-        } else {
-            s = (pos >> 2) & 1;
-            g = ((pos >> 3) << 2) | (pos & 3);
-        }
+        const int s = (pos >> 2) & 1, g = ((pos >> 3) << 2) | (pos & 3);
         cp_async16(tab_u32 + word * kRowBytes + pos * 16, src + ((size_t)(s * 16 + g) * kWords + word) * 8);
     }
 }
 
+template <int R>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcodes, const uint8_t *__restrict__ vcodes,
                        const __half *__restrict__ ktab, const __half *__restrict__ vtab, const __half *__restrict__ rope,
                        const int32_t *__restrict__ seq_start, const int32_t *__restrict__ seq_end, float *__restrict__ part,
                        int B, int Hq, int Hkv, int64_t T_cap, int splits) {
+    constexpr int kPos = kPositions<R>, kStride = kProbStride<R>;
+    constexpr int kRowWarps = kWarps / R, kRowThreads = kThreads / R;  // softmax and pass V: warps of one batch row
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *tab_s = smem_raw;
-    float *score_s = reinterpret_cast<float *>(smem_raw + kTabBytes);
+    float *score_s = reinterpret_cast<float *>(smem_raw + kTabBytes);  // [R][kPos][4 heads]
     float *red_s = reinterpret_cast<float *>(smem_raw + kTabBytes + kScoreBytes);  // [2][warps][4]
+    int4 *limit_s = reinterpret_cast<int4 *>(red_s + 2 * kRedFloats);  // per row: first and last + 1 visible token, both ends for code reads
     const uint32_t tab_u32 = smem_u32(tab_s), score_u32 = smem_u32(score_s);
 
-    const int split = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+    const int split = blockIdx.x, h = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rep = Hq / Hkv;  // 1, 2 or 4 query heads per KV head
+    const int b0 = (int)((int64_t)blockIdx.z * B / gridDim.z), n_rows = (int)((int64_t)(blockIdx.z + 1) * B / gridDim.z) - b0;
 
-    const int lo_all = seq_start ? max(seq_start[b], 0) : 0;
-    const int hi_all = seq_end ? min(seq_end[b], (int)T_cap) : (int)T_cap;
+    // positions that some row of the block sees, and this split's share of them
+    int lo_all = 0x7fffffff, hi_all = 0;
+    for (int r = 0; r < n_rows; ++r) {
+        const int lo = seq_start ? max(seq_start[b0 + r], 0) : 0;
+        const int hi = seq_end ? min(seq_end[b0 + r], (int)T_cap) : (int)T_cap;
+        if (hi > lo) lo_all = min(lo_all, lo), hi_all = max(hi_all, hi);
+    }
     const int n_all = hi_all > lo_all ? hi_all - lo_all : 0;
     const int per = (n_all + splits - 1) / splits;
-    const int chunk = lo_all + split * per;
-    const int n = max(min(chunk + per, lo_all + n_all) - chunk, 0);  // at most kChunk: the launcher picks the split count
+    const int chunk = n_all > 0 ? lo_all + split * per : 0;
+    const int n = n_all > 0 ? max(min(chunk + per, hi_all) - chunk, 0) : 0;  // at most kPos: the launcher picks the split count
     const int64_t rows = (int64_t)B * Hq;
-    const size_t code_row = ((size_t)b * Hkv + h) * (size_t)T_cap;
 
     if (n <= 0) {  // an empty range contributes the neutral state
-        for (int idx = tid; idx < rep * (kDim + 2); idx += kThreads) {
+        for (int idx = tid; idx < n_rows * rep * (kDim + 2); idx += kThreads) {
             const int r = idx / (kDim + 2), col = idx % (kDim + 2);
-            part[((int64_t)split * rows + (int64_t)b * Hq + h * rep + r) * (kDim + 2) + col] = col == 0 ? -INFINITY : 0.0f;
+            part[((int64_t)split * rows + (int64_t)(b0 + r / rep) * Hq + h * rep + r % rep) * (kDim + 2) + col] = col == 0 ? -INFINITY : 0.0f;
         }
         return;
     }
+    const size_t row_step = (size_t)Hkv * (size_t)T_cap * 32;  // code bytes from one batch row to the next
+    const size_t code_at = (((size_t)b0 * Hkv + h) * (size_t)T_cap + chunk) * 32;
 
-    copy_tables<true>(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, tid);
+    copy_tables(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, tid);
+    if (tid < n_rows) {
+        const int lo = seq_start ? max(seq_start[b0 + tid], 0) : 0;
+        const int hi = seq_end ? min(seq_end[b0 + tid], (int)T_cap) : (int)T_cap;
+        const int first = max(lo - chunk, 0), end = min(hi - chunk, n);
+        // a row without a token here reads the codes of some position of the chunk and drops them
+        limit_s[tid] = first < end ? make_int4(first, end, first, end - 1) : make_int4(n, 0, 0, n - 1);
+    }
 
     // ---- pass K ------------------------------------------------------------------------------------
     const int g8 = lane >> 2, j4 = lane & 3;
     {
-        // B operand: column n = g8 is (head n & 3, channel half n >> 2); this lane's 16 channels of it
-        uint32_t qf[8];
-        {
+        // B operand: column n = g8 is (head n & 3, channel half n >> 2); this lane's 16 channels of it, for every row
+        uint32_t qf[R][8];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
             const int head = g8 & 3, half = g8 >> 2;
             uint4 lo4 = make_uint4(0u, 0u, 0u, 0u), hi4 = lo4;
-            if (head < rep) {
-                const uint4 *src = reinterpret_cast<const uint4 *>(q + ((size_t)b * Hq + h * rep + head) * kDim + half * 64 + 16 * j4);
+            if (head < rep && r < n_rows) {
+                const uint4 *src = reinterpret_cast<const uint4 *>(q + ((size_t)(b0 + r) * Hq + h * rep + head) * kDim + half * 64 + 8 * j4);
                 lo4 = __ldg(src);
-                hi4 = __ldg(src + 1);
+                hi4 = __ldg(src + 4);
             }
-            qf[0] = lo4.x, qf[1] = lo4.y, qf[2] = lo4.z, qf[3] = lo4.w, qf[4] = hi4.x, qf[5] = hi4.y, qf[6] = hi4.z, qf[7] = hi4.w;
+            qf[r][0] = lo4.x, qf[r][1] = lo4.y, qf[r][2] = lo4.z, qf[r][3] = lo4.w;
+            qf[r][4] = hi4.x, qf[r][5] = hi4.y, qf[r][6] = hi4.z, qf[r][7] = hi4.w;
         }
-        // gather addresses: step (ci, sf) reads group 2j + {0,1,8,9}[ci] of stage sf ^ (token parity)
+        // step (ci, sf) gathers group j + 4 ci of stage sf ^ (token parity), which lies 128 ci bytes behind that of ci = 0
         const int first_stage = g8 & 1;
-        uint32_t k_off[4][2];
-#pragma unroll
-        for (int ci = 0; ci < 4; ++ci)
-#pragma unroll
-            for (int sf = 0; sf < 2; ++sf)
-                k_off[ci][sf] = tab_u32 + key_pos(sf ^ first_stage, 2 * j4 + (ci & 1) + (ci >> 1) * 8) * 16;
-        // a token's 32 code bytes: stage s at bytes 16s..16s+15; this lane wants bytes 2j, 2j+1 and 8+2j, 9+2j of each
-        const int code_a = first_stage * 16 + 2 * j4, code_b = (first_stage ^ 1) * 16 + 2 * j4;
-        const uint8_t *kc = kcodes + (code_row + chunk) * 32;
-        const __half *rp = rope + (size_t)chunk * kDim + 16 * j4;
+        const uint32_t k_off[2] = {tab_u32 + word_pos(first_stage, j4) * 16, tab_u32 + word_pos(first_stage ^ 1, j4) * 16};
+        const uint32_t k_sel = 0x4404u | ((uint32_t)j4 << 4);  // byte j of a word -> bits 8..15
+        // a token's 32 code bytes: stage s at bytes 16s..16s+15; group j + 4 ci is byte j of word ci
+        const uint8_t *kc = kcodes + code_at + first_stage * 16;
+        const int other_stage = 16 - 32 * first_stage;
+        const ptrdiff_t v_from_k = reinterpret_cast<intptr_t>(vcodes) - reinterpret_cast<intptr_t>(kcodes);
+        const __half *rp = rope + (size_t)chunk * kDim + 8 * j4;
 
         const int trips = (n + 8 * kWarps - 1) / (8 * kWarps);
-        uint32_t cn[4];
-        uint4 rn[4];
-        auto fetch = [&](int local) {
-            const int t = min(local, n - 1);
-            const uint8_t *row = kc + (size_t)t * 32;
-            cn[0] = *reinterpret_cast<const unsigned short *>(row + code_a);
-            cn[1] = *reinterpret_cast<const unsigned short *>(row + code_a + 8);
-            cn[2] = *reinterpret_cast<const unsigned short *>(row + code_b);
-            cn[3] = *reinterpret_cast<const unsigned short *>(row + code_b + 8);
-            const uint4 *cs = reinterpret_cast<const uint4 *>(rp + (size_t)t * kDim);
-            rn[0] = __ldg(cs), rn[1] = __ldg(cs + 1);          // cosines of frequencies 16j .. 16j+15
-            rn[2] = __ldg(cs + 8), rn[3] = __ldg(cs + 9);      // sines
+        uint4 cn[2], rn[4];
+        int4 limit;
+        auto fetch_codes = [&](int r, int local) {
+            limit = limit_s[r];
+            const int t = min(max(local, limit.z), limit.w);
+            const uint8_t *src = kc + (size_t)r * row_step + (size_t)t * 32;
+            cn[0] = __ldg(reinterpret_cast<const uint4 *>(src));
+            cn[1] = __ldg(reinterpret_cast<const uint4 *>(src + other_stage));
+            // to L2: the key codes two trips on, and the value codes of this one for pass V
+            const int ahead = max(min(local + 16 * kWarps, limit.w), 0);
+            if (j4 < 2) prefetch_l2(j4 == 0 ? kc + (size_t)r * row_step + (size_t)ahead * 32 : src + v_from_k);
         };
-        fetch(warp * 8 + g8);
+        auto fetch_rope = [&](int local) {
+            const uint4 *cs = reinterpret_cast<const uint4 *>(rp + (size_t)min(local, n - 1) * kDim);
+            rn[0] = __ldg(cs), rn[1] = __ldg(cs + 4);          // cosines of frequencies 8j .. and 32 + 8j ..
+            rn[2] = __ldg(cs + 8), rn[3] = __ldg(cs + 12);     // sines
+        };
+        fetch_rope(warp * 8 + g8);
         cp_async_wait_all();
         __syncthreads();
+        fetch_codes(0, warp * 8 + g8);
+#pragma unroll 1
         for (int trip = 0; trip < trips; ++trip) {
             const int local = (trip * kWarps + warp) * 8 + g8;
-            const uint32_t c0 = cn[0], c1 = cn[1], c2 = cn[2], c3 = cn[3];
             const uint32_t cosv[8] = {rn[0].x, rn[0].y, rn[0].z, rn[0].w, rn[1].x, rn[1].y, rn[1].z, rn[1].w};
             const uint32_t sinv[8] = {rn[2].x, rn[2].y, rn[2].z, rn[2].w, rn[3].x, rn[3].y, rn[3].z, rn[3].w};
-            if (trip + 1 < trips) fetch(local + 8 * kWarps);
-            // first stage of this lane's order, then the other; the packed fp16 sum does not depend on the order
-            const uint4 a0 = lds128(k_off[0][0] + (c0 & 0xffu) * kRowBytes), a1 = lds128(k_off[1][0] + (c0 >> 8) * kRowBytes);
-            const uint4 a2 = lds128(k_off[2][0] + (c1 & 0xffu) * kRowBytes), a3 = lds128(k_off[3][0] + (c1 >> 8) * kRowBytes);
-            const uint4 b0 = lds128(k_off[0][1] + (c2 & 0xffu) * kRowBytes), b1 = lds128(k_off[1][1] + (c2 >> 8) * kRowBytes);
-            const uint4 b2 = lds128(k_off[2][1] + (c3 & 0xffu) * kRowBytes), b3 = lds128(k_off[3][1] + (c3 >> 8) * kRowBytes);
-            const uint32_t lo[8] = {hadd2(a0.x, b0.x), hadd2(a0.y, b0.y), hadd2(a0.z, b0.z), hadd2(a0.w, b0.w),
-                                    hadd2(a1.x, b1.x), hadd2(a1.y, b1.y), hadd2(a1.z, b1.z), hadd2(a1.w, b1.w)};
-            const uint32_t hi[8] = {hadd2(a2.x, b2.x), hadd2(a2.y, b2.y), hadd2(a2.z, b2.z), hadd2(a2.w, b2.w),
-                                    hadd2(a3.x, b3.x), hadd2(a3.y, b3.y), hadd2(a3.z, b3.z), hadd2(a3.w, b3.w)};
-            // k'_c = k_c cos - k_{c+64} sin ;  k'_{c+64} = k_{c+64} cos + k_c sin
-            uint32_t rl[8], rh[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                rl[i] = hfma2(hi[i] ^ 0x80008000u, sinv[i], hmul2(lo[i], cosv[i]));
-                rh[i] = hfma2(lo[i], sinv[i], hmul2(hi[i], cosv[i]));
+            for (int r = 0; r < R; ++r) {
+                if (r >= n_rows) break;
+                const uint32_t first[4] = {cn[0].x, cn[0].y, cn[0].z, cn[0].w}, second[4] = {cn[1].x, cn[1].y, cn[1].z, cn[1].w};
+                const bool seen = local >= limit.x && local < limit.y;
+                if (r + 1 < n_rows && r + 1 < R) fetch_codes(r + 1, local);
+                else if (trip + 1 < trips) fetch_codes(0, local + 8 * kWarps);
+                float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                if (__any_sync(0xffffffffu, seen)) {
+                    // first stage of this lane's order, then the other; the packed fp16 sum does not depend on the order
+                    uint32_t k[4][4];
+#pragma unroll
+                    for (int ci = 0; ci < 4; ++ci) {
+                        const uint32_t at0 = prmt(first[ci], 0u, k_sel), at1 = prmt(second[ci], 0u, k_sel);
+                        const uint4 a = lds128(k_off[0] + at0 + at0 + ci * 128), b = lds128(k_off[1] + at1 + at1 + ci * 128);
+                        k[ci][0] = hadd2(a.x, b.x), k[ci][1] = hadd2(a.y, b.y), k[ci][2] = hadd2(a.z, b.z), k[ci][3] = hadd2(a.w, b.w);
+                    }
+                    // k'_c = k_c cos - k_{c+64} sin ;  k'_{c+64} = k_{c+64} cos + k_c sin
+                    uint32_t rl[8], rh[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t lo = k[i >> 2][i & 3], hi = k[2 + (i >> 2)][i & 3];
+                        rl[i] = hfma2(hi ^ 0x80008000u, sinv[i], hmul2(lo, cosv[i]));
+                        rh[i] = hfma2(lo, sinv[i], hmul2(hi, cosv[i]));
+                    }
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)
+                        mma16816(d, rl[2 * ks], rh[2 * ks], rl[2 * ks + 1], rh[2 * ks + 1], qf[r][2 * ks], qf[r][2 * ks + 1]);
+                }
+                // rows 0-7 x columns 0-3 hold the lower halves of the scores (lanes j < 2), rows 8-15 x columns 4-7
+                // the upper halves (lanes j >= 2)
+                const float up0 = __shfl_xor_sync(0xffffffffu, d[2], 2), up1 = __shfl_xor_sync(0xffffffffu, d[3], 2);
+                if (j4 < 2 && local < n)
+                    *reinterpret_cast<float2 *>(score_s + ((size_t)r * kPos + local) * 4 + 2 * j4) =
+                        seen ? make_float2(d[0] + up0, d[1] + up1) : make_float2(-INFINITY, -INFINITY);
             }
-            float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) mma16816(d, rl[2 * ks], rh[2 * ks], rl[2 * ks + 1], rh[2 * ks + 1], qf[2 * ks], qf[2 * ks + 1]);
-            // rows 0-7 x columns 0-3 hold the lower halves of the scores (lanes j < 2), rows 8-15 x columns 4-7
-            // the upper halves (lanes j >= 2)
-            const float up0 = __shfl_xor_sync(0xffffffffu, d[2], 2), up1 = __shfl_xor_sync(0xffffffffu, d[3], 2);
-            if (j4 < 2 && local < n) *reinterpret_cast<float2 *>(score_s + (size_t)local * 4 + 2 * j4) = make_float2(d[0] + up0, d[1] + up1);
+            if (trip + 1 < trips) fetch_rope(local + 8 * kWarps);
         }
     }
     __syncthreads();
 
-    // ---- softmax over the block's tokens; value tables arrive meanwhile -------------------------------
-    copy_tables<false>(tab_u32, vtab + (size_t)h * 2 * 16 * kWords * 8, tid);
+    // ---- softmax over the block's tokens, kRowWarps warps a batch row; value tables arrive meanwhile ---
+    copy_tables(tab_u32, vtab + (size_t)h * 2 * 16 * kWords * 8, tid);
     const int n_pad = (n + 31) & ~31;
+    const int row = warp / kRowWarps, row_warp = warp % kRowWarps;
+    const bool row_live = row < n_rows;
     float m[4], l[4];
     {
-        float4 sv[kChunk / kThreads];
+        float4 sv[kPos / kRowThreads];
         float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int k = 0; k < kChunk / kThreads; ++k) {
-            const int i = tid + k * kThreads;
-            if (i < n) {
-                sv[k] = *reinterpret_cast<const float4 *>(score_s + (size_t)i * 4);
+        for (int k = 0; k < kPos / kRowThreads; ++k) {
+            const int i = row_warp * 32 + lane + k * kRowThreads;
+            if (i < n && row_live) {
+                sv[k] = *reinterpret_cast<const float4 *>(score_s + ((size_t)row * kPos + i) * 4);
                 top[0] = fmaxf(top[0], sv[k].x), top[1] = fmaxf(top[1], sv[k].y), top[2] = fmaxf(top[2], sv[k].z), top[3] = fmaxf(top[3], sv[k].w);
             }
         }
@@ -258,22 +292,22 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             m[r] = -INFINITY;
-            for (int w = 0; w < kWarps; ++w) m[r] = fmaxf(m[r], red_s[w * 4 + r]);
+            for (int w = 0; w < kRowWarps; ++w) m[r] = fmaxf(m[r], red_s[(row * kRowWarps + w) * 4 + r]);
             l[r] = 0.0f;
         }
-        __half *prob = reinterpret_cast<__half *>(score_s);
+        __half *prob = reinterpret_cast<__half *>(score_s) + (size_t)row * 4 * (kStride / 2);
 #pragma unroll
-        for (int k = 0; k < kChunk / kThreads; ++k) {
-            const int i = tid + k * kThreads;
-            if (i < n_pad) {
+        for (int k = 0; k < kPos / kRowThreads; ++k) {
+            const int i = row_warp * 32 + lane + k * kRowThreads;
+            if (i < n_pad && row_live) {
                 float p[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                if (i < n) {
+                if (i < n) {  // a token that the row does not see scored -inf: weight 0 as long as the row has a maximum
                     p[0] = __expf(sv[k].x - m[0]), p[1] = __expf(sv[k].y - m[1]), p[2] = __expf(sv[k].z - m[2]), p[3] = __expf(sv[k].w - m[3]);
                 }
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     l[r] += p[r];
-                    prob[(size_t)r * (kProbStride / 2) + i] = __float2half_rn(p[r]);
+                    prob[(size_t)r * (kStride / 2) + i] = __float2half_rn(p[r]);
                 }
             }
         }
@@ -293,7 +327,7 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
 #pragma unroll
         for (int gsel = 0; gsel < 2; ++gsel) {
             const int s = sp ^ (kq & 1), gh = gsel ^ (kq >> 1);
-            v_off[sp][gsel] = tab_u32 + value_pos(s, 2 * r8 + gh) * 16;
+            v_off[sp][gsel] = tab_u32 + word_pos(s, 2 * r8 + gh) * 16;
         }
 #pragma unroll
     for (int tk = 0; tk < 2; ++tk)
@@ -301,37 +335,36 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
         for (int gsel = 0; gsel < 2; ++gsel) v_sel[tk][gsel] = 0x4404u | ((uint32_t)(tk * 2 + (gsel ^ (kq >> 1))) << 4);  // code byte -> bits 8..15
     const int b_head = r8 & 3;                       // B-operand column n = r8: head n & 3, visiting order n >> 2
     const bool b_valid = (r8 >> 2) == (kq >> 1);
-    const uint32_t vstage_u32 = score_u32 + 4 * kProbStride + warp * kVStagePerWarp;
-    // landing place of this lane's (= token's) two 16-byte stage halves: odd token pairs swap the halves (stage
+    const uint32_t vstage_u32 = score_u32 + R * 4 * kStride + warp * kVStagePerWarp;
+    // landing place of a token's two 16-byte stage halves: odd token pairs swap the halves (stage
     // order of the value look-ups), tokens 4..7 of every eight swap them once more so that the eight rows of an
-    // ldmatrix tile cover all banks
-    const uint32_t v_land = vstage_u32 + lane * 32 + ((((lane >> 1) ^ (lane >> 2)) & 1) * 16);
+    // ldmatrix tile cover all banks (a request takes sixteen tokens, two lanes a token: whole sectors)
+    const uint32_t v_land = vstage_u32 + (lane >> 1) * 32 + ((((lane >> 2) ^ (lane >> 3) ^ lane) & 1) * 16);
     const uint32_t v_row0 = vstage_u32 + (8 * (lane >> 4) + (lane & 7)) * 32 + ((((lane >> 3) & 1) ^ ((lane >> 2) & 1)) * 16);
-    const uint32_t p_read = score_u32 + (uint32_t)(b_head * kProbStride + kq * 4);
-    const uint8_t *vc = vcodes + (code_row + chunk) * 32;
+    const uint32_t p_read = score_u32 + (uint32_t)((row * 4 + b_head) * kStride + kq * 4);
+    // a row that sees nothing of this chunk has no maximum and no weights
+    const int4 own = row_live ? limit_s[row] : make_int4(0, 0, 0, 0);
+    const int tiles = own.x < own.y ? n_pad >> 5 : 0;
+    const uint8_t *vc = vcodes + code_at + (size_t)(row_live ? row : 0) * row_step;
+    auto land_codes = [&](int tile) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            cp_async16(v_land + u * 512, vc + (size_t)min(max(tile * 32 + u * 16 + (lane >> 1), own.z), own.w) * 32 + (lane & 1) * 16);
+    };
 
     float acc[8][4];
 #pragma unroll
     for (int mm = 0; mm < 8; ++mm) acc[mm][0] = acc[mm][1] = acc[mm][2] = acc[mm][3] = 0.0f;
-    const int tiles = n_pad >> 5;
     __syncthreads();  // probabilities written; nobody reads scores any more
-    if (warp < tiles) {
-        const uint8_t *src = vc + (size_t)min(warp * 32 + lane, n - 1) * 32;
-        cp_async16(v_land, src);
-        cp_async16(v_land ^ 16u, src + 16);
-    }
+    if (row_warp < tiles) land_codes(row_warp);
     cp_async_wait_all();  // the value tables and the first tile of codes
     __syncthreads();
-    for (int tile = warp; tile < tiles; tile += kWarps) {
+    for (int tile = row_warp; tile < tiles; tile += kRowWarps) {
         uint32_t vm_lo[4], vm_hi[4];  // tokens 0..15 and 16..31 of the tile
         ldmatrix_x4_trans(vm_lo, v_row0);
         ldmatrix_x4_trans(vm_hi, v_row0 + 512);
         __syncwarp();
-        if (tile + kWarps < tiles) {
-            const uint8_t *src = vc + (size_t)min((tile + kWarps) * 32 + lane, n - 1) * 32;
-            cp_async16(v_land, src);
-            cp_async16(v_land ^ 16u, src + 16);
-        }
+        if (tile + kRowWarps < tiles) land_codes(tile + kRowWarps);
         const uint32_t p_tile = p_read + (uint32_t)tile * 64;
 #pragma unroll 1
         for (int a = 0; a < 2; ++a) {
@@ -383,8 +416,9 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
         }
     }
     __syncthreads();
-    for (int o = tid; o < 4 * kDim; o += kThreads) {
-        // output o <-> (product mm, register j, lane of visiting order 0); its twin of order 1 is (mm, j^2, lane^2)
+    for (int oo = tid; oo < n_rows * 4 * kDim; oo += kThreads) {
+        // output o of a row <-> (product mm, register j, lane of visiting order 0); its twin of order 1 is (mm, j^2, lane^2)
+        const int br = oo >> 9, o = oo & 511;
         const int mm = o >> 6, j = (o >> 4) & 3, l16 = o & 15;
         const int src_r8 = l16 >> 1, src_kq = l16 & 1;
         const int lane0 = src_r8 * 4 + src_kq;
@@ -392,19 +426,49 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
         if (r >= rep) continue;
         const int dim = (2 * src_r8 + (j >> 1)) * 8 + mm;
         float asum = 0.0f;
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = br * kRowWarps; w < (br + 1) * kRowWarps; ++w) {
             const float *src = wacc + (size_t)w * 1024;
             asum += src[(mm * 4 + j) * 32 + lane0] + src[(mm * 4 + (j ^ 2)) * 32 + (lane0 ^ 2)];
         }
-        float *dst = part + ((int64_t)split * rows + (int64_t)b * Hq + h * rep + r) * (kDim + 2);
+        float *dst = part + ((int64_t)split * rows + (int64_t)(b0 + br) * Hq + h * rep + r) * (kDim + 2);
         dst[2 + dim] = asum;
         if (dim == 0) {
-            float lsum = 0.0f;
-            for (int w = 0; w < kWarps; ++w) lsum += red_s[kRedFloats + w * 4 + r];
-            dst[0] = m[r];
-            dst[1] = lsum;
+            float top = -INFINITY, lsum = 0.0f;
+            for (int w = br * kRowWarps; w < (br + 1) * kRowWarps; ++w) {
+                top = fmaxf(top, red_s[w * 4 + r]);
+                lsum += red_s[kRedFloats + w * 4 + r];
+            }
+            dst[0] = top;
+            dst[1] = top == -INFINITY ? 0.0f : lsum;
         }
     }
+}
+
+// Rows a block, and splits of the positions, for `visible` positions a row.  One block per SM; a block costs its
+// table copies and merge (kFixed) and its tokens, whose price falls with the rows that share a position's cos/sin; the pair with
+// the least waves x block is taken.  In clocks, from the measured kernel.
+struct Plan {
+    int rows, splits;
+};
+
+inline Plan plan(int B, int Hkv, int64_t visible, int sms) {
+    constexpr double kFixed = 14000.0;
+    Plan best = {0, 0};
+    double least_cost = 0.0;
+    for (int rows = 4; rows >= 1; rows >>= 1) {
+        if (rows > 1 && B <= rows / 2) continue;  // fewer rows than that share a block
+        const int groups = (B + rows - 1) / rows, share = (B + groups - 1) / groups;
+        const double token = rows == 4 ? 19.0 : rows == 2 ? 20.0 : 22.0;
+        const int64_t least = (visible + kChunk / rows - 1) / (kChunk / rows);
+        for (int splits = least < 1 ? 1 : (int)(least > 65 ? 65 : least); splits <= 64; ++splits) {
+            const int64_t per = (visible + splits - 1) / splits;
+            const int64_t waves = ((int64_t)groups * Hkv * splits + sms - 1) / sms;
+            const double cost = (double)waves * (kFixed + (double)(share * per) * token) + 40.0 * splits;
+            if (best.rows == 0 || cost < least_cost) least_cost = cost, best = {rows, splits};
+            if (per * share <= 256) break;
+        }
+    }
+    return best;
 }
 
 }  // namespace rotmma
@@ -414,18 +478,32 @@ bool attn_rotary_mma_supported(int Hq, int Hkv, int D, int G, int S, int K) {
     return D == 128 && G == 16 && S == 2 && K == 256 && (rep == 1 || rep == 2 || rep == 4);
 }
 
-// Same grid and partial-state layout as the staged kernel: grid (splits, KV heads, batch rows), at most 4096
-// tokens per block, partial states [split][B*Hq][2 + D] for attn_combine_kernel.
-int attn_rotary_mma_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
+template <int R>
+static int launch_rotary_mma(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
                              const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
                              int Hkv, int64_t T_cap, int splits, cudaStream_t stream) {
-    static_assert(rotmma::kChunk == 4096, "the split count is chosen for 4096 tokens per block");
-    cudaError_t e = cudaFuncSetAttribute(rotmma::attn_rotary_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rotmma::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(rotmma::attn_rotary_mma_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, rotmma::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
-    dim3 grid((unsigned)splits, (unsigned)Hkv, (unsigned)B);
-    rotmma::attn_rotary_mma_kernel<<<grid, rotmma::kThreads, rotmma::kSmemBytes, stream>>>(q, kcodes, vcodes, ktab, vtab, rope, seq_start,
-                                                                                          seq_end, part, B, Hq, Hkv, T_cap, splits);
+    dim3 grid((unsigned)splits, (unsigned)Hkv, (unsigned)((B + R - 1) / R));
+    rotmma::attn_rotary_mma_kernel<R><<<grid, rotmma::kThreads, rotmma::kSmemBytes, stream>>>(q, kcodes, vcodes, ktab, vtab, rope, seq_start,
+                                                                                             seq_end, part, B, Hq, Hkv, T_cap, splits);
     return launch_status();
+}
+
+// Partial states [split][B*Hq][2 + D] for attn_combine_kernel; *splits is how many (0: `visible` positions are too many for
+// the score areas of 64 splits, nothing was launched).  No row may see more than `visible` positions, nor may two rows of
+// the batch together span more.
+int attn_rotary_mma_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
+                             const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
+                             int Hkv, int64_t T_cap, int64_t visible, int sms, int *splits, cudaStream_t stream) {
+    const rotmma::Plan plan = rotmma::plan(B, Hkv, visible, sms);
+    *splits = plan.splits;
+    switch (plan.rows) {
+        case 1: return launch_rotary_mma<1>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, stream);
+        case 2: return launch_rotary_mma<2>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, stream);
+        case 4: return launch_rotary_mma<4>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, stream);
+        default: return TACVQ_OK;
+    }
 }
 
 }  // namespace tacvq

@@ -97,6 +97,38 @@ def test_rotary_attention_matches_the_oracle(device, b, hq, hkv, t, groups, stag
     _check(state[..., 2:] / state[..., 1:2], acc / l[..., None])
 
 
+@pytest.mark.parametrize(
+    "b,hq,hkv,t,ranges",
+    [
+        (3, 8, 2, 700, [(0, 700), (100, 333), (5, 5)]),                                   # one block's rows: whole, part, nothing
+        (4, 4, 4, 2049, [(0, 1), (2048, 2049), (7, 1500), (1024, 1032)]),                 # ranges that hardly meet
+        (5, 8, 4, 4100, [(0, 4100), (4, 4099), (4000, 4100), (300, 100), (0, 8)]),        # rows spread over two unequal groups
+        (2, 8, 2, 6150, [(0, 6150), (3, 6149)]),                                          # more positions than one chunk of two rows
+        (9, 2, 2, 31, [(0, 31)] * 8 + [(30, 31)]),                                        # less than a tile
+    ],
+)
+def test_rotary_rows_of_a_batch_that_share_positions(device, b, hq, hkv, t, ranges):
+    """Rows of one block stand at the same positions but see ranges of their own; a row that sees nothing gets zeros."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(b * t)
+    kcodes, vcodes = (torch.randint(0, 256, (b, hkv, t, 2, 16), generator=gen, dtype=torch.uint8) for _ in range(2))
+    ktab, vtab = make_tables(gen, hkv, 2, 16, 8), make_tables(gen, hkv, 2, 16, 8)
+    q = (torch.randn(b, hq, 128, generator=gen) / 128**0.5).half()
+    start, end = [r[0] for r in ranges], [r[1] for r in ranges]
+    live = [i for i in range(b) if end[i] > start[i]]
+    want, *_ = O.attention_over_codes(q[live], kcodes[live], vcodes[live], ktab, vtab, [start[i] for i in live], [end[i] for i in live], rope_theta=1e6)
+    out, state = ops.attn_decode(
+        q.to(device), kcodes.to(device), vcodes.to(device), ktab.to(device), vtab.to(device),
+        torch.tensor(start, dtype=torch.int32, device=device), torch.tensor(end, dtype=torch.int32, device=device),
+        rope=ops.rope_table(t, 128, 1e6, device), want_state=True,
+    )
+    out, state = out.float().cpu(), state.cpu()
+    for i, row in enumerate(live):
+        _check(out[row], want[i])
+    for row in set(range(b)) - set(live):
+        assert not out[row].any() and (state[row, :, 0] == -float("inf")).all() and not state[row, :, 1:].any()
+
+
 def test_code_cache_with_rope_follows_the_reference_decode_loop(device):
     """Prefill + three decode steps through VQCodeCache(rope_theta=...): codes of pre-rotary keys are
     appended in place, the query arrives rotated; compared with the oracle on the cache's own codes."""
