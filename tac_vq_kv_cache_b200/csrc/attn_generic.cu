@@ -171,6 +171,7 @@ attn_combine_kernel(const float *__restrict__ states, int n_parts, int64_t rows,
     const int64_t stride = rows * W;
     const float *own = states + row * W;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    wait_for_previous_kernel();
     float top = -INFINITY;
     for (int p = tid; p < n_parts; p += blockDim.x) top = fmaxf(top, own[p * stride]);
 #pragma unroll
@@ -220,8 +221,9 @@ int attn_combine_dispatch(const float *states, int n_parts, __half *out, float *
     if (rows == 0) return TACVQ_OK;
     // a group for every eight parts: more would have less than one round of loads each
     const int groups = n_parts > 8 * kCombineGroups ? kCombineGroups : n_parts > 8 ? (n_parts + 7) / 8 : 1;
-    attn_combine_kernel<<<(unsigned)rows, kCombineLanes * groups, 0, stream>>>(states, n_parts, rows, D, out, merged);
-    return launch_status();
+    const cudaError_t e = launch_dependent(true, attn_combine_kernel, dim3((unsigned)rows), dim3(kCombineLanes * groups), 0, stream, states,
+                                           n_parts, rows, D, out, merged);
+    return e == cudaSuccess ? launch_status() : (int)e;
 }
 
 int attn_generic_splits(int B, int Hkv, int64_t T_cap, int sms) {

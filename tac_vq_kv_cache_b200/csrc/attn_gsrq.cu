@@ -162,9 +162,6 @@ __device__ __forceinline__ uint4 ldg_stream(const void *p) {
                  : "l"(p));
     return v;
 }
-// Programmatic dependent launch: a kernel launched with the stream-serialization attribute may start
-// before its predecessor has finished; it must not touch the predecessor's results before this wait.
-__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ float fast_exp2(float x) {  // 2^x, ex2.approx: 2^-inf = +0
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -192,8 +189,6 @@ __device__ __forceinline__ long long block_first_tile(long long total, int block
 
 // position of slot (stage s, group g) inside a code's 512-byte row of the value table
 __device__ __forceinline__ int value_pos(int s, int g) { return (g >> 2) * 8 + s * 4 + (g & 3); }
-
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 using NewToken = GsrqNewToken;
 
@@ -939,24 +934,6 @@ bool attn_gsrq_supported(int Hq, int Hkv, int D, int G, int S, int K) {
     return D == gsrq::kDim && G == gsrq::kGroups && S == gsrq::kStages && K == gsrq::kWords && Hq == Hkv * gsrq::kRep;
 }
 
-// Launch `kernel` so that it may be scheduled while the previous kernel of the stream drains
-// (the kernel itself waits, see wait_for_previous_kernel).
-template <typename... Params, typename... Args>
-static cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                    Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-}
-
 static size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 struct GsrqWorkspace {  // offsets into the caller's scratch; slot index = pair + scan block
@@ -1019,11 +996,11 @@ int attn_gsrq_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vc
     const unsigned long long epoch = g_epoch.fetch_add(2, std::memory_order_relaxed);  // odd, so never 0 (= cleared)
     GsrqNewToken token = {};
     if (fresh) token = *fresh;
-    cudaError_t e = launch_dependent(gsrq::attn_gsrq_prepare_kernel, dim3(2 * B * Hkv), dim3(gsrq::kPrepThreads), 0, stream, q,
+    cudaError_t e = launch_dependent(true, gsrq::attn_gsrq_prepare_kernel, dim3(2 * B * Hkv), dim3(gsrq::kPrepThreads), 0, stream, q,
                                      ktab, vtab, lut, scale, (uint4 *)(base + ws.vperm), B, Hkv, token);
     int st = e == cudaSuccess ? launch_status() : (int)e;
     if (st != TACVQ_OK) return st;
-    e = launch_dependent(gsrq::attn_gsrq_scan_kernel, dim3(sms), dim3(gsrq::kThreads), gsrq::kSmemBytes, stream, kcodes, vcodes,
+    e = launch_dependent(true, gsrq::attn_gsrq_scan_kernel, dim3(sms), dim3(gsrq::kThreads), gsrq::kSmemBytes, stream, kcodes, vcodes,
                          (const uint2 *)lut, (const float *)scale, vtab, (const uint4 *)(base + ws.vperm), seq_start, seq_end, part, marks, out,
                          state_out, B, Hkv, (int)T_cap, epoch);
     return e == cudaSuccess ? launch_status() : (int)e;

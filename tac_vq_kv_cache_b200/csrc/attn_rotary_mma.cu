@@ -138,6 +138,9 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
     const int rep = Hq / Hkv;  // 1, 2 or 4 query heads per KV head
     const int b0 = (int)((int64_t)blockIdx.z * B / gridDim.z), n_rows = (int)((int64_t)(blockIdx.z + 1) * B / gridDim.z) - b0;
 
+    // A decode step's new codes and ranges come from the kernel before this one; the tables and the query do not.
+    copy_tables(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, tid);
+    wait_for_previous_kernel();
     // positions that some row of the block sees, and this split's share of them
     int lo_all = 0x7fffffff, hi_all = 0;
     for (int r = 0; r < n_rows; ++r) {
@@ -156,12 +159,12 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
             const int r = idx / (kDim + 2), col = idx % (kDim + 2);
             part[((int64_t)split * rows + (int64_t)(b0 + r / rep) * Hq + h * rep + r % rep) * (kDim + 2) + col] = col == 0 ? -INFINITY : 0.0f;
         }
+        cp_async_wait_all();  // no copy outlives the block
         return;
     }
     const size_t row_step = (size_t)Hkv * (size_t)T_cap * 32;  // code bytes from one batch row to the next
     const size_t code_at = (((size_t)b0 * Hkv + h) * (size_t)T_cap + chunk) * 32;
 
-    copy_tables(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, tid);
     if (tid < n_rows) {
         const int lo = seq_start ? max(seq_start[b0 + tid], 0) : 0;
         const int hi = seq_end ? min(seq_end[b0 + tid], (int)T_cap) : (int)T_cap;
@@ -481,13 +484,13 @@ bool attn_rotary_mma_supported(int Hq, int Hkv, int D, int G, int S, int K) {
 template <int R>
 static int launch_rotary_mma(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
                              const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
-                             int Hkv, int64_t T_cap, int splits, cudaStream_t stream) {
+                             int Hkv, int64_t T_cap, int splits, bool after_prologue, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(rotmma::attn_rotary_mma_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, rotmma::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     dim3 grid((unsigned)splits, (unsigned)Hkv, (unsigned)((B + R - 1) / R));
-    rotmma::attn_rotary_mma_kernel<R><<<grid, rotmma::kThreads, rotmma::kSmemBytes, stream>>>(q, kcodes, vcodes, ktab, vtab, rope, seq_start,
-                                                                                             seq_end, part, B, Hq, Hkv, T_cap, splits);
-    return launch_status();
+    e = launch_dependent(after_prologue, rotmma::attn_rotary_mma_kernel<R>, grid, dim3(rotmma::kThreads), rotmma::kSmemBytes, stream, q, kcodes,
+                         vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, splits);
+    return e == cudaSuccess ? launch_status() : (int)e;
 }
 
 // Partial states [split][B*Hq][2 + D] for attn_combine_kernel; *splits is how many (0: `visible` positions are too many for
@@ -495,13 +498,14 @@ static int launch_rotary_mma(const __half *q, const uint8_t *kcodes, const uint8
 // the batch together span more.
 int attn_rotary_mma_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
                              const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
-                             int Hkv, int64_t T_cap, int64_t visible, int sms, int *splits, cudaStream_t stream) {
+                             int Hkv, int64_t T_cap, int64_t visible, int sms, bool after_prologue, int *splits,
+                             cudaStream_t stream) {
     const rotmma::Plan plan = rotmma::plan(B, Hkv, visible, sms);
     *splits = plan.splits;
     switch (plan.rows) {
-        case 1: return launch_rotary_mma<1>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, stream);
-        case 2: return launch_rotary_mma<2>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, stream);
-        case 4: return launch_rotary_mma<4>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, stream);
+        case 1: return launch_rotary_mma<1>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, after_prologue, stream);
+        case 2: return launch_rotary_mma<2>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, after_prologue, stream);
+        case 4: return launch_rotary_mma<4>(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, plan.splits, after_prologue, stream);
         default: return TACVQ_OK;
     }
 }

@@ -144,6 +144,28 @@ struct GsrqNewToken {
     long long position, T_cap;
 };
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may start before its predecessor has finished; it must
+// not read the predecessor's results, nor overwrite what that reads, before it has waited.  A predecessor that lets it start early
+// calls launch_dependents.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 inline int launch_status() {
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TACVQ_OK : static_cast<int>(e);

@@ -230,7 +230,7 @@ decode_prologue_kernel(const XT *__restrict__ k_rows, const XT *__restrict__ v_r
                        const __half *__restrict__ ktab, const __half *__restrict__ vtab, uint8_t *__restrict__ kcodes,
                        uint8_t *__restrict__ vcodes, int32_t *__restrict__ seq_start, int32_t *__restrict__ seq_end, int start,
                        int end, int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    launch_dependents();
     if (blockIdx.x == 0) {
         for (int b = threadIdx.x; b < B; b += blockDim.x) {
             seq_start[b] = start;

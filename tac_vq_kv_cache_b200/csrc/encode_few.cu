@@ -195,6 +195,7 @@ encode_few_wide_kernel(FewSide first, FewSide second, int64_t sxb, int64_t sxh, 
                          : "=r"(ok) : "r"(bar0 + slot * 8), "r"((uint32_t)phase) : "memory");
         return ok != 0;
     };
+    if (seq_start != nullptr) launch_dependents();  // a decode step: its attention is next, and waits for this grid where it has to
     if (tid == 0) {
         for (int i = 0; i < ring; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + i * 8) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
