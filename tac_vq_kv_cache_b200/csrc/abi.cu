@@ -24,12 +24,11 @@ int attn_generic_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t 
                           int Hq, int Hkv, int D, int G, int S, int K, int64_t T_cap, int splits, cudaStream_t stream);
 int attn_combine_dispatch(const float *states, int n_parts, __half *out, float *merged, int64_t rows, int D,
                           cudaStream_t stream);
-bool attn_fullwidth_supported(int Hq, int Hkv, int D, int G, int S, int K);
-int attn_fullwidth_splits(int B, int Hkv, int64_t T_cap, int sms);
-int attn_fullwidth_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab,
-                            const __half *vtab, const int32_t *seq_start, const int32_t *seq_end, float *part,
-                            __half *out, float *state_out, int B, int Hq, int Hkv, int S, int64_t T_cap, int splits,
-                            cudaStream_t stream);
+bool attn_slots_supported(int B, int Hq, int Hkv, int D, int G, int S, int K);
+int attn_slots_splits(int B, int Hq, int Hkv, int G, int S, int64_t visible, int sms);
+int attn_slots_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
+                        const int32_t *seq_start, const int32_t *seq_end, float *part, __half *out, float *state_out, int B, int Hq,
+                        int Hkv, int G, int S, int64_t T_cap, int splits, bool after_prologue, cudaStream_t stream);
 bool attn_gsrq_supported(int Hq, int Hkv, int D, int G, int S, int K);
 size_t attn_gsrq_workspace_bytes(int B, int Hq, int Hkv, int D, int sms);
 int attn_gsrq_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab,
@@ -293,10 +292,11 @@ size_t tacvq_attn_workspace_bytes(int B, int Hq, int Hkv, int D, int G, int S) {
     return (need + 255) & ~(size_t)255;
 }
 
-int tacvq_attn_decode(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
-                      const uint16_t *vtab_f16, const int32_t *seq_start, const int32_t *seq_end, void *workspace,
-                      size_t workspace_bytes, uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv, int D,
-                      int G, int S, int K, int64_t T_cap, tacvq_stream_t stream) {
+// `visible`: the most positions that a row sees, as far as the host knows (T_cap otherwise).
+static int attn_decode(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
+                       const uint16_t *vtab_f16, const int32_t *seq_start, const int32_t *seq_end, void *workspace,
+                       size_t workspace_bytes, uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv, int D, int G, int S, int K,
+                       int64_t T_cap, int64_t visible, bool after_prologue, tacvq_stream_t stream) {
     if (!q_f16 || !kcodes || !vcodes || !ktab_f16 || !vtab_f16) return TACVQ_ERR_NULL;
     if (!out_f16 && !state_out) return TACVQ_ERR_NULL;
     const int g = check_attn_geometry(B, Hq, Hkv, D, G, S, K);
@@ -306,42 +306,35 @@ int tacvq_attn_decode(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_
         return TACVQ_ERR_WORKSPACE;
     if ((((uintptr_t)kcodes | (uintptr_t)vcodes) & 15) != 0) return TACVQ_ERR_ALIGN;
     cudaStream_t s = (cudaStream_t)stream;
-    if (attn_gsrq_supported(Hq, Hkv, D, G, S, K) && gsrq_batch_ok(B, Hkv) && gsrq_aligned(q_f16, ktab_f16, vtab_f16)) {
-        const int fast = attn_gsrq_dispatch((const __half *)q_f16, kcodes, vcodes, (const __half *)ktab_f16,
-                                            (const __half *)vtab_f16, seq_start, seq_end, workspace, (__half *)out_f16,
-                                            state_out, B, Hq, Hkv, T_cap, sm_count(), s);
-        if (fast != TACVQ_ERR_UNSUPPORTED) return fast;  // sizes beyond the specialised scan: the generic kernel below
+    const __half *q = (const __half *)q_f16, *ktab = (const __half *)ktab_f16, *vtab = (const __half *)vtab_f16;
+    const bool aligned = (((uintptr_t)q_f16 | (uintptr_t)ktab_f16 | (uintptr_t)vtab_f16) & 15) == 0;  // the generic kernel takes any place
+    if (aligned && attn_gsrq_supported(Hq, Hkv, D, G, S, K) && gsrq_batch_ok(B, Hkv)) {
+        const int fast = attn_gsrq_dispatch(q, kcodes, vcodes, ktab, vtab, seq_start, seq_end, workspace, (__half *)out_f16, state_out, B, Hq,
+                                            Hkv, T_cap, sm_count(), s);
+        if (fast != TACVQ_ERR_UNSUPPORTED) return fast;  // sizes beyond the specialised scan: the kernels below
     }
-    int splits = attn_generic_splits(B, Hkv, T_cap, sm_count());
-    if (attn_fullwidth_supported(Hq, Hkv, D, G, S, K) && (((uintptr_t)ktab_f16 | (uintptr_t)vtab_f16) & 15) == 0) {
-        splits = attn_fullwidth_splits(B, Hkv, T_cap, sm_count());
-        if (splits <= kGenericMaxSplits) {
-            // a single block per pair writes the result itself; several blocks leave partial states to merge
-            int fw = attn_fullwidth_dispatch((const __half *)q_f16, kcodes, vcodes, (const __half *)ktab_f16,
-                                             (const __half *)vtab_f16, seq_start, seq_end, (float *)workspace,
-                                             (__half *)out_f16, state_out, B, Hq, Hkv, S, T_cap, splits, s);
-            if (fw != TACVQ_OK || splits == 1) return fw;
-            return attn_combine_dispatch((const float *)workspace, splits, (__half *)out_f16, state_out, (int64_t)B * Hq, D, s);
-        }
+    float *part = (float *)workspace;
+    int splits, st;
+    if (aligned && attn_slots_supported(B, Hq, Hkv, D, G, S, K)) {
+        // a single block per row and head writes the result itself; several blocks leave partial states to merge
+        splits = attn_slots_splits(B, Hq, Hkv, G, S, visible, sm_count());
+        st = attn_slots_dispatch(q, kcodes, vcodes, ktab, vtab, seq_start, seq_end, part, (__half *)out_f16, state_out, B, Hq, Hkv, G, S, T_cap,
+                                 splits, after_prologue, s);
+        if (splits == 1) return st;
+    } else {
         splits = attn_generic_splits(B, Hkv, T_cap, sm_count());
+        st = attn_generic_dispatch(q, kcodes, vcodes, ktab, vtab, seq_start, seq_end, part, B, Hq, Hkv, D, G, S, K, T_cap, splits, s);
     }
-    if (attn_rotary_staged_supported(Hq, Hkv, D, G, S, K) && (((uintptr_t)ktab_f16 | (uintptr_t)vtab_f16) & 15) == 0) {
-        // head_dim 128 in pieces of 8 channels, at most two stages (e.g. one-stage grouped CQ): score table and
-        // value tables in shared memory, two passes (the staged kernel of attn_rotary.cu without its rotary step)
-        const int staged = attn_rotary_staged_splits(B, Hkv, T_cap, sm_count());
-        if (staged > 0) {
-            int st = attn_rotary_staged_dispatch((const __half *)q_f16, kcodes, vcodes, (const __half *)ktab_f16,
-                                                 (const __half *)vtab_f16, nullptr, seq_start, seq_end, (float *)workspace,
-                                                 B, Hq, Hkv, G, S, T_cap, staged, s);
-            if (st != TACVQ_OK) return st;
-            return attn_combine_dispatch((const float *)workspace, staged, (__half *)out_f16, state_out, (int64_t)B * Hq, D, s);
-        }
-    }
-    int st = attn_generic_dispatch((const __half *)q_f16, kcodes, vcodes, (const __half *)ktab_f16,
-                                   (const __half *)vtab_f16, seq_start, seq_end, (float *)workspace, B, Hq, Hkv, D, G,
-                                   S, K, T_cap, splits, s);
     if (st != TACVQ_OK) return st;
-    return attn_combine_dispatch((const float *)workspace, splits, (__half *)out_f16, state_out, (int64_t)B * Hq, D, s);
+    return attn_combine_dispatch(part, splits, (__half *)out_f16, state_out, (int64_t)B * Hq, D, s);
+}
+
+int tacvq_attn_decode(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
+                      const uint16_t *vtab_f16, const int32_t *seq_start, const int32_t *seq_end, void *workspace,
+                      size_t workspace_bytes, uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv, int D,
+                      int G, int S, int K, int64_t T_cap, tacvq_stream_t stream) {
+    return attn_decode(q_f16, kcodes, vcodes, ktab_f16, vtab_f16, seq_start, seq_end, workspace, workspace_bytes, out_f16, state_out, B, Hq,
+                       Hkv, D, G, S, K, T_cap, T_cap, false, stream);
 }
 
 int tacvq_rope_table(uint16_t *table_f16, int64_t T, int D, double theta, int64_t first_position, tacvq_stream_t stream) {
@@ -456,8 +449,8 @@ static int decode_step(const tacvq_step_plan &p, const uint16_t *q_f16, const vo
         return attn_decode_rotary(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.rope_table_f16, p.seq_start, p.seq_end,
                                   p.workspace, p.workspace_bytes, out_f16, state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K, p.T_cap,
                                   end - start, one_launch, stream);
-    return tacvq_attn_decode(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.seq_start, p.seq_end, p.workspace,
-                             p.workspace_bytes, out_f16, state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K, p.T_cap, stream);
+    return attn_decode(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.seq_start, p.seq_end, p.workspace, p.workspace_bytes, out_f16,
+                       state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K, p.T_cap, end - start, one_launch, stream);
 }
 
 int tacvq_decode_step_planned(const tacvq_step_plan *plan, const uint16_t *q_f16, const void *k_rows, const void *v_rows,

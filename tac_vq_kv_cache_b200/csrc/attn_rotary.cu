@@ -306,13 +306,10 @@ static int rotary_dpl(const __half *q, const uint8_t *kcodes, const uint8_t *vco
 constexpr int kRotBigThreads = TACVQ_ROT_THREADS;
 constexpr int kRotChunk = 4096;
 
-// ROTARY = false: the same two passes without the rotary step.  The key pass then needs no key rows at
-// all: the block first fills the table area with scores, lut[stage][code][piece] = q_r . (8 channels of the
-// word), r < REP, and a token's score is the sum of its S x 16 entries.
 // NARROW = true: one stage of 32 groups of 4 channels.  A lane's eight channels are then two whole words of
-// neighbouring groups; tables and score table are stored [code][group] (8-byte words, 16-byte scores) and the
+// neighbouring groups; the tables are stored [code][group] (8-byte words) and the
 // lane's two codes take the place of the two stage codes.
-template <int REP, bool ROTARY, bool NARROW>
+template <int REP, bool NARROW>
 __global__ void __launch_bounds__(kRotBigThreads, 1)
 attn_rotary_staged_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcodes, const uint8_t *__restrict__ vcodes,
                           const __half *__restrict__ ktab, const __half *__restrict__ vtab, const __half *__restrict__ rope,
@@ -321,7 +318,7 @@ attn_rotary_staged_kernel(const __half *__restrict__ q, const uint8_t *__restric
     constexpr int D = 128, K = 256, kWarps = kRotBigThreads / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint4 *tab = reinterpret_cast<uint4 *>(smem_raw);                                   // [S][256][16]
-    const size_t table_bytes = NARROW ? (ROTARY ? (size_t)K * 32 * 8 : (size_t)K * 32 * 16) : (size_t)S * K * 16 * 16;
+    const size_t table_bytes = NARROW ? (size_t)K * 32 * 8 : (size_t)S * K * 16 * 16;
     float *score = reinterpret_cast<float *>(smem_raw + table_bytes);                   // [kRotChunk][REP]
     float *red = score + (size_t)kRotChunk * REP;                                       // [kWarps][REP], later merge scratch
 
@@ -355,52 +352,6 @@ attn_rotary_staged_kernel(const __half *__restrict__ q, const uint8_t *__restric
                 const int g = (8 * p) / d, off = (8 * p) % d;
                 tab[idx] = __ldg(reinterpret_cast<const uint4 *>(src + ((((int64_t)h * S + s) * G + g) * K + code) * d + off));
             }
-        }
-    };
-    auto build_score_table = [&]() {  // ROTARY = false only; the query rows sit at the start of the score area
-        float *q_s = score;
-        for (int i = tid; i < REP * D; i += kRotBigThreads)
-            q_s[i] = __half2float(q[((int64_t)b * Hq + h * REP + i / D) * D + i % D]);
-        __syncthreads();
-        float4 *lut = reinterpret_cast<float4 *>(tab);
-        if constexpr (NARROW) {
-            for (int idx = tid; idx < K * 32; idx += kRotBigThreads) {
-                const int g = idx & 31, code = idx >> 5;
-                const uint2 w = __ldg(reinterpret_cast<const uint2 *>(ktab + (((int64_t)h * G + g) * K + code) * 4));
-                const __half2 *hp = reinterpret_cast<const __half2 *>(&w);
-                float dot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const float2 f = __half22float2(hp[i]);
-#pragma unroll
-                    for (int r = 0; r < REP; ++r)
-                        dot[r] = fmaf(q_s[r * D + 4 * g + 2 * i + 1], f.y, fmaf(q_s[r * D + 4 * g + 2 * i], f.x, dot[r]));
-                }
-                lut[idx] = make_float4(dot[0], dot[1], dot[2], dot[3]);
-            }
-            return;
-        }
-        // the block size is a multiple of 16, so a thread meets the same piece p on every trip: its query
-        // channels are read once
-        const int p = tid & 15;
-        const int g = (8 * p) / d, off = (8 * p) % d;
-        float qp[REP][8];
-#pragma unroll
-        for (int r = 0; r < REP; ++r)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) qp[r][i] = q_s[r * D + 8 * p + i];
-        for (int idx = tid; idx < S * K * 16; idx += kRotBigThreads) {
-            const int code = (idx >> 4) & 255, s = idx >> 12;
-            const uint4 w = __ldg(reinterpret_cast<const uint4 *>(ktab + ((((int64_t)h * S + s) * G + g) * K + code) * d + off));
-            const __half2 *hp = reinterpret_cast<const __half2 *>(&w);
-            float dot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 f = __half22float2(hp[i]);
-#pragma unroll
-                for (int r = 0; r < REP; ++r) dot[r] = fmaf(qp[r][2 * i + 1], f.y, fmaf(qp[r][2 * i], f.x, dot[r]));
-            }
-            lut[idx] = make_float4(dot[0], dot[1], dot[2], dot[3]);
         }
     };
     // This lane's eight channels of a token from the resident tables, as the fp16 row the reference
@@ -439,12 +390,10 @@ attn_rotary_staged_kernel(const __half *__restrict__ q, const uint8_t *__restric
     };
 
     float qv[REP][8];
-    if constexpr (ROTARY) {
 #pragma unroll
-        for (int r = 0; r < REP; ++r)
+    for (int r = 0; r < REP; ++r)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) qv[r][i] = __half2float(q[((int64_t)b * Hq + h * REP + r) * D + c0 + i]);
-    }
+        for (int i = 0; i < 8; ++i) qv[r][i] = __half2float(q[((int64_t)b * Hq + h * REP + r) * D + c0 + i]);
     float m[REP], l[REP], acc[REP][8];  // the sums are only live in the value pass: registers for the key pass
 #pragma unroll
     for (int r = 0; r < REP; ++r) m[r] = -INFINITY;
@@ -453,8 +402,7 @@ attn_rotary_staged_kernel(const __half *__restrict__ q, const uint8_t *__restric
     const int n = hi - lo;  // at most kRotChunk: the launcher picks the split count for that
 
     if (n > 0) {
-        if constexpr (ROTARY) load_tables(ktab);
-        else build_score_table();
+        load_tables(ktab);
         __syncthreads();
         // ---- pass K: scores of the chunk ------------------------------------------------------------
         int code_next[2];
@@ -462,10 +410,8 @@ attn_rotary_staged_kernel(const __half *__restrict__ q, const uint8_t *__restric
         {
             const int t = chunk + min(2 * warp + sub, n - 1);
             fetch_codes(kcodes + (code_row + t) * slots, code_next);
-            if constexpr (ROTARY) {
-                cos_next = __ldg(reinterpret_cast<const uint4 *>(rope + (int64_t)t * D + f0));
-                sin_next = __ldg(reinterpret_cast<const uint4 *>(rope + (int64_t)t * D + D / 2 + f0));
-            }
+            cos_next = __ldg(reinterpret_cast<const uint4 *>(rope + (int64_t)t * D + f0));
+            sin_next = __ldg(reinterpret_cast<const uint4 *>(rope + (int64_t)t * D + D / 2 + f0));
         }
         for (int base = 0; base < n; base += 2 * kWarps) {
             const int local = base + 2 * warp + sub;  // lanes past the end redo the last token and drop it
@@ -474,43 +420,22 @@ attn_rotary_staged_kernel(const __half *__restrict__ q, const uint8_t *__restric
             if (base + 2 * kWarps < n) {
                 const int t = chunk + min(local + 2 * kWarps, n - 1);
                 fetch_codes(kcodes + (code_row + t) * slots, code_next);
-                if constexpr (ROTARY) {
-                    cos_next = __ldg(reinterpret_cast<const uint4 *>(rope + (int64_t)t * D + f0));
-                    sin_next = __ldg(reinterpret_cast<const uint4 *>(rope + (int64_t)t * D + D / 2 + f0));
-                }
+                cos_next = __ldg(reinterpret_cast<const uint4 *>(rope + (int64_t)t * D + f0));
+                sin_next = __ldg(reinterpret_cast<const uint4 *>(rope + (int64_t)t * D + D / 2 + f0));
             }
             float sc[REP];
-            if constexpr (ROTARY) {
-                __half2 krow[4];
-                rebuild8(code_now, krow);
-                const __half2 *cosv = reinterpret_cast<const __half2 *>(&cos_now), *sinv = reinterpret_cast<const __half2 *>(&sin_now);
+            __half2 krow[4];
+            rebuild8(code_now, krow);
+            const __half2 *cosv = reinterpret_cast<const __half2 *>(&cos_now), *sinv = reinterpret_cast<const __half2 *>(&sin_now);
 #pragma unroll
-                for (int r = 0; r < REP; ++r) sc[r] = 0.0f;
+            for (int r = 0; r < REP; ++r) sc[r] = 0.0f;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const __half2 other = __shfl_xor_sync(0xffffffffu, krow[i], 8);
-                    const __half2 turned = upper ? other : __hneg2(other);
-                    const float2 kf = __half22float2(__hadd2(__hmul2(krow[i], cosv[i]), __hmul2(turned, sinv[i])));
+            for (int i = 0; i < 4; ++i) {
+                const __half2 other = __shfl_xor_sync(0xffffffffu, krow[i], 8);
+                const __half2 turned = upper ? other : __hneg2(other);
+                const float2 kf = __half22float2(__hadd2(__hmul2(krow[i], cosv[i]), __hmul2(turned, sinv[i])));
 #pragma unroll
-                    for (int r = 0; r < REP; ++r) sc[r] = fmaf(qv[r][2 * i + 1], kf.y, fmaf(qv[r][2 * i], kf.x, sc[r]));
-                }
-            } else {
-                const float4 *lut = reinterpret_cast<const float4 *>(tab);
-                float4 e;
-                if constexpr (NARROW) {
-                    e = lut[code_now[0] * 32 + 2 * l16];
-                    const float4 e1 = lut[code_now[1] * 32 + 2 * l16 + 1];
-                    e = make_float4(e.x + e1.x, e.y + e1.y, e.z + e1.z, e.w + e1.w);
-                } else {
-                    e = lut[code_now[0] * 16 + l16];
-                    if (S > 1) {
-                        const float4 e1 = lut[(K + code_now[1]) * 16 + l16];
-                        e = make_float4(e.x + e1.x, e.y + e1.y, e.z + e1.z, e.w + e1.w);
-                    }
-                }
-                const float ev[4] = {e.x, e.y, e.z, e.w};
-#pragma unroll
-                for (int r = 0; r < REP; ++r) sc[r] = ev[r];
+                for (int r = 0; r < REP; ++r) sc[r] = fmaf(qv[r][2 * i + 1], kf.y, fmaf(qv[r][2 * i], kf.x, sc[r]));
             }
             // sum over the token's 16 lanes; with 4 or 2 heads the lanes first trade heads, so that fewer
             // values travel: head (bit 3, bit 2) of the lane index ends up in the lanes with those bits
@@ -643,12 +568,11 @@ static int launch_rotary_staged(const __half *q, const uint8_t *kcodes, const ui
                                 float *part, int B, int Hq, int Hkv, int G, int S, int64_t T_cap, int splits,
                                 cudaStream_t stream) {
     const bool narrow = G == 32;
-    const size_t tables = narrow ? (rope != nullptr ? (size_t)256 * 32 * 8 : (size_t)256 * 32 * 16) : (size_t)S * 256 * 16 * 16;
+    const size_t tables = narrow ? (size_t)256 * 32 * 8 : (size_t)S * 256 * 16 * 16;
     const size_t merge = ((size_t)(kRotBigThreads / 16) * REP + (size_t)(kRotBigThreads / 16) * REP * 128) * sizeof(float);
     size_t smem = tables + ((size_t)kRotChunk * REP + (size_t)(kRotBigThreads / 32) * REP) * sizeof(float);
     if (smem < merge) smem = merge;
-    auto kernel = narrow ? (rope != nullptr ? attn_rotary_staged_kernel<REP, true, true> : attn_rotary_staged_kernel<REP, false, true>)
-                         : (rope != nullptr ? attn_rotary_staged_kernel<REP, true, false> : attn_rotary_staged_kernel<REP, false, false>);
+    auto kernel = narrow ? attn_rotary_staged_kernel<REP, true> : attn_rotary_staged_kernel<REP, false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     dim3 grid((unsigned)splits, (unsigned)Hkv, (unsigned)B);

@@ -133,6 +133,40 @@ def test_two_pass_kernel_for_head_dim_128_geometries(device, b, hq, hkv, t, grou
         assert bool((out.cpu()[dead] == 0).all()) and bool((state.cpu()[dead][..., 1:] == 0).all())
 
 
+@pytest.mark.parametrize(
+    "b,hq,hkv,t,groups,stages,sub,order",
+    [
+        (1, 4, 1, 33000, 1, 1, 128, "random"),   # one slot, eight copies of the tables; bins folded because they could overflow
+        (1, 2, 2, 2047, 1, 3, 128, "rising"),    # slots that are no power of two, the reference score grows in every segment
+        (2, 8, 2, 4099, 1, 5, 128, "falling"),   # a first token far above the rest: small weights
+        (1, 4, 2, 5000, 2, 4, 64, "rising"),     # eight slots
+        (2, 4, 1, 1025, 4, 3, 32, "random"),     # twelve
+        (1, 8, 2, 513, 8, 3, 16, "falling"),     # 24: two heads a block
+        (3, 4, 2, 9001, 16, 2, 8, "rising"),     # 32, two query heads per KV head
+        (9, 4, 2, 700, 32, 1, 4, "falling"),     # 4-wide words, a row per block
+        (2, 8, 2, 6000, 1, 16, 128, "falling"),
+    ],
+)
+def test_tables_of_up_to_32_slots(device, b, hq, hkv, t, groups, stages, sub, order):
+    """Every rounding of the slot count, rows that end inside a segment, and scores in an order that moves the softmax reference."""
+    q, kcodes, vcodes, ktab, vtab = _workload(t + stages, b, hq, hkv, t, groups, stages, sub, [0.3 * 0.8**s for s in range(stages)] if sub >= 16 else None)
+    if order != "random":
+        q = q * 3  # logits over a range of about ten
+        for row in range(b):
+            for h in range(hkv):
+                score = torch.zeros(t)
+                for s in range(stages):
+                    for g in range(groups):
+                        score += (ktab[h, s, g].float() @ q[row, h * (hq // hkv), g * sub : (g + 1) * sub].float())[kcodes[row, h, :, s, g].long()]
+                kcodes[row, h] = kcodes[row, h, score.argsort(descending=order == "falling")]
+    start, end = [5 * i for i in range(b)], [t - 3 * i for i in range(b)]
+    work = (q, kcodes, vcodes, ktab, vtab)
+    out, state = _run(device, work, start, end, want_state=True)
+    want, want_state = C.attention(*work, start, end)
+    _check(out, want)
+    _check_state(state.cpu(), want_state)
+
+
 def test_partial_states_merge_to_the_whole(device):
     """Sequence split as ranks would do it: per-range states, then the log-sum-exp merge."""
     ops = _ops()
