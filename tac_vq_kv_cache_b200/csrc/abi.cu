@@ -52,6 +52,10 @@ int attn_rotary_mma_dispatch(const __half *q, const uint8_t *kcodes, const uint8
                              const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
                              int Hkv, int64_t T_cap, int64_t visible, int sms, bool after_prologue, int *splits,
                              cudaStream_t stream);
+bool attn_rotary_ladder_supported(int Hq, int Hkv, int D, int G, int S, int K);
+int attn_rotary_ladder_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
+                                const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
+                                int Hkv, int S, int64_t T_cap, int64_t visible, const LadderStep &step, int *splits, cudaStream_t stream);
 int rope_table_dispatch(__half *table, int64_t tokens, int D, double theta, int64_t first, cudaStream_t stream);
 int attn_rotary_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab,
                          const __half *vtab, const __half *rope, const int32_t *seq_start, const int32_t *seq_end,
@@ -350,7 +354,7 @@ int tacvq_rope_table(uint16_t *table_f16, int64_t T, int D, double theta, int64_
 static int attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
                               const uint16_t *vtab_f16, const uint16_t *rope_table, const int32_t *seq_start, const int32_t *seq_end,
                               void *workspace, size_t workspace_bytes, uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv,
-                              int D, int G, int S, int K, int64_t T_cap, int64_t visible, bool after_prologue, tacvq_stream_t stream) {
+                              int D, int G, int S, int K, int64_t T_cap, int64_t visible, const LadderStep &step, tacvq_stream_t stream) {
     if (!q_f16 || !kcodes || !vcodes || !ktab_f16 || !vtab_f16 || !rope_table) return TACVQ_ERR_NULL;
     if (!out_f16 && !state_out) return TACVQ_ERR_NULL;
     const int g = check_attn_geometry(B, Hq, Hkv, D, G, S, K);
@@ -367,7 +371,10 @@ static int attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, cons
     if ((((uintptr_t)ktab_f16 | (uintptr_t)vtab_f16 | (uintptr_t)rope_table) & 15) == 0) {
         if (attn_rotary_mma_supported(Hq, Hkv, D, G, S, K) && (((uintptr_t)kcodes | (uintptr_t)vcodes | (uintptr_t)q_f16) & 15) == 0) {
             st = attn_rotary_mma_dispatch(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, T_cap, visible,
-                                          sm_count(), after_prologue, &splits, s);
+                                          sm_count(), step.fresh != 0, &splits, s);
+        } else if (attn_rotary_ladder_supported(Hq, Hkv, D, G, S, K) && (((uintptr_t)kcodes | (uintptr_t)q_f16) & 3) == 0) {
+            st = attn_rotary_ladder_dispatch(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, S, T_cap, visible,
+                                             step, &splits, s);
         } else if (attn_rotary_staged_supported(Hq, Hkv, D, G, S, K)) {
             splits = attn_rotary_staged_splits(B, Hkv, T_cap, sm_count());
             if (splits > 0)
@@ -389,7 +396,7 @@ int tacvq_attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, const
                              uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv, int D, int G, int S, int K,
                              int64_t T_cap, tacvq_stream_t stream) {
     return attn_decode_rotary(q_f16, kcodes, vcodes, ktab_f16, vtab_f16, rope_table, seq_start, seq_end, workspace, workspace_bytes,
-                              out_f16, state_out, B, Hq, Hkv, D, G, S, K, T_cap, T_cap, false, stream);
+                              out_f16, state_out, B, Hq, Hkv, D, G, S, K, T_cap, T_cap, LadderStep{0, 0, 0}, stream);
 }
 
 int tacvq_set_ranges(int32_t *seq_start, int32_t *seq_end, int B, int start, int end, tacvq_stream_t stream) {
@@ -448,7 +455,7 @@ static int decode_step(const tacvq_step_plan &p, const uint16_t *q_f16, const vo
     if (p.rope_table_f16)
         return attn_decode_rotary(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.rope_table_f16, p.seq_start, p.seq_end,
                                   p.workspace, p.workspace_bytes, out_f16, state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K, p.T_cap,
-                                  end - start, one_launch, stream);
+                                  end - start, LadderStep{start, end, one_launch ? T_new : 0}, stream);
     return attn_decode(q_f16, p.kcodes, p.vcodes, p.ktab_f16, p.vtab_f16, p.seq_start, p.seq_end, p.workspace, p.workspace_bytes, out_f16,
                        state_out, p.B, p.Hq, p.Hkv, p.D, p.G, p.S, p.K, p.T_cap, end - start, one_launch, stream);
 }

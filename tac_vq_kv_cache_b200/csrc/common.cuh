@@ -144,6 +144,12 @@ struct GsrqNewToken {
     long long position, T_cap;
 };
 
+// What the host knows of the decode step that a launch belongs to, when the launch before it is that step's prologue: the range that every
+// row sees, and how many positions at its end have codes that the prologue writes.  fresh = 0: nothing.
+struct LadderStep {
+    int start, end, fresh;
+};
+
 // Programmatic dependent launch: a kernel launched with launch_dependent may start before its predecessor has finished; it must
 // not read the predecessor's results, nor overwrite what that reads, before it has waited.  A predecessor that lets it start early
 // calls launch_dependents.

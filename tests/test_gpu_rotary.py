@@ -129,6 +129,44 @@ def test_rotary_rows_of_a_batch_that_share_positions(device, b, hq, hkv, t, rang
         assert not out[row].any() and (state[row, :, 0] == -float("inf")).all() and not state[row, :, 1:].any()
 
 
+@pytest.mark.parametrize(
+    "b,hq,hkv,stages,t,ranges,peak",
+    [
+        (1, 4, 1, 16, 1, [(0, 1)], 1.0),                                                  # one token, one cluster
+        (1, 8, 2, 4, 17, [(0, 17)], 1.0),                                                 # a tile and a token, four stages
+        (2, 16, 4, 8, 511, [(3, 500), (10, 10)], 1.0),                                    # a row that sees nothing
+        (1, 8, 8, 12, 4097, [(0, 4097)], 1.0),                                            # a token more than a cluster holds at a time
+        (5, 8, 4, 16, 300, [(0, 300), (299, 300), (0, 1), (17, 250), (100, 164)], 1.0),   # more items than clusters, heads change inside one
+        (1, 4, 2, 16, 3000, [(0, 3000)], 12.0),                                           # one token carries most of the weight
+    ],
+)
+def test_rotary_attention_over_deep_ladders(device, b, hq, hkv, stages, t, ranges, peak):
+    """Full-width ladders of 4 to 16 stages; ``peak``: by how much the first token's logit stands out."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(stages * t)
+    kcodes, vcodes = (torch.randint(0, 256, (b, hkv, t, stages, 1), generator=gen, dtype=torch.uint8) for _ in range(2))
+    scales = [0.3 * 0.85**s for s in range(stages)]
+    ktab, vtab = make_tables(gen, hkv, stages, 1, 128, scales), make_tables(gen, hkv, stages, 1, 128, scales)
+    q = (torch.randn(b, hq, 128, generator=gen) / 128**0.5).half()
+    if peak > 1.0:  # queries along the first token's key, which stands at position 0: no rotation
+        key = ktab[:, torch.arange(stages), 0, kcodes[0, :, 0, :, 0].long()][torch.arange(hkv), torch.arange(hkv)].float().sum(1)
+        q = (peak * key / (key * key).sum(-1, keepdim=True)).half().repeat_interleave(hq // hkv, 0)[None].expand(b, -1, -1).contiguous()
+    start, end = [r[0] for r in ranges], [r[1] for r in ranges]
+    live = [i for i in range(b) if end[i] > start[i]]
+    want, m, l, acc = O.attention_over_codes(q[live], kcodes[live], vcodes[live], ktab, vtab, [start[i] for i in live], [end[i] for i in live], rope_theta=1e6)
+    out, state = ops.attn_decode(
+        q.to(device), kcodes.to(device), vcodes.to(device), ktab.to(device), vtab.to(device),
+        torch.tensor(start, dtype=torch.int32, device=device), torch.tensor(end, dtype=torch.int32, device=device),
+        rope=ops.rope_table(t, 128, 1e6, device), want_state=True,
+    )
+    out, state = out.float().cpu(), state.cpu()
+    for i, row in enumerate(live):
+        _check(out[row], want[i])
+    torch.testing.assert_close(state[live][..., 0] + state[live][..., 1].log(), m + l.log(), rtol=0, atol=2e-3)
+    for row in set(range(b)) - set(live):
+        assert not out[row].any() and (state[row, :, 0] == -float("inf")).all() and not state[row, :, 1:].any()
+
+
 def test_code_cache_with_rope_follows_the_reference_decode_loop(device):
     """Prefill + three decode steps through VQCodeCache(rope_theta=...): codes of pre-rotary keys are
     appended in place, the query arrives rotated; compared with the oracle on the cache's own codes."""
