@@ -107,14 +107,16 @@ __device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1,
 // position of the codeword (stage s, group g) inside a code's 512-byte row; the bank is s*4 + g%4 (as in attn_gsrq.cu)
 __device__ __forceinline__ int word_pos(int s, int g) { return (g >> 2) * 8 + s * 4 + (g & 3); }
 
-// A head's tables [stage][group][word][8] -> shared memory rows [word][position]; a warp copies, per trip,
-// 4 neighbouring words of 8 positions with different banks: full 32-byte sectors in, no conflicts out.
-__device__ __forceinline__ void copy_tables(uint32_t tab_u32, const __half *__restrict__ src, int tid) {
+// A head's tables [stage][group][word][8] -> shared memory rows [word][position].  The copies of eight neighbouring lanes go
+// out together: they take two neighbouring words of four positions, whole 32-byte sectors (eight positions of one word, without
+// the two-way conflict on arrival, asked L2 for every sector twice).  Blocks of one head start at different places (`first`), so
+// that they do not all ask for the same lines at the same time.
+__device__ __forceinline__ void copy_tables(uint32_t tab_u32, const __half *__restrict__ src, int tid, int first) {
+#pragma unroll 4
     for (int idx = tid; idx < kWords * 32; idx += kThreads) {
-        const int pos = ((idx >> 5) & 3) * 8 + (idx & 7);
-        const int word = ((idx >> 7) << 2) | ((idx >> 3) & 3);
-        const int s = (pos >> 2) & 1, g = ((pos >> 3) << 2) | (pos & 3);
-        cp_async16(tab_u32 + word * kRowBytes + pos * 16, src + ((size_t)(s * 16 + g) * kWords + word) * 8);
+        const int lane = idx & 31, rest = ((idx >> 5) + (first & 15) * (kThreads / 32)) & 255;
+        const int word = (rest >> 2) * 4 + (lane >> 4) * 2 + (lane & 1), s = (lane >> 3) & 1, g = (rest & 3) * 4 + ((lane >> 1) & 3);
+        cp_async16(tab_u32 + word * kRowBytes + word_pos(s, g) * 16, src + ((size_t)(s * 16 + g) * kWords + word) * 8);
     }
 }
 
@@ -139,7 +141,7 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
     const int b0 = (int)((int64_t)blockIdx.z * B / gridDim.z), n_rows = (int)((int64_t)(blockIdx.z + 1) * B / gridDim.z) - b0;
 
     // A decode step's new codes and ranges come from the kernel before this one; the tables and the query do not.
-    copy_tables(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, tid);
+    copy_tables(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, tid, split);
     wait_for_previous_kernel();
     // positions that some row of the block sees, and this split's share of them
     int lo_all = 0x7fffffff, hi_all = 0;
@@ -269,7 +271,7 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
     __syncthreads();
 
     // ---- softmax over the block's tokens, kRowWarps warps a batch row; value tables arrive meanwhile ---
-    copy_tables(tab_u32, vtab + (size_t)h * 2 * 16 * kWords * 8, tid);
+    copy_tables(tab_u32, vtab + (size_t)h * 2 * 16 * kWords * 8, tid, split);
     const int n_pad = (n + 31) & ~31;
     const int row = warp / kRowWarps, row_warp = warp % kRowWarps;
     const bool row_live = row < n_rows;
