@@ -24,14 +24,6 @@ import torch
 from . import _lib, ops
 
 
-
-def _raw_stream(index: int) -> int:
-    """Handle of torch's current stream on device ``index`` (the quick accessor when this torch has it)."""
-    try:
-        return torch._C._cuda_getCurrentRawStream(index)
-    except AttributeError:  # older or newer torch without the accessor
-        return torch.cuda.current_stream(index).cuda_stream
-
 class VQCodeCache:
     """K and V codes of one layer for a batch of sequences that advance in lockstep."""
 
@@ -157,7 +149,7 @@ class VQCodeCache:
             heads, dim, self.groups, self.stages, words,
         )
         args = (record, query.data_ptr(), raw_key.data_ptr(), raw_value.data_ptr(), ops._DTYPE_TAG[dtype], tokens, self.length, out.data_ptr(),
-                None, _raw_stream(index))
+                None, ops._raw_stream(index))
         if index == torch.cuda.current_device():
             status = _lib.load().tacvq_decode_step_planned(*args)
         else:
@@ -168,11 +160,6 @@ class VQCodeCache:
         self.length += tokens
         self._range_is = self.visible()
         return out
-
-    def _result_fits(self, out: torch.Tensor, query: torch.Tensor) -> bool:
-        """Whether attention may write its result to ``out`` while it reads ``query``."""
-        apart = out.data_ptr() + 2 * out.numel() <= query.data_ptr() or query.data_ptr() + 2 * query.numel() <= out.data_ptr()
-        return apart and out.shape == query.shape and out.dtype == torch.float16 and out.is_contiguous() and out.device == query.device
 
     @staticmethod
     def _result_fits(out: torch.Tensor, query: torch.Tensor) -> bool:
@@ -253,7 +240,7 @@ class VQCodeCache:
         args[3:7] = ktab.data_ptr(), vtab.data_ptr(), codes_k.data_ptr(), codes_v.data_ptr()
         args[9], args[10] = self.length, self.window or 0
         args[24] = 1 if synchronize else 0
-        args[25] = _raw_stream(index)
+        args[25] = ops._raw_stream(index)
         if index == torch.cuda.current_device():
             status = call(*args)
         else:

@@ -66,6 +66,7 @@ class _HardGroupedResidualVQ(torch.autograd.Function):
         ctx.table_dtype = tables.dtype
         ctx.straight_through = bool(straight_through)
         ctx.mark_non_differentiable(codes)
+        ctx.set_materialize_grads(False)  # no zeros in the place of the codes' gradient, or of an exit's that nobody used
         return (*exits, codes)
 
     @staticmethod

@@ -52,15 +52,24 @@ def _ptr(t: torch.Tensor | None) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+def _raw_stream(index: int) -> int:
+    """Handle of torch's current stream on device ``index`` (the quick accessor when this torch has it)."""
+    try:
+        return torch._C._cuda_getCurrentRawStream(index)
+    except AttributeError:  # older or newer torch without the accessor
+        return torch.cuda.current_stream(index).cuda_stream
+
+
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def _rows_view(x: torch.Tensor) -> torch.Tensor:
-    """States usable in place: last axis contiguous and rows 16-byte aligned, else a packed copy."""
+    """States ``[B,H,T,D]`` usable in place: last axis contiguous and rows 16-byte aligned, else a packed copy."""
     if x.dtype not in _DTYPE_TAG:
         raise ValueError("states must be float16 or float32")
-    ok = x.stride(-1) == 1 and x.data_ptr() % 16 == 0 and all((s * x.element_size()) % 16 == 0 for s in x.stride()[:-1])
+    b, h, t, last = x.stride()
+    ok = last == 1 and (x.data_ptr() | (b | h | t) * x.element_size()) & 15 == 0
     return x if ok else x.contiguous()
 
 
