@@ -293,7 +293,8 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     };
     // the norms and seeds of a share of use u's words, by a warp; the first share's also fetches all the words by TMA (or plain
     // copies without a tensor map)
-    auto load_table = [&](uint32_t u, int share) {
+    // (`ahead`: norms of words k_begin + lane and 32 further that are in registers already)
+    auto load_table = [&](uint32_t u, int share, const float *ahead) {
         const int s = (int)(u % (uint32_t)S), buf = (int)(u & 1u);
         const int64_t first = head_words + s * stage_words;
         if (share != 0) {
@@ -311,7 +312,10 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         }
         const int k_begin = share * (kMaxWords / shares), k_end = k_begin + kMaxWords / shares;
         float *nrm = nrms + buf * kMaxWords;
-        if (a.sqnorm != nullptr) {
+        if (ahead != nullptr) {
+            nrm[k_begin + lane] = ahead[0];
+            nrm[k_begin + 32 + lane] = ahead[1];
+        } else if (a.sqnorm != nullptr) {
 #pragma unroll 1
             for (int k = k_begin + lane; k < k_end; k += 32) nrm[k] = k < K ? __ldg(a.sqnorm + first + k) : inf;
         } else {
@@ -349,7 +353,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     };
 #pragma unroll 1
     for (int i = warp; i < 2 * shares; i += GROUPS * 16)
-        if ((uint32_t)(i / shares) < uses) load_table((uint32_t)(i / shares), i % shares);
+        if ((uint32_t)(i / shares) < uses) load_table((uint32_t)(i / shares), i % shares, nullptr);
 
     const int grp = warp >> 4, part = warp & 3, q = (warp >> 2) & 3;
     const int row = part * 32 + lane;                     // of the group's tile
@@ -437,6 +441,17 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             const __half *tab = tabs + (size_t)buf * (L::kTabBytes / 2);
             const float *nrm = nrms + buf * kMaxWords;
             const int64_t first = head_words + s * stage_words;
+            // One group a block: the norms of the next stage's words are asked for here and wait in registers, because the four warps
+            // that fill its buffer hold up the other twelve meanwhile.
+            float ahead[2] = {inf, inf};
+            if constexpr (GROUPS == 1) {
+                if (a.sqnorm != nullptr && q == 0 && !resident && u >= 1 && u + 1 < uses) {
+                    const float *from = a.sqnorm + head_words + (int64_t)((u + 1) % (uint32_t)S) * stage_words;
+                    const int k = part * 64 + lane;
+                    if (k < K) ahead[0] = __ldg(from + k);
+                    if (k + 32 < K) ahead[1] = __ldg(from + k + 32);
+                }
+            }
             {
                 float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // |r|^2 for the margins; the exact one is taken where it decides
 #pragma unroll
@@ -475,7 +490,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                 if (lane == 0) n = atomicAdd(left + ((u - 1) & 1u) * 16 + q * 4 + part, 1u) + 1u;
                 __threadfence_block();
                 n = __shfl_sync(0xffffffffu, n, 0);
-                if (n % (unsigned int)groups == 0u) load_table(u + 1, q * 4 + part);
+                if (n % (unsigned int)groups == 0u) load_table(u + 1, q * 4 + part, GROUPS == 1 && a.sqnorm != nullptr ? ahead : nullptr);
             }
             const float xx = (xxs[0] + xxs[kRows]) + (xxs[2 * kRows] + xxs[3 * kRows]);
             const float *share_tops = cc_tops + buf * 16;
