@@ -62,6 +62,11 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     return d;
 }
 __device__ __forceinline__ void add_shared(uint32_t addr, uint32_t v) { asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {  // two fp32 sums
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -120,6 +125,22 @@ __device__ __forceinline__ void permute_words(uint32_t (&w)[NW], int x) {
     }
 }
 
+// adds a token's weights w[r] at offsets to[r], heads in the lane's order; ALL: none of the block's heads is missing
+template <int P, bool FULL, bool ALL>
+__device__ __forceinline__ void add_weights(const uint32_t (&codes)[Shape<P>::kCodeWords], const uint32_t (&w)[Shape<P>::kHeads],
+                                            const uint32_t (&to)[Shape<P>::kHeads], const uint32_t (&sel)[4], uint32_t lane_xor, int x,
+                                            int slots, int rot, int heads) {
+    constexpr int H = Shape<P>::kHeads;
+#pragma unroll
+    for (int k = 0; k < P; ++k) {
+        if (!FULL && (k ^ x) >= slots) continue;
+        const uint32_t at = (prmt(codes[k >> 2], 0u, sel[k & 3]) | (uint32_t)(k * Shape<P>::kEntry)) ^ lane_xor;
+#pragma unroll
+        for (int r = 0; r < H; ++r)
+            if (ALL || ((r + rot) & (H - 1)) < heads) add_shared(at + to[r], w[r]);
+    }
+}
+
 template <int P, bool FULL>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_slots_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcodes, const uint8_t *__restrict__ vcodes,
@@ -131,7 +152,7 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcod
     extern __shared__ __align__(256) unsigned char smem[];
     float *q_s = reinterpret_cast<float *>(smem + 3 * kAreaBytes);
     float *red = q_s + kQueryFloats;  // [warps][H] maxima, [warps][H] sums
-    const uint32_t lut = smem_u32(smem), hist = lut + kAreaBytes;
+    const uint32_t hist = smem_u32(smem) + kAreaBytes;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rep = Hq / Hkv, head_groups = (rep + H - 1) / H;
@@ -273,38 +294,43 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcod
         }
     };
     int pending = 0;
-    for (int base = lo; base < hi; base += NT * kThreads) {
+#pragma unroll 1
+    for (int base = lo;; base += NT * kThreads) {
+        const bool more = base < hi;
         float sc[NT][H];
         bool grow = false;
+        if (more) {
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            permute_words<NW>(kc[j], x);
+            for (int j = 0; j < NT; ++j) {
+                permute_words<NW>(kc[j], x);
+                unsigned long long pair[H / 2];  // two heads an addition
 #pragma unroll
-            for (int r = 0; r < H; ++r) sc[j][r] = 0.0f;
+                for (int r = 0; r < H / 2; ++r) pair[r] = 0ull;
 #pragma unroll
-            for (int k = 0; k < P; ++k) {
-                if (!FULL && (k ^ x) >= slots) continue;
-                const uint32_t at = ((prmt(kc[j][k >> 2], 0u, sel[k & 3]) | (uint32_t)(k * L::kEntry)) ^ lane_xor) + lut;
-                if constexpr (H == 4) {
-                    float4 e;
-                    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(e.x), "=f"(e.y), "=f"(e.z), "=f"(e.w) : "r"(at));
-                    sc[j][0] += e.x, sc[j][1] += e.y, sc[j][2] += e.z, sc[j][3] += e.w;
-                } else {
-                    float2 e;
-                    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(e.x), "=f"(e.y) : "r"(at));
-                    sc[j][0] += e.x, sc[j][1] += e.y;
+                for (int k = 0; k < P; ++k) {
+                    if (!FULL && (k ^ x) >= slots) continue;
+                    const unsigned char *entry = smem + ((prmt(kc[j][k >> 2], 0u, sel[k & 3]) | (uint32_t)(k * L::kEntry)) ^ lane_xor);
+                    if constexpr (H == 4) {
+                        const ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(entry);
+                        pair[0] = add2(pair[0], e.x);
+                        pair[1] = add2(pair[1], e.y);
+                    } else {
+                        pair[0] = add2(pair[0], *reinterpret_cast<const unsigned long long *>(entry));
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < H; ++r) {
+                    sc[j][r] = __uint_as_float((uint32_t)(pair[r / 2] >> (32 * (r & 1))));
+                    if (base + j * kThreads + tid >= hi) sc[j][r] = -INFINITY;
+                    grow |= sc[j][r] > m[r];
                 }
             }
-#pragma unroll
-            for (int r = 0; r < H; ++r) {
-                if (base + j * kThreads + tid >= hi) sc[j][r] = -INFINITY;
-                grow |= sc[j][r] > m[r];
-            }
+            if (base + NT * kThreads < hi) fetch(kc_row, base + NT * kThreads, kc);
         }
-        if (base + NT * kThreads < hi) fetch(kc_row, base + NT * kThreads, kc);
         // every thread has added its weights of the segment before when this returns
-        if (__syncthreads_or(grow)) {
-            float f[H];
+        const bool grown = __syncthreads_or(grow);
+        float mine = 1.0f;  // what a fold multiplies this thread's bins by, which are all of one head
+        if (grown) {
 #pragma unroll
             for (int r = 0; r < H; ++r) {
                 float v = sc[0][r];
@@ -320,23 +346,18 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcod
                 float top = m[r];
                 for (int w = 0; w < kWarps; ++w) top = fmaxf(top, red[w * H + r]);
                 top = top > m[r] ? top + kHeadroom : m[r];
-                f[r] = top == -INFINITY ? 1.0f : __expf(m[r] - top);  // 0 for the first tokens
+                const float f = top == -INFINITY ? 1.0f : __expf(m[r] - top);  // 0 for the first tokens
                 m[r] = top;
-                l[r] *= f[r];
+                l[r] *= f;
+                mine = (tid & (H - 1)) == r ? f : mine;
             }
-            if (pending > 0) {
-                float mine = f[0];  // a thread's bins are all of one head
-#pragma unroll
-                for (int r = 1; r < H; ++r) mine = (tid & (H - 1)) == r ? f[r] : mine;
-                fold(mine);
-            }
+        }
+        if (grown || !more || pending + NT * kThreads > L::kFold) {
+            if (pending > 0) fold(mine);
             pending = 0;
             __syncthreads();  // bins are empty, maxima are read
-        } else if (pending + NT * kThreads > L::kFold) {
-            fold(1.0f);
-            pending = 0;
-            __syncthreads();
         }
+        if (!more) break;
         pending += NT * kThreads;
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
@@ -348,7 +369,8 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcod
                 const float p = __expf(sc[j][r] - m[r]);
                 l[r] += p;
                 const bool small = p < kBorder;
-                w[r] = __float2uint_rn(p * (small ? kSmall : kLarge));  // a NaN becomes 0, and its sum spoils the result
+                // to the nearest integer by adding 2^23 (a conversion runs at a quarter of the rate); a NaN's sum spoils the result
+                w[r] = __float_as_uint(fmaf(p, small ? kSmall : kLarge, 8388608.0f)) & 0x7fffffu;
                 to[r] = hist + r * 4 + (small ? kAreaBytes : 0);
             }
             if (rot & 1) {
@@ -367,19 +389,11 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcod
                     }
                 }
             }
-#pragma unroll
-            for (int k = 0; k < P; ++k) {
-                if (!FULL && (k ^ x) >= slots) continue;
-                const uint32_t at = (prmt(vc[j][k >> 2], 0u, sel[k & 3]) | (uint32_t)(k * L::kEntry)) ^ lane_xor;
-#pragma unroll
-                for (int r = 0; r < H; ++r)
-                    if (heads == H || ((r + rot) & (H - 1)) < heads) add_shared(at + to[r], w[r]);
-            }
+            if (heads == H) add_weights<P, FULL, true>(vc[j], w, to, sel, lane_xor, x, slots, rot, heads);
+            else add_weights<P, FULL, false>(vc[j], w, to, sel, lane_xor, x, slots, rot, heads);
         }
         if (base + NT * kThreads < hi) fetch(vc_row, base + NT * kThreads, vc);
     }
-    __syncthreads();
-    if (pending > 0) fold(1.0f);
     // the score table is done with: its place takes the folded weights, [code][slot][head]
 #pragma unroll
     for (int i = 0; i < L::kBins; ++i) {
