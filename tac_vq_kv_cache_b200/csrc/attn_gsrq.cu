@@ -37,9 +37,11 @@
 //   prepare  one block per (batch row, KV head, stage): the score table of the pair (q . codeword for
 //            4096 codewords x 4 heads straight from the fp16 K tables, quantised to 13 bits), written to
 //            scratch in the order the scan's shared memory wants; its share of the V codewords in that
-//            order; and, in a decode step, the codes of the pair's new K or V row and the visible ranges.  A build costs about 5 us of a 512-thread
+//            order; and, in a decode step, the codes of the pair's new K or V row and the visible ranges.  Blocks on SMs
+//            without a pair only share the V codewords.  A build costs about 3.5 us of a 512-thread
 //            block per stage (64 values per thread, quarter-rate conversions); building inside the scan
 //            was measured twice and repeats that for every block that enters a pair (3.3 per pair).
+//            It is a chain of latencies: row 1.3 us, two encode stages 0.8 and 1.4, scores 1.4, quantising 2.0.
 //   scan     a persistent grid (one block per SM) walks the flattened (KV head, batch row, 32-token
 //            tile) space; every block gets an equal share of work units.  When it enters a new (batch
 //            row, KV head) pair it copies that pair's score table (64 KB, flat) and, when the head
@@ -208,18 +210,46 @@ constexpr int kPrepCodes = kWords / (2 * kPrepWarps);  // codes per thread
 __global__ void __launch_bounds__(kPrepThreads)
 attn_gsrq_prepare_kernel(const __half *__restrict__ q, const __half *__restrict__ ktab, const __half *__restrict__ vtab,
                          uint2 *__restrict__ lut_g, float *__restrict__ scale_g, uint4 *__restrict__ vperm_g, int B, int Hkv, const NewToken fresh) {
-    __shared__ float red[kPrepWarps * 8 * 32];  // [warp][min x4, max x4][lane]
-    __shared__ float red2[8 * 32];
+    __shared__ float red[kPrepWarps * 8 * kGroups];  // [warp][min x4, max x4][group]
+    __shared__ __align__(16) float low_s[kGroups * kRep], step_s[12];  // smallest entry per group and head; per head 1 / step, step, offset
     launch_dependents();  // the scan may be scheduled as soon as SMs free up; it waits for this grid itself
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int pair = blockIdx.x >> 1, stage = blockIdx.x & 1;
     const int h = pair / B, b = pair % B;
     const int Hq = Hkv * kRep;
     const int g = lane & 15, half = lane >> 4;
+#if TACVQ_GSRQ_VPERM
+    auto permute_values = [&]() {  // this block's share of the V codewords, in the scan's order
+        const int perm_total = Hkv * kWords * kSlots;
+        const int perm_per_block = (perm_total + (int)gridDim.x - 1) / (int)gridDim.x;
+        for (int local = tid; local < perm_per_block; local += kPrepThreads) {
+            const int e = blockIdx.x * perm_per_block + local;
+            if (e < perm_total) {
+                const int hh = e >> 13, code = (e >> 5) & 255, pos = e & 31;
+                const int s = (pos >> 2) & 1, gg = ((pos >> 3) << 2) | (pos & 3);
+                vperm_g[e] = __ldg(reinterpret_cast<const uint4 *>(vtab + ((((size_t)hh * kStages + s) * kGroups + gg) * kWords + code) * kSub));
+            }
+        }
+    };
+    if (pair >= B * Hkv) {  // few pairs: blocks that only share the permutation
+        wait_for_previous_kernel();
+        permute_values();
+        return;
+    }
+#endif
     // A decode step's new token: this block (pair, side = stage) encodes the 16 groups of the pair's new K
     // (side 0) or V (side 1) row, a warp per group, with the arithmetic of the row-at-a-time encode kernel.
     // The words of both stages are requested at once (one memory latency instead of two); the codes are kept
     // in registers and stored after the wait below.  None of these inputs is produced by this chain.
+    // inputs of the table build, which are not produced by the kernels of this chain either
+    const uint4 *tab = reinterpret_cast<const uint4 *>(ktab + (((size_t)h * kStages + stage) * kGroups + g) * kWords * kSub);
+    uint4 raw[kPrepCodes], qraw[kRep];
+    auto fetch_build = [&]() {
+#pragma unroll
+        for (int c = 0; c < kPrepCodes; ++c) raw[c] = __ldg(tab + warp * 2 + half + 2 * kPrepWarps * c);
+#pragma unroll
+        for (int r = 0; r < kRep; ++r) qraw[r] = __ldg(reinterpret_cast<const uint4 *>(q + ((size_t)b * Hq + h * kRep + r) * kDim + g * kSub));
+    };
     int fresh_code[kStages] = {0, 0};
     if (fresh.k_rows != nullptr) {
         static_assert(kPrepWarps == kGroups && kStages == 2 && kWords == 256, "a warp per group, 8 words per lane and stage");
@@ -242,21 +272,26 @@ attn_gsrq_prepare_kernel(const __half *__restrict__ q, const __half *__restrict_
         }
         fresh_code[0] = nearest_of_fetched_words(res, w0, lane);
         {
+            // the chosen word from the lane that has it: a trip to L2 would be 0.4 us of this chain
+            auto either = [](bool second, const uint4 &a, const uint4 &b) {
+                return make_uint4(second ? b.x : a.x, second ? b.y : a.y, second ? b.z : a.z, second ? b.w : a.w);
+            };
+            const bool b5 = (fresh_code[0] & 32) != 0, b6 = (fresh_code[0] & 64) != 0, b7 = (fresh_code[0] & 128) != 0;
+            uint4 mine = either(b7, either(b6, either(b5, w0[0], w0[1]), either(b5, w0[2], w0[3])),
+                                either(b6, either(b5, w0[4], w0[5]), either(b5, w0[6], w0[7])));
+            const int from = fresh_code[0] & 31;
+            mine = make_uint4(__shfl_sync(0xffffffffu, mine.x, from), __shfl_sync(0xffffffffu, mine.y, from),
+                              __shfl_sync(0xffffffffu, mine.z, from), __shfl_sync(0xffffffffu, mine.w, from));
+            fetch_build();
             float c[kSub];
-            unpack8(__ldg(words0 + fresh_code[0]), c);
+            unpack8(mine, c);
 #pragma unroll
             for (int i = 0; i < kSub; ++i) res[i] = __fsub_rn(res[i], c[i]);
         }
         fresh_code[1] = nearest_of_fetched_words(res, w1, lane);
+    } else {
+        fetch_build();
     }
-    // inputs of the table build (q and the K tables) are not produced by the kernels of this chain either
-    const uint4 *tab = reinterpret_cast<const uint4 *>(ktab + (((size_t)h * kStages + stage) * kGroups + g) * kWords * kSub);
-    uint4 raw[kPrepCodes];
-#pragma unroll
-    for (int c = 0; c < kPrepCodes; ++c) raw[c] = __ldg(tab + warp * 2 + half + 2 * kPrepWarps * c);
-    uint4 qraw[kRep];
-#pragma unroll
-    for (int r = 0; r < kRep; ++r) qraw[r] = __ldg(reinterpret_cast<const uint4 *>(q + ((size_t)b * Hq + h * kRep + r) * kDim + g * kSub));
     float qv[kRep][kSub];
 #pragma unroll
     for (int r = 0; r < kRep; ++r) {
@@ -293,44 +328,46 @@ attn_gsrq_prepare_kernel(const __half *__restrict__ q, const __half *__restrict_
             mx[r] = fmaxf(mx[r], dot);
         }
     }
-    // range of every (group, head) over the 256 codes: over warps through shared memory in two levels
-    // (8 x 32 threads fold the warps), then over the two lane halves and, for the common step, over the
-    // 16 groups by shuffles
+    // range of every (group, head) over the 256 codes: the two lane halves by shuffles, the warps through shared memory, where a
+    // thread per (head, group) also folds the groups into the head's common step
 #pragma unroll
     for (int r = 0; r < kRep; ++r) {
-        red[(warp * 8 + r) * 32 + lane] = mn[r];       // lane-major: conflict-free writes and reads
-        red[(warp * 8 + 4 + r) * 32 + lane] = mx[r];
-    }
-    __syncthreads();
-    if (tid < 8 * 32) {
-        const int v = tid >> 5;
-        float t = red[v * 32 + lane];
-        for (int w = 1; w < kPrepWarps; ++w) {
-            const float o = red[(w * 8 + v) * 32 + lane];
-            t = v < 4 ? fminf(t, o) : fmaxf(t, o);
-        }
-        red2[v * 32 + lane] = t;
-    }
-    __syncthreads();
-    float inv_step[kRep], scale_step[kRep], scale_offs[kRep];
-#pragma unroll
-    for (int r = 0; r < kRep; ++r) {
-        mn[r] = red2[r * 32 + lane];
-        mx[r] = red2[(4 + r) * 32 + lane];
-        // the two lane halves hold the two codes of a round for the same group: fold them first
         mn[r] = fminf(mn[r], __shfl_xor_sync(0xffffffffu, mn[r], 16));
         mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 16));
-        float range = mx[r] - mn[r];
-        float offs = mn[r];
+        if (half == 0) {
+            red[(warp * 8 + r) * kGroups + g] = mn[r];
+            red[(warp * 8 + 4 + r) * kGroups + g] = mx[r];
+        }
+    }
+    __syncthreads();
+    if (tid < kRep * kGroups) {
+        const int r = tid >> 4;
+        float lo = red[r * kGroups + g], hi = red[(4 + r) * kGroups + g];
 #pragma unroll
-        for (int off = 8; off >= 1; off >>= 1) {  // over the 16 groups
+        for (int w = 1; w < kPrepWarps; ++w) {
+            lo = fminf(lo, red[(w * 8 + r) * kGroups + g]);
+            hi = fmaxf(hi, red[(w * 8 + 4 + r) * kGroups + g]);
+        }
+        low_s[g * kRep + r] = lo;
+        float range = hi - lo, offs = lo;
+#pragma unroll
+        for (int off = 8; off >= 1; off >>= 1) {
             range = fmaxf(range, __shfl_xor_sync(0xffffffffu, range, off));
             offs += __shfl_xor_sync(0xffffffffu, offs, off);
         }
-        const float step = range > 0.0f ? range / (float)kEntryMax : 1.0f;
-        inv_step[r] = 1.0f / step;
-        scale_step[r] = step * kLog2e;
-        scale_offs[r] = offs * kLog2e;
+        if (g == 0) {
+            const float step = range > 0.0f ? range / (float)kEntryMax : 1.0f;
+            step_s[r] = 1.0f / step;
+            step_s[4 + r] = step * kLog2e;
+            step_s[8 + r] = offs * kLog2e;
+        }
+    }
+    __syncthreads();
+    float inv_step[kRep];
+    {
+        const float4 low = *reinterpret_cast<const float4 *>(low_s + g * kRep), inv = *reinterpret_cast<const float4 *>(step_s);
+        mn[0] = low.x, mn[1] = low.y, mn[2] = low.z, mn[3] = low.w;
+        inv_step[0] = inv.x, inv_step[1] = inv.y, inv_step[2] = inv.z, inv_step[3] = inv.w;
     }
     uint32_t packed[kPrepCodes][2];
 #pragma unroll
@@ -368,26 +405,9 @@ attn_gsrq_prepare_kernel(const __half *__restrict__ q, const __half *__restrict_
         const int code = warp * 2 + half + 2 * kPrepWarps * c;
         lut_g[((size_t)pair * kWords + code) * kSlots + stage * kGroups + g] = make_uint2(packed[c][0], packed[c][1]);
     }
-    if (tid == 0) {
-#pragma unroll
-        for (int r = 0; r < kRep; ++r) {
-            scale_g[((size_t)pair * kStages + stage) * 8 + r] = scale_step[r];
-            scale_g[((size_t)pair * kStages + stage) * 8 + 4 + r] = scale_offs[r];
-        }
-    }
+    if (tid < 2 * kRep) scale_g[((size_t)pair * kStages + stage) * 8 + tid] = step_s[4 + tid];  // steps, then offsets
 #if TACVQ_GSRQ_VPERM
-    {
-        const int perm_total = Hkv * kWords * kSlots;
-        const int perm_per_block = (perm_total + (int)gridDim.x - 1) / (int)gridDim.x;
-        for (int local = tid; local < perm_per_block; local += kPrepThreads) {
-            const int e = blockIdx.x * perm_per_block + local;
-            if (e < perm_total) {
-                const int hh = e >> 13, code = (e >> 5) & 255, pos = e & 31;
-                const int s = (pos >> 2) & 1, gg = ((pos >> 3) << 2) | (pos & 3);
-                vperm_g[e] = __ldg(reinterpret_cast<const uint4 *>(vtab + ((((size_t)hh * kStages + s) * kGroups + gg) * kWords + code) * kSub));
-            }
-        }
-    }
+    permute_values();
 #endif
 }
 
@@ -464,7 +484,7 @@ attn_gsrq_scan_kernel(const uint8_t *__restrict__ kcodes, const uint8_t *__restr
                       const __half *__restrict__ vtab, const uint4 *__restrict__ vperm_g, const int32_t *__restrict__ seq_start,
                       const int32_t *__restrict__ seq_end, float *__restrict__ part, unsigned long long *__restrict__ marks,
                       __half *__restrict__ out, float *__restrict__ state_out, int B, int Hkv, int T_cap,
-                      unsigned long long epoch) {
+                      unsigned long long epoch, int known_start, int known_end) {
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *lut_s = smem;
     unsigned char *vtab_s = smem + kLutBytes;
@@ -475,6 +495,9 @@ attn_gsrq_scan_kernel(const uint8_t *__restrict__ kcodes, const uint8_t *__restr
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Hq = Hkv * kRep;
 
+    // visible range of a row: a decode step's is known to the host, the same for all rows, and needs no trip to memory
+    auto first_token = [&](int b) { return known_end > 0 ? known_start : max(seq_start ? seq_start[b] : 0, 0); };
+    auto tokens_of = [&](int b) { return known_end > 0 ? known_end - known_start : row_tokens(seq_start, seq_end, b, T_cap); };
     // ---- work prefix over batch rows: a non-empty row costs its tiles plus kItemCost units (table
     //      copies, pipeline fill and drain, merge), so blocks that enter more pairs get fewer tiles ------
     auto work_prefix = [&]() {
@@ -482,7 +505,7 @@ attn_gsrq_scan_kernel(const uint8_t *__restrict__ kcodes, const uint8_t *__restr
             int running = 0;
             for (int b0 = 0; b0 < B; b0 += 32) {
                 const int b = b0 + lane;
-                int tiles = (b < B) ? (row_tokens(seq_start, seq_end, b, T_cap) + kTile - 1) / kTile : 0;
+                int tiles = (b < B) ? (tokens_of(b) + kTile - 1) / kTile : 0;
                 if (tiles > 0) tiles += kItemCost;
                 int incl = tiles;
 #pragma unroll
@@ -600,8 +623,8 @@ attn_gsrq_scan_kernel(const uint8_t *__restrict__ kcodes, const uint8_t *__restr
             cursor = item_end;
             continue;
         }
-        const int tok_lo_row = max(seq_start ? seq_start[b] : 0, 0);
-        const int n_tokens = row_tokens(seq_start, seq_end, b, T_cap);
+        const int tok_lo_row = first_token(b);
+        const int n_tokens = tokens_of(b);
         const int pair = h * B + b;
 
         __syncthreads();  // previous item fully merged: tables and staging may be overwritten
@@ -996,13 +1019,16 @@ int attn_gsrq_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vc
     const unsigned long long epoch = g_epoch.fetch_add(2, std::memory_order_relaxed);  // odd, so never 0 (= cleared)
     GsrqNewToken token = {};
     if (fresh) token = *fresh;
-    cudaError_t e = launch_dependent(true, gsrq::attn_gsrq_prepare_kernel, dim3(2 * B * Hkv), dim3(gsrq::kPrepThreads), 0, stream, q,
+    // a block per pair and stage; where that leaves SMs without one, further blocks share the permutation of the V codewords (16
+    // blocks alone take 4.5 us for 8 heads' 1 MB)
+    const int prepare_blocks = TACVQ_GSRQ_VPERM && 2 * B * Hkv < sms ? sms : 2 * B * Hkv;
+    cudaError_t e = launch_dependent(true, gsrq::attn_gsrq_prepare_kernel, dim3(prepare_blocks), dim3(gsrq::kPrepThreads), 0, stream, q,
                                      ktab, vtab, lut, scale, (uint4 *)(base + ws.vperm), B, Hkv, token);
     int st = e == cudaSuccess ? launch_status() : (int)e;
     if (st != TACVQ_OK) return st;
     e = launch_dependent(true, gsrq::attn_gsrq_scan_kernel, dim3(sms), dim3(gsrq::kThreads), gsrq::kSmemBytes, stream, kcodes, vcodes,
                          (const uint2 *)lut, (const float *)scale, vtab, (const uint4 *)(base + ws.vperm), seq_start, seq_end, part, marks, out,
-                         state_out, B, Hkv, (int)T_cap, epoch);
+                         state_out, B, Hkv, (int)T_cap, epoch, token.start, token.end);
     return e == cudaSuccess ? launch_status() : (int)e;
 }
 
