@@ -520,6 +520,16 @@ static int dispatch_d(const EncodeArgs &a) {
             if (st != TACVQ_ERR_UNSUPPORTED) return st;
         }
     }
+    // Whitened search of 8- and 4-wide groups, whatever the number of rows.  Whole calls, us through the fp32 scan of launch_small /
+    // this one, for one head; for eight heads:
+    //   16 x 8, two stages  33 rows 42.1/12.9; 44.7/16.6  256 rows 43.3/14.4; 49.1/20.6  4096 rows 52.3/22.6; 226.2/101.6
+    //   32 x 4, one stage   33 rows 19.1/11.1; 27.3/16.9  256 rows 20.6/12.3; 31.2/20.9  4096 rows 33.6/26.6; 185.4/121.4
+    if constexpr (sizeof(TT) == 4) {
+        if (TACVQ_ENCODE_TC && (a.D / a.G == 8 || a.D / a.G == 4)) {
+            const int st = encode_narrow_launch(a);
+            if (st != TACVQ_ERR_UNSUPPORTED) return st;
+        }
+    }
     if (TACVQ_ENCODE_TC && a.D / a.G >= 64) {
         const int st = encode_wide_launch(a);
         if (st != TACVQ_ERR_UNSUPPORTED) return st;

@@ -15,7 +15,8 @@
 // enter it, so the chip stays full whatever the number of pairs; a table costs about one tile's time.
 //
 // Bound by latency between the phases of a stage at 16 warps an SM (issue 48 % busy).  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
-// stages, rows wanted: 435 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.
+// stages, rows wanted: 435 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.  Whitened (fp32 words, a third product a
+// half): 3001 fp32 rows x 8 heads, 32 x 4, one stage 68 us against 125 for the fp32 scan of all words.
 //
 // Reference statements: src/jointkv/closed_loop_vq.py:52-76 (search), :343-395 (stage recursion),
 // src/jointkv/cq_tac.py:86-105.
@@ -30,6 +31,9 @@ constexpr int kRows = 128, kGroups = 4, kThreads = kRows * kGroups, kHalf = kMax
 constexpr uint32_t kSpan = 64;  // tiles
 constexpr size_t kWordBytes = kMaxWords * 32, kSeedBytes = kMaxWords * 32, kNormBytes = kMaxWords * 4;
 constexpr size_t kStageBytes = kWordBytes + kSeedBytes + kNormBytes;  // (word | word), seeds, |word|^2
+// fp32 words: their fp16 rounding takes the place of the words above; what it leaves follows, (low | 0), and the words themselves
+template <int DSUB, bool EXACT32>
+constexpr size_t kStage = EXACT32 ? kStageBytes + kWordBytes + kMaxWords * DSUB * 4 : kStageBytes;
 constexpr size_t kABytes = kRows * 32;                                // a group's (hi | lo) rows
 constexpr size_t kFixedBytes = (1 + kGroups) * kABytes + 256;         // ones, rows, barriers
 constexpr int kMaxStages = 12;                                        // and the length of the queue of codes
@@ -103,14 +107,25 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
     return *reinterpret_cast<const uint4 *>(h);
 }
 
+template <int DSUB>
+__device__ __forceinline__ void load_word(float (&w)[8], const unsigned char *from) {
+#pragma unroll
+    for (int j = 0; j < DSUB; j += 4) *reinterpret_cast<float4 *>(w + j) = *reinterpret_cast<const float4 *>(from + j * 4);
+}
+
 // DSUB = 8, or 4 run as 8 with the upper four elements of rows and words held at zero: appending zeros changes neither the
 // FMA chain of a dot product nor the left-to-right sum of squares.
-template <int DSUB, typename XT>
+// EXACT32: the words that decide are fp32 (transformed by a whitener); they are scored by three products, of the row's high and low
+// halves with the word's high one and of the high halves with the word's low one, which drops 2^-21 |r||c| and, where the low halves
+// are subnormal, 2^-22 |r|.  The rows of the reconstruction are summed from `plain`.
+template <int DSUB, typename XT, bool EXACT32>
 __global__ void __launch_bounds__(kThreads, 1)
-encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t sxt, const __half *__restrict__ tables,
-                     const float *__restrict__ sqnorm_in, uint8_t *__restrict__ codes, void *__restrict__ recon, int recon_dtype,
+encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t sxt, const void *__restrict__ tables_in,
+                     const __half *__restrict__ plain, const float *__restrict__ sqnorm_in, uint8_t *__restrict__ codes, void *__restrict__ recon, int recon_dtype,
                      int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap, int vec_ok, int spins) {
     extern __shared__ __align__(1024) unsigned char smem[];
+    constexpr size_t kStageBytes = kStage<DSUB, EXACT32>, kExactAt = narrow::kStageBytes + kWordBytes;
+    const __half *tables = reinterpret_cast<const __half *>(tables_in);
     unsigned char *ones = smem + (size_t)S * kStageBytes, *misc = ones + (1 + kGroups) * kABytes;
     const uint32_t bars = smem_u32(misc);                               // [kGroups]
     uint32_t *in_flight = reinterpret_cast<uint32_t *>(misc + 32);      // [kGroups] phase of the last product asked for; 2: none
@@ -155,6 +170,7 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
             const uint32_t words_a = smem_u32(stage) + half * (kHalf * 32);
             mma(tmem, descriptor(smem_u32(ones)), descriptor(words_a + (uint32_t)kWordBytes), 0u);
             mma(tmem, descriptor(smem_u32(A)), descriptor(words_a), 1u);
+            if constexpr (EXACT32) mma(tmem, descriptor(smem_u32(A)), descriptor(words_a + (uint32_t)narrow::kStageBytes), 1u);
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
             in_flight[grp] = phase;
         }
@@ -185,17 +201,31 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
         for (int i = tid; i < S * kMaxWords; i += kThreads) {
             const int s = i / kMaxWords, k = i % kMaxWords;
             unsigned char *stage = smem + (size_t)s * kStageBytes;
-            uint4 w = make_uint4(0u, 0u, 0u, 0u);
+            uint4 w = make_uint4(0u, 0u, 0u, 0u), low = w;
             float cc = inf;  // padding words can never be chosen
             if (k < K) {
                 const int64_t word = (((int64_t)h * S + s) * G + g) * K + k;
-                if constexpr (DSUB == 8) {
+                if constexpr (EXACT32) {
+                    const float *from = reinterpret_cast<const float *>(tables_in) + word * DSUB;
+                    float e[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, back[8];
+#pragma unroll
+                    for (int j = 0; j < DSUB; j += 4) *reinterpret_cast<float4 *>(e + j) = __ldg(reinterpret_cast<const float4 *>(from + j));
+#pragma unroll
+                    for (int j = 0; j < DSUB; j += 4) *reinterpret_cast<float4 *>(stage + kExactAt + (k * DSUB + j) * 4) = *reinterpret_cast<const float4 *>(e + j);
+                    cc = sqnorm_in != nullptr ? sqnorm_in[word] : sqnorm_ordered<DSUB>([&](int j) { return e[j]; });
+                    w = pack8(e);
+                    unpack8(w, back);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) e[j] -= back[j];
+                    low = pack8(e);
+                } else if constexpr (DSUB == 8) {
                     w = __ldg(reinterpret_cast<const uint4 *>(tables + word * 8));
                 } else {
                     const uint2 half_word = __ldg(reinterpret_cast<const uint2 *>(tables + word * 4));
                     w = make_uint4(half_word.x, half_word.y, 0u, 0u);
                 }
-                if (sqnorm_in != nullptr) {
+                if constexpr (EXACT32) {
+                } else if (sqnorm_in != nullptr) {
                     cc = sqnorm_in[word];
                 } else {
                     float e[8];
@@ -206,6 +236,11 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
             }
             *reinterpret_cast<uint4 *>(stage + k * 32) = w;
             *reinterpret_cast<uint4 *>(stage + k * 32 + 16) = w;
+            if constexpr (EXACT32) {
+                unsigned char *to = stage + narrow::kStageBytes + k * 32;
+                *reinterpret_cast<uint4 *>(to + ((k >> 2) & 1) * 16) = low;
+                *reinterpret_cast<uint4 *>(to + (((k >> 2) & 1) ^ 1) * 16) = make_uint4(0u, 0u, 0u, 0u);
+            }
             const float t = -0.5f * cc;
             const __half p1 = __float2half_rn(t);
             const float r1 = k < K ? t - __half2float(p1) : 0.0f;
@@ -288,7 +323,9 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                 const float cc_top = __int_as_float(cc_tops[s]);
                 float rough;
                 asm("sqrt.approx.f32 %0, %1;" : "=f"(rough) : "f"(cc_top));
-                const float margin = 3.0517578125e-05f * (xx + cc_top) + 3.82e-06f * rough + 1.1920929e-07f;
+                float rough_row = 0.0f;
+                if constexpr (EXACT32) asm("sqrt.approx.f32 %0, %1;" : "=f"(rough_row) : "f"(xx));
+                const float margin = 3.0517578125e-05f * (xx + cc_top) + (EXACT32 ? 3.82e-06f * rough_row : 0.0f) + 3.82e-06f * rough + 1.1920929e-07f;
 
                 // ---- half by half: the largest score of every four words, their largest, and the fours close to that.  The first half's
                 // are looked at while the second half's product runs, against the first half's own maximum: at worst a few too many.
@@ -351,7 +388,8 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                     for (int j = 0; j < 4; ++j) {
                         const int k = 4 * p + ((j + tid) & 3);
                         float w[8];
-                        unpack8(*reinterpret_cast<const uint4 *>(stage + k * 32 + copy), w);
+                        if constexpr (EXACT32) load_word<DSUB>(w, stage + kExactAt + k * DSUB * 4);
+                        else unpack8(*reinterpret_cast<const uint4 *>(stage + k * 32 + copy), w);
                         float dot = __fmaf_rn(r[0], w[0], 0.0f);
 #pragma unroll
                         for (int i = 1; i < DSUB; ++i) dot = __fmaf_rn(r[i], w[i], dot);
@@ -362,7 +400,8 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                 __syncwarp();
                 if (arg >= K) arg = 0;  // no distance was finite
                 float sel[8];
-                unpack8(*reinterpret_cast<const uint4 *>(stage + arg * 32 + copy), sel);
+                if constexpr (EXACT32) load_word<DSUB>(sel, stage + kExactAt + arg * DSUB * 4);
+                else unpack8(*reinterpret_cast<const uint4 *>(stage + arg * 32 + copy), sel);
 #pragma unroll
                 for (int i = 0; i < DSUB; ++i) r[i] = __fsub_rn(r[i], sel[i]);
                 picks = (picks >> 8) | ((uint64_t)(later & 255u) << 56);  // a queue of 12 bytes
@@ -376,7 +415,19 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                     const int byte = kMaxStages - S + s;
                     const int code = (int)((byte < 8 ? (uint32_t)(picks >> (8 * byte)) : later >> (8 * (byte - 8))) & 255u);
                     float w[8];
-                    unpack8(*reinterpret_cast<const uint4 *>(smem + (size_t)s * kStageBytes + code * 32 + copy), w);
+                    if constexpr (EXACT32) {
+                        const __half *from = plain + ((((int64_t)h * S + s) * G + g) * K + code) * DSUB;
+                        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                        if constexpr (DSUB == 8) {
+                            v = __ldg(reinterpret_cast<const uint4 *>(from));
+                        } else {
+                            const uint2 half_word = __ldg(reinterpret_cast<const uint2 *>(from));
+                            v.x = half_word.x, v.y = half_word.y;
+                        }
+                        unpack8(v, w);
+                    } else {
+                        unpack8(*reinterpret_cast<const uint4 *>(smem + (size_t)s * kStageBytes + code * 32 + copy), w);
+                    }
 #pragma unroll
                     for (int i = 0; i < DSUB; ++i) dec[i] = __fadd_rn(dec[i], w[i]);
                 }
@@ -412,7 +463,8 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
 int encode_narrow_launch(const EncodeArgs &a) {
     using namespace narrow;
     const int sub = a.D / a.G;
-    if (a.tables_f32 || (sub != 8 && sub != 4) || a.K > kMaxWords || a.S > kMaxStages) return TACVQ_ERR_UNSUPPORTED;
+    if ((sub != 8 && sub != 4) || a.K > kMaxWords || a.S > kMaxStages) return TACVQ_ERR_UNSUPPORTED;
+    if (a.tables_f32 && (a.x_dtype != TACVQ_F32 || (reinterpret_cast<uintptr_t>(a.recon_tables) & 15u) != 0)) return TACVQ_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(a.tables) & 15u) != 0) return TACVQ_ERR_UNSUPPORTED;
     if (a.recon != nullptr && (reinterpret_cast<uintptr_t>(a.recon) & 15u) != 0) return TACVQ_ERR_UNSUPPORTED;
     const int64_t rows = (int64_t)a.B * a.T;
@@ -420,24 +472,36 @@ int encode_narrow_launch(const EncodeArgs &a) {
     const int64_t tiles = (rows + kRows - 1) / kRows, all_tiles = tiles * a.H * a.G;
     const int elem = a.x_dtype == TACVQ_F16 ? 2 : 4, vec = sub * elem < 16 ? sub * elem : 16, per_vec = vec / elem;
     const int vec_ok = (reinterpret_cast<uintptr_t>(a.x) % vec) == 0 && a.sxb % per_vec == 0 && a.sxh % per_vec == 0 && a.sxt % per_vec == 0;
-    const size_t smem = (size_t)a.S * kStageBytes + kFixedBytes + (size_t)a.S * 4;
+    const size_t stage = a.tables_f32 ? (sub == 8 ? kStage<8, true> : kStage<4, true>) : kStageBytes;
+    const size_t smem = (size_t)a.S * stage + kFixedBytes + (size_t)a.S * 4;
+    if (smem > 227 * 1024) return TACVQ_ERR_UNSUPPORTED;
     // one block an SM; fewer where that would leave less than a tile for every group
     int64_t blocks = (all_tiles + kGroups - 1) / kGroups;
+    // Few rows: whole pairs, as copying another pair's words costs more than idle threads.  Whitened 16 x 8, two stages, us with tiles / 4
+    // blocks and so: one head x 33 rows 28.9 / 12.9, eight 32.5 / 16.6.
+    if (tiles < kGroups) {
+        const int64_t pairs = (int64_t)a.H * a.G, turns = (pairs + 147) / 148;
+        blocks = (pairs + turns - 1) / turns;
+    }
     if (blocks > 148) blocks = 148;
     auto launch = [&](auto kernel, auto *xp) -> int {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        kernel<<<(unsigned)blocks, kThreads, smem, a.stream>>>(xp, a.sxb, a.sxh, a.sxt, (const __half *)a.tables, a.sqnorm, a.codes, a.recon,
+        kernel<<<(unsigned)blocks, kThreads, smem, a.stream>>>(xp, a.sxb, a.sxh, a.sxt, a.tables, a.recon_tables, a.sqnorm, a.codes, a.recon,
                                                                a.recon_dtype, a.B, a.H, a.T, a.G, a.S, a.K, a.t0, a.T_cap, vec_ok,
                                                                a.wait_spins < 0 ? kSpins : a.wait_spins);
         return launch_status();
     };
-    if (sub == 8) {
-        if (a.x_dtype == TACVQ_F16) return launch(encode_narrow_kernel<8, __half>, (const __half *)a.x);
-        return launch(encode_narrow_kernel<8, float>, (const float *)a.x);
+    if (a.tables_f32) {
+        if (sub == 8) return launch(encode_narrow_kernel<8, float, true>, (const float *)a.x);
+        return launch(encode_narrow_kernel<4, float, true>, (const float *)a.x);
     }
-    if (a.x_dtype == TACVQ_F16) return launch(encode_narrow_kernel<4, __half>, (const __half *)a.x);
-    return launch(encode_narrow_kernel<4, float>, (const float *)a.x);
+    if (sub == 8) {
+        if (a.x_dtype == TACVQ_F16) return launch(encode_narrow_kernel<8, __half, false>, (const __half *)a.x);
+        return launch(encode_narrow_kernel<8, float, false>, (const float *)a.x);
+    }
+    if (a.x_dtype == TACVQ_F16) return launch(encode_narrow_kernel<4, __half, false>, (const __half *)a.x);
+    return launch(encode_narrow_kernel<4, float, false>, (const float *)a.x);
 }
 
 int narrow_timeouts(unsigned int *out) { return (int)cudaMemcpyFromSymbol(out, narrow::g_timeouts, sizeof(unsigned int)); }

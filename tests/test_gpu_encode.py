@@ -117,6 +117,21 @@ def test_whitened_assignment_is_bit_exact_with_the_c_oracle(device, name, shape,
     assert int((plain != want_codes).sum()) > 0  # the matrix does change assignments: the test is not vacuous
 
 
+@pytest.mark.parametrize("sub,groups,stages,words", [(8, 16, 2, 256), (8, 2, 6, 99), (8, 2, 7, 256), (4, 32, 1, 256), (4, 4, 7, 130)])
+@pytest.mark.parametrize("heads,tokens,dtype", [(1, 1, torch.float16), (3, 127, torch.float32), (8, 129, torch.float16), (2, 385, torch.float32), (1, 8321, torch.float16)])
+def test_whitened_search_of_narrow_groups_is_bit_exact(device, sub, groups, stages, words, heads, tokens, dtype):
+    """Edges of tiles, of blocks and of spans; stages whose tables just fit in shared memory and one more; words too large for fp16."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(sub * stages + tokens)
+    states = make_states(gen, (1, heads, tokens, sub * groups), dtype)
+    tables = make_tables(gen, heads, stages, groups, sub, [0.5 * 0.7**s for s in range(stages)])[:, :, :, :words].contiguous()
+    w = torch.eye(sub).expand(heads, groups, sub, sub) + 0.3 * torch.randn(heads, groups, sub, sub, generator=gen) / sub**0.5
+    w[0, groups - 1] *= 3e5 if tokens == 129 else 1.0
+    want, want_recon = C.encode_whitened(states, tables, w)
+    codes, recon = ops.encode(states.to(device), tables.to(device), whitener=w.to(device))
+    assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
+
+
 def test_modules_match_reference_golden(golden, device):
     from tac_vq_kv_cache_b200.jointkv.cq_tac import ClosedLoopGroupedCQ
     from tac_vq_kv_cache_b200.jointkv.uniform_depth_tac import ClosedLoopUniformResidualVQ
