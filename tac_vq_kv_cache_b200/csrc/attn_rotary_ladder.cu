@@ -25,6 +25,9 @@
 // in units of 2^-20, smaller ones in units of 2^-30 and in bins of their own, so that the many small weights beside a large one
 // keep ten bits down to 2^-20.  The sums are exact.
 //
+// us a decode step of 16 stages and 8 KV heads, against attn_rotary_kernel: one row of 6144 tokens with a window of 4096 51.4 / 114.5 (27 are the
+// new token's encode), 600 tokens 44 / 89, 16384 tokens 119 / 240, 8 x 2000 156 / 230, 16 x 1000 189 / 201.
+//
 // Semantics replaced: experiments_followup_mistral/evaluate_mistral_longbench.py:112-122 including the rotary step
 // (:113-118); the query arrives rotated at its own position and scaled.
 
