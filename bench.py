@@ -554,7 +554,7 @@ def run_cq32layers(args) -> dict:
         "decode": {"ms_per_layer_step": round(dec_ms, 4), "tokens_per_s": round(CQ_BATCH * world / (dec_ms * 1e-3), 1)},
         "roofline": {"bound": "hbm", "achieved": round(dec_bytes / (dec_ms * 1e-3) / 1e9, 1), "peak": peaks["hbm"], "unit": "GB/s",
                      "frac": round(dec_bytes / (dec_ms * 1e-3) / 1e9 / peaks["hbm"], 4), "peak_source": f"{peaks['kind']} copy bandwidth",
-                     "algorithmic_bytes_per_launch": dec_bytes, "kernel": "attn_fullwidth_kernel (decode side of a layer-step)", "traffic": None},
+                     "algorithmic_bytes_per_launch": dec_bytes, "kernel": "attn_slots_kernel (decode side of a layer-step)", "traffic": None},
         "parity": parity, "gpu_launches": 4 * args.steps, "clocks": clocks.summary(),
     }
 
