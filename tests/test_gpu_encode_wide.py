@@ -52,6 +52,23 @@ def test_wide_encode_is_bit_exact(device, batch, heads, tokens, sub, groups, sta
     assert ops.encode_tensor_memory_timeouts(device) == 0
 
 
+@pytest.mark.parametrize("sub,groups,heads,tokens", [(128, 1, 2, 1), (128, 1, 3, 127), (128, 1, 60, 645), (64, 2, 2, 129), (64, 2, 40, 647)])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+def test_fp32_rows_at_any_alignment(device, sub, groups, heads, tokens, shift):
+    """Rows that are fetched together, 16 bytes a lane, and rows that start elsewhere; heads and tokens exchanged, with a gap between rows."""
+    from tac_vq_kv_cache_b200 import ops
+
+    gen = torch.Generator().manual_seed(sub + tokens)
+    tables = make_tables(gen, heads, 2, groups, sub, [0.1, 0.08])
+    states = make_states(gen, (2, heads, tokens, sub * groups), torch.float32, 4)
+    room = torch.full((2, tokens, heads, sub * groups + 8), float("nan"), device=device)
+    x = room[..., shift : shift + sub * groups].transpose(1, 2)
+    x.copy_(states)
+    want, want_recon = C.encode(states, tables)
+    codes, recon = ops.encode(x, tables.to(device))
+    assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
+
+
 def test_rows_between_words_take_the_exact_chains(device):
     """Every row lies on a bisector of two words, or at a word that occurs three times: nothing but the exact order decides."""
     from tac_vq_kv_cache_b200 import ops
