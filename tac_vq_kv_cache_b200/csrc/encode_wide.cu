@@ -415,7 +415,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
         } else {
             if (DSUB == 128 && a.vec_ok) {
                 // The same in two halves, for which the place of the fp16 rows is just large enough.  Against 32 bytes of its own row a
-                // thread, us: 131072 rows x 8 heads, two stages 315 / 290, 16 stages x 2048 rows 107 / 101.  64 wide it is 181 / 183.
+                // thread, us: 65536 rows x 8 heads, two stages 318 / 288, 16 stages x 2048 rows 109 / 103.  64 wide it is 181 / 183.
                 constexpr int kAtOnce = 32 / kPieces, kEach = 8 / kAtOnce;
                 const unsigned long long mine = live ? (unsigned long long)src : 0ull;
                 uint4 v[2][kEach];

@@ -69,6 +69,24 @@ def test_fp32_rows_at_any_alignment(device, sub, groups, heads, tokens, shift):
     assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
 
 
+@pytest.mark.parametrize("sub,groups", [(128, 1), (64, 2), (32, 4)])
+@pytest.mark.parametrize("batch,tokens,words,shift,dtype", [(1, 1, 256, 0, torch.float16), (1, 129, 256, 1, torch.float32), (1, 601, 99, 0, torch.float32), (3, 333, 256, 0, torch.float16), (1, 1500, 256, 1, torch.float16), (1, 2049, 256, 0, torch.float16)])
+def test_whitener_at_every_tile_height(device, sub, groups, batch, tokens, words, shift, dtype):
+    """One bit of a transformed row or word shows in the codes: four to eight rows a thread, ragged tiles, rows of several batch entries."""
+    from tac_vq_kv_cache_b200 import ops
+
+    gen = torch.Generator().manual_seed(sub + tokens)
+    heads = 20
+    tables = make_tables(gen, heads, 1, groups, sub, [0.1])[:, :, :, :words].contiguous()
+    states = make_states(gen, (batch, heads, tokens, sub * groups), dtype)
+    w = torch.eye(sub).expand(heads, groups, sub, sub) + 0.3 * torch.randn(heads, groups, sub, sub, generator=gen) / sub**0.5
+    x = torch.zeros(batch, tokens, heads, sub * groups + 8, dtype=dtype, device=device)[..., shift : shift + sub * groups].transpose(1, 2)
+    x.copy_(states)
+    want, want_recon = C.encode_whitened(states, tables, w)
+    codes, recon = ops.encode(x, tables.to(device), whitener=w.to(device))
+    assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
+
+
 def test_rows_between_words_take_the_exact_chains(device):
     """Every row lies on a bisector of two words, or at a word that occurs three times: nothing but the exact order decides."""
     from tac_vq_kv_cache_b200 import ops
