@@ -19,7 +19,9 @@
 // apply_rotary_pos_emb, transposed by movmatrix, and the result is the A operand of the product with the query heads.
 //
 // In a decode step the ladder's new token takes longer to encode (16 stages one after the other on a few SMs) than everything
-// here up to the scores of the old ones, so those go first and the kernel waits for the new codes where it needs them.
+// here up to the scores of the old ones, so those go first and the kernel waits for the new codes where it needs them.  Codes are
+// read from L2 (code_word, code_byte): a line of the first-level cache that was fetched for an old token before the wait may hold the
+// place of the new one, and would still hold its old bytes after it.
 //
 // Weights enter the histograms as integers, because shared-memory integer adds are single instructions: weights from 2^-10 on
 // in units of 2^-20, smaller ones in units of 2^-30 and in bins of their own, so that the many small weights beside a large one
@@ -84,6 +86,18 @@ __device__ __forceinline__ uint4 ldg_in_place(const void *p) {  // a load that s
     asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
+// Code bytes as they are in L2, which is where the kernel before this one has left them by the time its end was waited for.  Not
+// ld.global.nc: that is for memory which nobody writes while the kernel runs.
+__device__ __forceinline__ uint32_t code_word(const uint8_t *p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t code_byte(const uint8_t *p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 // all blocks of the cluster: writes before are seen by reads after, in every block's shared memory
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -111,7 +125,7 @@ constexpr uint32_t kIsSmall = 0x80000000u;
 // Clusters of 8 blocks share the KV heads x B x splits items (a split of a row's visible tokens) evenly, head by head; a
 // cluster loads the key tables when the head changes.
 __global__ void __launch_bounds__(kThreads, 1)
-attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcodes, const uint8_t *__restrict__ vcodes,
+attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uint8_t *vcodes,
                           const __half *__restrict__ ktab, const __half *__restrict__ vtab, const __half *__restrict__ rope,
                           const int32_t *__restrict__ seq_start, const int32_t *__restrict__ seq_end, float *__restrict__ part,
                           int B, int Hq, int Hkv, int S, int64_t T_cap, int splits, const LadderStep step) {
@@ -191,7 +205,7 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *__restric
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const int t = min(tile * 16 + u * 8 + r8, n - 1);
-                    cn[u] = kq < words_per_token ? __ldg(reinterpret_cast<const uint32_t *>(kc + (int64_t)t * S) + kq) : 0u;
+                    cn[u] = kq < words_per_token ? code_word(kc + (int64_t)t * S + 4 * kq) : 0u;
                     const int t0 = min(tile * 16 + u * 8 + 2 * kq, n - 1), t1 = min(tile * 16 + u * 8 + 2 * kq + 1, n - 1);
                     const unsigned short *c0 = reinterpret_cast<const unsigned short *>(rp + (int64_t)t0 * kDim), *c1 = reinterpret_cast<const unsigned short *>(rp + (int64_t)t1 * kDim);
                     rn[u][0] = __ldg(c0) | (uint32_t)__ldg(c1) << 16;
@@ -253,8 +267,8 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *__restric
             const int t = tid + i * kThreads;
             v_codes[i] = 0u;
             if (t < n && stages > 0) {
-                v_codes[i] = __ldg(vc + (int64_t)t * S + slice);
-                if (stages > 1) v_codes[i] |= (uint32_t)__ldg(vc + (int64_t)t * S + slice + 8) << 8;
+                v_codes[i] = code_byte(vc + (int64_t)t * S + slice);
+                if (stages > 1) v_codes[i] |= code_byte(vc + (int64_t)t * S + slice + 8) << 8;
             }
         }
         uint4 v_words[2 * kWords / 32];

@@ -11,8 +11,9 @@ from __future__ import annotations
 import pytest
 import torch
 
+from oracle import c_oracle as C
 from oracle import jointkv_oracle as O
-from tests.util import make_tables, max_rel, rel_l2
+from tests.util import make_states, make_tables, max_rel, rel_l2
 
 pytestmark = pytest.mark.gpu
 TOL = 2e-3
@@ -166,6 +167,46 @@ def test_rotary_attention_over_deep_ladders(device, b, hq, hkv, stages, t, range
     for row in set(range(b)) - set(live):
         assert not out[row].any() and (state[row, :, 0] == -float("inf")).all() and not state[row, :, 1:].any()
 
+
+@pytest.mark.parametrize(
+    "batch,heads,q_heads,groups,stages,sub,max_tokens,window,first,new",
+    [
+        (1, 8, 32, 1, 16, 128, 513, None, 295, 1),   # rows of odd length: every position's codes begin inside a sector in some head
+        (1, 8, 32, 1, 16, 128, 4097, None, 4081, 1),
+        (3, 8, 16, 1, 16, 128, 337, None, 310, 1),   # more items than clusters, heads change inside one
+        (1, 2, 8, 1, 4, 128, 45, None, 0, 1),        # from the first token on: a new token alone in its tile
+        (5, 3, 3, 1, 8, 128, 271, 100, 250, 1),      # the range moves against the tiles
+        (2, 4, 16, 1, 12, 128, 303, None, 240, 3),   # several new tokens, across the end of a tile
+        (1, 1, 4, 1, 16, 128, 1023, None, 500, 2),
+        (3, 2, 8, 16, 2, 8, 333, None, 305, 1),
+        (5, 2, 4, 16, 2, 8, 97, 40, 60, 2),
+    ],
+)
+def test_a_step_sees_the_codes_of_its_own_token(device, batch, heads, q_heads, groups, stages, sub, max_tokens, window, first, new):
+    """Attention starts before the new token's codes are written over others: whatever was there before must not be seen.  The new
+    key carries most of the weight, and steps go over the edges of tiles, sectors and splits."""
+    from tac_vq_kv_cache_b200.code_cache import VQCodeCache
+
+    gen = torch.Generator().manual_seed(max_tokens + stages)
+    scales = [0.5 * 0.85**s for s in range(stages)] if groups == 1 else None
+    tables = [make_tables(gen, heads, stages, groups, sub, scales) for _ in range(2)]
+    cache = VQCodeCache(*tables, batch=batch, max_tokens=max_tokens, window=window, device=device, rope_theta=1e6)
+    kept = [torch.randint(0, 256, cache.key.shape, generator=gen, dtype=torch.uint8) for _ in range(2)]
+    cache.key.copy_(kept[0]), cache.value.copy_(kept[1])
+    cache.length = first
+    last = min(first + 34, max_tokens)
+    for end in range(first + new, last + 1, new):
+        rows = [make_states(gen, (batch, heads, new, 128)) for _ in range(2)]
+        for store, table, row in zip(kept, tables, rows):
+            C.encode(row, table, codes=store, t0=end - new, want_recon=False)
+        key = O.reconstruct(kept[0][:, :, end - 1 : end], tables[0], torch.float16)
+        key = O.apply_rotary_fp16(key, *O.rotary_table(1, 128, 1e6, end - 1)).float()[:, :, 0]
+        query = (9.0 * key / (key * key).sum(-1, keepdim=True)).half().repeat_interleave(q_heads // heads, 1)
+        out = cache.decode_step(query.to(device), *(row.to(device) for row in rows))
+        start, stop = cache.visible()
+        want, *_ = O.attention_over_codes(query, *kept, *tables, [start] * batch, [stop] * batch, rope_theta=1e6)
+        assert torch.equal(cache.key.cpu(), kept[0]) and torch.equal(cache.value.cpu(), kept[1])
+        _check(out.float().cpu(), want)
 
 def test_code_cache_with_rope_follows_the_reference_decode_loop(device):
     """Prefill + three decode steps through VQCodeCache(rope_theta=...): codes of pre-rotary keys are
