@@ -162,7 +162,7 @@ attn_generic_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kc
 constexpr int kCombineLanes = 128, kCombineGroups = 8;
 
 __global__ void __launch_bounds__(kCombineLanes * kCombineGroups)
-attn_combine_kernel(const float *__restrict__ states, int n_parts, int64_t rows, int D, __half *__restrict__ out,
+attn_combine_kernel(const float *states, int n_parts, int64_t rows, int D, __half *__restrict__ out,
                     float *__restrict__ merged) {
     __shared__ float red[2 * kCombineLanes * kCombineGroups / 32];
     __shared__ float sums[kCombineGroups * kCombineLanes];

@@ -160,7 +160,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ uint4 ldg_stream(const void *p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;
@@ -480,10 +480,8 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 // scan kernel
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads, 1)
-attn_gsrq_scan_kernel(const uint8_t *__restrict__ kcodes, const uint8_t *__restrict__ vcodes,
-                      const uint2 *__restrict__ lut_g, const float *__restrict__ scale_g,
-                      const __half *__restrict__ vtab, const uint4 *__restrict__ vperm_g, const int32_t *__restrict__ seq_start,
-                      const int32_t *__restrict__ seq_end, float *__restrict__ part, unsigned long long *__restrict__ marks,
+attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 *lut_g, const float *scale_g,
+                      const __half *__restrict__ vtab, const uint4 *vperm_g, const int32_t *seq_start, const int32_t *seq_end, float *__restrict__ part, unsigned long long *__restrict__ marks,
                       __half *__restrict__ out, float *__restrict__ state_out, int B, int Hkv, int T_cap,
                       unsigned long long epoch, int known_start, int known_end) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -644,7 +642,7 @@ attn_gsrq_scan_kernel(const uint8_t *__restrict__ kcodes, const uint8_t *__restr
         // twelve registers of every thread: scale_s = step of stage 0 x4, step of stage 1 x4, total offset x4
         if (tid < 12) {
             const float *sg = scale_g + (size_t)pair * 16;
-            scale_s[tid] = tid < 4 ? __ldg(sg + tid) : tid < 8 ? __ldg(sg + 4 + tid) : __ldg(sg + tid - 4) + __ldg(sg + tid + 4);
+            scale_s[tid] = tid < 4 ? sg[tid] : tid < 8 ? sg[4 + tid] : sg[tid - 4] + sg[tid + 4];
         }
         cp_async_wait_all();
         __syncthreads();  // tables ready

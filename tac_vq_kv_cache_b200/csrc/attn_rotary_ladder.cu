@@ -127,7 +127,7 @@ constexpr uint32_t kIsSmall = 0x80000000u;
 __global__ void __launch_bounds__(kThreads, 1)
 attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uint8_t *vcodes,
                           const __half *__restrict__ ktab, const __half *__restrict__ vtab, const __half *__restrict__ rope,
-                          const int32_t *__restrict__ seq_start, const int32_t *__restrict__ seq_end, float *__restrict__ part,
+                          const int32_t *seq_start, const int32_t *seq_end, float *__restrict__ part,
                           int B, int Hq, int Hkv, int S, int64_t T_cap, int splits, const LadderStep step) {
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *area = smem + kTabBytes;                              // scores, then weights, then sums

@@ -126,9 +126,9 @@ __device__ __forceinline__ void copy_tables(uint32_t tab_u32, const __half *__re
 
 template <int R>
 __global__ void __launch_bounds__(kThreads, 1)
-attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcodes, const uint8_t *__restrict__ vcodes,
+attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uint8_t *vcodes,
                        const __half *__restrict__ ktab, const __half *__restrict__ vtab, const __half *__restrict__ rope,
-                       const int32_t *__restrict__ seq_start, const int32_t *__restrict__ seq_end, float *__restrict__ part,
+                       const int32_t *seq_start, const int32_t *seq_end, float *__restrict__ part,
                        int B, int Hq, int Hkv, int64_t T_cap, int splits) {
     constexpr int kPos = kPositions<R>, kStride = kProbStride<R>;
     constexpr int kRowWarps = kWarps / R, kRowThreads = kThreads / R;  // softmax and pass V: warps of one batch row
@@ -213,8 +213,8 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *__restrict__
             limit = limit_s[r];
             const int t = min(max(local, limit.z), limit.w);
             const uint8_t *src = kc + (size_t)r * row_step + (size_t)t * 32;
-            cn[0] = __ldg(reinterpret_cast<const uint4 *>(src));
-            cn[1] = __ldg(reinterpret_cast<const uint4 *>(src + other_stage));
+            cn[0] = *reinterpret_cast<const uint4 *>(src);
+            cn[1] = *reinterpret_cast<const uint4 *>(src + other_stage);
             // to L2: the key codes two trips on, and the value codes of this one for pass V
             const int ahead = max(min(local + 16 * kWarps, limit.w), 0);
             if (j4 < 2) prefetch_l2(j4 == 0 ? kc + (size_t)r * row_step + (size_t)ahead * 32 : src + v_from_k);

@@ -80,26 +80,26 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 
 // a token's code bytes; slots that are a power of two have rows that one or two aligned loads fetch
 template <int P, bool FULL>
-__device__ __forceinline__ void load_codes(const uint8_t *__restrict__ p, int slots, uint32_t (&w)[Shape<P>::kCodeWords]) {
+__device__ __forceinline__ void load_codes(const uint8_t *p, int slots, uint32_t (&w)[Shape<P>::kCodeWords]) {
     if constexpr (!FULL || P == 1) {
 #pragma unroll
         for (int i = 0; i < Shape<P>::kCodeWords; ++i) {
             w[i] = 0u;
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (4 * i + j < P && 4 * i + j < slots) w[i] |= (uint32_t)__ldg(p + 4 * i + j) << (8 * j);
+                if (4 * i + j < P && 4 * i + j < slots) w[i] |= (uint32_t)p[4 * i + j] << (8 * j);
         }
     } else if constexpr (P == 2) {
-        w[0] = __ldg(reinterpret_cast<const unsigned short *>(p));
+        w[0] = *reinterpret_cast<const unsigned short *>(p);
     } else if constexpr (P == 4) {
-        w[0] = __ldg(reinterpret_cast<const uint32_t *>(p));
+        w[0] = *reinterpret_cast<const uint32_t *>(p);
     } else if constexpr (P == 8) {
-        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+        const uint2 v = *reinterpret_cast<const uint2 *>(p);
         w[0] = v.x, w[1] = v.y;
     } else {
 #pragma unroll
         for (int i = 0; i < P / 16; ++i) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p) + i);
+            const uint4 v = reinterpret_cast<const uint4 *>(p)[i];
             w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
         }
     }
@@ -147,9 +147,8 @@ __device__ __forceinline__ void add_weights(const uint32_t (&codes)[Shape<P>::kC
 
 template <int P, bool FULL>
 __global__ void __launch_bounds__(kThreads, 1)
-attn_slots_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kcodes, const uint8_t *__restrict__ vcodes,
-                  const __half *__restrict__ ktab, const __half *__restrict__ vtab, const int32_t *__restrict__ seq_start,
-                  const int32_t *__restrict__ seq_end, float *__restrict__ part, __half *__restrict__ out,
+attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *__restrict__ ktab,
+                  const __half *__restrict__ vtab, const int32_t *seq_start, const int32_t *seq_end, float *__restrict__ part, __half *__restrict__ out,
                   float *__restrict__ state_out, int B, int Hq, int Hkv, int G, int S, int64_t T_cap, int splits) {
     using L = Shape<P>;
     constexpr int H = L::kHeads, NW = L::kCodeWords, NT = L::kTokens;

@@ -153,6 +153,8 @@ struct LadderStep {
 // Programmatic dependent launch: a kernel launched with launch_dependent may start before its predecessor has finished; it must
 // not read the predecessor's results, nor overwrite what that reads, before it has waited.  A predecessor that lets it start early
 // calls launch_dependents.
+// What the predecessor writes is read through pointers without __restrict__ and never by __ldg or ld.global.nc: those count as reads of
+// memory that nobody changes while the kernel runs, which the compiler may move above the wait.
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
