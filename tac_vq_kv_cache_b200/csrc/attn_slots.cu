@@ -16,9 +16,10 @@
 // gains.
 //
 // Weights are added as integers, because shared-memory integer adds are single instructions (a float add is a
-// compare-and-swap loop): weights from 2^-10 on in units of 2^-20, smaller ones in units of 2^-30 and in bins of their own, so that
-// the many small weights beside a large one keep ten bits down to 2^-20.  Integer sums are exact and the result does not depend on
-// the order.  A weight is relative to a reference that lies a little (kHeadroom) above the largest score when it was last set; when a
+// compare-and-swap loop).  FINE: a weight's multiple of 2^-19 goes to one bin and what that leaves, in units of 2^-38, to another,
+// which keeps all 24 bits of a weight down to 2^-15 and costs two adds.  Otherwise weights from 2^-10 on are added in units of 2^-20, smaller ones in units of
+// 2^-30 and in bins of their own, one add each; ladders of up to 16 full-width stages with four query heads are content with that, as their weights had 18 bits before.
+// Integer sums are exact and the result does not depend on the order.  A weight is relative to a reference that lies a little (kHeadroom) above the largest score when it was last set; when a
 // score exceeds it, or the bins could overflow, they are folded into fp32 sums that every thread keeps in registers.  (With the
 // largest score itself as the reference, ten of the first sixteen segments set it anew.)
 //
@@ -42,7 +43,8 @@ constexpr int kDim = 128, kWords = 256, kRowBytes = 256;
 constexpr int kAreaBytes = kWords * kRowBytes;  // score table; histogram of large weights; of small weights
 // 4096 weights of at most 1 x kLarge, or of less than 2^-10 x kSmall, add up below 2^32
 constexpr float kLarge = 1048575.0f, kSmall = 1073740800.0f, kBorder = 0.0009765625f;
-constexpr float kHeadroom = 1.0f, kBack = 2.718281828459045f;  // natural-log units; e to that
+constexpr float kFine = 524288.0f, kRound = 8388608.0f, kRoundSigned = 12582912.0f;  // 2^19; adding them rounds to an integer
+constexpr float kHeadroom = 1.0f;  // natural-log units
 constexpr int kQueryFloats = kDim * 4 + 32 * 4;  // [group][channel of the group, one more][head]
 constexpr int kSmemBytes = 3 * kAreaBytes + (kQueryFloats + kWarps * 8 + 8) * 4;
 static_assert(kWarps * 4 * kDim * 4 <= kAreaBytes, "the warps' sums reuse a histogram");
@@ -129,10 +131,11 @@ __device__ __forceinline__ void permute_words(uint32_t (&w)[NW], int x) {
     }
 }
 
-// adds a token's weights w[r] at offsets to[r], heads in the lane's order; ALL: none of the block's heads is missing
-template <int P, bool FULL, bool ALL>
+// adds a token's weights w[r] (FINE: and rest[r] to the second bins) at offsets to[r], heads in the lane's order; ALL: none of the
+// block's heads is missing
+template <int P, bool FULL, bool FINE, bool ALL>
 __device__ __forceinline__ void add_weights(const uint32_t (&codes)[Shape<P>::kCodeWords], const uint32_t (&w)[Shape<P>::kHeads],
-                                            const uint32_t (&to)[Shape<P>::kHeads], const uint32_t (&sel)[4], uint32_t lane_xor, int x,
+                                            const uint32_t (&rest)[Shape<P>::kHeads], const uint32_t (&to)[Shape<P>::kHeads], const uint32_t (&sel)[4], uint32_t lane_xor, int x,
                                             int slots, int rot, int heads) {
     constexpr int H = Shape<P>::kHeads;
 #pragma unroll
@@ -141,11 +144,14 @@ __device__ __forceinline__ void add_weights(const uint32_t (&codes)[Shape<P>::kC
         const uint32_t at = (prmt(codes[k >> 2], 0u, sel[k & 3]) | (uint32_t)(k * Shape<P>::kEntry)) ^ lane_xor;
 #pragma unroll
         for (int r = 0; r < H; ++r)
-            if (ALL || ((r + rot) & (H - 1)) < heads) add_shared(at + to[r], w[r]);
+            if (ALL || ((r + rot) & (H - 1)) < heads) {
+                add_shared(at + to[r], w[r]);
+                if constexpr (FINE) add_shared(at + to[r] + kAreaBytes, rest[r]);
+            }
     }
 }
 
-template <int P, bool FULL>
+template <int P, bool FULL, bool FINE>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *__restrict__ ktab,
                   const __half *__restrict__ vtab, const int32_t *seq_start, const int32_t *seq_end, float *__restrict__ part, __half *__restrict__ out,
@@ -190,12 +196,15 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
             uint4 a[4], c8[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) a[c] = __ldg(row + 4 * c), c8[c] = __ldg(row + 8 * (kDim / 8) + 4 * c);
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            float part[4][4], acc[4];  // 32 channels each, added in fp32: the tensor core cuts off what it adds to a sum that is there
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                mma16816(acc, a[c].x, c8[c].x, a[c].y, c8[c].y, qf[c].x, qf[c].y);
-                mma16816(acc, a[c].z, c8[c].z, a[c].w, c8[c].w, qf[c].z, qf[c].w);
+                part[c][0] = part[c][1] = part[c][2] = part[c][3] = 0.0f;
+                mma16816(part[c], a[c].x, c8[c].x, a[c].y, c8[c].y, qf[c].x, qf[c].y);
+                mma16816(part[c], a[c].z, c8[c].z, a[c].w, c8[c].w, qf[c].z, qf[c].w);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] = (part[0][i] + part[1][i]) + (part[2][i] + part[3][i]);
             if (2 * kq < H) {
                 const int slot = tile / (kWords / 16), code = (tile % (kWords / 16)) * 16 + r8;
 #pragma unroll
@@ -289,7 +298,8 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
 #pragma unroll
             for (int u = 0; u < L::kCopies; ++u) {
                 uint32_t *large = reinterpret_cast<uint32_t *>(smem + kAreaBytes + at + u * P * L::kEntry), *small = large + kAreaBytes / 4;
-                v += fmaf((float)*small, 1.0f / kSmall, (float)*large * (1.0f / kLarge));
+                if constexpr (FINE) v += fmaf((float)(int32_t)*small, 1.0f / (kFine * kFine), (float)*large * (1.0f / kFine));
+                else v += fmaf((float)*small, 1.0f / kSmall, (float)*large * (1.0f / kLarge));
                 *large = 0u;
                 *small = 0u;
             }
@@ -306,20 +316,30 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
                 permute_words<NW>(kc[j], x);
-                unsigned long long pair[H / 2];  // two heads an addition
+                // two heads an addition; several short sums have less rounding than a long one
+                constexpr int kSums = P == 32 ? 4 : P >= 4 ? 2 : 1;
+                unsigned long long part[kSums][H / 2], pair[H / 2];
 #pragma unroll
-                for (int r = 0; r < H / 2; ++r) pair[r] = 0ull;
+                for (int r = 0; r < H / 2; ++r)
+#pragma unroll
+                    for (int i = 0; i < kSums; ++i) part[i][r] = 0ull;
 #pragma unroll
                 for (int k = 0; k < P; ++k) {
                     if (!FULL && (k ^ x) >= slots) continue;
                     const unsigned char *entry = smem + ((prmt(kc[j][k >> 2], 0u, sel[k & 3]) | (uint32_t)(k * L::kEntry)) ^ lane_xor);
                     if constexpr (H == 4) {
                         const ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(entry);
-                        pair[0] = add2(pair[0], e.x);
-                        pair[1] = add2(pair[1], e.y);
+                        part[k % kSums][0] = add2(part[k % kSums][0], e.x);
+                        part[k % kSums][1] = add2(part[k % kSums][1], e.y);
                     } else {
-                        pair[0] = add2(pair[0], *reinterpret_cast<const unsigned long long *>(entry));
+                        part[k % kSums][0] = add2(part[k % kSums][0], *reinterpret_cast<const unsigned long long *>(entry));
                     }
+                }
+#pragma unroll
+                for (int r = 0; r < H / 2; ++r) {
+                    pair[r] = part[0][r];
+                    if constexpr (kSums == 2) pair[r] = add2(pair[r], part[1][r]);
+                    if constexpr (kSums == 4) pair[r] = add2(add2(pair[r], part[1][r]), add2(part[2][r], part[3][r]));
                 }
 #pragma unroll
                 for (int r = 0; r < H; ++r) {
@@ -366,34 +386,42 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
         for (int j = 0; j < NT; ++j) {
             if (base + j * kThreads + tid >= hi) continue;
             permute_words<NW>(vc[j], x);
-            uint32_t w[H], to[H];
+            uint32_t w[H], rest[H], to[H];
 #pragma unroll
             for (int r = 0; r < H; ++r) {
                 const float p = __expf(sc[j][r] - m[r]);
                 l[r] += p;
-                const bool small = p < kBorder;
                 // to the nearest integer by adding 2^23 (a conversion runs at a quarter of the rate); a NaN's sum spoils the result
-                w[r] = __float_as_uint(fmaf(p, small ? kSmall : kLarge, 8388608.0f)) & 0x7fffffu;
-                to[r] = hist + r * 4 + (small ? kAreaBytes : 0);
+                if constexpr (FINE) {
+                    const float near = fmaf(p, kFine, kRound);
+                    w[r] = __float_as_uint(near) & 0x7fffffu;
+                    rest[r] = __float_as_uint(fmaf(fmaf(p, kFine, kRound - near), kFine, kRoundSigned)) - __float_as_uint(kRoundSigned);
+                    to[r] = hist + r * 4;
+                } else {
+                    const bool small = p < kBorder;
+                    w[r] = __float_as_uint(fmaf(p, small ? kSmall : kLarge, kRound)) & 0x7fffffu;
+                    rest[r] = 0u;
+                    to[r] = hist + r * 4 + (small ? kAreaBytes : 0);
+                }
             }
             if (rot & 1) {
-                const uint32_t w0 = w[0], t0 = to[0];
+                const uint32_t w0 = w[0], r0 = rest[0], t0 = to[0];
 #pragma unroll
-                for (int r = 0; r + 1 < H; ++r) w[r] = w[r + 1], to[r] = to[r + 1];
-                w[H - 1] = w0, to[H - 1] = t0;
+                for (int r = 0; r + 1 < H; ++r) w[r] = w[r + 1], rest[r] = rest[r + 1], to[r] = to[r + 1];
+                w[H - 1] = w0, rest[H - 1] = r0, to[H - 1] = t0;
             }
             if constexpr (H == 4) {
                 if (rot & 2) {
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
-                        const uint32_t wr = w[r], tr = to[r];
-                        w[r] = w[r + 2], to[r] = to[r + 2];
-                        w[r + 2] = wr, to[r + 2] = tr;
+                        const uint32_t wr = w[r], rr = rest[r], tr = to[r];
+                        w[r] = w[r + 2], rest[r] = rest[r + 2], to[r] = to[r + 2];
+                        w[r + 2] = wr, rest[r + 2] = rr, to[r + 2] = tr;
                     }
                 }
             }
-            if (heads == H) add_weights<P, FULL, true>(vc[j], w, to, sel, lane_xor, x, slots, rot, heads);
-            else add_weights<P, FULL, false>(vc[j], w, to, sel, lane_xor, x, slots, rot, heads);
+            if (heads == H) add_weights<P, FULL, FINE, true>(vc[j], w, rest, to, sel, lane_xor, x, slots, rot, heads);
+            else add_weights<P, FULL, FINE, false>(vc[j], w, rest, to, sel, lane_xor, x, slots, rot, heads);
         }
         if (base + NT * kThreads < hi) fetch(vc_row, base + NT * kThreads, vc);
     }
@@ -485,10 +513,11 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
         float top = m[0];
 #pragma unroll
         for (int k = 1; k < H; ++k) top = r == k ? m[k] : top;
-        // the state's reference is a score that was there
-        top -= kHeadroom;
-        lsum *= kBack;
-        asum *= kBack;
+        // the state's reference is a score that was there, as exactly as fp32 has it: the sums follow what the subtraction gave
+        const float ref = top - kHeadroom, back = top == -INFINITY ? 1.0f : expf(top - ref);
+        top = ref;
+        lsum *= back;
+        asum *= back;
         const int64_t row = (int64_t)b * Hq + head0 + r;
         if (splits == 1) {  // the whole row was handled here: this is the result
             if (out) out[row * kDim + channel] = __float2half_rn(lsum > 0.0f ? asum / lsum : 0.0f);
@@ -505,11 +534,11 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
     }
 }
 
-template <int P>
+template <int P, bool FINE>
 static int launch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
                   const int32_t *seq_start, const int32_t *seq_end, float *part, __half *out, float *state_out, int B, int Hq, int Hkv,
                   int G, int S, int64_t T_cap, int splits, bool after_prologue, cudaStream_t stream) {
-    auto kernel = S * G == P ? attn_slots_kernel<P, true> : attn_slots_kernel<P, false>;
+    auto kernel = S * G == P ? attn_slots_kernel<P, true, FINE> : attn_slots_kernel<P, false, FINE>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     const int rep = Hq / Hkv, head_groups = (rep + Shape<P>::kHeads - 1) / Shape<P>::kHeads;
@@ -548,17 +577,20 @@ int attn_slots_splits(int B, int Hq, int Hkv, int G, int S, int64_t visible, int
 int attn_slots_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
                         const int32_t *seq_start, const int32_t *seq_end, float *part, __half *out, float *state_out, int B, int Hq,
                         int Hkv, int G, int S, int64_t T_cap, int splits, bool after_prologue, cudaStream_t stream) {
-#define TACVQ_CASE(P)                                                                                                                 \
-    return slots::launch<P>(q, kcodes, vcodes, ktab, vtab, seq_start, seq_end, part, out, state_out, B, Hq, Hkv, G, S, T_cap, splits, \
-                            after_prologue, stream);
+#define TACVQ_LAUNCH(P, FINE)                                                                                                               \
+    slots::launch<P, FINE>(q, kcodes, vcodes, ktab, vtab, seq_start, seq_end, part, out, state_out, B, Hq, Hkv, G, S, T_cap, splits, \
+                           after_prologue, stream)
+#define TACVQ_CASE(P) return coarse ? TACVQ_LAUNCH(P, false) : TACVQ_LAUNCH(P, true);
     const int n = S * G;
+    const bool coarse = G == 1 && Hq == 4 * Hkv && n <= 16;
     if (n == 1) TACVQ_CASE(1)
     if (n == 2) TACVQ_CASE(2)
     if (n <= 4) TACVQ_CASE(4)
     if (n <= 8) TACVQ_CASE(8)
     if (n <= 16) TACVQ_CASE(16)
-    TACVQ_CASE(32)
+    return TACVQ_LAUNCH(32, true);
 #undef TACVQ_CASE
+#undef TACVQ_LAUNCH
 }
 
 }  // namespace tacvq

@@ -167,6 +167,40 @@ def test_tables_of_up_to_32_slots(device, b, hq, hkv, t, groups, stages, sub, or
     _check_state(state.cpu(), want_state)
 
 
+@pytest.mark.parametrize(
+    "b,hq,hkv,t,groups,stages,sub",
+    [
+        (2, 8, 2, 700, 16, 1, 8),
+        (2, 16, 4, 9000, 16, 1, 8),
+        (1, 4, 2, 2000, 32, 1, 4),
+        (2, 4, 2, 5000, 16, 2, 8),
+        (1, 8, 8, 3000, 16, 2, 8),
+        (1, 4, 2, 16384, 1, 2, 128),
+        (1, 8, 8, 8192, 1, 16, 128),
+        (2, 8, 2, 5000, 8, 3, 16),
+        (1, 4, 1, 3000, 1, 20, 128),
+    ],
+)
+def test_weights_have_the_precision_of_fp32(device, b, hq, hkv, t, groups, stages, sub):
+    """The state of attention without a rotary step against 64 bits, for logits over a range of about 30.
+
+    A weight is exp of an fp32 difference of at most 30 (2^-24 of it, 1.8e-6) by exp2 with two units in the last place (1.2e-7 each); the
+    errors of different tokens are not alike, so a weighted mean has less than a single weight's.
+    """
+    gen = torch.Generator().manual_seed(t + stages)
+    scales = [0.5 * 0.8**s for s in range(stages)] if sub <= 16 else [0.6 / stages**0.5] * stages
+    ktab, vtab = (make_tables(gen, hkv, stages, groups, sub, scales) for _ in range(2))
+    codes = [torch.randint(0, 256, (b, hkv, t, stages, groups), generator=gen, dtype=torch.uint8) for _ in range(2)]
+    q = (4 * torch.randn(b, hq, 128, generator=gen) / 128**0.5).half()
+    _, state = _run(device, (q, *codes, ktab, vtab), want_out=False, want_state=True)
+    heads, at = torch.arange(hkv)[None, :, None, None], torch.arange(groups)
+    rows = [sum(tab.double()[heads, s, at, c[:, :, :, s].long()] for s in range(stages)).flatten(3).repeat_interleave(hq // hkv, 1) for c, tab in zip(codes, (ktab, vtab))]
+    score = torch.einsum("bhd,bhtd->bht", q.double(), rows[0])
+    weight = score.softmax(-1)
+    state = state.cpu().double()
+    assert rel_l2(state[..., 2:] / state[..., 1:2], torch.einsum("bht,bhtd->bhd", weight, rows[1])) <= 1.5e-6
+    torch.testing.assert_close(state[..., 0] + state[..., 1].log(), score.logsumexp(-1), rtol=0, atol=4e-6)
+
 def test_partial_states_merge_to_the_whole(device):
     """Sequence split as ranks would do it: per-range states, then the log-sum-exp merge."""
     ops = _ops()
