@@ -168,6 +168,29 @@ def test_rotary_attention_over_deep_ladders(device, b, hq, hkv, stages, t, range
         assert not out[row].any() and (state[row, :, 0] == -float("inf")).all() and not state[row, :, 1:].any()
 
 
+@pytest.mark.parametrize("b,hq,hkv,stages,t", [(1, 4, 1, 16, 4096), (2, 8, 4, 16, 700), (1, 2, 2, 8, 3000), (2, 8, 2, 4, 9000)])
+def test_ladder_weights_have_the_precision_of_fp32(device, b, hq, hkv, stages, t):
+    """The state against 64 bits, for logits over a range of about 30 and a rotary table that turns nothing: keys are the sums of their
+    words in fp16, values the sums themselves.
+
+    A weight is exp of an fp32 difference of at most 30 (2^-24 of it, 1.8e-6) by exp2 with two units in the last place (1.2e-7 each); the
+    errors of different tokens are not alike, so a weighted mean has less than a single weight's.
+    """
+    ops = _ops()
+    gen = torch.Generator().manual_seed(stages * t)
+    ktab, vtab = (make_tables(gen, hkv, stages, 1, 128, [1.2 / stages] * stages) for _ in range(2))
+    codes = [torch.randint(0, 256, (b, hkv, t, stages, 1), generator=gen, dtype=torch.uint8) for _ in range(2)]
+    q = (6 * torch.randn(b, hq, 128, generator=gen) / 128**0.5).half()
+    still = torch.zeros(t, 2, 64, dtype=torch.float16, device=device)
+    still[:, 0] = 1.0
+    _, state = ops.attn_decode(q.to(device), *(x.to(device) for x in (*codes, ktab, vtab)), rope=still, want_out=False, want_state=True)
+    heads = torch.arange(hkv)[None, :, None]
+    key, value = (sum(tab[:, s, 0].double()[heads, c[:, :, :, s, 0].long()] for s in range(stages)).repeat_interleave(hq // hkv, 1) for c, tab in zip(codes, (ktab, vtab)))
+    score = torch.einsum("bhd,bhtd->bht", q.double(), key.half().double())
+    state = state.cpu().double()
+    assert rel_l2(state[..., 2:] / state[..., 1:2], torch.einsum("bht,bhtd->bhd", score.softmax(-1), value)) <= 1.5e-6
+    torch.testing.assert_close(state[..., 0] + state[..., 1].log(), score.logsumexp(-1), rtol=0, atol=4e-6)
+
 @pytest.mark.parametrize(
     "batch,heads,q_heads,groups,stages,sub,max_tokens,window,first,new",
     [
