@@ -243,6 +243,21 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                         const uint32_t one = r8 == t ? 0x3c003c00u : 0u;
                         mma16816(sum, m[t][0], m[t][2], m[t][1], m[t][3], one, one);
                     }
+                    // The zeros in the other tokens' columns do not hide a word that is not finite (0 x inf): then every token's words
+                    // are added without the others'.
+                    if (__any_sync(0xffffffffu, !(fabsf((sum[0] + sum[1]) + (sum[2] + sum[3])) < INFINITY))) {
+#pragma unroll 1
+                        for (int j = 0; j < 4; ++j) {  // channel r8 or its partner of token 2kq + j % 2
+                            float alone = 0.0f;
+#pragma unroll 1
+                            for (int st = 0; st < S; ++st) {
+                                const uint32_t word = __shfl_sync(0xffffffffu, code[u], (2 * kq + (j & 1)) * 4 + (st >> 2)) >> (8 * (st & 3)) & 255u;
+                                alone += __half2float(*reinterpret_cast<const __half *>(smem + word * kRowBytes + (j >> 1) * (kStages * 16) + st * 16 + r8 * 2));
+                            }
+                            sum[0] = j == 0 ? alone : sum[0], sum[1] = j == 1 ? alone : sum[1];
+                            sum[2] = j == 2 ? alone : sum[2], sum[3] = j == 3 ? alone : sum[3];
+                        }
+                    }
                     // round, rotate (k cos + rotate_half(k) sin, products and sum in fp16)
                     const __half2 kl = __floats2half2_rn(sum[0], sum[1]), kh = __floats2half2_rn(sum[2], sum[3]);
                     const __half2 cosv = *reinterpret_cast<const __half2 *>(&turn[u][0]), sinv = *reinterpret_cast<const __half2 *>(&turn[u][1]);

@@ -168,6 +168,22 @@ def test_rotary_attention_over_deep_ladders(device, b, hq, hkv, stages, t, range
         assert not out[row].any() and (state[row, :, 0] == -float("inf")).all() and not state[row, :, 1:].any()
 
 
+@pytest.mark.parametrize("stages,word", [(4, float("inf")), (16, float("inf")), (12, float("-inf"))])
+def test_an_infinite_key_word_of_a_ladder_stays_with_its_token(device, stages, word):
+    """A token whose score is -inf has no weight; the tokens beside it keep theirs."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(stages)
+    kcodes, vcodes = (torch.randint(0, 255, (1, 2, 100, stages, 1), generator=gen, dtype=torch.uint8) for _ in range(2))
+    ktab, vtab = (make_tables(gen, 2, stages, 1, 128, [0.3 * 0.85**s for s in range(stages)]) for _ in range(2))
+    q = (torch.randn(1, 8, 128, generator=gen) / 128**0.5).half()
+    q[:, :, [5, 69]] = -0.1 if word > 0 else 0.1  # at position 1 channel 5 and its partner both get words of that sign
+    ktab[:, stages - 2, 0, 255, 5] = word
+    kcodes[:, :, 1, stages - 2, 0] = 255
+    want, *_ = O.attention_over_codes(q, kcodes, vcodes, ktab, vtab, rope_theta=1e6)
+    assert bool(want.isfinite().all())
+    out, _ = ops.attn_decode(*(x.to(device) for x in (q, kcodes, vcodes, ktab, vtab)), rope=ops.rope_table(100, 128, 1e6, device))
+    _check(out.float().cpu(), want)
+
 @pytest.mark.parametrize("b,hq,hkv,stages,t", [(1, 4, 1, 16, 4096), (2, 8, 4, 16, 700), (1, 2, 2, 8, 3000), (2, 8, 2, 4, 9000)])
 def test_ladder_weights_have_the_precision_of_fp32(device, b, hq, hkv, stages, t):
     """The state against 64 bits, for logits over a range of about 30 and a rotary table that turns nothing: keys are the sums of their
