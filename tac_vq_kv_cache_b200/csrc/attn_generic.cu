@@ -146,7 +146,7 @@ attn_generic_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kc
         } else {
             for (int w = 0; w < kAttnWarps; ++w) {
                 const float mw = wm[w * REP + r];
-                if (mw == -INFINITY) continue;
+                if (wl[w * REP + r] == 0.0f) continue;  // no token; a sum that is NaN spoils the others
                 const float scale = __expf(mw - top);
                 sum += scale * (col == 1 ? wl[w * REP + r] : wacc[((size_t)w * REP + r) * D + (col - 2)]);
             }
@@ -181,8 +181,8 @@ attn_combine_kernel(const float *states, int n_parts, int64_t rows, int D, __hal
     for (int w = 0; w < warps; ++w) top = fmaxf(top, red[w]);
     float l = 0.0f;
     for (int p = tid; p < n_parts; p += blockDim.x) {
-        const float m = own[p * stride];
-        if (m != -INFINITY) l += __expf(m - top) * own[p * stride + 1];
+        const float part = own[p * stride + 1];
+        if (part != 0.0f) l += __expf(own[p * stride] - top) * part;  // 0: no token there
     }
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
@@ -206,7 +206,7 @@ attn_combine_kernel(const float *states, int n_parts, int64_t rows, int D, __hal
         if (group == 0 && i < D) {
             for (int g = 1; g < groups; ++g) a += sums[g * kCombineLanes + at];
             if (merged) merged[row * W + 2 + i] = a;
-            if (out) out[row * D + i] = __float2half_rn(l > 0.0f ? a / l : 0.0f);
+            if (out) out[row * D + i] = __float2half_rn(l == 0.0f ? 0.0f : a / l);
         }
         __syncthreads();
     }

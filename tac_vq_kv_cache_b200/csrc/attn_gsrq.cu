@@ -443,14 +443,18 @@ __device__ void merge_pair_parts(const float *part, int first, int n_parts, int 
 #pragma unroll
             for (int i = 0; i < 8; ++i)
                 if (i0 + i < n_parts) ntop = fmaxf(ntop, mc[i]);
-            if (ntop == -INFINITY) continue;
+            if (ntop == -INFINITY) {  // no score above -inf so far: sums that are 0 or NaN
+                for (int i = 0; i < 8; ++i)
+                    if (i0 + i < n_parts) lsum += lc[i];
+                continue;
+            }
             const float f = __expf(top - ntop);  // 0 while nothing has been added yet
             lsum *= f;
             asum *= f;
             top = ntop;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                if (i0 + i < n_parts && mc[i] != -INFINITY) {
+                if (i0 + i < n_parts && lc[i] != 0.0f) {
                     const float sc = __expf(mc[i] - top);
                     lsum += sc * lc[i];
                     asum += sc * ac[i];
@@ -458,7 +462,7 @@ __device__ void merge_pair_parts(const float *part, int first, int n_parts, int 
             }
         }
         const size_t row = (size_t)b * Hq + h * kRep + r;
-        if (out) out[row * kDim + dim] = __float2half_rn(lsum > 0.0f ? asum / lsum : 0.0f);
+        if (out) out[row * kDim + dim] = __float2half_rn(lsum == 0.0f ? 0.0f : asum / lsum);
         if (state_out) {
             float *dst = state_out + row * kStateWidth;
             if (dim == 0) {
@@ -884,7 +888,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             float lsum = 0.0f, asum = 0.0f;
             for (int w = 0; w < kWarps; ++w) {
                 const float mw = wm[w * kRep + r];
-                if (mw == -INFINITY) continue;
+                if (wl[w * kRep + r] == 0.0f) continue;  // no token; a sum that is NaN spoils the others
                 const float sc = fast_exp2(mw - top);
                 lsum += sc * wl[w * kRep + r];
                 const float *src = wacc + (size_t)w * 1024;
@@ -892,7 +896,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             }
             if (n_parts == 1) {  // the whole pair was scanned here: this is the result
                 const size_t row = (size_t)b * Hq + h * kRep + r;
-                if (out) out[row * kDim + dim] = __float2half_rn(lsum > 0.0f ? asum / lsum : 0.0f);
+                if (out) out[row * kDim + dim] = __float2half_rn(lsum == 0.0f ? 0.0f : asum / lsum);
                 if (state_out) {
                     float *dst = state_out + row * kStateWidth;
                     if (dim == 0) {

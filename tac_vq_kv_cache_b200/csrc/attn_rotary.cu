@@ -222,7 +222,7 @@ attn_rotary_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kco
         } else {
             for (int w = 0; w < kHalfWarps; ++w) {
                 const float mw = wm[w * REP + r];
-                if (mw == -INFINITY) continue;
+                if (wl[w * REP + r] == 0.0f) continue;  // no token; a sum that is NaN spoils the others
                 const float scale = __expf(mw - top);
                 sum += scale * (col == 1 ? wl[w * REP + r] : wacc[((size_t)w * REP + r) * D + (col - 2)]);
             }

@@ -448,7 +448,7 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
                 lsum += red_s[kRedFloats + w * 4 + r];
             }
             dst[0] = top;
-            dst[1] = top == -INFINITY ? 0.0f : lsum;
+            dst[1] = limit_s[br].x < limit_s[br].y ? lsum : 0.0f;  // without a token there is no maximum, and weights that mean nothing
         }
     }
 }

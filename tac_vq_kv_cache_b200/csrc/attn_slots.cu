@@ -520,7 +520,7 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
         asum *= back;
         const int64_t row = (int64_t)b * Hq + head0 + r;
         if (splits == 1) {  // the whole row was handled here: this is the result
-            if (out) out[row * kDim + channel] = __float2half_rn(lsum > 0.0f ? asum / lsum : 0.0f);
+            if (out) out[row * kDim + channel] = __float2half_rn(lsum == 0.0f ? 0.0f : asum / lsum);
             if (state_out) {
                 float *dst = state_out + row * (kDim + 2);
                 if (channel == 0) dst[0] = top, dst[1] = lsum;

@@ -201,6 +201,40 @@ def test_weights_have_the_precision_of_fp32(device, b, hq, hkv, t, groups, stage
     assert rel_l2(state[..., 2:] / state[..., 1:2], torch.einsum("bht,bhtd->bhd", weight, rows[1])) <= 1.5e-6
     torch.testing.assert_close(state[..., 0] + state[..., 1].log(), score.logsumexp(-1), rtol=0, atol=4e-6)
 
+@pytest.mark.parametrize("t", [40, 3000])  # one block a row and head, several
+@pytest.mark.parametrize(
+    "hq,hkv,groups,stages,sub,rotary",
+    [
+        (8, 2, 16, 2, 8, False),
+        (4, 2, 16, 2, 8, False),
+        (8, 2, 1, 2, 128, False),
+        (8, 2, 1, 16, 128, False),
+        (2, 2, 32, 1, 4, False),
+        (8, 2, 8, 2, 8, False),     # head_dim 64
+        (16, 2, 8, 1, 16, False),   # eight query heads per KV head
+        (8, 2, 16, 2, 8, True),
+        (8, 2, 1, 16, 128, True),
+        (8, 2, 1, 2, 128, True),
+        (8, 2, 1, 3, 128, True),
+    ],
+)
+def test_a_query_that_is_not_a_number_spoils_its_own_rows_only(device, hq, hkv, groups, stages, sub, rotary, t):
+    ops = _ops()
+    q, kcodes, vcodes, ktab, vtab = _workload(t, 3, hq, hkv, t, groups, stages, sub, [0.3 * 0.8**s for s in range(stages)] if sub >= 16 else None)
+    start, end = [0, 0, 5], [t, t - 3, 5]
+    rope = ops.rope_table(t, groups * sub, 1e6, device) if rotary else None
+    want, _ = _run(device, (q, kcodes, vcodes, ktab, vtab), start, end, rope=rope)
+    q[0, hq - 1, 7] = float("nan")
+    q[1, 0] = float("nan")
+    q[2, 1, 0] = float("nan")
+    out, state = _run(device, (q, kcodes, vcodes, ktab, vtab), start, end, rope=rope, want_state=True)
+    bad = torch.zeros(3, hq, dtype=torch.bool)
+    bad[0, hq - 1] = bad[1, 0] = True
+    out, state = out.cpu(), state.cpu()
+    assert bool(out[bad].isnan().all()) and bool(state[..., 1][bad].isnan().all())
+    _check(out[:2][~bad[:2]], want.cpu()[:2][~bad[:2]])
+    assert bool((out[2] == 0).all()) and bool((state[2, :, 1] == 0).all())  # a row that sees nothing has no use for its query
+
 def test_partial_states_merge_to_the_whole(device):
     """Sequence split as ranks would do it: per-range states, then the log-sum-exp merge."""
     ops = _ops()
