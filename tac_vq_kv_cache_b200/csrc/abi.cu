@@ -382,7 +382,7 @@ static int attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, cons
                                                  splits, s);
         }
     }
-    if (splits == 0) {
+    if (st == TACVQ_OK && splits == 0) {  // none of these kernels took the call
         splits = attn_rotary_splits(B, Hkv, T_cap, sm_count());
         st = attn_rotary_dispatch(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, D, G, S, K, T_cap, splits, s);
     }

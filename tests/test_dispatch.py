@@ -1,0 +1,131 @@
+"""Which kernel the C ABI hands a call to, and what it makes of its status (CPU).
+
+abi.cu is compiled by itself and linked with stand-ins for the kernels' launchers, which write down how they were called and
+return what the test tells them to.
+"""
+
+from __future__ import annotations
+
+import ctypes
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+PACKAGE = ROOT / "tac_vq_kv_cache_b200"
+
+STAND_INS = r"""
+#include <map>
+#include <string>
+#include "common.cuh"
+namespace {
+std::string calls;
+std::map<std::string, int> told;  // status, or number of splits
+int called(const char *name, long long a = -1, long long b = -1) {
+    calls += std::string(name) + " " + std::to_string(a) + " " + std::to_string(b) + "\n";
+    auto it = told.find(name);
+    return it == told.end() ? 0 : it->second;
+}
+int splits_of(const char *name) { auto it = told.find(std::string(name) + ".splits"); return it == told.end() ? 3 : it->second; }
+}
+extern "C" __attribute__((visibility("default"))) const char *stand_in_calls() { return calls.c_str(); }
+extern "C" __attribute__((visibility("default"))) void stand_in_reset() { calls.clear(); told.clear(); }
+extern "C" __attribute__((visibility("default"))) void stand_in_tell(const char *name, int value) { told[name] = value; }
+namespace tacvq {
+int encode_dispatch(const EncodeArgs &) { return called("encode"); }
+int decode_dispatch(const uint8_t *, const __half *, void *, int, int, int, int, int, int, int, int, int, int64_t, int64_t, cudaStream_t) { return called("decode"); }
+int codeword_grad_dispatch(const uint8_t *, const float *, float *, int, int, int, int, int, int, int, int, int64_t, int64_t, cudaStream_t) { return called("grad"); }
+int table_sqnorm_dispatch(const __half *, float *, int64_t, int, cudaStream_t) { return called("sqnorm"); }
+int tensor_memory_timeouts(unsigned int *) { return 0; }
+int round_words_dispatch(const float *, __half *, float *, int64_t, int, cudaStream_t) { return called("round_words"); }
+int whiten_dispatch(const void *, int, int64_t, int64_t, int64_t, const __half *, const float *, float *, float *, int, int, int, int, int, int, int, cudaStream_t) { return called("whiten"); }
+int rope_table_dispatch(__half *, int64_t, int, double, int64_t, cudaStream_t) { return called("rope"); }
+int decode_prologue_dispatch(const void *, const void *, int, int64_t, int64_t, int64_t, const __half *, const __half *, uint8_t *, uint8_t *, int32_t *,
+                             int32_t *, int start, int end, int, int, int, int, int, int, int, int64_t, int64_t, cudaStream_t) { return called("prologue", start, end); }
+int attn_generic_splits(int, int, int64_t, int) { return splits_of("generic"); }
+int attn_generic_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const int32_t *, const int32_t *, float *, int,
+                          int, int, int, int, int, int, int64_t, int, cudaStream_t) { return called("generic"); }
+int attn_combine_dispatch(const float *, int n, __half *, float *, int64_t, int, cudaStream_t) { return called("combine", n); }
+bool attn_slots_supported(int, int Hq, int Hkv, int D, int G, int S, int K) { return D == 128 && K == 256 && S * G <= 32 && Hq / Hkv <= 4; }
+int attn_slots_splits(int, int, int, int, int, int64_t visible, int) { calls += "slots.plan " + std::to_string(visible) + "\n"; return splits_of("slots"); }
+int attn_slots_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const int32_t *, const int32_t *, float *, __half *,
+                        float *, int, int, int, int, int, int64_t, int splits, bool after, cudaStream_t) { return called("slots", splits, after); }
+bool attn_gsrq_supported(int Hq, int Hkv, int D, int G, int S, int K) { return D == 128 && G == 16 && S == 2 && K == 256 && Hq == 4 * Hkv; }
+size_t attn_gsrq_workspace_bytes(int, int, int, int, int) { return 0; }
+int attn_gsrq_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const int32_t *, const int32_t *, void *, __half *,
+                       float *, int, int, int, int64_t, int, cudaStream_t, const GsrqNewToken *) { return called("gsrq"); }
+int attn_rotary_splits(int, int, int64_t, int) { return splits_of("rotary"); }
+int attn_rotary_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const __half *, const int32_t *, const int32_t *,
+                         float *, int, int, int, int, int, int, int, int64_t, int, cudaStream_t) { return called("rotary"); }
+bool attn_rotary_staged_supported(int, int, int D, int G, int S, int) { return D == 128 && S <= 2 && D / G >= 4; }
+int attn_rotary_staged_splits(int, int, int64_t, int) { return splits_of("staged"); }
+int attn_rotary_staged_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const __half *, const int32_t *,
+                                const int32_t *, float *, int, int, int, int, int, int64_t, int, cudaStream_t) { return called("staged"); }
+bool attn_rotary_mma_supported(int, int, int D, int G, int S, int) { return D == 128 && G == 16 && S == 2; }
+int attn_rotary_mma_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const __half *, const int32_t *, const int32_t *,
+                             float *, int, int, int, int64_t, int64_t visible, int, bool, int *splits, cudaStream_t) { *splits = splits_of("mma"); return called("mma", visible); }
+bool attn_rotary_ladder_supported(int, int, int D, int G, int S, int) { return D == 128 && G == 1 && S >= 4 && S <= 16; }
+int attn_rotary_ladder_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const __half *, const int32_t *, const int32_t *,
+                                float *, int, int, int, int, int64_t, int64_t visible, const LadderStep &step, int *splits, cudaStream_t) {
+    *splits = splits_of("ladder");
+    return called("ladder", visible, step.fresh);
+}
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    from tac_vq_kv_cache_b200 import _lib, build
+
+    if not (shutil.which("nvcc") or Path("/usr/local/cuda/bin/nvcc").exists()):
+        pytest.skip("no nvcc")
+    folder = tmp_path_factory.mktemp("dispatch")
+    (folder / "stand_ins.cu").write_text(STAND_INS)
+    target = folder / "libdispatch.so"
+    done = subprocess.run([build.nvcc(), *build.NVCC_FLAGS, "-shared", str(PACKAGE / "csrc" / "abi.cu"), str(folder / "stand_ins.cu"), "-o", str(target)],
+                          capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr
+    lib = ctypes.CDLL(str(target), mode=ctypes.RTLD_LOCAL)
+    for name, (restype, argtypes) in _lib._SIGNATURES.items():
+        getattr(lib, name).restype, getattr(lib, name).argtypes = restype, argtypes
+    lib.stand_in_calls.restype = ctypes.c_char_p
+    lib.stand_in_tell.argtypes = [ctypes.c_char_p, ctypes.c_int]
+    return lib
+
+
+def _calls(lib):
+    return [line.split() for line in lib.stand_in_calls().decode().splitlines()]
+
+
+def _attend(lib, groups, stages, *, rope, t_cap=1000, batch=1, hq=8, hkv=2):
+    dim, at = 128, 1 << 20  # addresses that nobody follows
+    need = lib.tacvq_attn_workspace_bytes(batch, hq, hkv, dim, groups, stages)
+    tail = (at, need, at, 0, batch, hq, hkv, dim, groups, stages, 256, t_cap, 0)
+    if rope:
+        return lib.tacvq_attn_decode_rotary(at, at, at, at, at, at, 0, 0, *tail)
+    return lib.tacvq_attn_decode(at, at, at, at, at, 0, 0, *tail)
+
+
+@pytest.mark.parametrize("kernel,groups,stages", [("ladder", 1, 16), ("mma", 16, 2), ("staged", 16, 1)])
+def test_a_rotary_launch_that_fails_is_the_calls_status(library, kernel, groups, stages):
+    """No other kernel is tried after an error: it would hide it, or fail for it."""
+    for splits in (0, 3):
+        library.stand_in_reset()
+        library.stand_in_tell(kernel.encode(), 98)
+        library.stand_in_tell(f"{kernel}.splits".encode(), splits)
+        status = _attend(library, groups, stages, rope=True)
+        if kernel == "staged" and splits == 0:  # does not take such a size, and is not launched
+            assert status == 0 and [c[0] for c in _calls(library)] == ["rotary", "combine"]
+        else:
+            assert status == 98 and [c[0] for c in _calls(library)] == [kernel]
+
+
+@pytest.mark.parametrize("kernel,groups,stages", [("ladder", 1, 16), ("mma", 16, 2), ("staged", 16, 1)])
+def test_a_rotary_kernel_that_steps_aside_leaves_the_call_to_the_general_one(library, kernel, groups, stages):
+    library.stand_in_reset()
+    library.stand_in_tell(f"{kernel}.splits".encode(), 0)
+    assert _attend(library, groups, stages, rope=True) == 0
+    assert [c[0] for c in _calls(library) if c[0] != kernel] == ["rotary", "combine"]
