@@ -38,7 +38,7 @@
 //            4096 codewords x 4 heads straight from the fp16 K tables, quantised to 13 bits), written to
 //            scratch in the order the scan's shared memory wants; its share of the V codewords in that
 //            order; and, in a decode step, the codes of the pair's new K or V row and the visible ranges.  Blocks on SMs
-//            without a pair only share the V codewords.  A build costs about 3.5 us of a 512-thread
+//            without a pair encode the rows and share the V codewords.  A build costs about 3.5 us of a 512-thread
 //            block per stage (64 values per thread, quarter-rate conversions); building inside the scan
 //            was measured twice and repeats that for every block that enters a pair (3.3 per pair).
 //            One row of 777 tokens takes 13.0 us a step (16.0 before the V codewords were shared by all SMs and
@@ -208,14 +208,23 @@ constexpr int kPrepThreads = 512;
 constexpr int kPrepWarps = kPrepThreads / 32;
 constexpr int kPrepCodes = kWords / (2 * kPrepWarps);  // codes per thread
 
+// APART: a block of the first 2 * B * Hkv builds a table, and one of as many again encodes a row beside it, which makes the chain of a small
+// batch shorter (one row of 777 tokens 15.8 us a step, 17.4 with both in one block, one after the other).
+template <bool APART>
 __global__ void __launch_bounds__(kPrepThreads)
-attn_gsrq_prepare_kernel(const __half *__restrict__ q, const __half *__restrict__ ktab, const __half *__restrict__ vtab,
+attn_gsrq_prepare_kernel(const __half *q, const __half *ktab, const __half *vtab,
                          uint2 *__restrict__ lut_g, float *__restrict__ scale_g, uint4 *__restrict__ vperm_g, int B, int Hkv, const NewToken fresh) {
     __shared__ float red[kPrepWarps * 8 * kGroups];  // [warp][min x4, max x4][group]
     __shared__ __align__(16) float low_s[kGroups * kRep], step_s[12];  // smallest entry per group and head; per head 1 / step, step, offset
     launch_dependents();  // the scan may be scheduled as soon as SMs free up; it waits for this grid itself
+    // The launch before this one may be what computes the query, the rows or the tables, and let this grid start before it has stored
+    // them (a scan does, and so may a matrix product of another library); a scan also still reads the scratch that is written here.
+    wait_for_previous_kernel();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int pair = blockIdx.x >> 1, stage = blockIdx.x & 1;
+    const int tables = 2 * B * Hkv, own = (int)blockIdx.x % tables;
+    const bool builds = (int)blockIdx.x < tables;
+    const bool encodes = fresh.k_rows != nullptr && (APART ? (int)blockIdx.x / tables == 1 : builds);
+    const int pair = own >> 1, stage = own & 1;
     const int h = pair / B, b = pair % B;
     const int Hq = Hkv * kRep;
     const int g = lane & 15, half = lane >> 4;
@@ -228,40 +237,35 @@ attn_gsrq_prepare_kernel(const __half *__restrict__ q, const __half *__restrict_
             if (e < perm_total) {
                 const int hh = e >> 13, code = (e >> 5) & 255, pos = e & 31;
                 const int s = (pos >> 2) & 1, gg = ((pos >> 3) << 2) | (pos & 3);
-                vperm_g[e] = __ldg(reinterpret_cast<const uint4 *>(vtab + ((((size_t)hh * kStages + s) * kGroups + gg) * kWords + code) * kSub));
+                vperm_g[e] = *reinterpret_cast<const uint4 *>(vtab + ((((size_t)hh * kStages + s) * kGroups + gg) * kWords + code) * kSub);
             }
         }
     };
-    if (pair >= B * Hkv) {  // few pairs: blocks that only share the permutation
-        wait_for_previous_kernel();
-        permute_values();
-        return;
-    }
 #endif
     // A decode step's new token: this block (pair, side = stage) encodes the 16 groups of the pair's new K
     // (side 0) or V (side 1) row, a warp per group, with the arithmetic of the row-at-a-time encode kernel.
-    // The words of both stages are requested at once (one memory latency instead of two); the codes are kept
-    // in registers and stored after the wait below.  None of these inputs is produced by this chain.
-    // inputs of the table build, which are not produced by the kernels of this chain either
+    // The words of both stages are requested at once (one memory latency instead of two).
+    // inputs of the table build
     const uint4 *tab = reinterpret_cast<const uint4 *>(ktab + (((size_t)h * kStages + stage) * kGroups + g) * kWords * kSub);
     uint4 raw[kPrepCodes], qraw[kRep];
     auto fetch_build = [&]() {
 #pragma unroll
-        for (int c = 0; c < kPrepCodes; ++c) raw[c] = __ldg(tab + warp * 2 + half + 2 * kPrepWarps * c);
+        for (int c = 0; c < kPrepCodes; ++c) raw[c] = tab[warp * 2 + half + 2 * kPrepWarps * c];
 #pragma unroll
-        for (int r = 0; r < kRep; ++r) qraw[r] = __ldg(reinterpret_cast<const uint4 *>(q + ((size_t)b * Hq + h * kRep + r) * kDim + g * kSub));
+        for (int r = 0; r < kRep; ++r) qraw[r] = *reinterpret_cast<const uint4 *>(q + ((size_t)b * Hq + h * kRep + r) * kDim + g * kSub);
     };
-    int fresh_code[kStages] = {0, 0};
-    if (fresh.k_rows != nullptr) {
+    if (builds && (APART || !encodes)) fetch_build();
+    if (encodes) {
+        int fresh_code[kStages] = {0, 0};
         static_assert(kPrepWarps == kGroups && kStages == 2 && kWords == 256, "a warp per group, 8 words per lane and stage");
         const __half *side_tab = stage ? vtab : ktab;
         const uint4 *words0 = reinterpret_cast<const uint4 *>(side_tab + (((size_t)h * kStages + 0) * kGroups + warp) * kWords * kSub);
         const uint4 *words1 = words0 + (size_t)kGroups * kWords;
         uint4 w0[8], w1[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) w0[i] = __ldg(words0 + lane + 32 * i);
+        for (int i = 0; i < 8; ++i) w0[i] = words0[lane + 32 * i];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) w1[i] = __ldg(words1 + lane + 32 * i);
+        for (int i = 0; i < 8; ++i) w1[i] = words1[lane + 32 * i];
         const size_t at = ((size_t)b * Hkv + h) * kDim + warp * kSub;
         float res[kSub];
         if (fresh.rows_f32) {
@@ -283,15 +287,30 @@ attn_gsrq_prepare_kernel(const __half *__restrict__ q, const __half *__restrict_
             const int from = fresh_code[0] & 31;
             mine = make_uint4(__shfl_sync(0xffffffffu, mine.x, from), __shfl_sync(0xffffffffu, mine.y, from),
                               __shfl_sync(0xffffffffu, mine.z, from), __shfl_sync(0xffffffffu, mine.w, from));
-            fetch_build();
+            if (!APART) fetch_build();
             float c[kSub];
             unpack8(mine, c);
 #pragma unroll
             for (int i = 0; i < kSub; ++i) res[i] = __fsub_rn(res[i], c[i]);
         }
         fresh_code[1] = nearest_of_fetched_words(res, w1, lane);
-    } else {
-        fetch_build();
+        if (lane == 0) {
+            uint8_t *dst = (stage ? fresh.vcodes : fresh.kcodes) + (((size_t)b * Hkv + h) * (size_t)fresh.T_cap + (size_t)fresh.position) * kSlots;
+#pragma unroll
+            for (int s = 0; s < kStages; ++s) dst[s * kGroups + warp] = (uint8_t)fresh_code[s];
+        }
+    }
+    if (fresh.k_rows != nullptr && blockIdx.x == 0) {
+        for (int i = tid; i < B; i += kPrepThreads) {
+            fresh.seq_start[i] = fresh.start;
+            fresh.seq_end[i] = fresh.end;
+        }
+    }
+    if (!builds) {
+#if TACVQ_GSRQ_VPERM
+        permute_values();
+#endif
+        return;
     }
     float qv[kRep][kSub];
 #pragma unroll
@@ -383,23 +402,6 @@ attn_gsrq_prepare_kernel(const __half *__restrict__ q, const __half *__restrict_
         }
         packed[c][0] = e[0] | (e[1] << 16);
         packed[c][1] = e[2] | (e[3] << 16);
-    }
-    // The scratch written below is read by the scan of the call before this one, which may still be
-    // running when this grid starts: wait for everything before this grid, then write.
-    wait_for_previous_kernel();
-    if (fresh.k_rows != nullptr) {
-        // the scan before this grid read the ranges and the code buffers up to its own end; both may change now
-        if (lane == 0) {
-            uint8_t *dst = (stage ? fresh.vcodes : fresh.kcodes) + (((size_t)b * Hkv + h) * (size_t)fresh.T_cap + (size_t)fresh.position) * kSlots;
-#pragma unroll
-            for (int s = 0; s < kStages; ++s) dst[s * kGroups + warp] = (uint8_t)fresh_code[s];
-        }
-        if (blockIdx.x == 0) {
-            for (int i = tid; i < B; i += kPrepThreads) {
-                fresh.seq_start[i] = fresh.start;
-                fresh.seq_end[i] = fresh.end;
-            }
-        }
     }
 #pragma unroll
     for (int c = 0; c < kPrepCodes; ++c) {
@@ -1008,9 +1010,10 @@ int attn_gsrq_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vc
         e = cudaFuncSetAttribute(gsrq::attn_gsrq_scan_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return (int)e;
-        e = cudaFuncSetAttribute(gsrq::attn_gsrq_prepare_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return (int)e;
+        for (auto prepare : {gsrq::attn_gsrq_prepare_kernel<false>, gsrq::attn_gsrq_prepare_kernel<true>}) {
+            e = cudaFuncSetAttribute(prepare, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            if (e != cudaSuccess) return (int)e;
+        }
         if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
     }
     const GsrqWorkspace ws(B, Hkv, sms);
@@ -1022,10 +1025,11 @@ int attn_gsrq_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vc
     const unsigned long long epoch = g_epoch.fetch_add(2, std::memory_order_relaxed);  // odd, so never 0 (= cleared)
     GsrqNewToken token = {};
     if (fresh) token = *fresh;
-    // a block per pair and stage; where that leaves SMs without one, further blocks share the permutation of the V codewords (16
-    // blocks alone take 4.5 us for 8 heads' 1 MB)
+    // a block per pair and stage; where that leaves SMs without one, further blocks encode the new token's rows, as far as there are enough for all, and
+    // share the permutation of the V codewords (16 blocks alone take 4.5 us for 8 heads' 1 MB)
     const int prepare_blocks = TACVQ_GSRQ_VPERM && 2 * B * Hkv < sms ? sms : 2 * B * Hkv;
-    cudaError_t e = launch_dependent(true, gsrq::attn_gsrq_prepare_kernel, dim3(prepare_blocks), dim3(gsrq::kPrepThreads), 0, stream, q,
+    auto prepare = fresh && prepare_blocks >= 4 * B * Hkv ? gsrq::attn_gsrq_prepare_kernel<true> : gsrq::attn_gsrq_prepare_kernel<false>;
+    cudaError_t e = launch_dependent(true, prepare, dim3(prepare_blocks), dim3(gsrq::kPrepThreads), 0, stream, q,
                                      ktab, vtab, lut, scale, (uint4 *)(base + ws.vperm), B, Hkv, token);
     int st = e == cudaSuccess ? launch_status() : (int)e;
     if (st != TACVQ_OK) return st;

@@ -20,8 +20,8 @@ WRITTEN_BEFORE = {
     "attn_rotary_ladder_kernel": {"kcodes", "vcodes", "seq_start", "seq_end"},
     "attn_gsrq_scan_kernel": {"kcodes", "vcodes", "lut_g", "scale_g", "vperm_g", "seq_start", "seq_end"},
     "attn_combine_kernel": {"states"},
+    "attn_gsrq_prepare_kernel": {"q", "ktab", "vtab"},
 }
-WAITS_BEFORE_WRITING_ONLY = {"attn_gsrq_prepare_kernel"}
 
 
 def _kernels():
@@ -37,7 +37,7 @@ def _kernels():
 
 def test_every_kernel_that_waits_is_listed():
     waiting = {name for name, _, body, _ in _kernels() if "wait_for_previous_kernel()" in body}
-    assert waiting == set(WRITTEN_BEFORE) | WAITS_BEFORE_WRITING_ONLY
+    assert waiting == set(WRITTEN_BEFORE)
 
 
 @pytest.mark.parametrize("name", sorted(WRITTEN_BEFORE))
@@ -52,3 +52,10 @@ def test_results_of_the_kernel_before_are_not_constant_memory(name):
         assert not aliases & set(re.findall(r"\w+", load)), load
     stream = re.search(r"ldg_stream\(const void \*p\) \{(.*?)\n\}", text, re.S)
     assert stream is None or ".nc" not in stream.group(1)
+
+
+def test_the_table_preparation_waits_before_it_reads_anything():
+    """It follows whatever kernel computed the query and the rows, also one that lets it start before they are stored."""
+    ((_, body, _),) = [found[1:] for found in _kernels() if found[0] == "attn_gsrq_prepare_kernel"]
+    head = body[: body.index("wait_for_previous_kernel()")]
+    assert not {"q", "ktab", "vtab", "fresh"} & set(re.findall(r"\w+", head))

@@ -226,3 +226,24 @@ def test_a_host_step_uses_the_buffers_tables_and_window_that_the_cache_has_now(d
     for cache in (stepped, plain):
         cache.key_tables, cache.value_tables = tables[0].clone(), tables[1].clone()
     step()
+
+
+def test_a_result_may_be_the_next_steps_query(device):
+    """Nothing runs between the steps: the second one's table preparation follows the first one's attention directly."""
+    from tac_vq_kv_cache_b200.code_cache import VQCodeCache
+
+    gen = torch.Generator().manual_seed(8615)
+    tables = [make_tables(gen, 2, 2, 16, 8) for _ in range(2)]
+    caches = [VQCodeCache(*tables, batch=2, max_tokens=4200, device=device) for _ in range(2)]
+    prompt = [make_states(gen, (2, 2, 4096, 128)).to(device) for _ in range(2)]
+    rows = [[make_states(gen, (2, 2, 1, 128)).to(device) for _ in range(2)] for _ in range(60)]
+    first = (torch.randn(2, 8, 128, generator=gen) / 128**0.5).half().to(device)
+    results = []
+    for cache, alone in zip(caches, (False, True)):
+        cache.append(*prompt)
+        query, outs = first, [torch.empty_like(first) for _ in rows]
+        for out, (key, value) in zip(outs, rows):
+            torch.cuda.synchronize() if alone else None
+            query = cache.decode_step(query, key, value, out=out)
+        results.append(torch.stack(outs))
+    assert torch.equal(*results)
