@@ -341,6 +341,18 @@ TACVQ_API int tacvq_attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kco
                                        size_t workspace_bytes, uint16_t *out_f16, float *state_out, int B, int Hq,
                                        int Hkv, int D, int G, int S, int K, int64_t T_cap, tacvq_stream_t stream);
 
+/*
+ * tacvq_attn_decode (rope_table_f16 NULL) or tacvq_attn_decode_rotary for a caller that knows how much of the buffer is visible: the
+ * rows' ranges lie within `visible` positions.  Work is divided for that many positions instead of T_cap, exactly as a decode step
+ * divides it, so attention after tacvq_encode and tacvq_set_ranges gives a step's result bit for bit.  Positions of a longer
+ * range may be left out (nothing is read or written out of range for them).
+ */
+TACVQ_API int tacvq_attn_decode_within(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
+                                       const uint16_t *vtab_f16, const uint16_t *rope_table_f16, const int32_t *seq_start,
+                                       const int32_t *seq_end, void *workspace, size_t workspace_bytes, uint16_t *out_f16,
+                                       float *state_out, int B, int Hq, int Hkv, int D, int G, int S, int K, int64_t T_cap,
+                                       int64_t visible, tacvq_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -44,6 +44,7 @@ _SIGNATURES = {
     "tacvq_attn_decode_static": (c_int, [c_void_p] * 7 + [c_void_p, c_void_p] + [c_int] * 7 + [c_int64, c_void_p]),
     "tacvq_attn_combine": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "tacvq_rope_table": (c_int, [c_void_p, c_int64, c_int, c_double, c_int64, c_void_p]),
+    "tacvq_attn_decode_within": (c_int, [c_void_p] * 9 + [c_size_t, c_void_p, c_void_p] + [c_int] * 7 + [c_int64, c_int64, c_void_p]),
     "tacvq_attn_decode_rotary": (c_int, [c_void_p] * 9 + [c_size_t, c_void_p, c_void_p] + [c_int] * 7 + [c_int64, c_void_p]),
 }
 

@@ -102,9 +102,11 @@ class VQCodeCache:
         if (start, end) != self._range_is:
             ops.set_ranges(self._range[0], self._range[1], start, end)
             self._range_is = (start, end)
+        # work is divided as decode_step divides it; a captured call may see other ranges when it is replayed
+        seen = None if torch.cuda.is_current_stream_capturing() else end - start
         out, state = ops.attn_decode(
             query, self.key, self.value, self.key_tables, self.value_tables, self._range[0], self._range[1],
-            workspace=self._scratch(int(query.shape[1])), want_state=want_state, rope=self.rope,
+            workspace=self._scratch(int(query.shape[1])), want_state=want_state, rope=self.rope, visible=seen,
         )
         return (out, state) if want_state else out
 

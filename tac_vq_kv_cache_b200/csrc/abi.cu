@@ -399,6 +399,19 @@ int tacvq_attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, const
                               out_f16, state_out, B, Hq, Hkv, D, G, S, K, T_cap, T_cap, LadderStep{0, 0, 0}, stream);
 }
 
+int tacvq_attn_decode_within(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
+                             const uint16_t *vtab_f16, const uint16_t *rope_table, const int32_t *seq_start, const int32_t *seq_end,
+                             void *workspace, size_t workspace_bytes, uint16_t *out_f16, float *state_out, int B, int Hq, int Hkv, int D,
+                             int G, int S, int K, int64_t T_cap, int64_t visible, tacvq_stream_t stream) {
+    if (visible < 0) return TACVQ_ERR_RANGE;
+    if (visible > T_cap) visible = T_cap;
+    if (rope_table)
+        return attn_decode_rotary(q_f16, kcodes, vcodes, ktab_f16, vtab_f16, rope_table, seq_start, seq_end, workspace, workspace_bytes,
+                                  out_f16, state_out, B, Hq, Hkv, D, G, S, K, T_cap, visible, LadderStep{0, 0, 0}, stream);
+    return attn_decode(q_f16, kcodes, vcodes, ktab_f16, vtab_f16, seq_start, seq_end, workspace, workspace_bytes, out_f16, state_out, B, Hq,
+                       Hkv, D, G, S, K, T_cap, visible, false, stream);
+}
+
 int tacvq_set_ranges(int32_t *seq_start, int32_t *seq_end, int B, int start, int end, tacvq_stream_t stream) {
     if (!seq_start || !seq_end) return TACVQ_ERR_NULL;
     if (B <= 0 || start < 0 || end < start) return TACVQ_ERR_GEOMETRY;

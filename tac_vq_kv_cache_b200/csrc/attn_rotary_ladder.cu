@@ -180,9 +180,9 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
         const int lo_all = step.fresh != 0 ? step.start : seq_start ? max(seq_start[b], 0) : 0;
         const int hi_all = step.fresh != 0 ? step.end : seq_end ? min(seq_end[b], (int)T_cap) : (int)T_cap;
         const int n_all = hi_all > lo_all ? hi_all - lo_all : 0;
-        const int per = (n_all + splits - 1) / splits;
+        const int per = min((n_all + splits - 1) / splits, kChunk);  // the split count is for the range that the launcher was told
         const int first = lo_all + split * per;
-        const int n = max(min(first + per, lo_all + n_all) - first, 0);  // at most kChunk: the launcher picks the split count
+        const int n = max(min(first + per, lo_all + n_all) - first, 0);
         float *dst = part + ((int64_t)split * rows + (int64_t)b * Hq + h * rep) * (kDim + 2);
         if (n == 0) {  // the same for the whole cluster: the neutral state
             if (slice == 0)

@@ -155,9 +155,9 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
         if (hi > lo) lo_all = min(lo_all, lo), hi_all = max(hi_all, hi);
     }
     const int n_all = hi_all > lo_all ? hi_all - lo_all : 0;
-    const int per = (n_all + splits - 1) / splits;
+    const int per = min((n_all + splits - 1) / splits, kPos);  // the split count is for the range that the launcher was told
     const int chunk = n_all > 0 ? lo_all + split * per : 0;
-    const int n = n_all > 0 ? max(min(chunk + per, hi_all) - chunk, 0) : 0;  // at most kPos: the launcher picks the split count
+    const int n = n_all > 0 ? max(min(chunk + per, hi_all) - chunk, 0) : 0;
     const int64_t rows = (int64_t)B * Hq;
 
     if (n <= 0) {  // an empty range contributes the neutral state

@@ -257,13 +257,15 @@ def attn_decode(
     out: torch.Tensor | None = None,
     state: torch.Tensor | None = None,
     rope: torch.Tensor | None = None,
+    visible: int | None = None,
 ) -> tuple[torch.Tensor | None, torch.Tensor | None]:
     """Decode-step attention over codes -> ``(out fp16 [B,Hq,D] | None, state fp32 [B,Hq,2+D] | None)``.
 
     ``q [B,Hq,D]`` fp16 pre-scaled; ``seq_start/seq_end`` int32 ``[B]`` on the device (None = whole buffer).
     With ``rope`` (from :func:`rope_table`, ``[T_cap, 2, D/2]`` fp16) the key codes are taken as
     pre-rotary keys and every rebuilt key row is rotated at its token index, as the reference's decode
-    branch does; ``q`` is then the query already rotated at its own position.
+    branch does; ``q`` is then the query already rotated at its own position.  ``visible``: the rows' ranges are known to
+    lie within that many positions, and the work is divided for them instead of the whole buffer.
     """
     device = _require_cuda(q, kcodes, vcodes, ktab_f16, vtab_f16, seq_start, seq_end, workspace, rope)
     b, hq, hkv, dim, g, s, k, t_cap = _attn_geometry(q, kcodes, vcodes, ktab_f16, vtab_f16, seq_start, seq_end)
@@ -282,9 +284,18 @@ def attn_decode(
         raise ValueError("out must be contiguous fp16 [B,Hq,D]")
     if state is not None and (state.dtype != torch.float32 or tuple(state.shape) != (b, hq, dim + 2) or not state.is_contiguous()):
         raise ValueError("state must be contiguous fp32 [B,Hq,2+D]")
+    if rope is not None and (rope.dtype != torch.float16 or tuple(rope.shape) != (t_cap, 2, dim // 2) or not rope.is_contiguous()):
+        raise ValueError("rope must be contiguous fp16 [T_cap, 2, D/2] (cosines, sines)")
+    if visible is not None:
+        with _on(device):
+            status = _lib.load().tacvq_attn_decode_within(
+                _ptr(q), _ptr(kcodes), _ptr(vcodes), _ptr(ktab_f16), _ptr(vtab_f16), _ptr(rope),
+                _ptr(seq_start), _ptr(seq_end), _ptr(workspace), workspace.numel() * workspace.element_size(), _ptr(out),
+                _ptr(state), b, hq, hkv, dim, g, s, k, t_cap, int(visible), _stream(device),
+            )
+        _lib.check("tacvq_attn_decode_within", status)
+        return out, state
     if rope is not None:
-        if rope.dtype != torch.float16 or tuple(rope.shape) != (t_cap, 2, dim // 2) or not rope.is_contiguous():
-            raise ValueError("rope must be contiguous fp16 [T_cap, 2, D/2] (cosines, sines)")
         with _on(device):
             status = _lib.load().tacvq_attn_decode_rotary(
                 _ptr(q), _ptr(kcodes), _ptr(vcodes), _ptr(ktab_f16), _ptr(vtab_f16), _ptr(rope),

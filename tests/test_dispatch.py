@@ -129,3 +129,24 @@ def test_a_rotary_kernel_that_steps_aside_leaves_the_call_to_the_general_one(lib
     library.stand_in_tell(f"{kernel}.splits".encode(), 0)
     assert _attend(library, groups, stages, rope=True) == 0
     assert [c[0] for c in _calls(library) if c[0] != kernel] == ["rotary", "combine"]
+
+
+@pytest.mark.parametrize("groups,stages,rope", [(1, 2, False), (1, 16, False), (16, 1, False), (1, 16, True), (16, 2, True)])
+def test_a_step_and_attention_after_it_divide_the_work_alike(library, groups, stages, rope):
+    """Both are told what is visible: 300 of 5000 positions."""
+    from tac_vq_kv_cache_b200 import _lib
+
+    at, batch, hq, hkv, dim, t_cap, length, window = 1 << 20, 2, 8, 2, 128, 5000, 4000, 300
+    need = library.tacvq_attn_workspace_bytes(batch, hq, hkv, dim, groups, stages)
+    plan = _lib.STEP_PLAN.pack(at, at, at if rope else 0, at, at, at, at, at, need, window, t_cap, batch, hq, hkv, dim, groups, stages, 256)
+    library.stand_in_reset()
+    assert library.tacvq_decode_step_planned(plan, at, at, at, 0, 1, length, at, 0, 0) == 0
+    step = [c[:2] for c in _calls(library) if c[0] != "prologue"]
+    library.stand_in_reset()
+    assert library.tacvq_attn_decode_within(at, at, at, at, at, at if rope else 0, at, at, at, need, at, 0, batch, hq, hkv, dim, groups, stages, 256,
+                                            t_cap, window, 0) == 0
+    assert [c[:2] for c in _calls(library)] == step
+    assert step[0][1] == "300" and step[-1][0] == "combine"
+    library.stand_in_reset()
+    assert _attend(library, groups, stages, rope=rope, t_cap=t_cap) == 0  # nothing is known: the whole buffer
+    assert _calls(library)[0][1] == "5000"

@@ -111,6 +111,44 @@ def _step_equals_append_and_attend(stepped, plain, query, key, value):
 
 
 @pytest.mark.parametrize("rope", [None, 1e6])
+@pytest.mark.parametrize(
+    "batch,heads,q_heads,groups,stages,sub,tokens,window",
+    [
+        (4, 2, 8, 16, 2, 8, 5000, 700),
+        (3, 2, 4, 16, 2, 8, 5000, None),
+        (1, 2, 8, 1, 16, 128, 9000, 900),
+        (5, 2, 8, 1, 2, 128, 4000, 600),
+        (2, 4, 8, 16, 1, 8, 6000, 1500),
+        (2, 2, 8, 2, 3, 64, 3000, 100),
+    ],
+)
+def test_a_step_equals_append_and_attend_bit_for_bit(device, batch, heads, q_heads, groups, stages, sub, tokens, window, rope):
+    """However little of the buffer is visible; also while it fills, and after a captured call of either kind."""
+    from tac_vq_kv_cache_b200.code_cache import VQCodeCache
+
+    gen = torch.Generator().manual_seed(tokens + stages)
+    tables = [make_tables(gen, heads, stages, groups, sub, [0.3 * 0.8**s for s in range(stages)] if sub >= 16 else None) for _ in range(2)]
+    pair = [VQCodeCache(*tables, batch=batch, max_tokens=tokens, window=window, device=device, rope_theta=rope) for _ in range(2)]
+    codes = [torch.randint(0, 256, pair[0].key.shape, generator=gen, dtype=torch.uint8) for _ in range(2)]
+    for cache in pair:
+        cache.key.copy_(codes[0]), cache.value.copy_(codes[1])
+    for length in (1, 250, tokens // 2, tokens - 1):
+        query = (2 * torch.randn(batch, q_heads, 128, generator=gen) / 128**0.5).half().to(device)
+        rows = [make_states(gen, (batch, heads, 1, 128)).to(device) for _ in range(2)]
+        for cache in pair:
+            cache.length = length
+        out = pair[0].decode_step(query, *rows)
+        pair[1].append(*rows)
+        want = pair[1].attend(query)
+        assert torch.equal(out, want), (length, rel_l2(out, want))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = pair[1].attend(query)
+        graph.replay()
+        assert rel_l2(captured, want) <= 1e-3
+
+
+@pytest.mark.parametrize("rope", [None, 1e6])
 @pytest.mark.parametrize("groups,stages,sub", [(16, 2, 8), (1, 2, 128)])
 def test_a_step_uses_the_buffers_tables_and_window_that_the_cache_has_now(device, groups, stages, sub, rope):
     gen = torch.Generator().manual_seed(8611)
