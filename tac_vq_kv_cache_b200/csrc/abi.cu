@@ -4,6 +4,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "ladder_plan.cuh"
 
 namespace tacvq {
 
@@ -40,7 +41,6 @@ int decode_prologue_dispatch(const void *k_rows, const void *v_rows, int rows_dt
                              uint8_t *vcodes, int32_t *seq_start, int32_t *seq_end, int start, int end, int B, int H, int T, int D,
                              int G, int S, int K, int64_t t0, int64_t T_cap, cudaStream_t stream);
 
-int attn_rotary_splits(int B, int Hkv, int64_t T_cap, int sms);
 bool attn_rotary_staged_supported(int Hq, int Hkv, int D, int G, int S, int K);
 int attn_rotary_staged_splits(int B, int Hkv, int64_t T_cap, int sms);
 int attn_rotary_staged_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab,
@@ -55,7 +55,7 @@ int attn_rotary_mma_dispatch(const __half *q, const uint8_t *kcodes, const uint8
 bool attn_rotary_ladder_supported(int Hq, int Hkv, int D, int G, int S, int K);
 int attn_rotary_ladder_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
                                 const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
-                                int Hkv, int S, int64_t T_cap, int64_t visible, const LadderStep &step, int *splits, cudaStream_t stream);
+                                int Hkv, int S, int64_t T_cap, int64_t visible, int sms, const LadderStep &step, int *splits, cudaStream_t stream);
 int rope_table_dispatch(__half *table, int64_t tokens, int D, double theta, int64_t first, cudaStream_t stream);
 int attn_rotary_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab,
                          const __half *vtab, const __half *rope, const int32_t *seq_start, const int32_t *seq_end,
@@ -374,7 +374,7 @@ static int attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, cons
                                           sm_count(), step.fresh != 0, &splits, s);
         } else if (attn_rotary_ladder_supported(Hq, Hkv, D, G, S, K) && (((uintptr_t)kcodes | (uintptr_t)q_f16) & 3) == 0) {
             st = attn_rotary_ladder_dispatch(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, S, T_cap, visible,
-                                             step, &splits, s);
+                                             sm_count(), step, &splits, s);
         } else if (attn_rotary_staged_supported(Hq, Hkv, D, G, S, K)) {
             splits = attn_rotary_staged_splits(B, Hkv, T_cap, sm_count());
             if (splits > 0)
@@ -383,7 +383,7 @@ static int attn_decode_rotary(const uint16_t *q_f16, const uint8_t *kcodes, cons
         }
     }
     if (st == TACVQ_OK && splits == 0) {  // none of these kernels took the call
-        splits = attn_rotary_splits(B, Hkv, T_cap, sm_count());
+        splits = rotary_splits(B, Hkv, T_cap, sm_count());
         st = attn_rotary_dispatch(q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, D, G, S, K, T_cap, splits, s);
     }
     if (st != TACVQ_OK) return st;

@@ -616,17 +616,6 @@ int attn_rotary_staged_splits(int B, int Hkv, int64_t T_cap, int sms) {
     return best;
 }
 
-// About four waves of blocks (two resident per SM), at least 256 tokens per block, at most 64 splits.
-int attn_rotary_splits(int B, int Hkv, int64_t T_cap, int sms) {
-    const int pairs = B * Hkv;
-    int splits = (8 * sms + pairs - 1) / pairs;
-    const int64_t by_len = (T_cap + 255) / 256;
-    if (splits > by_len) splits = (int)by_len;
-    if (splits > 64) splits = 64;
-    if (splits < 1) splits = 1;
-    return splits;
-}
-
 int attn_rotary_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab,
                          const __half *vtab, const __half *rope, const int32_t *seq_start, const int32_t *seq_end,
                          float *part, int B, int Hq, int Hkv, int D, int G, int S, int K, int64_t T_cap, int splits,

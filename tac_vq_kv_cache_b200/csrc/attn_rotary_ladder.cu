@@ -42,6 +42,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "ladder_plan.cuh"
 
 namespace tacvq {
 
@@ -51,7 +52,6 @@ constexpr int kThreads = 512, kWarps = kThreads / 32;
 constexpr int kDim = 128, kWords = 256, kStages = 16, kSlices = 8, kHeads = 4;
 constexpr int kRowBytes = kStages * 2 * 16;           // a code's words of all stages, this block's 16 channels
 constexpr int kTabBytes = kWords * kRowBytes;         // 131072
-constexpr int kChunk = 4096;                          // tokens of a cluster at a time at most
 constexpr int kScoreBytes = kChunk * kHeads * 4;      // parts of the scores, then weights, then per-warp sums
 constexpr int kHistBytes = 2 * 2 * kWords * kHeads * 4;  // [multiples | rest][stage j or j + 8][word][head]
 constexpr int kOutBytes = kSlices * 64 * 4;           // [source block][64 of the 512 outputs]
@@ -460,10 +460,11 @@ bool attn_rotary_ladder_supported(int Hq, int Hkv, int D, int G, int S, int K) {
     return D == 128 && G == 1 && K == 256 && S >= 4 && S <= 16 && S % 4 == 0 && (rep == 1 || rep == 2 || rep == 4);
 }
 
-// Partial states [split][B*Hq][2 + D] for attn_combine_kernel; *splits is how many (0: nothing was launched).
+// Partial states [split][B*Hq][2 + D] for attn_combine_kernel; *splits is how many (0: nothing was launched, the call is
+// for the general kernel).
 int attn_rotary_ladder_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
                                 const __half *rope, const int32_t *seq_start, const int32_t *seq_end, float *part, int B, int Hq,
-                                int Hkv, int S, int64_t T_cap, int64_t visible, const LadderStep &step, int *splits, cudaStream_t stream) {
+                                int Hkv, int S, int64_t T_cap, int64_t visible, int sms, const LadderStep &step, int *splits, cudaStream_t stream) {
     using namespace ladder;
     *splits = 0;
     cudaError_t e = cudaFuncSetAttribute(attn_rotary_ladder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
@@ -493,30 +494,10 @@ int attn_rotary_ladder_dispatch(const __half *q, const uint8_t *kcodes, const ui
         if (most < 1) return TACVQ_OK;
         if (dev >= 0 && dev < 64) cached[dev].store(most, std::memory_order_relaxed);
     }
-    // the cheapest way to deal the items out, in tokens: an item costs its barriers, histograms and products (kFixed) and its
-    // tokens, a change of head the table (kTable)
-    constexpr double kFixed = 1500.0, kTable = 1500.0;
-    const int64_t least = (visible + kChunk - 1) / kChunk;
-    int clusters = 0;
-    double least_cost = 0.0;
-    for (int s = least < 1 ? 1 : (int)(least > 65 ? 65 : least); s <= 64; ++s) {
-        const int64_t per = (visible + s - 1) / s, items = (int64_t)Hkv * B * s, per_head = (int64_t)B * s;
-        const int64_t heads_at_once = most / Hkv;  // clusters a head, when every head has some
-        const int64_t options[2] = {items < most ? items : most, heads_at_once > 0 ? Hkv * (heads_at_once < per_head ? heads_at_once : per_head) : 0};
-        for (const int64_t c : options) {
-            if (c < 1) continue;
-            const int64_t rounds = (items + c - 1) / c;
-            const int64_t tables = items % c == 0 && per_head % (items / c) == 0 ? 1 : 1 + (rounds + per_head - 2) / per_head;
-            const double cost = (double)rounds * (kFixed + (double)per) + (double)tables * kTable + 20.0 * s;
-            if (clusters == 0 || cost < least_cost) least_cost = cost, clusters = (int)c, *splits = s;
-        }
-        if (per <= 256) break;
-    }
-    if (clusters == 0 || (int64_t)Hkv * B * *splits > 0x7fffffff) {
-        *splits = 0;
-        return TACVQ_OK;
-    }
-    cfg.gridDim = dim3((unsigned)(kSlices * clusters));
+    const Plan dealt = plan(B, Hq, Hkv, S, T_cap, visible, sms, most);
+    if (dealt.splits == 0) return TACVQ_OK;
+    *splits = dealt.splits;
+    cfg.gridDim = dim3((unsigned)(kSlices * dealt.clusters));
     cfg.numAttrs = step.fresh != 0 ? 2 : 1;
     e = cudaLaunchKernelEx(&cfg, attn_rotary_ladder_kernel, q, kcodes, vcodes, ktab, vtab, rope, seq_start, seq_end, part, B, Hq, Hkv, S,
                            T_cap, *splits, step);

@@ -20,6 +20,7 @@ STAND_INS = r"""
 #include <map>
 #include <string>
 #include "common.cuh"
+#include "ladder_plan.cuh"
 namespace {
 std::string calls;
 std::map<std::string, int> told;  // status, or number of splits
@@ -33,6 +34,9 @@ int splits_of(const char *name) { auto it = told.find(std::string(name) + ".spli
 extern "C" __attribute__((visibility("default"))) const char *stand_in_calls() { return calls.c_str(); }
 extern "C" __attribute__((visibility("default"))) void stand_in_reset() { calls.clear(); told.clear(); }
 extern "C" __attribute__((visibility("default"))) void stand_in_tell(const char *name, int value) { told[name] = value; }
+extern "C" __attribute__((visibility("default"))) int ladder_splits(int B, int Hq, int Hkv, int S, int64_t T_cap, int64_t visible) {
+    return tacvq::ladder::plan(B, Hq, Hkv, S, T_cap, visible, 148, 15).splits;
+}
 namespace tacvq {
 int encode_dispatch(const EncodeArgs &) { return called("encode"); }
 int decode_dispatch(const uint8_t *, const __half *, void *, int, int, int, int, int, int, int, int, int, int64_t, int64_t, cudaStream_t) { return called("decode"); }
@@ -56,7 +60,6 @@ bool attn_gsrq_supported(int Hq, int Hkv, int D, int G, int S, int K) { return D
 size_t attn_gsrq_workspace_bytes(int, int, int, int, int) { return 0; }
 int attn_gsrq_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const int32_t *, const int32_t *, void *, __half *,
                        float *, int, int, int, int64_t, int, cudaStream_t, const GsrqNewToken *) { return called("gsrq"); }
-int attn_rotary_splits(int, int, int64_t, int) { return splits_of("rotary"); }
 int attn_rotary_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const __half *, const int32_t *, const int32_t *,
                          float *, int, int, int, int, int, int, int, int64_t, int, cudaStream_t) { return called("rotary"); }
 bool attn_rotary_staged_supported(int, int, int D, int G, int S, int) { return D == 128 && S <= 2 && D / G >= 4; }
@@ -68,7 +71,7 @@ int attn_rotary_mma_dispatch(const __half *, const uint8_t *, const uint8_t *, c
                              float *, int, int, int, int64_t, int64_t visible, int, bool, int *splits, cudaStream_t) { *splits = splits_of("mma"); return called("mma", visible); }
 bool attn_rotary_ladder_supported(int, int, int D, int G, int S, int) { return D == 128 && G == 1 && S >= 4 && S <= 16; }
 int attn_rotary_ladder_dispatch(const __half *, const uint8_t *, const uint8_t *, const __half *, const __half *, const __half *, const int32_t *, const int32_t *,
-                                float *, int, int, int, int, int64_t, int64_t visible, const LadderStep &step, int *splits, cudaStream_t) {
+                                float *, int, int, int, int, int64_t, int64_t visible, int, const LadderStep &step, int *splits, cudaStream_t) {
     *splits = splits_of("ladder");
     return called("ladder", visible, step.fresh);
 }
@@ -150,3 +153,26 @@ def test_a_step_and_attention_after_it_divide_the_work_alike(library, groups, st
     library.stand_in_reset()
     assert _attend(library, groups, stages, rope=rope, t_cap=t_cap) == 0  # nothing is known: the whole buffer
     assert _calls(library)[0][1] == "5000"
+
+
+# us a decode step through attn_rotary_kernel / the ladder kernel: 8 KV heads; stages, rows, query heads per KV head, tokens
+LADDER_TIMES = """
+4 1 4 600 43.6 19.9; 4 1 1 600 33.6 19.3; 4 4 4 2000 54.7 78.7; 4 4 1 2000 42.9 78.8; 4 8 4 300 39.2 61.8; 4 2 4 8192 101.1 124.9; 4 16 1 300 34.1 100.9
+4 1 2 2500 40.6 31.7; 4 1 4 2500 49.1 31.8; 4 16 4 1000 95.7 144.7; 8 1 4 600 63.5 27.3; 8 1 2 6000 70.2 54.5; 8 4 1 2000 64.4 86.7; 8 8 4 300 55.3 70.0
+8 16 4 300 64.1 111.6; 8 2 4 1000 69.7 41.3; 8 16 2 1000 115.2 156.4; 12 1 1 600 67.7 36.3; 12 8 4 2000 180.8 150.6; 12 16 4 300 80.5 134.1
+12 4 2 2000 89.9 102.2; 16 1 4 130 81.8 39.6; 16 1 4 6000 130.2 72.7; 16 16 4 300 100.9 144.1; 16 16 1 300 85.9 144.6; 16 8 4 2000 223.3 159.3
+16 2 1 8192 185.8 157.9; 16 8 2 300 72.5 94.9; 16 16 4 1000 227.8 192.9
+"""
+
+
+def test_ladders_go_to_the_kernel_that_is_quicker_for_them(library):
+    library.ladder_splits.argtypes = [ctypes.c_int] * 4 + [ctypes.c_int64] * 2
+    for line in LADDER_TIMES.replace("\n", ";").split(";"):
+        if line.strip():
+            stages, rows, rep, tokens, general, ladder = map(float, line.split())
+            taken = library.ladder_splits(int(rows), int(8 * rep), 8, int(stages), int(tokens), int(tokens)) > 0
+            assert taken == (ladder < general), line
+    assert library.ladder_splits(1, 8, 2, 16, 1 << 20, 300000) == 0  # more than 64 splits of 4096
+    for visible in (1, 4096, 4097):
+        splits = library.ladder_splits(1, 32, 8, 16, 262144, visible)
+        assert splits >= 1 and -(-visible // splits) <= 4096
