@@ -103,7 +103,7 @@ class VQCodeCache:
             ops.set_ranges(self._range[0], self._range[1], start, end)
             self._range_is = (start, end)
         # work is divided as decode_step divides it; a captured call may see other ranges when it is replayed
-        seen = None if torch.cuda.is_current_stream_capturing() else end - start
+        seen = None if self.key.is_cuda and ops._capturing(self.key.device) else end - start
         out, state = ops.attn_decode(
             query, self.key, self.value, self.key_tables, self.value_tables, self._range[0], self._range[1],
             workspace=self._scratch(int(query.shape[1])), want_state=want_state, rope=self.rope, visible=seen,

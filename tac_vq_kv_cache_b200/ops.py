@@ -64,6 +64,12 @@ def _stream(device: torch.device) -> int:
     return _raw_stream(torch.cuda.current_device() if device.index is None else device.index)
 
 
+def _capturing(device: torch.device) -> bool:
+    """Whether what is launched on ``device`` now goes into a CUDA graph."""
+    with _on(device):
+        return torch.cuda.is_current_stream_capturing()
+
+
 def _rows_view(x: torch.Tensor) -> torch.Tensor:
     """States ``[B,H,T,D]`` usable in place: last axis contiguous and rows 16-byte aligned, else a packed copy."""
     if x.dtype not in _DTYPE_TAG:

@@ -94,6 +94,17 @@ def test_argument_errors_need_no_device():
     assert lib.tacvq_attn_workspace_bytes(8, 32, 8, 128, 16, 2) > 0
 
 
+@pytest.mark.parametrize("length", [0, 2])
+def test_a_cache_on_the_cpu_refuses_to_attend(length):
+    from tac_vq_kv_cache_b200.code_cache import VQCodeCache
+
+    tables = torch.zeros(2, 2, 1, 256, 128)
+    cache = VQCodeCache(tables, tables, batch=1, max_tokens=4, device="cpu")
+    cache.length = length
+    with pytest.raises(RuntimeError, match="no CPU fallback"):
+        cache.attend(torch.zeros(1, 2, 128).half())
+
+
 def test_host_validation_and_no_cpu_fallback():
     from tac_vq_kv_cache_b200.jointkv.closed_loop_vq import hard_residual_vq_exits
     from tac_vq_kv_cache_b200.jointkv.cq_tac import ClosedLoopGroupedCQ, hard_grouped_cq
