@@ -27,6 +27,12 @@
 // rows for groups): 2 x 128, 16 rows x 16384 tokens 36.7 / 50.8; 16 x 128, 2 x 32768 82 / 150; 16 x 8, 8 x 32768 81 / 240; 32 x 4 154 / 317;
 // 16 x 2 x 8 with two query heads a KV head 101 / 309, with one 150 / 303.
 //
+// Short calls are bound by what a block does besides its tokens.  In clocks, one row of 100 tokens, 2 x 2 x 64: empty bins 1.6 k, score
+// table 17 k, folding the bins once 2.7 k (8 k for one slot), V words 7 k.  The table is a tensor-core product for every width from 16
+// on and has its query channels in registers below, bins are folded a row a warp, lanes take neighbouring words of 4 channels: us a call,
+// one row, before / now: 2 x 2 x 64 with one head 19.7 / 13.0, 1 x 128 15.4 / 11.0, 16 x 8 18.4 / 15.9, 8 x 2 x 16 22.8 / 18.7; 16 rows of 300
+// tokens, 32 x 4 43.2 / 34.2 a step.
+//
 // Semantics replaced: experiments_followup_mistral/evaluate_mistral_longbench.py:112-122 (no rotary step).  Differences from the
 // dense path inside the 2e-3 tolerance: the V row is the exact sum of its words (the reference rounds that sum to fp16 once), a
 // score is the sum of partial dot products (the reference rounds the rebuilt key to fp16 first).
@@ -58,7 +64,8 @@ struct Shape {
     static constexpr int kCodeWords = P < 4 ? 1 : P / 4;
     static constexpr int kTokens = P >= 16 ? 2 : P == 8 ? 4 : 8;       // a thread's tokens of a segment
     static constexpr int kFold = 4096 * kCopies;                       // tokens after which the bins are folded: a copy takes 4096 weights
-    static constexpr int kBins = P * kHeads * kWords / kThreads;       // a thread's bins
+    static constexpr int kUsed = kCopies * P * kHeads;                 // words of a code's row that are used
+    static constexpr int kBins = kUsed * kWords / kThreads;            // a thread's bins, of all copies
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -180,84 +187,121 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
     const uint8_t *kc_row = kcodes + ((int64_t)b * Hkv + h) * T_cap * slots, *vc_row = vcodes + ((int64_t)b * Hkv + h) * T_cap * slots;
 
     // ---- score table, and empty bins ----------------------------------------------------------------------------------
-    for (int i = tid; i < 2 * kAreaBytes / 16; i += kThreads) reinterpret_cast<uint4 *>(smem + kAreaBytes)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (G == 1) {
-        // tensor cores: A = 16 words, B = the heads; a lane's 16 bytes are channels 32 c + 8 kq .. of its two words, which
-        // makes them the operands of two products over a channel order that the query follows
+#pragma unroll
+    for (int i = tid; i < 2 * kWords * L::kUsed / 4; i += kThreads)
+        *reinterpret_cast<uint4 *>(smem + kAreaBytes + i / (L::kUsed / 4) * kRowBytes + i % (L::kUsed / 4) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    auto put_entry = [&](int code, int slot, int pair, float first, float second) {  // heads 2 * pair and the next, every copy
+#pragma unroll
+        for (int u = 0; u < L::kCopies; ++u)
+            *(reinterpret_cast<float2 *>(smem + code * kRowBytes + (u * P + slot) * L::kEntry) + pair) = make_float2(first, second);
+    };
+    const __half *q_rows = q + ((int64_t)b * Hq + head0) * kDim;
+    if (d >= 16) {
+        // tensor cores: A = 16 words, B = the heads; warp w takes words 16 w .. 16 w + 15 of every slot.  A lane's 16 bytes are channels
+        // 32 c + 8 kq .. of its two words (8 bytes, channels 4 kq .., for words of 16), which makes them the operands of two
+        // products (one) over a channel order that the query follows.  32 channels at a time, added in fp32: the tensor core cuts off what
+        // it adds to a sum that is there.
         const int r8 = lane >> 2, kq = lane & 3;
-        uint4 qf[4];
+        auto products = [&](auto width) {
+            constexpr int D = decltype(width)::value, C = D / 32;
+            uint4 qf[C];
+            auto load_query = [&](int g) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-            qf[c] = r8 < heads ? __ldg(reinterpret_cast<const uint4 *>(q + ((int64_t)b * Hq + head0 + r8) * kDim + 32 * c + 8 * kq)) : make_uint4(0u, 0u, 0u, 0u);
-        const uint4 *words = reinterpret_cast<const uint4 *>(ktab + (int64_t)h * slots * kWords * kDim) + kq;
+                for (int c = 0; c < C; ++c) qf[c] = r8 < heads ? __ldg(reinterpret_cast<const uint4 *>(q_rows + r8 * kDim + g * D + 32 * c + 8 * kq)) : make_uint4(0u, 0u, 0u, 0u);
+            };
+            if (G == 1) load_query(0);
 #pragma unroll 2
-        for (int tile = warp; tile < slots * (kWords / 16); tile += kWarps) {
-            const uint4 *row = words + (tile * 16 + r8) * (kDim / 8);
-            uint4 a[4], c8[4];
+            for (int slot = 0; slot < slots; ++slot) {
+                const uint4 *row = reinterpret_cast<const uint4 *>(ktab + (((int64_t)h * slots + slot) * kWords + warp * 16 + r8) * D) + kq;
+                if (G > 1) load_query(slot % G);
+                uint4 a[C], c8[C];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) a[c] = __ldg(row + 4 * c), c8[c] = __ldg(row + 8 * (kDim / 8) + 4 * c);
-            float part[4][4], acc[4];  // 32 channels each, added in fp32: the tensor core cuts off what it adds to a sum that is there
+                for (int c = 0; c < C; ++c) a[c] = __ldg(row + 4 * c), c8[c] = __ldg(row + D + 4 * c);
+                float part[C][4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                part[c][0] = part[c][1] = part[c][2] = part[c][3] = 0.0f;
-                mma16816(part[c], a[c].x, c8[c].x, a[c].y, c8[c].y, qf[c].x, qf[c].y);
-                mma16816(part[c], a[c].z, c8[c].z, a[c].w, c8[c].w, qf[c].z, qf[c].w);
+                for (int c = 0; c < C; ++c) {
+                    part[c][0] = part[c][1] = part[c][2] = part[c][3] = 0.0f;
+                    mma16816(part[c], a[c].x, c8[c].x, a[c].y, c8[c].y, qf[c].x, qf[c].y);
+                    mma16816(part[c], a[c].z, c8[c].z, a[c].w, c8[c].w, qf[c].z, qf[c].w);
+                }
+#pragma unroll
+                for (int step = 1; step < C; step *= 2)
+#pragma unroll
+                    for (int c = 0; c < C; c += 2 * step)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) part[c][i] += part[c + step][i];
+                if (2 * kq < H) {
+                    put_entry(warp * 16 + r8, slot, kq, part[0][0], part[0][1]);
+                    put_entry(warp * 16 + r8 + 8, slot, kq, part[0][2], part[0][3]);
+                }
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i] = (part[0][i] + part[1][i]) + (part[2][i] + part[3][i]);
-            if (2 * kq < H) {
-                const int slot = tile / (kWords / 16), code = (tile % (kWords / 16)) * 16 + r8;
-#pragma unroll
-                for (int u = 0; u < L::kCopies; ++u) {
-                    float2 *to = reinterpret_cast<float2 *>(smem + code * kRowBytes + (u * P + slot) * L::kEntry) + kq;
-                    to[0] = make_float2(acc[0], acc[1]);
-                    to[8 * kRowBytes / 8] = make_float2(acc[2], acc[3]);
+        };
+        if (d == 128) products(std::integral_constant<int, 128>());
+        else if (d == 64) products(std::integral_constant<int, 64>());
+        else if (d == 32) products(std::integral_constant<int, 32>());
+        else {
+#pragma unroll 4
+            for (int slot = 0; slot < slots; ++slot) {
+                const uint2 *row = reinterpret_cast<const uint2 *>(ktab + (((int64_t)h * slots + slot) * kWords + warp * 16 + r8) * 16) + kq;
+                const uint2 a = __ldg(row), c8 = __ldg(row + 8 * 4);
+                const uint2 qf = r8 < heads ? __ldg(reinterpret_cast<const uint2 *>(q_rows + r8 * kDim + slot % G * 16) + kq) : make_uint2(0u, 0u);
+                float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                mma16816(sum, a.x, c8.x, a.y, c8.y, qf.x, qf.y);
+                if (2 * kq < H) {
+                    put_entry(warp * 16 + r8, slot, kq, sum[0], sum[1]);
+                    put_entry(warp * 16 + r8 + 8, slot, kq, sum[2], sum[3]);
                 }
             }
         }
-    } else {
+    } else if constexpr (P >= 16) {
         for (int i = tid; i < kDim * H; i += kThreads) {
             const int r = i / kDim, c = i % kDim;
-            q_s[(c / d * (d + 1) + c % d) * H + r] = r < heads ? __half2float(q[((int64_t)b * Hq + head0 + r) * kDim + c]) : 0.0f;
+            q_s[(c / d * (d + 1) + c % d) * H + r] = r < heads ? __half2float(q_rows[r * kDim + c]) : 0.0f;
         }
         __syncthreads();
         // neighbouring lanes take different slots (no conflicts where they write and where they read the query), the next
-        // lanes neighbouring codes (whole sectors of the table)
-        constexpr int kNear = P < L::kSpread ? P : L::kSpread;
+        // lanes neighbouring codes (whole sectors of the table); a thread stays with a slot and has the query's channels in registers
+        constexpr int kNear = L::kSpread, kTrips = kNear * kWords / kThreads;
         auto entries = [&](auto width) {
-            constexpr int C = decltype(width)::value;  // channels at a time
-#pragma unroll 4
-            for (int i = 0; i < P * kWords / kThreads; ++i) {
-                const int idx = tid + i * kThreads;
-                const int slot = idx % kNear + idx / (kNear * kWords) * kNear, code = idx / kNear % kWords;
-                if (!FULL && slot >= slots) continue;
-                const __half *word = ktab + (((int64_t)h * slots + slot) * kWords + code) * d;
-                const float *qv = q_s + slot % G * (d + 1) * H;
-                float dot[H];
+            constexpr int C = decltype(width)::value;  // channels of a word
+#pragma unroll 1
+            for (int slot = tid % kNear; slot < (FULL ? P : slots); slot += kNear) {
+                const __half *words = ktab + (((int64_t)h * slots + slot) * kWords + tid / kNear) * C;
+                uint32_t raw[kTrips][C / 2];
 #pragma unroll
-                for (int r = 0; r < H; ++r) dot[r] = 0.0f;
-                for (int c = 0; c < d; c += C) {
-                    uint32_t raw[C / 2];
+                for (int i = 0; i < kTrips; ++i) {
+                    const __half *word = words + i * (kThreads / kNear) * C;
                     if constexpr (C == 8) {
-                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(word + c));
-                        raw[0] = v.x, raw[1] = v.y, raw[2] = v.z, raw[3] = v.w;
+                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(word));
+                        raw[i][0] = v.x, raw[i][1] = v.y, raw[i][2] = v.z, raw[i][3] = v.w;
                     } else {
-                        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(word + c));
-                        raw[0] = v.x, raw[1] = v.y;
-                    }
-#pragma unroll
-                    for (int e = 0; e < C; ++e) {
-                        const __half2 pair = *reinterpret_cast<const __half2 *>(&raw[e / 2]);
-                        const float f = __half2float(e & 1 ? __high2half(pair) : __low2half(pair));
-#pragma unroll
-                        for (int r = 0; r < H; ++r) dot[r] = fmaf(qv[(c + e) * H + r], f, dot[r]);
+                        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(word));
+                        raw[i][0] = v.x, raw[i][1] = v.y;
                     }
                 }
+                const float2 *qv = reinterpret_cast<const float2 *>(q_s + slot % G * (C + 1) * H);
+                float qr[C][H];
 #pragma unroll
-                for (int u = 0; u < L::kCopies; ++u) {
-                    float *to = reinterpret_cast<float *>(smem + code * kRowBytes + (u * P + slot) * L::kEntry);
+                for (int e = 0; e < C; ++e)
 #pragma unroll
-                    for (int r = 0; r < H; r += 2) *reinterpret_cast<float2 *>(to + r) = make_float2(dot[r], dot[r + 1]);
+                    for (int r = 0; r < H; r += 2) {
+                        const float2 v = qv[(e * H + r) / 2];
+                        qr[e][r] = v.x, qr[e][r + 1] = v.y;
+                    }
+#pragma unroll
+                for (int i = 0; i < kTrips; ++i) {
+                    float dot[H];
+#pragma unroll
+                    for (int r = 0; r < H; ++r) dot[r] = 0.0f;
+#pragma unroll
+                    for (int e = 0; e < C; ++e) {
+                        const __half2 pair = *reinterpret_cast<const __half2 *>(&raw[i][e / 2]);
+                        const float f = __half2float(e & 1 ? __high2half(pair) : __low2half(pair));
+#pragma unroll
+                        for (int r = 0; r < H; ++r) dot[r] = fmaf(qr[e][r], f, dot[r]);
+                    }
+#pragma unroll
+                    for (int r = 0; r < H; r += 2) put_entry(tid / kNear + i * (kThreads / kNear), slot, r / 2, dot[r], dot[r + 1]);
                 }
             }
         };
@@ -285,25 +329,32 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
     __syncthreads();
 
     // ---- tokens, a segment of NT x 512 at a time ------------------------------------------------------------------------
-    float m[H], l[H], sums[L::kBins];  // reference score, this thread's weights; its folded bins tid + 512 i of [code][slot][head]
+    float m[H], l[H], sums[L::kBins];  // reference score, this thread's weights; its folded bins tid + 512 i of [code][copy][slot][head]
 #pragma unroll
     for (int r = 0; r < H; ++r) m[r] = -INFINITY, l[r] = 0.0f;
 #pragma unroll
     for (int i = 0; i < L::kBins; ++i) sums[i] = 0.0f;
     auto fold = [&](float f) {  // what is in the bins joins the sums, times f; the bins become empty
+        constexpr int kAtOnce = 8;
 #pragma unroll
-        for (int i = 0; i < L::kBins; ++i) {
-            const int bin = tid + i * kThreads, at = bin / (P * H) * kRowBytes + bin % (P * H) * 4;
-            float v = 0.0f;
+        for (int i0 = 0; i0 < L::kBins; i0 += kAtOnce) {
+            uint32_t large[kAtOnce], small[kAtOnce];
 #pragma unroll
-            for (int u = 0; u < L::kCopies; ++u) {
-                uint32_t *large = reinterpret_cast<uint32_t *>(smem + kAreaBytes + at + u * P * L::kEntry), *small = large + kAreaBytes / 4;
-                if constexpr (FINE) v += fmaf((float)(int32_t)*small, 1.0f / (kFine * kFine), (float)*large * (1.0f / kFine));
-                else v += fmaf((float)*small, 1.0f / kSmall, (float)*large * (1.0f / kLarge));
-                *large = 0u;
-                *small = 0u;
+            for (int i = 0; i < kAtOnce; ++i) {
+                const int bin = tid + (i0 + i) * kThreads, at = kAreaBytes + bin / L::kUsed * kRowBytes + bin % L::kUsed * 4;
+                large[i] = *reinterpret_cast<uint32_t *>(smem + at);
+                small[i] = *reinterpret_cast<uint32_t *>(smem + at + kAreaBytes);
             }
-            sums[i] = (sums[i] + v) * f;
+#pragma unroll
+            for (int i = 0; i < kAtOnce; ++i) {
+                const int bin = tid + (i0 + i) * kThreads, at = kAreaBytes + bin / L::kUsed * kRowBytes + bin % L::kUsed * 4;
+                *reinterpret_cast<uint32_t *>(smem + at) = 0u;
+                *reinterpret_cast<uint32_t *>(smem + at + kAreaBytes) = 0u;
+                float v;
+                if constexpr (FINE) v = fmaf((float)(int32_t)small[i], 1.0f / (kFine * kFine), (float)large[i] * (1.0f / kFine));
+                else v = fmaf((float)small[i], 1.0f / kSmall, (float)large[i] * (1.0f / kLarge));
+                sums[i0 + i] = (sums[i0 + i] + v) * f;
+            }
         }
     };
     int pending = 0;
@@ -315,6 +366,11 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
         if (more) {
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
+                if (j > 0 && base + j * kThreads >= hi) {  // nobody has a token here
+#pragma unroll
+                    for (int r = 0; r < H; ++r) sc[j][r] = -INFINITY;
+                    continue;
+                }
                 permute_words<NW>(kc[j], x);
                 // two heads an addition; several short sums have less rounding than a long one
                 constexpr int kSums = P == 32 ? 4 : P >= 4 ? 2 : 1;
@@ -425,11 +481,15 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
         }
         if (base + NT * kThreads < hi) fetch(vc_row, base + NT * kThreads, vc);
     }
-    // the score table is done with: its place takes the folded weights, [code][slot][head]
+    // the score table is done with: its place takes the folded weights, [code][slot][head]; a row's copies are in neighbouring lanes
 #pragma unroll
     for (int i = 0; i < L::kBins; ++i) {
-        const int bin = tid + i * kThreads;
-        *reinterpret_cast<float *>(smem + bin / (P * H) * kRowBytes + bin % (P * H) * 4) = sums[i];
+        const int bin = tid + i * kThreads, col = bin % L::kUsed;
+        if constexpr (L::kCopies > 1) {
+#pragma unroll
+            for (int off = P * H; off < L::kUsed; off *= 2) sums[i] += __shfl_xor_sync(0xffffffffu, sums[i], off);
+        }
+        if (col < P * H) *reinterpret_cast<float *>(smem + bin / L::kUsed * kRowBytes + col * 4) = sums[i];
     }
 #pragma unroll
     for (int r = 0; r < H; ++r) {
@@ -444,7 +504,9 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
     float *warp_sums = reinterpret_cast<float *>(smem + kAreaBytes);  // [warp][H][128]
     auto product = [&](auto width) {
         constexpr int C = decltype(width)::value, kPieces = kDim / C, kSlices = kThreads / kPieces;
-        const int piece = tid % kPieces, g = piece * C / d, off = piece * C % d;
+        // words of four channels: neighbouring lanes take the words of a sector, a warp eight groups (a group a lane would be 32 lines a load)
+        const int piece = C == 4 ? (warp & 3) * 8 + (lane >> 2) : tid % kPieces, g = piece * C / d, off = piece * C % d;
+        const int first = C == 4 ? (warp >> 2) * 4 + (lane & 3) : tid / kPieces;  // of this thread's words, kSlices apart
         float acc[H][C];
 #pragma unroll
         for (int r = 0; r < H; ++r)
@@ -459,7 +521,7 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
                 uint32_t raw[kAtOnce][C / 2];
 #pragma unroll
                 for (int k = 0; k < kAtOnce; ++k) {
-                    const __half *from = words + (tid / kPieces + (trip + k) * kSlices) * d;
+                    const __half *from = words + (first + (trip + k) * kSlices) * d;
                     if constexpr (C == 8) {
                         const uint4 v = __ldg(reinterpret_cast<const uint4 *>(from));
                         raw[k][0] = v.x, raw[k][1] = v.y, raw[k][2] = v.z, raw[k][3] = v.w;
@@ -474,7 +536,7 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
                     bool used = false;  // a word that no token refers to may hold anything
 #pragma unroll
                     for (int r = 0; r < H; r += 2) {
-                        const float2 v = *reinterpret_cast<const float2 *>(weights + (tid / kPieces + (trip + k) * kSlices) * kRowBytes + r * 4);
+                        const float2 v = *reinterpret_cast<const float2 *>(weights + (first + (trip + k) * kSlices) * kRowBytes + r * 4);
                         w[r] = v.x, w[r + 1] = v.y;
                         used |= v.x != 0.0f || v.y != 0.0f;
                     }
@@ -492,23 +554,35 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
             }
         }
 #pragma unroll
-        for (int r = 0; r < H; ++r)
+        for (int r = 0; r < H; ++r) {
 #pragma unroll
             for (int i = 0; i < C; ++i) {
-                if constexpr (kPieces == 16) acc[r][i] += __shfl_xor_sync(0xffffffffu, acc[r][i], 16);
-                if (kPieces == 32 || lane < 16) warp_sums[(warp * H + r) * kDim + piece * C + i] = acc[r][i];
+                if constexpr (C == 4) {
+                    acc[r][i] += __shfl_xor_sync(0xffffffffu, acc[r][i], 1);
+                    acc[r][i] += __shfl_xor_sync(0xffffffffu, acc[r][i], 2);
+                } else {
+                    acc[r][i] += __shfl_xor_sync(0xffffffffu, acc[r][i], 16);
+                }
             }
+            if (C == 4 ? (lane & 3) == 0 : lane < 16) {
+#pragma unroll
+                for (int i = 0; i < C; i += 4)
+                    *reinterpret_cast<float4 *>(warp_sums + (warp * H + r) * kDim + piece * C + i) = make_float4(acc[r][i], acc[r][i + 1], acc[r][i + 2], acc[r][i + 3]);
+            }
+        }
     };
-    if (d == 4) product(std::integral_constant<int, 4>());
+    if (P == 32 && d == 4) product(std::integral_constant<int, P == 32 ? 4 : 8>());
     else product(std::integral_constant<int, 8>());
     __syncthreads();
     const int64_t rows = (int64_t)B * Hq;
     for (int o = tid; o < heads * kDim; o += kThreads) {
         const int r = o / kDim, channel = o % kDim;
         float lsum = 0.0f, asum = 0.0f;
+        // words of four channels: a channel is in every fourth warp's sums
+#pragma unroll
         for (int w = 0; w < kWarps; ++w) {
             lsum += red[(kWarps + w) * H + r];
-            asum += warp_sums[(w * H + r) * kDim + channel];
+            if (P < 32 || d > 4 || w % 4 == channel / 32) asum += warp_sums[(w * H + r) * kDim + channel];
         }
         float top = m[0];
 #pragma unroll
