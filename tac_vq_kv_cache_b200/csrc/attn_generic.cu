@@ -158,8 +158,9 @@ attn_generic_kernel(const __half *__restrict__ q, const uint8_t *__restrict__ kc
 
 // Merge n_parts states laid out [n_parts][rows][2+D]; one block per row.  What bounds it is the memory latency of a row's
 // n_parts states, so nothing walks them one after the other: the threads take a part's (m, l) each and reduce, then groups
-// of 128 threads (a thread per channel) take every groups-th part, up to eight loads in flight.
-constexpr int kCombineLanes = 128, kCombineGroups = 8;
+// of 128 threads (a thread per channel) take every groups-th part, up to eight loads in flight.  Up to eight parts are requested at
+// once by every thread, which then needs no other: us a merge of 32 rows of eight parts 3.6 with the reduction, 2.5 one part after the other.
+constexpr int kCombineLanes = 128, kCombineGroups = 8, kCombineFew = 8;
 
 __global__ void __launch_bounds__(kCombineLanes * kCombineGroups)
 attn_combine_kernel(const float *states, int n_parts, int64_t rows, int D, __half *__restrict__ out,
@@ -172,6 +173,32 @@ attn_combine_kernel(const float *states, int n_parts, int64_t rows, int D, __hal
     const float *own = states + row * W;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
     wait_for_previous_kernel();
+    if (n_parts <= kCombineFew) {
+        for (int i = tid; i < D; i += blockDim.x) {
+            float m[kCombineFew], part[kCombineFew], v[kCombineFew];
+#pragma unroll
+            for (int p = 0; p < kCombineFew; ++p) {
+                const float *from = own + (p < n_parts ? p : 0) * stride;
+                m[p] = from[0], part[p] = p < n_parts ? from[1] : 0.0f, v[p] = from[2 + i];
+            }
+            float top = m[0], l = 0.0f, a = 0.0f;
+#pragma unroll
+            for (int p = 1; p < kCombineFew; ++p) top = fmaxf(top, m[p]);
+#pragma unroll
+            for (int p = 0; p < kCombineFew; ++p) {
+                if (part[p] == 0.0f) continue;  // no token there
+                const float f = __expf(m[p] - top);
+                l += f * part[p];
+                if (m[p] != -INFINITY) a += f * v[p];
+            }
+            if (merged) {
+                merged[row * W + 2 + i] = a;
+                if (i == 0) merged[row * W] = top, merged[row * W + 1] = l;
+            }
+            if (out) out[row * D + i] = __float2half_rn(l == 0.0f ? 0.0f : a / l);
+        }
+        return;
+    }
     float top = -INFINITY;
     for (int p = tid; p < n_parts; p += blockDim.x) top = fmaxf(top, own[p * stride]);
 #pragma unroll

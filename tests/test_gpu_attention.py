@@ -253,6 +253,32 @@ def test_partial_states_merge_to_the_whole(device):
     _check(merged_out, c_out)
 
 
+@pytest.mark.parametrize("parts", [1, 2, 7, 8, 9, 17, 64, 65, 200])
+@pytest.mark.parametrize("dim", [32, 128, 256])
+def test_merges_of_few_and_many_parts(device, parts, dim):
+    """Both ways to merge, at their border; parts without a token, a row without any, one part of a row that is not a number."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(parts + dim)
+    states = torch.randn(parts, 2, 5, dim + 2, generator=gen)
+    states[..., 0] *= 20
+    states[..., 1] = states[..., 1].abs() + 0.1
+    empty = torch.rand(parts, 2, 5, generator=gen) < 0.3
+    empty[:, 1, 4] = True
+    empty[0, 0, 0] = False
+    states[empty] = 0.0
+    states[..., 0][empty] = -float("inf")
+    out, merged = ops.attn_combine(states.to(device), want_state=True)
+    want, want_merged = C.merge(states)
+    torch.testing.assert_close(out.cpu().float(), want.float(), rtol=2e-3, atol=2e-3)
+    torch.testing.assert_close(merged.cpu(), want_merged, rtol=2e-5, atol=2e-5)
+    assert bool((out[1, 4] == 0).all()) and float(merged[1, 4, 1]) == 0
+    states[parts // 2, 0, 0, 1] = float("nan")
+    states[parts // 2, 0, 0, 0] = -float("inf")
+    out, merged = ops.attn_combine(states.to(device), want_state=True)
+    assert bool(out[0, 0].isnan().all()) and bool(merged[0, 0, 1].isnan())
+    assert not bool(out[0, 1:].isnan().any()) and not bool(out[1].isnan().any())
+
+
 def test_benchmark_size_32k_context(device):
     """Full benchmark shape: batch 8, 32 query / 8 KV heads, 32768 tokens, 2x16 code bytes per token."""
     work = _workload(8601, 8, 32, 8, 32768, 16, 2, 8)
