@@ -455,14 +455,15 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
 
 // Rows a block, and splits of the positions, for `visible` positions a row.  One block per SM; a block costs its
 // table copies and merge (kFixed) and its tokens, whose price falls with the rows that share a position's cos/sin; the pair with
-// the least waves x block is taken.  In clocks, from the measured kernel.  (Splits for the buffer instead of the visible range: 8 rows
+// the least waves x block is taken.  Up to eight parts a row are merged in one round of loads, more take kMerge longer.  In clocks, from the
+// measured kernel.  (Splits for the buffer instead of the visible range: 8 rows
 // with 4096 of 30001 tokens visible 91 us a step against 45.)
 struct Plan {
     int rows, splits;
 };
 
 inline Plan plan(int B, int Hkv, int64_t visible, int sms) {
-    constexpr double kFixed = 14000.0;
+    constexpr double kFixed = 14000.0, kMerge = 3000.0;
     Plan best = {0, 0};
     double least_cost = 0.0;
     for (int rows = 4; rows >= 1; rows >>= 1) {
@@ -473,7 +474,7 @@ inline Plan plan(int B, int Hkv, int64_t visible, int sms) {
         for (int splits = least < 1 ? 1 : (int)(least > 65 ? 65 : least); splits <= 64; ++splits) {
             const int64_t per = (visible + splits - 1) / splits;
             const int64_t waves = ((int64_t)groups * Hkv * splits + sms - 1) / sms;
-            const double cost = (double)waves * (kFixed + (double)(share * per) * token) + 40.0 * splits;
+            const double cost = (double)waves * (kFixed + (double)(share * per) * token) + 40.0 * splits + (splits > 8 ? kMerge : 0.0);
             if (best.rows == 0 || cost < least_cost) least_cost = cost, best = {rows, splits};
             if (per * share <= 256) break;
         }
