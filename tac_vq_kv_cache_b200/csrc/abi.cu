@@ -79,7 +79,7 @@ static int sm_count() {
 }
 
 // the specialised scan keeps a work prefix over at most 512 batch rows in shared memory and reads its
-// query rows and tables in 16-byte pieces; other calls are served by the generic kernel
+// query rows and tables in 16-byte pieces; other calls are served by the kernels for at most 32 slots (which want the pieces too) and by the generic kernel
 static bool gsrq_batch_ok(int B, int Hkv) { return B <= 512 && (int64_t)B * Hkv <= 1024; }
 static bool gsrq_aligned(const void *q, const void *ktab, const void *vtab) {
     return (((uintptr_t)q | (uintptr_t)ktab | (uintptr_t)vtab) & 15) == 0;

@@ -87,7 +87,7 @@ def test_sliding_window_and_empty_rows(device):
 @pytest.mark.parametrize(
     "b,hq,hkv,t,groups,stages,sub",
     [
-        (2, 8, 2, 700, 1, 2, 128),   # two additive full-width codebooks (histogram kernel)
+        (2, 8, 2, 700, 1, 2, 128),   # two additive full-width codebooks
         (2, 8, 2, 1, 1, 2, 128),     # ... a single token
         (1, 32, 8, 5000, 1, 16, 128),  # the reference's own GSRQ layout at depth 16, 4 query heads per KV head
         (1, 8, 8, 300, 1, 16, 128),  # the reference's own GSRQ layout, depth 16, no query-head sharing
@@ -115,9 +115,8 @@ def test_other_geometries(device, b, hq, hkv, t, groups, stages, sub):
         (1, 2, 2, 300, 32, 1, 4),     # ... without head sharing
     ],
 )
-def test_two_pass_kernel_for_head_dim_128_geometries(device, b, hq, hkv, t, groups, stages, sub):
-    """head_dim 128, groups at least 8 wide, at most two stages, at most 4 query heads per KV head, other than
-    the two specialised layouts: score table and value tables in shared memory, two passes."""
+def test_grouped_codebooks_of_one_and_two_stages_at_head_dim_128(device, b, hq, hkv, t, groups, stages, sub):
+    """The kernel for at most 32 slots: groups of every width, ragged ranges, an empty row."""
     work = _workload(31 + t, b, hq, hkv, t, groups, stages, sub, [0.2] * stages if sub >= 32 else None)
     start = [(7 * i) % 50 for i in range(b)]
     end = [t - (11 * i) % 40 for i in range(b)]
@@ -337,9 +336,31 @@ def test_attention_argument_errors(device):
         ops.attn_decode(work[0][:, :3].contiguous(), *work[1:])  # 3 query heads over 1 KV head is fine? no: rep=3 unsupported
 
 
-def test_very_large_batch_uses_the_generic_kernel(device):
-    """More than 1024 (row, head) pairs: the specialised scan steps aside (its per-pair tables would need > 64 MB)."""
+def test_very_large_batch_is_not_the_scans(device):
+    """More than 1024 (row, head) pairs: the benchmark layout's scan steps aside (its per-pair tables would need > 64 MB)."""
     work = _workload(21, 300, 16, 4, 70, 16, 2, 8)
     out, _ = _run(device, work)
     want, _ = C.attention(*work)
+    _check(out, want)
+
+
+@pytest.mark.parametrize(
+    "b,hq,hkv,t,groups,stages,sub,shift",
+    [
+        (2, 8, 2, 600, 1, 40, 128, 0),     # more than 32 slots
+        (2, 16, 2, 600, 8, 2, 16, 0),      # eight query heads per KV head
+        (2, 8, 2, 600, 16, 2, 8, 4),       # a query that does not start at a multiple of 16 bytes
+        (3, 2, 2, 1500, 1, 2, 128, 1),
+        (1, 2, 1, 900, 32, 2, 4, 0),       # 64 slots
+    ],
+)
+def test_head_dim_128_calls_that_only_the_general_kernel_takes(device, b, hq, hkv, t, groups, stages, sub, shift):
+    ops = _ops()
+    q, *rest = _workload(t + stages, b, hq, hkv, t, groups, stages, sub, [0.5 / stages**0.5] * stages if sub >= 16 else None)
+    start, end = [3 * i for i in range(b)], [t - 5 * i for i in range(b)]
+    room = torch.zeros(q.numel() + shift, dtype=torch.float16, device=device)
+    out, _ = ops.attn_decode(
+        room[shift:].view(q.shape).copy_(q), *(x.to(device) for x in rest), torch.tensor(start, dtype=torch.int32, device=device), torch.tensor(end, dtype=torch.int32, device=device)
+    )
+    want, _ = C.attention(q, *rest, start, end)
     _check(out, want)

@@ -32,9 +32,9 @@ def _workload(device, seed, b, hq, hkv, t, groups, stages, sub):
     "geometry",
     [
         (2, 8, 2, 1500, 16, 2, 8),   # the specialised scan (16 groups x 2 stages)
-        (2, 4, 2, 700, 1, 2, 128),   # full-width codebooks (histogram kernel)
-        (2, 4, 2, 500, 16, 1, 8),    # one-stage grouped codebooks (two-pass kernel)
-        (2, 16, 2, 333, 8, 2, 8),    # 8 query heads per KV head, head_dim 64 (generic kernel)
+        (2, 4, 2, 700, 1, 2, 128),   # full-width codebooks (at most 32 slots)
+        (2, 4, 2, 500, 16, 1, 8),    # one-stage grouped codebooks (at most 32 slots)
+        (2, 16, 2, 333, 8, 2, 8),    # 8 query heads per KV head, head_dim 64 (the general kernel)
     ],
 )
 def test_static_scratch_entry_point_matches_the_ordinary_one(device, geometry):

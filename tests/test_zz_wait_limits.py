@@ -50,6 +50,9 @@ def _encode(device, states, tables, spins, norms=None, whitener=None):
         (2, 5, 32, 4, 2, 256, True, False),
         (4, 1700, 8, 16, 2, 256, False, False),    # narrow groups, many rows
         (4, 1700, 4, 32, 1, 100, True, False),
+        (2, 33, 8, 16, 2, 256, False, True),       # ... and fp32 words, whole pairs a block
+        (4, 1700, 8, 16, 3, 200, False, True),
+        (3, 700, 4, 32, 1, 256, False, True),
     ],
 )
 def test_codes_do_not_depend_on_waits_that_run_out(device, heads, tokens, sub, groups, stages, words, norms, whitened, spins):
