@@ -188,8 +188,10 @@ TACVQ_API size_t tacvq_attn_workspace_bytes(int B, int Hq, int Hkv, int D, int G
  *                      against: never above the maximum score and at most 8 ln 2 below it; m + ln l
  *                      (the log-sum-exp) and acc / l do not depend on it
  *   Hq % Hkv == 0, Hq/Hkv <= 8, K == 256, D % 32 == 0, D <= 256.
- * On the two-stage layout of 16 x 8 the query (and the new rows of a decode step) are read before the attention launch
- * that precedes on the stream has ended: they must not be its result buffers themselves.
+ * Scores and weights are fp32, with these exceptions: on the two-stage layout of 16 x 8 with four query heads per KV head score
+ * table entries have 13 bits and weights enter the product with V as fp16 (with a rotary step only the latter, whatever the heads); ladders of up
+ * to 16 full-width stages with four query heads and no rotary step add weights in units of 2^-20 of the largest, below 2^-10 of it in units of 2^-30.
+ * A weight that is not a number makes its row's results so.
  */
 TACVQ_API int tacvq_attn_decode(const uint16_t *q_f16, const uint8_t *kcodes, const uint8_t *vcodes, const uint16_t *ktab_f16,
                       const uint16_t *vtab_f16, const int32_t *seq_start, const int32_t *seq_end, void *workspace,

@@ -41,8 +41,9 @@
 //            without a pair encode the rows and share the V codewords.  A build costs about 3.5 us of a 512-thread
 //            block per stage (64 values per thread, quarter-rate conversions); building inside the scan
 //            was measured twice and repeats that for every block that enters a pair (3.3 per pair).
-//            One row of 777 tokens takes 13.0 us a step (16.0 before the V codewords were shared by all SMs and
-//            the table's inputs were requested during the encode).  It is a chain of latencies: row 1.3 us, two encode stages 0.8 and 1.4, scores 1.4, quantising 2.0.
+//            One row of 777 tokens takes 15.8 us a step when steps follow one another, 33 alone.  It is a chain of latencies: scores 1.4, quantising
+//            2.0, beside a row's 1.3 us and two encode stages' 0.8 and 1.4.  (13.8 when all this ran before the launch in
+//            front had ended, which is not sound: that launch may compute the query, the rows or the tables.)
 //   scan     a persistent grid (one block per SM) walks the flattened (KV head, batch row, 32-token
 //            tile) space; every block gets an equal share of work units.  When it enters a new (batch
 //            row, KV head) pair it copies that pair's score table (64 KB, flat) and, when the head

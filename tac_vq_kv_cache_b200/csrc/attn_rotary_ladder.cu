@@ -31,8 +31,9 @@
 // of equal spread and falling by 0.9 and 0.6 a stage, 3.5e-10 to 9.3e-9 in the 2-norm against 3.5e-10 to 1.3e-8, and the same fp16
 // value in every case.
 //
-// us a decode step of 16 stages and 8 KV heads, against attn_rotary_kernel: one row of 6144 tokens with a window of 4096 51.4 / 114.5 (27 are the
-// new token's encode), 600 tokens 44 / 89, 16384 tokens 119 / 240, 8 x 2000 156 / 230, 16 x 1000 189 / 201.
+// us a decode step of 16 stages and 8 KV heads, against attn_rotary_kernel: one row of 6144 tokens with a window of 4096 50 / 107 (27 are the
+// new token's encode), 600 tokens 41 / 103, 16384 tokens 120 / 232, 8 x 2000 159 / 225, 16 x 1000 193 / 228; ladder_plan.cuh has the sizes that
+// are left to that kernel.  Tables, gathers and products are 16 stages wide for fewer stages too.
 //
 // Semantics replaced: experiments_followup_mistral/evaluate_mistral_longbench.py:112-122 including the rotary step
 // (:113-118); the query arrives rotated at its own position and scaled.

@@ -24,8 +24,8 @@
 // largest score itself as the reference, ten of the first sixteen segments set it anew.)
 //
 // us a decode step with 8 KV heads, against the kernels this one replaced (tables ordered [slot][code] for full-width words, rebuilt value
-// rows for groups): 2 x 128, 16 rows x 16384 tokens 36.7 / 50.8; 16 x 128, 2 x 32768 82 / 150; 16 x 8, 8 x 32768 81 / 240; 32 x 4 154 / 317;
-// 16 x 2 x 8 with two query heads a KV head 101 / 309, with one 150 / 303.
+// rows for groups): 2 x 128, 16 rows x 16384 tokens 31.4 / 44.7; 16 x 128, 2 x 32768 78 / 142; 16 x 8, 8 x 32768 94 / 229; 32 x 4 164 / 309;
+// 16 x 2 x 8 with two query heads a KV head 103 / 302, with one 141 / 296.  The second add of a weight is 18 us of the 94 and 14 of the 164.
 //
 // Short calls are bound by what a block does besides its tokens.  In clocks, one row of 100 tokens, 2 x 2 x 64: empty bins 1.6 k, score
 // table 17 k, folding the bins once 2.7 k (8 k for one slot), V words 7 k.  The table is a tensor-core product for every width from 16
