@@ -15,13 +15,14 @@
 // ordered [slot][code], where random codes collide (2.6 wavefronts a look-up instead of 1, 3.6 an add), that is what this kernel
 // gains.
 //
-// Weights are added as integers, because shared-memory integer adds are single instructions (a float add is a
-// compare-and-swap loop).  FINE: a weight's multiple of 2^-19 goes to one bin and what that leaves, in units of 2^-38, to another,
-// which keeps all 24 bits of a weight down to 2^-15 and costs two adds.  Otherwise weights from 2^-10 on are added in units of 2^-20, smaller ones in units of
-// 2^-30 and in bins of their own, one add each; ladders of up to 16 full-width stages with four query heads are content with that, as their weights had 18 bits before.
-// Integer sums are exact and the result does not depend on the order.  A weight is relative to a reference that lies a little (kHeadroom) above the largest score when it was last set; when a
-// score exceeds it, or the bins could overflow, they are folded into fp32 sums that every thread keeps in registers.  (With the
-// largest score itself as the reference, ten of the first sixteen segments set it anew.)
+// Weights are added as integers, because shared-memory integer adds are single instructions (a float add is a compare-and-swap
+// loop).  FINE: a weight's multiple of 2^-19 goes to one bin and what that leaves, in units of 2^-38, to another, which keeps all 24
+// bits of a weight down to 2^-15 and costs two adds.  Otherwise weights from 2^-10 on are added in units of 2^-20, smaller ones in
+// units of 2^-30 and in bins of their own, one add each; ladders of up to 16 full-width stages with four query heads are content
+// with that, as their weights had 18 bits before. Integer sums are exact and the result does not depend on the order.  A weight is
+// relative to a reference that lies a little (kHeadroom) above the largest score when it was last set; when a score exceeds it, or
+// the bins could overflow, they are folded into fp32 sums that every thread keeps in registers.  (With the largest score itself as
+// the reference, ten of the first sixteen segments set it anew.)
 //
 // us a decode step with 8 KV heads, against the kernels this one replaced (tables ordered [slot][code] for full-width words, rebuilt value
 // rows for groups): 2 x 128, 16 rows x 16384 tokens 31.4 / 44.7; 16 x 128, 2 x 32768 78 / 142; 16 x 8, 8 x 32768 94 / 229; 32 x 4 164 / 309;
@@ -142,8 +143,8 @@ __device__ __forceinline__ void permute_words(uint32_t (&w)[NW], int x) {
 // block's heads is missing
 template <int P, bool FULL, bool FINE, bool ALL>
 __device__ __forceinline__ void add_weights(const uint32_t (&codes)[Shape<P>::kCodeWords], const uint32_t (&w)[Shape<P>::kHeads],
-                                            const uint32_t (&rest)[Shape<P>::kHeads], const uint32_t (&to)[Shape<P>::kHeads], const uint32_t (&sel)[4], uint32_t lane_xor, int x,
-                                            int slots, int rot, int heads) {
+                                            const uint32_t (&rest)[Shape<P>::kHeads], const uint32_t (&to)[Shape<P>::kHeads],
+                                            const uint32_t (&sel)[4], uint32_t lane_xor, int x, int slots, int rot, int heads) {
     constexpr int H = Shape<P>::kHeads;
 #pragma unroll
     for (int k = 0; k < P; ++k) {
