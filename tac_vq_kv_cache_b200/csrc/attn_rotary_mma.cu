@@ -10,7 +10,7 @@
 //            of the B operand are (4 heads) x (lower | upper query channels); the two halves of a score
 //            meet through one shuffle.  fp32 scores go to shared memory.
 //   softmax  maximum of every row and head, p = exp(score - max) as fp16 [row][head][token] over the score area.
-//   pass V   value tables loaded over the key tables (the copy overlaps the softmax step); P.V with
+//   pass V   value tables loaded over the key tables; P.V with
 //            m16n8k8 products exactly as in the kernel without rotary step (attn_gsrq.cu): rows =
 //            channels, columns = 4 heads x 2 visiting orders, contraction = tokens; value codes land by
 //            cp.async and are handed out by ldmatrix.trans.
@@ -19,8 +19,9 @@
 // long as the score area allows, because each one copies both tables (2 x 128 KB).
 //
 // What bounds it: wavefronts of the L1/shared pipe and the latency between them at 16 warps.  A block of 4856 tokens, in clocks: copies
-// and softmax 25 k, pass K 44 k (9.2 a token, 6.2 of them wavefronts), pass V 25 k (5.2, of which 4.4 are look-ups).  us a decode step with 8 KV
-// heads, against a row and at most 4096 tokens a block: 8 rows x 32768 183 / 205, a window of 4096 of them 45 / 91, 2 x 65536 115 / 148.
+// and softmax 16 k (25 k when scattered 16-byte cp.async filled the tables), pass K 44 k (9.2 a token, 6.2 of them wavefronts), pass V 25 k (5.2, of
+// which 4.4 are look-ups).  us a decode step with 8 KV heads, 8 rows x 32768: 165 (180 with those copies).  Against a row and at most 4096 tokens a
+// block, before: 8 rows x 32768 183 / 205, a window of 4096 of them 45 / 91, 2 x 65536 115 / 148.
 //
 // Every shared-memory gather is conflict-free for arbitrary codes: a code's 32 codewords lie in one
 // 512-byte row, the position of (stage, group) inside the row decides the bank, and the lanes that are
@@ -32,7 +33,7 @@
 // a packed multiply and a fused multiply-add per channel pair (the reference rounds both products), and
 // probabilities enter the P.V product as fp16.
 
-#include "common.cuh"
+#include "table_rows.cuh"
 
 namespace tacvq {
 
@@ -108,22 +109,6 @@ __device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1,
         : "r"(a0), "r"(a1), "r"(b0));
 }
 
-// position of the codeword (stage s, group g) inside a code's 512-byte row; the bank is s*4 + g%4 (as in attn_gsrq.cu)
-__device__ __forceinline__ int word_pos(int s, int g) { return (g >> 2) * 8 + s * 4 + (g & 3); }
-
-// A head's tables [stage][group][word][8] -> shared memory rows [word][position].  The copies of eight neighbouring lanes go
-// out together: they take two neighbouring words of four positions, whole 32-byte sectors (eight positions of one word, without
-// the two-way conflict on arrival, asked L2 for every sector twice).  Blocks of one head start at different places (`first`), so
-// that they do not all ask for the same lines at the same time.
-__device__ __forceinline__ void copy_tables(uint32_t tab_u32, const __half *__restrict__ src, int tid, int first) {
-#pragma unroll 4
-    for (int idx = tid; idx < kWords * 32; idx += kThreads) {
-        const int lane = idx & 31, rest = ((idx >> 5) + (first & 15) * (kThreads / 32)) & 255;
-        const int word = (rest >> 2) * 4 + (lane >> 4) * 2 + (lane & 1), s = (lane >> 3) & 1, g = (rest & 3) * 4 + ((lane >> 1) & 3);
-        cp_async16(tab_u32 + word * kRowBytes + word_pos(s, g) * 16, src + ((size_t)(s * 16 + g) * kWords + word) * 8);
-    }
-}
-
 template <int R>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uint8_t *vcodes,
@@ -145,7 +130,7 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
     const int b0 = (int)((int64_t)blockIdx.z * B / gridDim.z), n_rows = (int)((int64_t)(blockIdx.z + 1) * B / gridDim.z) - b0;
 
     // A decode step's new codes and ranges come from the kernel before this one; the tables and the query do not.
-    copy_tables(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, tid, split);
+    copy_table_rows<kWarps>(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, warp, lane);
     wait_for_previous_kernel();
     // positions that some row of the block sees, and this split's share of them
     int lo_all = 0x7fffffff, hi_all = 0;
@@ -165,7 +150,6 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
             const int r = idx / (kDim + 2), col = idx % (kDim + 2);
             part[((int64_t)split * rows + (int64_t)(b0 + r / rep) * Hq + h * rep + r % rep) * (kDim + 2) + col] = col == 0 ? -INFINITY : 0.0f;
         }
-        cp_async_wait_all();  // no copy outlives the block
         return;
     }
     const size_t row_step = (size_t)Hkv * (size_t)T_cap * 32;  // code bytes from one batch row to the next
@@ -198,7 +182,7 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
         }
         // step (ci, sf) gathers group j + 4 ci of stage sf ^ (token parity), which lies 128 ci bytes behind that of ci = 0
         const int first_stage = g8 & 1;
-        const uint32_t k_off[2] = {tab_u32 + word_pos(first_stage, j4) * 16, tab_u32 + word_pos(first_stage ^ 1, j4) * 16};
+        const uint32_t k_off[2] = {tab_u32 + word_place(first_stage, j4) * 16, tab_u32 + word_place(first_stage ^ 1, j4) * 16};
         const uint32_t k_sel = 0x4404u | ((uint32_t)j4 << 4);  // byte j of a word -> bits 8..15
         // a token's 32 code bytes: stage s at bytes 16s..16s+15; group j + 4 ci is byte j of word ci
         const uint8_t *kc = kcodes + code_at + first_stage * 16;
@@ -225,7 +209,6 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
             rn[2] = __ldg(cs + 8), rn[3] = __ldg(cs + 12);     // sines
         };
         fetch_rope(warp * 8 + g8);
-        cp_async_wait_all();
         __syncthreads();
         fetch_codes(0, warp * 8 + g8);
 #pragma unroll 1
@@ -274,8 +257,8 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
     }
     __syncthreads();
 
-    // ---- softmax over the block's tokens, kRowWarps warps a batch row; value tables arrive meanwhile ---
-    copy_tables(tab_u32, vtab + (size_t)h * 2 * 16 * kWords * 8, tid, split);
+    // ---- value tables; softmax over the block's tokens, kRowWarps warps a batch row ---
+    copy_table_rows<kWarps>(tab_u32, vtab + (size_t)h * 2 * 16 * kWords * 8, warp, lane);
     const int n_pad = (n + 31) & ~31;
     const int row = warp / kRowWarps, row_warp = warp % kRowWarps;
     const bool row_live = row < n_rows;
@@ -336,7 +319,7 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
 #pragma unroll
         for (int gsel = 0; gsel < 2; ++gsel) {
             const int s = sp ^ (kq & 1), gh = gsel ^ (kq >> 1);
-            v_off[sp][gsel] = tab_u32 + word_pos(s, 2 * r8 + gh) * 16;
+            v_off[sp][gsel] = tab_u32 + word_place(s, 2 * r8 + gh) * 16;
         }
 #pragma unroll
     for (int tk = 0; tk < 2; ++tk)
@@ -366,7 +349,7 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
     for (int mm = 0; mm < 8; ++mm) acc[mm][0] = acc[mm][1] = acc[mm][2] = acc[mm][3] = 0.0f;
     __syncthreads();  // probabilities written; nobody reads scores any more
     if (row_warp < tiles) land_codes(row_warp);
-    cp_async_wait_all();  // the value tables and the first tile of codes
+    cp_async_wait_all();  // the first tile of codes
     __syncthreads();
     for (int tile = row_warp; tile < tiles; tile += kRowWarps) {
         uint32_t vm_lo[4], vm_hi[4];  // tokens 0..15 and 16..31 of the tile
