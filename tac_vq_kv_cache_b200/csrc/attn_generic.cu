@@ -173,6 +173,7 @@ attn_combine_kernel(const float *states, int n_parts, int64_t rows, int D, __hal
     const float *own = states + row * W;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
     wait_for_previous_kernel();
+    launch_dependents();  // the next kernel may be scheduled; one that follows as a dependent waits for this grid itself
     if (n_parts <= kCombineFew) {
         for (int i = tid; i < D; i += blockDim.x) {
             float m[kCombineFew], part[kCombineFew], v[kCombineFew];

@@ -36,19 +36,19 @@
 // once; the successor waits for it before touching its results):
 //   prepare  one block per (batch row, KV head, stage): the score table of the pair (q . codeword for
 //            4096 codewords x 4 heads straight from the fp16 K tables, quantised to 13 bits), written to
-//            scratch in the order the scan's shared memory wants; its share of the V codewords in that
-//            order; and, in a decode step, the codes of the pair's new K or V row and the visible ranges.  Blocks on SMs
-//            without a pair encode the rows and share the V codewords.  A build costs about 3.5 us of a 512-thread
-//            block per stage (64 values per thread, quarter-rate conversions); building inside the scan
-//            was measured twice and repeats that for every block that enters a pair (3.3 per pair).
-//            One row of 777 tokens takes 15.8 us a step when steps follow one another, 33 alone.  It is a chain of latencies: scores 1.4, quantising
-//            2.0, beside a row's 1.3 us and two encode stages' 0.8 and 1.4.  (13.8 when all this ran before the launch in
-//            front had ended, which is not sound: that launch may compute the query, the rows or the tables.)
+//            scratch in the order the scan's shared memory wants; and, in a decode step, the codes of the pair's new K or V row
+//            (in blocks of their own where there are SMs enough) and the visible ranges.  Building the table
+//            inside the scan was measured twice and repeats that for every block that enters a pair (3.3 per pair).
+//            It waits for the launch in front of it before it reads anything: that launch may compute the query, the rows or the tables.
+//            Then it lets the scan start, which may therefore read whatever is older than this grid before its own wait is over.
+//            One row of 777 tokens takes 13.8 us a step when steps follow one another (15.8 before; the host needs as long to
+//            launch them), in us after the start: inputs there 1.0 (2.9 with a lane per group, whose loads are 16 lines each), products
+//            1.9, range 2.5, table stored 3.4, scan goes on 4.3, its tables and codes there 6.0, tiles 7.1, state stored 8.9, seen by the others 10.2, merged 11.8.
 //   scan     a persistent grid (one block per SM) walks the flattened (KV head, batch row, 32-token
 //            tile) space; every block gets an equal share of work units.  When it enters a new (batch
 //            row, KV head) pair it copies that pair's score table (64 KB, flat) and, when the head
-//            changed, the head's V codewords, which the prepare grid wrote in their bank-striped
-//            order (128 KB, flat).  It writes one partial
+//            changed, the head's V codewords in bank-striped order (128 KB, table_rows.cuh; the first ones while the
+//            prepare grid runs, where it leaves an SM free).  It writes one partial
 //            softmax state per pair it touches, then marks it; the block that finds every partial of a
 //            pair marked merges them (log-sum-exp) and writes fp16 output and/or fp32 state.  A pair
 //            that lies inside one block's share is written directly.
@@ -61,8 +61,8 @@
 
 #include <atomic>
 
-#include "common.cuh"
 #include "encode_rows.cuh"
+#include "table_rows.cuh"
 
 namespace tacvq {
 
@@ -88,9 +88,6 @@ constexpr int kMaxBatch = 512;
 #ifndef TACVQ_GSRQ_EARLY_K
 #define TACVQ_GSRQ_EARLY_K 0  // 1: the next tile's K codes are requested before the score phase (8 more registers live)
 #endif
-#ifndef TACVQ_GSRQ_VPERM
-#define TACVQ_GSRQ_VPERM 1  // 1: the prepare grid writes the V codewords in shared-memory order, the scan copies them flat
-#endif
 #ifndef TACVQ_GSRQ_LAZY_MAX
 #define TACVQ_GSRQ_LAZY_MAX 1  // 0: every tile reduces its maximum over the warp (20 shuffles)
 #endif
@@ -110,7 +107,7 @@ constexpr int kVCodeBytes = kTile * 32;                     // one tile of V cod
 constexpr int kProbStride = 72;                             // bytes per head of the fp16 probabilities: 64 + 8, so the four heads' reads hit different banks
 constexpr int kStagePerWarp = kVCodeBytes + 4 * kProbStride + 32;  // + fp16 probabilities [4 heads][32 tokens], 64-byte multiple
 constexpr int kStageBytes = kWarps * kStagePerWarp;         // 20480 at 16 warps (also scratch of the table build)
-constexpr int kPrefixBytes = (kMaxBatch + 8) * 4 + 12 * 4;
+constexpr int kPrefixBytes = (kMaxBatch + 8) * 4 + (12 + 2 * kWarps * kRep) * 4;  // the work prefix; steps and offset; the warps' references and weights
 constexpr int kSmemBytes = kLutBytes + kVtabBytes + kStageBytes + kPrefixBytes;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -191,9 +188,6 @@ __device__ __forceinline__ long long block_first_tile(long long total, int block
     return total * block / blocks;
 }
 
-// position of slot (stage s, group g) inside a code's 512-byte row of the value table
-__device__ __forceinline__ int value_pos(int s, int g) { return (g >> 2) * 8 + s * 4 + (g & 3); }
-
 using NewToken = GsrqNewToken;
 
 // ------------------------------------------------------------------------------------------------
@@ -201,64 +195,60 @@ using NewToken = GsrqNewToken;
 // ------------------------------------------------------------------------------------------------
 //   lut_g[p][code][slot]   8 bytes: four 13-bit fields, field r = round((q_r . word - min_slot_r) / step_stage_r)
 //   scale_g[p][stage*8+r]  step_stage_r * log2 e;  [stage*8+4+r] = sum over the stage's slots of min_slot_r * log2 e
-// A lane always works on group lane % 16 and on one of the two codes its warp covers per round, so the
-// 16 lanes of a half warp read sixteen 4 KB-strided table rows in 32-byte sectors that the other half
-// warp completes, and write 128 contiguous bytes.  Each stage has its own step, so the finer second
-// stage keeps its precision.
+// A warp works on one group, a lane on words lane + 32 i, so the words arrive in whole lines (a lane per group, which makes the stores
+// whole lines instead, has 16 lines a load and took 1.5 us longer); the entries are turned in shared memory.  Each stage has its own
+// step, so the finer second stage keeps its precision.
 constexpr int kPrepThreads = 512;
 constexpr int kPrepWarps = kPrepThreads / 32;
-constexpr int kPrepCodes = kWords / (2 * kPrepWarps);  // codes per thread
+constexpr int kPrepWords = kWords / 32;  // words per thread
+static_assert(kPrepWarps == kGroups && kStages == 2 && kWords == 256, "a warp per group, 8 words per lane and stage");
+
+__device__ __forceinline__ float warp_min(float v) {
+    float d;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(v));
+    return d;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float d;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(v));
+    return d;
+}
 
 // APART: a block of the first 2 * B * Hkv builds a table, and one of as many again encodes a row beside it, which makes the chain of a small
-// batch shorter (one row of 777 tokens 15.8 us a step, 17.4 with both in one block, one after the other).
+// batch shorter.
 template <bool APART>
 __global__ void __launch_bounds__(kPrepThreads)
 attn_gsrq_prepare_kernel(const __half *q, const __half *ktab, const __half *vtab,
-                         uint2 *__restrict__ lut_g, float *__restrict__ scale_g, uint4 *__restrict__ vperm_g, int B, int Hkv, const NewToken fresh) {
-    __shared__ float red[kPrepWarps * 8 * kGroups];  // [warp][min x4, max x4][group]
-    __shared__ __align__(16) float low_s[kGroups * kRep], step_s[12];  // smallest entry per group and head; per head 1 / step, step, offset
-    launch_dependents();  // the scan may be scheduled as soon as SMs free up; it waits for this grid itself
+                         uint2 *__restrict__ lut_g, float *__restrict__ scale_g, int B, int Hkv, const NewToken fresh) {
+    __shared__ __align__(16) float low_s[kGroups * kRep], range_s[kGroups * kRep];  // smallest entry and range per group and head
+    __shared__ __align__(16) unsigned char turn_s[kWords * kGroups * 8];            // entries [code][group ^ code % 16]
     // The launch before this one may be what computes the query, the rows or the tables, and let this grid start before it has stored
     // them (a scan does, and so may a matrix product of another library); a scan also still reads the scratch that is written here.
     wait_for_previous_kernel();
+    // The scan may be scheduled as SMs free up.  It waits for this grid itself, but not before that order to read what is older than this grid.
+    launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tables = 2 * B * Hkv, own = (int)blockIdx.x % tables;
     const bool builds = (int)blockIdx.x < tables;
-    const bool encodes = fresh.k_rows != nullptr && (APART ? (int)blockIdx.x / tables == 1 : builds);
+    const bool encodes = fresh.k_rows != nullptr && (APART ? !builds : builds);
     const int pair = own >> 1, stage = own & 1;
     const int h = pair / B, b = pair % B;
     const int Hq = Hkv * kRep;
-    const int g = lane & 15, half = lane >> 4;
-#if TACVQ_GSRQ_VPERM
-    auto permute_values = [&]() {  // this block's share of the V codewords, in the scan's order
-        const int perm_total = Hkv * kWords * kSlots;
-        const int perm_per_block = (perm_total + (int)gridDim.x - 1) / (int)gridDim.x;
-        for (int local = tid; local < perm_per_block; local += kPrepThreads) {
-            const int e = blockIdx.x * perm_per_block + local;
-            if (e < perm_total) {
-                const int hh = e >> 13, code = (e >> 5) & 255, pos = e & 31;
-                const int s = (pos >> 2) & 1, gg = ((pos >> 3) << 2) | (pos & 3);
-                vperm_g[e] = *reinterpret_cast<const uint4 *>(vtab + ((((size_t)hh * kStages + s) * kGroups + gg) * kWords + code) * kSub);
-            }
-        }
+    // inputs of the table build: the group's words and the heads' channels of it
+    const uint4 *tab = reinterpret_cast<const uint4 *>(ktab + (((size_t)h * kStages + stage) * kGroups + warp) * kWords * kSub);
+    uint4 raw[kPrepWords], qraw[kRep];
+    auto fetch_build = [&]() {
+#pragma unroll
+        for (int i = 0; i < kPrepWords; ++i) raw[i] = tab[lane + 32 * i];
+#pragma unroll
+        for (int r = 0; r < kRep; ++r) qraw[r] = *reinterpret_cast<const uint4 *>(q + ((size_t)b * Hq + h * kRep + r) * kDim + warp * kSub);
     };
-#endif
+    if (builds && (APART || !encodes)) fetch_build();
     // A decode step's new token: this block (pair, side = stage) encodes the 16 groups of the pair's new K
     // (side 0) or V (side 1) row, a warp per group, with the arithmetic of the row-at-a-time encode kernel.
     // The words of both stages are requested at once (one memory latency instead of two).
-    // inputs of the table build
-    const uint4 *tab = reinterpret_cast<const uint4 *>(ktab + (((size_t)h * kStages + stage) * kGroups + g) * kWords * kSub);
-    uint4 raw[kPrepCodes], qraw[kRep];
-    auto fetch_build = [&]() {
-#pragma unroll
-        for (int c = 0; c < kPrepCodes; ++c) raw[c] = tab[warp * 2 + half + 2 * kPrepWarps * c];
-#pragma unroll
-        for (int r = 0; r < kRep; ++r) qraw[r] = *reinterpret_cast<const uint4 *>(q + ((size_t)b * Hq + h * kRep + r) * kDim + g * kSub);
-    };
-    if (builds && (APART || !encodes)) fetch_build();
     if (encodes) {
         int fresh_code[kStages] = {0, 0};
-        static_assert(kPrepWarps == kGroups && kStages == 2 && kWords == 256, "a warp per group, 8 words per lane and stage");
         const __half *side_tab = stage ? vtab : ktab;
         const uint4 *words0 = reinterpret_cast<const uint4 *>(side_tab + (((size_t)h * kStages + 0) * kGroups + warp) * kWords * kSub);
         const uint4 *words1 = words0 + (size_t)kGroups * kWords;
@@ -307,112 +297,71 @@ attn_gsrq_prepare_kernel(const __half *q, const __half *ktab, const __half *vtab
             fresh.seq_end[i] = fresh.end;
         }
     }
-    if (!builds) {
-#if TACVQ_GSRQ_VPERM
-        permute_values();
-#endif
-        return;
-    }
-    float qv[kRep][kSub];
-#pragma unroll
-    for (int r = 0; r < kRep; ++r) {
-        const uint4 qr = qraw[r];
-        const __half2 *hp = reinterpret_cast<const __half2 *>(&qr);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 f = __half22float2(hp[i]);
-            qv[r][2 * i] = f.x;
-            qv[r][2 * i + 1] = f.y;
-        }
-    }
-    float val[kPrepCodes][kRep];
+    if (!builds) return;
+    float val[kPrepWords][kRep];
     float mn[kRep], mx[kRep];
 #pragma unroll
-    for (int r = 0; r < kRep; ++r) { mn[r] = INFINITY; mx[r] = -INFINITY; }
+    for (int r = 0; r < kRep; ++r) {
+        float qv[kSub];
+        unpack8(qraw[r], qv);
+        mn[r] = INFINITY;
+        mx[r] = -INFINITY;
 #pragma unroll
-    for (int c = 0; c < kPrepCodes; ++c) {
-        const __half2 *hp = reinterpret_cast<const __half2 *>(&raw[c]);
-        float w[kSub];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 f = __half22float2(hp[i]);
-            w[2 * i] = f.x;
-            w[2 * i + 1] = f.y;
-        }
-#pragma unroll
-        for (int r = 0; r < kRep; ++r) {
+        for (int i = 0; i < kPrepWords; ++i) {
+            float w[kSub];
+            unpack8(raw[i], w);
             float dot = 0.0f;
 #pragma unroll
-            for (int i = 0; i < kSub; ++i) dot = fmaf(qv[r][i], w[i], dot);
-            val[c][r] = dot;
+            for (int c = 0; c < kSub; ++c) dot = fmaf(qv[c], w[c], dot);
+            val[i][r] = dot;
             mn[r] = fminf(mn[r], dot);
             mx[r] = fmaxf(mx[r], dot);
         }
     }
-    // range of every (group, head) over the 256 codes: the two lane halves by shuffles, the warps through shared memory, where a
-    // thread per (head, group) also folds the groups into the head's common step
+    // range of the group and every head over the 256 codes; then, by every warp, the head's common step and the sum of its low ends
 #pragma unroll
-    for (int r = 0; r < kRep; ++r) {
-        mn[r] = fminf(mn[r], __shfl_xor_sync(0xffffffffu, mn[r], 16));
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 16));
-        if (half == 0) {
-            red[(warp * 8 + r) * kGroups + g] = mn[r];
-            red[(warp * 8 + 4 + r) * kGroups + g] = mx[r];
-        }
+    for (int r = 0; r < kRep; ++r) mn[r] = warp_min(mn[r]), mx[r] = warp_max(mx[r]);
+    if (lane == 0) {
+        *reinterpret_cast<float4 *>(low_s + warp * kRep) = make_float4(mn[0], mn[1], mn[2], mn[3]);
+        *reinterpret_cast<float4 *>(range_s + warp * kRep) = make_float4(mx[0] - mn[0], mx[1] - mn[1], mx[2] - mn[2], mx[3] - mn[3]);
     }
     __syncthreads();
-    if (tid < kRep * kGroups) {
-        const int r = tid >> 4;
-        float lo = red[r * kGroups + g], hi = red[(4 + r) * kGroups + g];
+    float range = fmaxf(range_s[lane], range_s[lane + 32]), offs = low_s[lane] + low_s[lane + 32];  // head lane % 4, groups lane / 4 and 8 on
 #pragma unroll
-        for (int w = 1; w < kPrepWarps; ++w) {
-            lo = fminf(lo, red[(w * 8 + r) * kGroups + g]);
-            hi = fmaxf(hi, red[(w * 8 + 4 + r) * kGroups + g]);
-        }
-        low_s[g * kRep + r] = lo;
-        float range = hi - lo, offs = lo;
-#pragma unroll
-        for (int off = 8; off >= 1; off >>= 1) {
-            range = fmaxf(range, __shfl_xor_sync(0xffffffffu, range, off));
-            offs += __shfl_xor_sync(0xffffffffu, offs, off);
-        }
-        if (g == 0) {
-            const float step = range > 0.0f ? range / (float)kEntryMax : 1.0f;
-            step_s[r] = 1.0f / step;
-            step_s[4 + r] = step * kLog2e;
-            step_s[8 + r] = offs * kLog2e;
-        }
+    for (int off = 16; off >= 4; off >>= 1) {
+        range = fmaxf(range, __shfl_xor_sync(0xffffffffu, range, off));
+        offs += __shfl_xor_sync(0xffffffffu, offs, off);
     }
-    __syncthreads();
+    const float step = range > 0.0f ? range / (float)kEntryMax : 1.0f, inv = 1.0f / step;
+    if (tid < kRep) {
+        float *scale = scale_g + ((size_t)pair * kStages + stage) * 8 + tid;  // steps, then offsets
+        scale[0] = step * kLog2e;
+        scale[kRep] = offs * kLog2e;
+    }
     float inv_step[kRep];
-    {
-        const float4 low = *reinterpret_cast<const float4 *>(low_s + g * kRep), inv = *reinterpret_cast<const float4 *>(step_s);
-        mn[0] = low.x, mn[1] = low.y, mn[2] = low.z, mn[3] = low.w;
-        inv_step[0] = inv.x, inv_step[1] = inv.y, inv_step[2] = inv.z, inv_step[3] = inv.w;
-    }
-    uint32_t packed[kPrepCodes][2];
 #pragma unroll
-    for (int c = 0; c < kPrepCodes; ++c) {
+    for (int r = 0; r < kRep; ++r) inv_step[r] = __shfl_sync(0xffffffffu, inv, r);
+#pragma unroll
+    for (int i = 0; i < kPrepWords; ++i) {
         uint32_t e[kRep];
 #pragma unroll
         for (int r = 0; r < kRep; ++r) {
             // round to nearest by adding 2^23 (full-rate add and mask instead of a quarter-rate conversion);
             // the argument is in [0, 8191.x]
-            const float t = fmaf(val[c][r] - mn[r], inv_step[r], 8388608.0f);
+            const float t = fmaf(val[i][r] - mn[r], inv_step[r], 8388608.0f);
             e[r] = min((uint32_t)kEntryMax, __float_as_uint(t) & 0x3fffu);
         }
-        packed[c][0] = e[0] | (e[1] << 16);
-        packed[c][1] = e[2] | (e[3] << 16);
+        const int code = lane + 32 * i;  // sixteen neighbouring codes store to sixteen different places of eight bytes
+        *reinterpret_cast<uint2 *>(turn_s + code * (kGroups * 8) + ((warp ^ (code & 15)) * 8)) = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
     }
+    __syncthreads();
 #pragma unroll
-    for (int c = 0; c < kPrepCodes; ++c) {
-        const int code = warp * 2 + half + 2 * kPrepWarps * c;
-        lut_g[((size_t)pair * kWords + code) * kSlots + stage * kGroups + g] = make_uint2(packed[c][0], packed[c][1]);
+    for (int i = 0; i < kWords * kGroups / 2 / kPrepThreads; ++i) {  // groups 2p and 2p + 1 of a code
+        const int u = tid + i * kPrepThreads, code = u >> 3, p = u & 7;
+        uint4 v = *reinterpret_cast<const uint4 *>(turn_s + code * (kGroups * 8) + ((p ^ ((code & 15) >> 1)) * 16));
+        if (code & 1) v = make_uint4(v.z, v.w, v.x, v.y);
+        *reinterpret_cast<uint4 *>(lut_g + ((size_t)pair * kWords + code) * kSlots + stage * kGroups + 2 * p) = v;
     }
-    if (tid < 2 * kRep) scale_g[((size_t)pair * kStages + stage) * 8 + tid] = step_s[4 + tid];  // steps, then offsets
-#if TACVQ_GSRQ_VPERM
-    permute_values();
-#endif
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -488,7 +437,7 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads, 1)
 attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 *lut_g, const float *scale_g,
-                      const __half *__restrict__ vtab, const uint4 *vperm_g, const int32_t *seq_start, const int32_t *seq_end, float *__restrict__ part, unsigned long long *__restrict__ marks,
+                      const __half *__restrict__ vtab, const int32_t *seq_start, const int32_t *seq_end, float *__restrict__ part, unsigned long long *__restrict__ marks,
                       __half *__restrict__ out, float *__restrict__ state_out, int B, int Hkv, int T_cap,
                       unsigned long long epoch, int known_start, int known_end) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -496,7 +445,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
     unsigned char *vtab_s = smem + kLutBytes;
     unsigned char *stage_s = vtab_s + kVtabBytes;
     int *prefix_s = reinterpret_cast<int *>(stage_s + kStageBytes);
-    float *scale_s = reinterpret_cast<float *>(prefix_s + kMaxBatch + 8);  // 16-byte aligned: 12 floats
+    float *scale_s = reinterpret_cast<float *>(prefix_s + kMaxBatch + 8);  // 16-byte aligned
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Hq = Hkv * kRep;
@@ -526,37 +475,10 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
         }
         __syncthreads();
     };
-    // value codewords of a head in the bank-striped rows [word][position].  Default: a flat 128 KB copy of what the
-    // prepare grid wrote in that order.  Without TACVQ_GSRQ_VPERM the block gathers them from the fp16 V tables
-    // [stage][group][word][8] itself (per trip a warp copies 4 neighbouring words of 8 positions with different
-    // banks: whole 32-byte sectors in, no conflicts out) and starts with the head it will most likely begin in
-    // before it waits for the prepare grid; measured 6 us per step slower than the flat copy.
-    auto copy_value_table = [&](int h) {
-#if TACVQ_GSRQ_VPERM
-        const uint4 *flat = vperm_g + (size_t)h * (kWords * kSlots);
-        for (int e = tid; e < kWords * kSlots; e += kThreads) cp_async16(smem_u32(vtab_s) + e * 16, flat + e);
-#else
-        const __half *src = vtab + (size_t)h * (kStages * kGroups * kWords * kSub);
-        const uint32_t dst = smem_u32(vtab_s);
-        for (int idx = tid; idx < kWords * kSlots; idx += kThreads) {
-            const int pos = ((idx >> 5) & 3) * 8 + (idx & 7);
-            const int word = ((idx >> 7) << 2) | ((idx >> 3) & 3);
-            const int s = (pos >> 2) & 1, g = ((pos >> 3) << 2) | (pos & 3);
-            cp_async16(dst + word * (kSlots * 16) + pos * 16, src + ((size_t)(s * kGroups + g) * kWords + word) * kSub);
-        }
-#endif
-    };
-
-    // The score and value tables come from the prepare grid, and the visible ranges and newest code rows may be
-    // written by it too (a decode step's new token): of the kernels of this chain, nothing is read before the wait.
-#if TACVQ_GSRQ_VPERM
-    int loaded_head = -1;
-#else
-    int loaded_head = min((int)(((long long)blockIdx.x * Hkv) / (long long)gridDim.x), Hkv - 1);
-    copy_value_table(loaded_head);
-#endif
-    wait_for_previous_kernel();
-    launch_dependents();  // the next kernel on the stream may take SMs as they free up; it waits for this grid itself
+    auto copy_value_table = [&](int h) { copy_table_rows<kWarps>(smem_u32(vtab_s), vtab + (size_t)h * (kStages * kGroups * kWords * kSub), warp, lane); };
+    // The score table, and a decode step's newest code rows, come from the prepare grid and are read after the wait.  What is older than
+    // that grid is there already, because it lets this one start only when its own wait is over: the visible ranges (a step's are
+    // known to the host), the V words.  The codes of the block's first tiles are brought to L2.
     work_prefix();
     const int tiles_per_head = prefix_s[B];
     const int total_tiles = tiles_per_head * Hkv;  // fits: checked by the dispatcher
@@ -566,6 +488,14 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
         cursor = (int)block_first_tile(total_tiles, blockIdx.x, blocks);
         my_end = (int)block_first_tile(total_tiles, blockIdx.x + 1, blocks);
     }
+    int loaded_head = -1;
+    bool waited = false;
+    auto wait_once = [&]() {
+        if (waited) return;
+        wait_for_previous_kernel();
+        launch_dependents();  // the next kernel on the stream may take SMs as they free up; it waits for this grid itself
+        waited = true;
+    };
 
     // ---- per-lane constants ------------------------------------------------------------------
     // score side: lane = token, slot visiting order permuted by XOR so a half warp covers 16 bank pairs
@@ -584,7 +514,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
 #pragma unroll
         for (int gsel = 0; gsel < 2; ++gsel) {
             const int s = sp ^ (kq & 1), gh = gsel ^ (kq >> 1);
-            v_off[sp][gsel] = smem_u32(vtab_s) + value_pos(s, 2 * r8 + gh) * 16;
+            v_off[sp][gsel] = smem_u32(vtab_s) + word_place(s, 2 * r8 + gh) * 16;
         }
 #pragma unroll
     for (int tk = 0; tk < 2; ++tk)
@@ -635,11 +565,32 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
 
         __syncthreads();  // previous item fully merged: tables and staging may be overwritten
 
-        // ---- tables of this item: the head's V codewords when the head changed, and the pair's score table,
-        //      which the prepare grid laid out for shared memory (a flat copy) ----------------------------------
+        const size_t row_base = ((size_t)b * Hkv + h) * (size_t)T_cap;
+
+        // codes of a tile: lane = token; rows past the end of the range re-read the last valid row
+        const uint8_t *k_row = kcodes + (row_base + (size_t)tok_lo_row) * 32, *v_row_g = vcodes + (row_base + (size_t)tok_lo_row) * 32;
+        auto code_offset = [=](int tile) -> uint32_t {  // byte offset of this lane's 32-byte code row (T_cap <= 2^26)
+            return (uint32_t)min(tile * kTile + lane, n_tokens - 1) * 32u;
+        };
+        // ---- tables of this item: the head's V codewords when the head changed; the pair's score table, which the prepare grid
+        //      laid out for shared memory (a flat copy); and the codes of every warp's first tile -----------------------------
+        const bool busy = tile_lo + warp < tile_hi;
+        if (!waited && busy) {
+            prefetch_l2(k_row + code_offset(tile_lo + warp));
+            prefetch_l2(v_row_g + code_offset(tile_lo + warp));
+        }
         if (h != loaded_head) {
             loaded_head = h;
             copy_value_table(h);
+        }
+        wait_once();
+        uint4 k0 = make_uint4(0, 0, 0, 0), k1 = k0;
+        if (busy) {
+            const uint32_t off = code_offset(tile_lo + warp);
+            const uint4 *kp = reinterpret_cast<const uint4 *>(k_row + off);
+            k0 = ldg_stream(kp); k1 = ldg_stream(kp + 1);
+            cp_async16(v_land, v_row_g + off);
+            cp_async16(v_land ^ 16u, v_row_g + off + 16);
         }
         {
             const unsigned char *l_src = reinterpret_cast<const unsigned char *>(lut_g) + (size_t)pair * kLutBytes;
@@ -651,7 +602,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             const float *sg = scale_g + (size_t)pair * 16;
             scale_s[tid] = tid < 4 ? sg[tid] : tid < 8 ? sg[4 + tid] : sg[tid - 4] + sg[tid + 4];
         }
-        cp_async_wait_all();
+        cp_async_wait_all();  // also the first tile's value codes
         __syncthreads();  // tables ready
 
         // ---- scan this block's tiles of the pair ----------------------------------------------
@@ -663,22 +614,6 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
         float m_ref[kRep], l_lane[kRep];
 #pragma unroll
         for (int r = 0; r < kRep; ++r) { m_ref[r] = -INFINITY; l_lane[r] = 0.0f; }
-
-        const size_t row_base = ((size_t)b * Hkv + h) * (size_t)T_cap;
-
-        // codes of a tile: lane = token; rows past the end of the range re-read the last valid row
-        const uint8_t *k_row = kcodes + (row_base + (size_t)tok_lo_row) * 32, *v_row_g = vcodes + (row_base + (size_t)tok_lo_row) * 32;
-        auto code_offset = [=](int tile) -> uint32_t {  // byte offset of this lane's 32-byte code row (T_cap <= 2^26)
-            return (uint32_t)min(tile * kTile + lane, n_tokens - 1) * 32u;
-        };
-        uint4 k0 = make_uint4(0, 0, 0, 0), k1 = k0;
-        if (tile_lo + warp < tile_hi) {
-            const uint32_t off = code_offset(tile_lo + warp);
-            const uint4 *kp = reinterpret_cast<const uint4 *>(k_row + off);
-            k0 = ldg_stream(kp); k1 = ldg_stream(kp + 1);
-            cp_async16(v_land, v_row_g + off);
-            cp_async16(v_land ^ 16u, v_row_g + off + 16);
-        }
 
         for (int tile = tile_lo + warp; tile < tile_hi; tile += kWarps) {
             const bool live = tile * kTile + lane < n_tokens;
@@ -851,27 +786,39 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             for (int off = 16; off >= 1; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
             l_warp[r] = t;
         }
+        // a warp's sums are relative to its own reference, which is within the rescale gap of its maximum
+        float *wm = scale_s + 12, *wl = wm + kWarps * kRep;  // [warps][4] each
+        if (lane == 0) *reinterpret_cast<float4 *>(wm + warp * kRep) = make_float4(m_ref[0], m_ref[1], m_ref[2], m_ref[3]);
         __syncthreads();  // every warp is done with the tables' score part and the staging area
         static_assert(kWarps * 32 * 32 * 4 <= kLutBytes, "merge scratch must fit in the score table");
-        float *wm = reinterpret_cast<float *>(stage_s);    // [warps][4]
-        float *wl = wm + kWarps * kRep;                     // [warps][4]
         float *wacc = reinterpret_cast<float *>(lut_s);    // [warps][8 products x 4 registers][32 lanes]
-        if (lane == 0) {
+        float top[kRep], factor[kRep];
+        {
+            float4 most = *reinterpret_cast<const float4 *>(wm);
+#pragma unroll 4  // (not further: this is run once or twice, and instructions come from far)
+            for (int w = 0; w < kWarps; ++w) {
+                const float4 v = *reinterpret_cast<const float4 *>(wm + w * kRep);
+                most = make_float4(fmaxf(most.x, v.x), fmaxf(most.y, v.y), fmaxf(most.z, v.z), fmaxf(most.w, v.w));
+            }
+            top[0] = most.x, top[1] = most.y, top[2] = most.z, top[3] = most.w;
 #pragma unroll
             for (int r = 0; r < kRep; ++r) {
-                wm[warp * kRep + r] = m_ref[r];  // reference of this warp's sums: within the rescale gap of its maximum
-                wl[warp * kRep + r] = l_warp[r];
+                // a warp without a token has nothing to add; a sum that is NaN spoils the others
+                factor[r] = l_warp[r] == 0.0f ? 0.0f : fast_exp2(m_ref[r] - top[r]);
+                l_warp[r] *= factor[r];
             }
         }
+        if (lane == 0) *reinterpret_cast<float4 *>(wl + warp * kRep) = make_float4(l_warp[0], l_warp[1], l_warp[2], l_warp[3]);
         {
             // accumulator register j of product mm: column 2kq + (j&1) -> head, row half j>>1; stored lane-major
+            const float f0 = (kq & 1) ? factor[2] : factor[0], f1 = (kq & 1) ? factor[3] : factor[1];
             float *base = wacc + (size_t)warp * 1024 + lane;
 #pragma unroll
             for (int mm = 0; mm < 8; ++mm) {
-                base[(mm * 4 + 0) * 32] = acc[mm][0];
-                base[(mm * 4 + 1) * 32] = acc[mm][1];
-                base[(mm * 4 + 2) * 32] = acc[mm][2];
-                base[(mm * 4 + 3) * 32] = acc[mm][3];
+                base[(mm * 4 + 0) * 32] = acc[mm][0] * f0;
+                base[(mm * 4 + 1) * 32] = acc[mm][1] * f1;
+                base[(mm * 4 + 2) * 32] = acc[mm][2] * f0;
+                base[(mm * 4 + 3) * 32] = acc[mm][3] * f1;
             }
         }
         // the blocks that hold a partial state of this pair (this block among them)
@@ -886,16 +833,13 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             const int lane0 = src_r8 * 4 + src_kq;
             const int r = 2 * src_kq + (j & 1);
             const int dim = (2 * src_r8 + (j >> 1)) * 8 + mm;  // row r8 holds group 2*r8, row r8+8 group 2*r8+1
-            float top = -INFINITY;
-            for (int w = 0; w < kWarps; ++w) top = fmaxf(top, wm[w * kRep + r]);
+            const float head_top = (j & 1) ? (src_kq ? top[3] : top[1]) : (src_kq ? top[2] : top[0]);
             float lsum = 0.0f, asum = 0.0f;
+#pragma unroll 4
             for (int w = 0; w < kWarps; ++w) {
-                const float mw = wm[w * kRep + r];
-                if (wl[w * kRep + r] == 0.0f) continue;  // no token; a sum that is NaN spoils the others
-                const float sc = fast_exp2(mw - top);
-                lsum += sc * wl[w * kRep + r];
                 const float *src = wacc + (size_t)w * 1024;
-                asum += sc * (src[(mm * 4 + j) * 32 + lane0] + src[(mm * 4 + (j ^ 2)) * 32 + (lane0 ^ 2)]);
+                lsum += wl[w * kRep + r];
+                asum += src[(mm * 4 + j) * 32 + lane0] + src[(mm * 4 + (j ^ 2)) * 32 + (lane0 ^ 2)];
             }
             if (n_parts == 1) {  // the whole pair was scanned here: this is the result
                 const size_t row = (size_t)b * Hq + h * kRep + r;
@@ -903,7 +847,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
                 if (state_out) {
                     float *dst = state_out + row * kStateWidth;
                     if (dim == 0) {
-                        dst[0] = top * kLn2;  // natural-log units outside the kernel
+                        dst[0] = head_top * kLn2;  // natural-log units outside the kernel
                         dst[1] = lsum;
                     }
                     dst[2 + dim] = asum;
@@ -911,7 +855,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             } else {
                 float *dst = part + ((size_t)(pair + blockIdx.x) * kRep + r) * kStateWidth;
                 if (dim == 0) {
-                    dst[0] = top * kLn2;
+                    dst[0] = head_top * kLn2;
                     dst[1] = lsum;
                 }
                 dst[2 + dim] = asum;
@@ -930,8 +874,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             }
             __syncthreads();
             const int seen = tid < n_parts ? (ld_acquire_u64(marks + pair + c_lo + tid) == epoch) : 1;
-            if (__syncthreads_and(seen)) {
-                __threadfence();
+            if (__syncthreads_and(seen)) {  // acquired above, for the whole block by the barrier
                 merge_pair_parts(part, pair + c_lo, n_parts, b, h, Hkv, out, state_out);
                 if (tid < n_parts) marks[pair + c_lo + tid] = 0ull;
             }
@@ -939,6 +882,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
         cursor = item_end;
     }
 
+    wait_once();  // a block without work; whoever waits for this grid may rely on the one before it
     // ---- rows with an empty range never enter the loop: their defined result (out 0, m -inf, l 0, acc 0) ----
     for (int pair = blockIdx.x; pair < B * Hkv; pair += gridDim.x) {
         const int h = pair / B, b = pair % B;
@@ -966,14 +910,13 @@ bool attn_gsrq_supported(int Hq, int Hkv, int D, int G, int S, int K) {
 static size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 struct GsrqWorkspace {  // offsets into the caller's scratch; slot index = pair + scan block
-    size_t part, marks, lut, vperm, scale, total;
+    size_t part, marks, lut, scale, total;
     GsrqWorkspace(int B, int Hkv, int sms) {
         const size_t pairs = (size_t)B * Hkv, slots = pairs + (size_t)sms;
         part = 0;  // one partial softmax state per (pair, scan block) incidence
         marks = align256(slots * gsrq::kRep * gsrq::kStateWidth * sizeof(float));
         lut = align256(marks + slots * sizeof(unsigned long long));
-        vperm = lut + pairs * gsrq::kLutBytes;
-        scale = vperm + (TACVQ_GSRQ_VPERM ? (size_t)Hkv * gsrq::kVtabBytes : 0);
+        scale = lut + pairs * gsrq::kLutBytes;
         total = align256(scale + pairs * gsrq::kStages * 8 * sizeof(float));
     }
 };
@@ -1026,16 +969,15 @@ int attn_gsrq_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vc
     const unsigned long long epoch = g_epoch.fetch_add(2, std::memory_order_relaxed);  // odd, so never 0 (= cleared)
     GsrqNewToken token = {};
     if (fresh) token = *fresh;
-    // a block per pair and stage; where that leaves SMs without one, further blocks encode the new token's rows, as far as there are enough for all, and
-    // share the permutation of the V codewords (16 blocks alone take 4.5 us for 8 heads' 1 MB)
-    const int prepare_blocks = TACVQ_GSRQ_VPERM && 2 * B * Hkv < sms ? sms : 2 * B * Hkv;
-    auto prepare = fresh && prepare_blocks >= 4 * B * Hkv ? gsrq::attn_gsrq_prepare_kernel<true> : gsrq::attn_gsrq_prepare_kernel<false>;
-    cudaError_t e = launch_dependent(true, prepare, dim3(prepare_blocks), dim3(gsrq::kPrepThreads), 0, stream, q,
-                                     ktab, vtab, lut, scale, (uint4 *)(base + ws.vperm), B, Hkv, token);
+    // a block per pair and stage; as many again encode the new token's rows, where there are SMs enough for both
+    const int tables = 2 * B * Hkv;
+    const bool apart = fresh != nullptr && 2 * tables <= sms;
+    cudaError_t e = launch_dependent(true, apart ? gsrq::attn_gsrq_prepare_kernel<true> : gsrq::attn_gsrq_prepare_kernel<false>,
+                                     dim3(apart ? 2 * tables : tables), dim3(gsrq::kPrepThreads), 0, stream, q, ktab, vtab, lut, scale, B, Hkv, token);
     int st = e == cudaSuccess ? launch_status() : (int)e;
     if (st != TACVQ_OK) return st;
     e = launch_dependent(true, gsrq::attn_gsrq_scan_kernel, dim3(sms), dim3(gsrq::kThreads), gsrq::kSmemBytes, stream, kcodes, vcodes,
-                         (const uint2 *)lut, (const float *)scale, vtab, (const uint4 *)(base + ws.vperm), seq_start, seq_end, part, marks, out,
+                         (const uint2 *)lut, (const float *)scale, vtab, seq_start, seq_end, part, marks, out,
                          state_out, B, Hkv, (int)T_cap, epoch, token.start, token.end);
     return e == cudaSuccess ? launch_status() : (int)e;
 }

@@ -59,3 +59,12 @@ def test_the_table_preparation_waits_before_it_reads_anything():
     ((_, body, _),) = [found[1:] for found in _kernels() if found[0] == "attn_gsrq_prepare_kernel"]
     head = body[: body.index("wait_for_previous_kernel()")]
     assert not {"q", "ktab", "vtab", "fresh"} & set(re.findall(r"\w+", head))
+
+
+def test_the_table_preparation_lets_the_scan_start_only_after_its_own_wait():
+    """The scan reads what is older than the preparation (V words, ranges) before its own wait."""
+    ((_, body, _),) = [found[1:] for found in _kernels() if found[0] == "attn_gsrq_prepare_kernel"]
+    assert body.index("wait_for_previous_kernel()") < body.index("launch_dependents()")
+    ((_, scan, _),) = [found[1:] for found in _kernels() if found[0] == "attn_gsrq_scan_kernel"]
+    before = scan[scan.index("while (cursor < my_end)") : scan.index("wait_once();\n        uint4 k0")]
+    assert not {"lut_g", "scale_g", "part", "marks", "out"} & set(re.findall(r"\w+", before))
