@@ -471,17 +471,15 @@ static int launch_large(const EncodeArgs &a) {
 
 constexpr int kFewRows = 32;  // at or below this many rows a warp per (row, head, group) wins
 
-// Whether 8- and 4-wide groups go to the tcgen05 kernel, whose blocks of four tiles each stay a while, or to the mma.sync kernel of
-// many small blocks.  Measured with fp16 rows wanted, us of the mma.sync / tcgen05 kernel; T = tiles of 128 rows, all heads and groups:
-//   16 x 8, two stages  640 rows: T 80 7.5/17.4, 320 14.2/18.1, 640 22.0/19.7, 1280 37.3/32.2, 2560 58.4/58.9
-//                       T = 512: 17.1/14.0 (1024, 2048 or 4096 rows); T = 256: 9.9/13.5
-//   16 x 8, one stage   T = 512 11.8/10.6; 640 rows: T 640 15.0/14.7, 1280 25.2/23.2, 2560 36.9/41.3; 1024 rows: T 4096 52.9/49.3
-//   32 x 4, one stage   640 rows: T 640 15.0/14.0, 1280 25.4/22.4, 2560 37.0/38.8, 5120 63.7/67.1; 1024 rows: T 8192 92.7/85.2
-// From T of about 2048 on a block goes through whole (head, group) pairs, and five or six tiles of a pair leave its four groups of
-// threads half idle in the second round, which one stage does not make up for.
-static bool narrow_pays(int64_t rows, int64_t pairs, int stages) {
-    const int64_t tiles = (rows + 127) / 128 * pairs;
-    return rows >= 640 && tiles >= 512 && (tiles < 2048 || rows >= 1024 || stages >= 2);
+// Whether 8- and 4-wide groups go to the tcgen05 kernel, whose 148 blocks take four tiles of 128 rows at a time, or to the mma.sync
+// kernel of many small blocks.  The former takes a round's time however few rows its tiles hold, the latter goes by rows: 33000 rows of a
+// (head, group) cost as much as a round.  us of the mma.sync / tcgen05 kernel, rows not wanted; n = rows x heads x groups:
+//   16 x 8, two stages  8 heads x 250 rows (n 32000) 9.7/8.6, 400 15.8/10.3, 640 21.3/14.9, 1000 30.1/18.5; one head x 1500 (24000) 8.6/10.2, 3000 14.7/10.3
+//   16 x 8, one stage   8 x 250 6.6/6.6, 400 10.8/7.8, 640 14.4/10.6; 1 x 1500 6.1/7.5, 3000 10.1/7.4
+//   32 x 4, one stage   8 x 130 (33280) 10.2/9.9, 250 11.4/10.1, 400 18.6/14.1, 1000 31.3/20.0; 1 x 1000 (32000) 6.7/7.7, 1500 10.0/7.9
+static bool narrow_pays(int64_t rows, int64_t pairs) {
+    const int64_t rounds = ((rows + 127) / 128 * pairs + 4 * 148 - 1) / (4 * 148);
+    return rows * pairs >= 33000 * rounds;
 }
 
 // 32-, 64- and 128-wide groups: a block per (head, group) and four rows while that is at most two blocks per SM, or one and a half
@@ -504,7 +502,7 @@ static int dispatch_d(const EncodeArgs &a) {
             }
         }
         if (TACVQ_ENCODE_TC && (a.D / a.G == 8 || a.D / a.G == 4)) {
-            if (narrow_pays((int64_t)a.B * a.T, (int64_t)a.H * a.G, a.S)) {
+            if (narrow_pays((int64_t)a.B * a.T, (int64_t)a.H * a.G)) {
                 const int st = encode_narrow_launch(a);
                 if (st != TACVQ_ERR_UNSUPPORTED) return st;
             }

@@ -14,9 +14,11 @@
 // Blocks split the tiles of all (head, group) pairs evenly, span by span of 8192 rows, and bring a pair's tables in when they
 // enter it, so the chip stays full whatever the number of pairs; a table costs about one tile's time.
 //
-// Bound by latency between the phases of a stage at 16 warps an SM (issue 48 % busy).  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
-// stages, rows wanted: 435 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.  Whitened (fp32 words, a third product a
-// half): 3001 fp32 rows x 8 heads, 32 x 4, one stage 68 us against 125 for the fp32 scan of all words.
+// Bound by latency between the phases of a stage at 16 warps an SM.  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
+// stages, rows wanted: 344 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.  Whitened (fp32 words, a third product a
+// half): 3001 fp32 rows x 8 heads, 32 x 4, one stage 51 us against 125 for the fp32 scan of all words.
+// (Words as fp32 pairs in copies without bank conflicts, two exact chains an instruction: 372 us where this takes 344, as look-ups are scarcer than
+// issue slots.)
 //
 // Reference statements: src/jointkv/closed_loop_vq.py:52-76 (search), :343-395 (stage recursion),
 // src/jointkv/cq_tac.py:86-105.
@@ -52,8 +54,8 @@ __device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, int 
                      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
 }
-// 32 columns; the registers are valid when it returns
-__device__ __forceinline__ void tmem_load32(float (&v)[32], uint32_t taddr) {
+// 32 or 16 columns; the registers are valid when it returns
+__device__ __forceinline__ void tmem_load(float (&v)[32], uint32_t taddr) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -63,6 +65,15 @@ __device__ __forceinline__ void tmem_load32(float (&v)[32], uint32_t taddr) {
           "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]),
           "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]),
           "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_load(float (&v)[16], uint32_t taddr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+          "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
         : "r"(taddr)
         : "memory");
 }
@@ -124,6 +135,11 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                      const __half *__restrict__ plain, const float *__restrict__ sqnorm_in, uint8_t *__restrict__ codes, void *__restrict__ recon, int recon_dtype,
                      int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap, int vec_ok, int spins) {
     extern __shared__ __align__(1024) unsigned char smem[];
+    // Columns of a load from tensor memory.  What is decided by them is registers: 32 at a time made the kernels keep part of a row's state in
+    // local memory in every stage.  us, 32 / 16 columns, 32768 rows x 8 heads with rows: 16 x 2 x 8 fp16 441 / 344, 16 x 8 286 / 207, 32 x 4
+    // 436 / 363; whitened 32 x 4, 3001 fp32 rows 106 / 85.  fp32 rows of 8-wide words fit either way: 360 / 383, whitened 73 / 74.  (8 columns: 364
+    // where 16 take 344; the next 16 asked for before these are looked at: 368.)
+    constexpr int kColumns = DSUB == 8 && sizeof(XT) == 4 ? 32 : 16;
     constexpr size_t kStageBytes = kStage<DSUB, EXACT32>, kExactAt = narrow::kStageBytes + kWordBytes;
     const __half *tables = reinterpret_cast<const __half *>(tables_in);
     unsigned char *ones = smem + (size_t)S * kStageBytes, *misc = ones + (1 + kGroups) * kABytes;
@@ -341,13 +357,13 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                     fail = __any_sync(0xffffffffu, fail);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                    for (int c = 0; c < kHalf / 32; ++c) {
-                        float v[32];
-                        tmem_load32(v, my_scores + c * 32);
+                    for (int c = 0; c < kHalf / kColumns; ++c) {
+                        float v[kColumns];
+                        tmem_load(v, my_scores + c * kColumns);
 #pragma unroll
-                        for (int p = 0; p < 8; ++p) {
-                            top4[c * 8 + p] = fmaxf(max3(v[4 * p], v[4 * p + 1], v[4 * p + 2]), v[4 * p + 3]);
-                            asm volatile("" : "+f"(top4[c * 8 + p]));  // before the next columns are loaded: all of them at once do not fit
+                        for (int p = 0; p < kColumns / 4; ++p) {
+                            top4[c * (kColumns / 4) + p] = fmaxf(max3(v[4 * p], v[4 * p + 1], v[4 * p + 2]), v[4 * p + 3]);
+                            asm volatile("" : "+f"(top4[c * (kColumns / 4) + p]));  // before the next columns are loaded: all of them at once do not fit
                         }
                     }
                     if (half == 0) issue(stage, 1);

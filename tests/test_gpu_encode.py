@@ -447,6 +447,23 @@ def test_narrow_groups_with_many_rows_are_bit_exact(device, batch, heads, tokens
     assert ops.encode_tensor_memory_timeouts(device) == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize(
+    "heads,tokens,sub,groups,stages",
+    [(8, 257, 8, 16, 2), (8, 258, 8, 16, 2), (8, 385, 8, 16, 1), (2, 1031, 8, 16, 3), (2, 1032, 4, 32, 1), (8, 129, 4, 32, 1), (17, 33, 4, 128, 1)],
+)
+def test_both_kernels_of_narrow_groups_where_one_takes_over_from_the_other(device, heads, tokens, sub, groups, stages, dtype):
+    """Rows x heads x groups a little below and above what a round of the tcgen05 kernel is worth; nearly empty tiles; a second round."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(heads + tokens)
+    tables = make_tables(gen, heads, stages, groups, sub, [0.5 * 0.8**s for s in range(stages)])
+    states = make_states(gen, (1, heads, tokens, sub * groups), dtype)
+    want, want_recon = C.encode(states, tables)
+    codes, recon = ops.encode(states.to(device), tables.to(device))
+    assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
+    assert ops.encode_tensor_memory_timeouts(device) == 0
+
+
 @pytest.mark.parametrize(
     "batch,tokens,sub,groups,stages,words,depth,dtype",
     [
