@@ -369,6 +369,36 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     const uint32_t my_mma = mma_bar + 8 * grp;
     uint32_t mma_phase = 0u;
     bool fail = false;
+    // fp32 vectors of 128, one a row, by the four warps of 32 rows together (whole lines): a thread gets its pieces of its row's.  In two halves,
+    // for which the place of the fp16 rows is just large enough.
+    auto fetch_fp32 = [&](unsigned long long mine, float *out) {
+        constexpr int kAtOnce = 32 / kPieces, kEach = 8 / kAtOnce;
+        uint4 v[2][kEach];
+#pragma unroll
+        for (int i = 0; i < kEach; ++i) {
+            const unsigned long long from = __shfl_sync(0xffffffffu, mine, q * 8 + i * kAtOnce + lane / kPieces);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                v[half][i] = make_uint4(0u, 0u, 0u, 0u);
+                if (from != 0ull) v[half][i] = __ldg(reinterpret_cast<const uint4 *>(from) + half * kPieces + lane % kPieces);
+            }
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            if (half == 1) sync_quad();
+#pragma unroll
+            for (int i = 0; i < kEach; ++i)
+                *reinterpret_cast<uint4 *>(A + L::template at<kRows>(part * 32 + q * 8 + i * kAtOnce + lane / kPieces, (lane % kPieces) * 8)) = v[half][i];
+            sync_quad();
+#pragma unroll
+            for (int m = half * (kOwn / 2); m < (half + 1) * (kOwn / 2); ++m)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    *reinterpret_cast<float4 *>(out + 8 * m + 4 * i) =
+                        *reinterpret_cast<const float4 *>(A + L::template at<kRows>(row, (2 * (4 * m + q) + i - half * kPieces) * 8));
+        }
+        sync_quad();
+    };
     // (batch entry, token) of this thread's row: divided out once, then advanced by the stride of the tiles
     const uint32_t step = gridDim.x * groups * kRows, step_b = step / (uint32_t)a.T, step_t = step % (uint32_t)a.T;
     uint32_t grow = (blockIdx.x * groups + grp) * kRows + row;
@@ -414,35 +444,9 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             for (int m = 0; m < kOwn; ++m) unpack8(*reinterpret_cast<const uint4 *>(A + L::template at<kRows>(row, (4 * m + q) * 8)), r + 8 * m);
         } else {
             if (DSUB == 128 && a.vec_ok) {
-                // The same in two halves, for which the place of the fp16 rows is just large enough.  Against 32 bytes of its own row a
-                // thread, us: 65536 rows x 8 heads, two stages 318 / 288, 16 stages x 2048 rows 109 / 103.  64 wide it is 181 / 183.
-                constexpr int kAtOnce = 32 / kPieces, kEach = 8 / kAtOnce;
-                const unsigned long long mine = live ? (unsigned long long)src : 0ull;
-                uint4 v[2][kEach];
-#pragma unroll
-                for (int i = 0; i < kEach; ++i) {
-                    const unsigned long long from = __shfl_sync(0xffffffffu, mine, q * 8 + i * kAtOnce + lane / kPieces);
-#pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        v[half][i] = make_uint4(0u, 0u, 0u, 0u);
-                        if (from != 0ull) v[half][i] = __ldg(reinterpret_cast<const uint4 *>(from) + half * kPieces + lane % kPieces);
-                    }
-                }
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    if (half == 1) sync_quad();
-#pragma unroll
-                    for (int i = 0; i < kEach; ++i)
-                        *reinterpret_cast<uint4 *>(A + L::template at<kRows>(part * 32 + q * 8 + i * kAtOnce + lane / kPieces, (lane % kPieces) * 8)) = v[half][i];
-                    sync_quad();
-#pragma unroll
-                    for (int m = half * (kOwn / 2); m < (half + 1) * (kOwn / 2); ++m)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            *reinterpret_cast<float4 *>(r + 8 * m + 4 * i) =
-                                *reinterpret_cast<const float4 *>(A + L::template at<kRows>(row, (2 * (4 * m + q) + i - half * kPieces) * 8));
-                }
-                sync_quad();
+                // The same in two halves.  Against 32 bytes of its own row a thread, us: 65536 rows x 8 heads, two stages 318 / 288, 16 stages x
+                // 2048 rows 109 / 103.  64 wide it is 181 / 183.
+                fetch_fp32(live ? (unsigned long long)src : 0ull, r);
             } else {
 #pragma unroll
                 for (int m = 0; m < kOwn; ++m) {
@@ -593,7 +597,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                 if (n >= 1) wb = wa, wa = i * 64 + (info & 63);
                 if (n >= 2) wb = wa, wa = i * 64 + ((info >> 6) & 63);
             }
-            int pick = wa;
+            int pick = min(wa, K - 1);  // (a row past the end may have listed padding words)
             // (rows past the end are all alike: one that is undecided would be 32 in a row)
             bool undecided = live && n_words != 1;
             if (__any_sync(0xffffffffu, undecided)) {  // the same in the four warps
@@ -739,7 +743,18 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                         *reinterpret_cast<uint4 *>(A + L::template at<kRows>(row, e)) = pack8(r + 8 * m);
                     }
                 };
-                if constexpr (EXACT32) {
+                if constexpr (EXACT32 && DSUB == 128 && GROUPS == 1) {
+                    // 16 bytes of 32 words a load are 32 lines; the words of 32 rows together are 4 lines a load.  Whole calls, us, 16 stages x 2048
+                    // fp16 rows x 8 heads with rows 217 / 206.  (With two groups a block another one hides it: 1154 / 1157 for 4 x 4096 rows.)
+                    float words[kOwn * 8];
+                    fetch_fp32((unsigned long long)(a.words32 + (first + pick) * DSUB), words);
+#pragma unroll
+                    for (int m = 0; m < kOwn; ++m) {
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2) sub2(r[8 * m + j], r[8 * m + j + 1], words[8 * m + j], words[8 * m + j + 1]);
+                        *reinterpret_cast<uint4 *>(A + L::template at<kRows>(row, 8 * (4 * m + q))) = pack8(r + 8 * m);
+                    }
+                } else if constexpr (EXACT32) {
                     subtract([&](int e, float *c) {
                         *reinterpret_cast<float4 *>(c) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + pick) * DSUB + e));
                         *reinterpret_cast<float4 *>(c + 4) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + pick) * DSUB + e + 4));
