@@ -72,6 +72,12 @@ TACVQ_API const char *tacvq_status_string(int status);
 TACVQ_API int tacvq_table_sqnorm(const uint16_t *tables_f16, float *out, int64_t words, int d, tacvq_stream_t stream);
 
 /*
+ * Whether all of matrices [count][n][n] are exactly the identity (-0 counts as 0, a NaN as another value): *answer = 1 or 0, in
+ * device memory, when the stream has got there.  A whitener that is the identity leaves rows and words unchanged bit for bit.
+ */
+TACVQ_API int tacvq_is_identity(const float *matrices, int64_t count, int n, uint8_t *answer, tacvq_stream_t stream);
+
+/*
  * Diagnostic of the encode kernels that wait for tensor-core products (tcgen05) or for table copies of the copy engine
  * (TMA): groups 32, 64 and 128 wide, and many rows of groups 4 and 8 wide.  *count = in how many blocks, on the current
  * device since the library was loaded, a wait was given up - the rows concerned are then searched word by word, from

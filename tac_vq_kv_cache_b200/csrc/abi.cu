@@ -4,6 +4,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "identity.cuh"
 #include "ladder_plan.cuh"
 
 namespace tacvq {
@@ -156,6 +157,12 @@ int tacvq_table_sqnorm(const uint16_t *tables_f16, float *out, int64_t words, in
     if (!tables_f16 || !out) return TACVQ_ERR_NULL;
     if (words < 0 || d <= 0 || d > 128) return TACVQ_ERR_GEOMETRY;
     return table_sqnorm_dispatch((const __half *)tables_f16, out, words, d, (cudaStream_t)stream);
+}
+
+int tacvq_is_identity(const float *matrices, int64_t count, int n, uint8_t *answer, tacvq_stream_t stream) {
+    if (!matrices || !answer) return TACVQ_ERR_NULL;
+    if (count < 0 || n <= 0 || n > 32768) return TACVQ_ERR_GEOMETRY;
+    return is_identity_launch(matrices, count, n, answer, (cudaStream_t)stream);
 }
 
 int tacvq_encode_tensor_memory_timeouts(unsigned int *count) {

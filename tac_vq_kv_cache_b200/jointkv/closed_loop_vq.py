@@ -18,7 +18,7 @@ from __future__ import annotations
 
 import math
 from dataclasses import dataclass
-from typing import Any, Sequence
+from typing import Any, Callable, Sequence
 
 import torch
 
@@ -46,6 +46,13 @@ def is_identity_whitener(w: torch.Tensor | None) -> bool:
         return True
     eye = torch.eye(w.shape[-1], dtype=w.dtype, device=w.device)
     return bool((w == eye).all())
+
+
+def ask_identity_whitener(w: torch.Tensor | None) -> Callable[[], bool]:
+    """:func:`is_identity_whitener` in two parts: the question now, the answer (and the host's wait for it) where it is needed."""
+    if w is not None and w.is_cuda and w.dtype == torch.float32 and w.is_contiguous():
+        return ops.ask_identity(w)
+    return lambda: is_identity_whitener(w)
 
 
 class _HardGroupedResidualVQ(torch.autograd.Function):

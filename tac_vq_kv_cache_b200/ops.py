@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import contextlib
 import functools
+from collections.abc import Callable
 
 import torch
 
@@ -91,6 +92,31 @@ def table_sqnorm(tables_f16: torch.Tensor) -> torch.Tensor:
     with _on(device):
         _lib.check("tacvq_table_sqnorm", _lib.load().tacvq_table_sqnorm(_ptr(tables_f16), _ptr(out), out.numel(), tables_f16.shape[-1], _stream(device)))
     return out
+
+
+def ask_identity(matrices: torch.Tensor) -> Callable[[], bool]:
+    """Asks the device whether contiguous fp32 ``[..., n, n]`` is a stack of identity matrices; the call that is returned waits for the answer.
+
+    What is launched between the two runs while the host waits.
+    """
+    device = _require_cuda(matrices)
+    if matrices.dtype != torch.float32 or matrices.ndim < 2 or matrices.shape[-1] != matrices.shape[-2] or not matrices.is_contiguous():
+        raise ValueError("matrices must be contiguous fp32 [..., n, n]")
+    n = int(matrices.shape[-1])
+    if n == 0 or matrices.numel() == 0:
+        return lambda: True
+    answer = torch.empty(1, dtype=torch.uint8, device=device)
+    with _on(device):
+        _lib.check("tacvq_is_identity", _lib.load().tacvq_is_identity(_ptr(matrices), matrices.numel() // (n * n), n, _ptr(answer), _stream(device)))
+        landed = torch.empty(1, dtype=torch.uint8, pin_memory=True).copy_(answer, non_blocking=True)
+        event = torch.cuda.Event()
+        event.record()
+
+    def wait() -> bool:
+        event.synchronize()
+        return bool(landed.item())
+
+    return wait
 
 
 def encode_tensor_memory_timeouts(device=None) -> int:

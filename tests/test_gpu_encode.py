@@ -543,3 +543,22 @@ def test_rebuilt_fp16_rows_equal_the_oracle_bit_for_bit(device, sub, groups, sta
     codes = torch.randint(0, words, (1, 3, tokens, stages, groups), generator=gen, dtype=torch.uint8)
     got = ops.decode(codes.to(device), tables.to(device), depth=depth).cpu()
     assert torch.equal(got.view(torch.int16), C.decode(codes, tables, torch.float16, depth=depth).view(torch.int16))
+
+
+@pytest.mark.parametrize("shape", [(8, 128, 128), (1, 1, 1), (3, 7, 7), (2, 2, 33, 33), (5, 64, 64)])
+def test_the_identity_is_told_from_its_neighbours(device, shape):
+    """Every corner, the element after the diagonal, another sign of zero, a NaN; the question goes out before the answer is waited for."""
+    ops = _ops()
+    eye = torch.eye(shape[-1], device=device).expand(shape).contiguous()
+    assert ops.ask_identity(eye)()
+    assert ops.ask_identity(torch.where(eye == 0, -eye, eye))()
+    asked = []
+    for at in {0, 1 % eye.numel(), shape[-1] - 1, shape[-1] + 1, eye.numel() // 2, eye.numel() - 1} - {eye.numel()}:
+        if at < eye.numel():
+            for value in (2.0, float("nan")):
+                other = eye.clone()
+                other.view(-1)[at] = value
+                asked.append(ops.ask_identity(other))
+    assert asked and not any(wait() for wait in asked)
+    with pytest.raises(ValueError):
+        ops.ask_identity(eye.double())
