@@ -466,7 +466,9 @@ static int launch_decode_rows(const uint8_t *codes, const __half *tables, OT *ou
     if (e != cudaSuccess) return (int)e;
     const int64_t rows = (int64_t)B * T;
     int64_t per_head = H < 148 ? 148 / H : 1;
-    if (per_head > rows / 512) per_head = rows / 512;  // a block keeps 512 rows to be worth its copy of the table
+    // A block keeps 128 rows; more blocks cost nothing while SMs are free.  us with 512 / 128 rows, 8 heads x 2000, 16 x 2 x 8: fp16 12.4 / 9.7, fp32 20.0 / 11.6;
+    // 8 heads x 4000 12.4 / 10.3, 19.8 / 13.7.
+    if (per_head > rows / 128) per_head = rows / 128;
     if (per_head < 1) per_head = 1;
     kernel<<<dim3((unsigned)per_head, (unsigned)H), kRowsThreads, bytes, stream>>>(codes, tables, out, B, H, T, D, G, S, K, t0, T_cap);
     return launch_status();
@@ -476,9 +478,13 @@ int decode_dispatch(const uint8_t *codes, const __half *tables, void *out, int o
                     int G, int S, int S_use, int K, int64_t t0, int64_t T_cap, cudaStream_t stream) {
     const int d = D / G;
     const size_t head_bytes = (size_t)S * G * K * d * 2;
+    // A copy of the table, 5 to 7 us with the launch, pays from about 16384 rows of 128 on, all heads together.  us without / with it, 8 heads x 1100
+    // rows, 2000, 4000: 16 x 2 x 8 fp16 4.2/9.6, 6.0/9.7, 9.4/10.3, fp32 7.7/11.5, 10.8/11.6, 17.1/13.7; 2 x 128 fp16 3.7/6.9, 5.1/7.0, 8.4/7.5;
+    // 32 x 4 fp16 5.1/7.2, 7.3/7.4, 12.0/7.8.
     const bool staged = (d % 8 == 0 || d == 4) && D % 8 == 0 && kStagedThreads % (D / 8) == 0 && (int64_t)B * T < 0x7f000000 &&
                         head_bytes <= (size_t)kStagedMaxBytes && head_bytes % 16 == 0 &&
-                        ((uintptr_t)tables & 15) == 0 && ((uintptr_t)out & 15) == 0 && (int64_t)B * T >= 1024;
+                        ((uintptr_t)tables & 15) == 0 && ((uintptr_t)out & 15) == 0 && (int64_t)B * T >= 1024 &&
+                        (int64_t)B * T * H * D > (int64_t)1 << 21;
     // (S_use stages are copied here, all S of them there; a row is 8 to 128 pieces)
     // fp32 rows only while the staged kernel could not fill the chip: 8 heads, 4096 rows 21 us against 54, 16384 rows 30 against 19
     const int64_t fills = (int64_t)512 * (H < 148 ? 148 / H : 1);

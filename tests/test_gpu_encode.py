@@ -485,6 +485,18 @@ def test_rows_of_one_or_two_stages_rebuild_exactly(device, batch, tokens, sub, g
     assert torch.equal(got.cpu(), C.decode(codes, tables, dtype, depth=depth, t0=1, tokens=tokens))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("batch,tokens", [(1, 2048), (1, 2049), (3, 701), (2, 2077)])
+@pytest.mark.parametrize("sub,groups,stages,words", [(8, 16, 2, 256), (4, 32, 1, 252), (128, 1, 2, 256), (8, 16, 1, 256)])
+def test_rows_rebuild_exactly_where_a_copy_of_the_table_begins_to_pay(device, sub, groups, stages, words, batch, tokens, dtype):
+    """Eight heads x 2048 rows is the last call without the copy; a few rows more, and blocks whose share of them is ragged."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(tokens)
+    tables = make_tables(gen, 8, stages, groups, sub)[:, :, :, :words].contiguous()
+    codes = torch.randint(0, words, (batch, 8, tokens, stages, groups), generator=gen, dtype=torch.uint8)
+    assert torch.equal(ops.decode(codes.to(device), tables.to(device), dtype).cpu(), C.decode(codes, tables, dtype))
+
+
 @pytest.mark.parametrize("sub,groups,stages,depth", [(128, 1, 16, 16), (4, 32, 1, 1), (8, 16, 2, 1), (2, 16, 2, 2)])
 def test_codeword_gradient_sums_the_rows_that_chose_a_word(device, sub, groups, stages, depth):
     """Against float64 index_add: at most 2^-23 times the number of addends relative to the sum of their magnitudes."""
