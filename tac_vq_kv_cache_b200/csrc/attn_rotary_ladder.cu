@@ -27,12 +27,16 @@
 // 2^-19 goes to one bin and what that leaves, in units of 2^-38, to another, which keeps all 24 bits of a weight down to 2^-15.  The sums
 // are exact.
 //
+// Where a cluster's time goes, us after its start, one row with 4096 tokens: tables there 5.9, scores of 64 SMs 27.8, parts exchanged 31.6, weights
+// exchanged 36.9, histograms 40.5, end 44.7.  The weights are relative to the maximum of the block that has their share of the tokens and put right by the
+// reader, which saves one of four exchanges (2 us); sums in two chains of products and rotary rows in whole channel pairs take 1 us off the scores.
+//
 // A sum of 16 words by the tensor core is no further from the exact one than fp32 adds in order: over 2^20 sums of 4, 8, 12 and 16 normal values,
 // of equal spread and falling by 0.9 and 0.6 a stage, 3.5e-10 to 9.3e-9 in the 2-norm against 3.5e-10 to 1.3e-8, and the same fp16
 // value in every case.
 //
-// us a decode step of 16 stages and 8 KV heads, against attn_rotary_kernel: one row of 6144 tokens with a window of 4096 50 / 107 (27 are the
-// new token's encode), 600 tokens 41 / 103, 16384 tokens 120 / 232, 8 x 2000 159 / 225, 16 x 1000 193 / 228; ladder_plan.cuh has the sizes that
+// us a decode step of 16 stages and 8 KV heads, against attn_rotary_kernel: one row of 6144 tokens with a window of 4096 48 / 107, 600
+// tokens 39 / 103 (27 are the new token's encode), 16384 tokens 120 / 232, 8 x 2000 159 / 225, 16 x 1000 193 / 228; ladder_plan.cuh has the sizes that
 // are left to that kernel.  Tables, gathers and products are 16 stages wide for fewer stages too.
 //
 // Semantics replaced: experiments_followup_mistral/evaluate_mistral_longbench.py:112-122 including the rotary step
@@ -56,7 +60,7 @@ constexpr int kTabBytes = kWords * kRowBytes;         // 131072
 constexpr int kScoreBytes = kChunk * kHeads * 4;      // parts of the scores, then weights, then per-warp sums
 constexpr int kHistBytes = 2 * 2 * kWords * kHeads * 4;  // [multiples | rest][stage j or j + 8][word][head]
 constexpr int kOutBytes = kSlices * 64 * 4;           // [source block][64 of the 512 outputs]
-constexpr int kSmallFloats = 2 * kSlices * kHeads + 2 * kWarps * kHeads;  // maxima and sums of the blocks, of the warps
+constexpr int kSmallFloats = 3 * kSlices * kHeads + 2 * kWarps * kHeads;  // maxima, sums and factors of the blocks, maxima and sums of the warps
 constexpr int kSmemBytes = kTabBytes + kScoreBytes + kHistBytes + kOutBytes + kSmallFloats * 4;
 static_assert(kWarps * kHeads * kDim * 4 <= kScoreBytes, "per-warp sums reuse the score area");
 static_assert(kSmemBytes <= 227 * 1024, "");
@@ -139,6 +143,7 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
     float *out_s = reinterpret_cast<float *>(area + kScoreBytes + kHistBytes);
     float *top_s = out_s + kSlices * 64, *sum_s = top_s + kSlices * kHeads;  // [block][head]
     float *warp_top = sum_s + kSlices * kHeads, *warp_sum = warp_top + kWarps * kHeads;
+    float *factor_s = warp_sum + kWarps * kHeads;  // [block][head]: from weights relative to a block's maximum to the largest of all
     const uint32_t tab_u32 = smem_u32(smem), area_u32 = smem_u32(area);
 
     const int slice = blockIdx.x % kSlices, cluster = blockIdx.x / kSlices, clusters = gridDim.x / kSlices;
@@ -172,7 +177,10 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
     // A decode step's new codes come from the kernel before this one, and nothing else that is read here; without one, all may.
     bool waited = false;
     auto wait_once = [&]() {
-        if (!waited) wait_for_previous_kernel();
+        if (!waited) {
+            wait_for_previous_kernel();
+            launch_dependents();
+        }
         waited = true;
     };
     if (step.fresh == 0) wait_once();
@@ -191,7 +199,7 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
             continue;
         }
         const uint8_t *kc = kcodes + (((int64_t)b * Hkv + h) * T_cap + first) * S, *vc = vcodes + (((int64_t)b * Hkv + h) * T_cap + first) * S;
-        const __half *rp = rope + (int64_t)first * kDim + slice * 8 + r8;
+        const __half *rp = rope + (int64_t)first * kDim + slice * 8 + 2 * kq;
         const int old_tiles = step.fresh != 0 ? max(min(step.end - step.fresh - first, n), 0) >> 4 : (n + 15) >> 4;  // without a new token
 
         load_table(h);
@@ -204,16 +212,15 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                 q1 = __ldg(src + 32);
             }
             const int tiles = (n + 15) >> 4;
-            uint32_t cn[2], rn[2][2];  // code words of tokens 0-7 and 8-15 (lane = 4 x token + word); cosines and sines of channel r8, tokens 2kq, 2kq + 1
+            uint32_t cn[2], rn[2][2];  // code words of tokens 0-7 and 8-15 (lane = 4 x token + word); cosines and sines of token r8, channels 2kq, 2kq + 1
             auto fetch = [&](int tile) {
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const int t = min(tile * 16 + u * 8 + r8, n - 1);
                     cn[u] = kq < words_per_token ? code_word(kc + (int64_t)t * S + 4 * kq) : 0u;
-                    const int t0 = min(tile * 16 + u * 8 + 2 * kq, n - 1), t1 = min(tile * 16 + u * 8 + 2 * kq + 1, n - 1);
-                    const unsigned short *c0 = reinterpret_cast<const unsigned short *>(rp + (int64_t)t0 * kDim), *c1 = reinterpret_cast<const unsigned short *>(rp + (int64_t)t1 * kDim);
-                    rn[u][0] = __ldg(c0) | (uint32_t)__ldg(c1) << 16;
-                    rn[u][1] = __ldg(c0 + 64) | (uint32_t)__ldg(c1 + 64) << 16;
+                    const uint32_t *turn = reinterpret_cast<const uint32_t *>(rp + (int64_t)t * kDim);
+                    rn[u][0] = __ldg(turn);
+                    rn[u][1] = __ldg(turn + 32);
                 }
             };
             for (int i = tid; i < kHistBytes / 4; i += kThreads) hist[i] = 0u;
@@ -238,12 +245,16 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                         const uint32_t at = prmt(__shfl_sync(0xffffffffu, code[u], t * 4 + k_lane), 0u, k_sel);
                         ldmatrix_x4_trans(m[t], k_base + at + at);
                     }
-                    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // channel r8 and its partner, tokens 2kq and 2kq + 1 of these eight
+                    // channel r8 and its partner, tokens 2kq and 2kq + 1 of these eight; in two chains, which hold zeros for each other's tokens
+                    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f}, odd[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
                     for (int t = 0; t < 8; ++t) {
                         const uint32_t one = r8 == t ? 0x3c003c00u : 0u;
-                        mma16816(sum, m[t][0], m[t][2], m[t][1], m[t][3], one, one);
+                        if (t & 1) mma16816(odd, m[t][0], m[t][2], m[t][1], m[t][3], one, one);
+                        else mma16816(sum, m[t][0], m[t][2], m[t][1], m[t][3], one, one);
                     }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[i] += odd[i];
                     // The zeros in the other tokens' columns do not hide a word that is not finite (0 x inf): then every token's words
                     // are added without the others'.
                     if (__any_sync(0xffffffffu, !(fabsf((sum[0] + sum[1]) + (sum[2] + sum[3])) < INFINITY))) {
@@ -259,13 +270,15 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                             sum[2] = j == 2 ? alone : sum[2], sum[3] = j == 3 ? alone : sum[3];
                         }
                     }
-                    // round, rotate (k cos + rotate_half(k) sin, products and sum in fp16)
-                    const __half2 kl = __floats2half2_rn(sum[0], sum[1]), kh = __floats2half2_rn(sum[2], sum[3]);
+                    // round, turn to row = token, k = channel; rotate (k cos + rotate_half(k) sin, products and sum in fp16)
+                    const __half2 low = __floats2half2_rn(sum[0], sum[1]), high = __floats2half2_rn(sum[2], sum[3]);
+                    const uint32_t lt = movmatrix(*reinterpret_cast<const uint32_t *>(&low)), ht = movmatrix(*reinterpret_cast<const uint32_t *>(&high));
+                    const __half2 kl = *reinterpret_cast<const __half2 *>(&lt), kh = *reinterpret_cast<const __half2 *>(&ht);
                     const __half2 cosv = *reinterpret_cast<const __half2 *>(&turn[u][0]), sinv = *reinterpret_cast<const __half2 *>(&turn[u][1]);
                     const __half2 tl = __hadd2(__hmul2(kl, cosv), __hmul2(__hneg2(kh), sinv));
                     const __half2 th = __hadd2(__hmul2(kh, cosv), __hmul2(kl, sinv));
-                    a[u] = movmatrix(*reinterpret_cast<const uint32_t *>(&tl));  // row = token, k = channel
-                    a[2 + u] = movmatrix(*reinterpret_cast<const uint32_t *>(&th));
+                    a[u] = *reinterpret_cast<const uint32_t *>(&tl);
+                    a[2 + u] = *reinterpret_cast<const uint32_t *>(&th);
                 }
                 float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 mma16816(d, a[0], a[1], a[2], a[3], q0, q1);
@@ -298,8 +311,8 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
         cluster_barrier();
 
         // ---- block j adds up the parts of its share of the tokens; weights go to every block ------------------------------
+        const int share = (n + kSlices - 1) / kSlices;  // at most kThreads
         {
-            const int share = (n + kSlices - 1) / kSlices;  // at most kThreads
             const int t = slice * share + tid;
             const bool mine = tid < share && t < n;
             float sc[kHeads] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -320,19 +333,14 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                 if (lane == 0) warp_top[warp * kHeads + r] = v;
             }
             __syncthreads();
-            if (tid < kSlices * kHeads) {  // this block's maximum of head tid % 4, to block tid / 4
-                float v = -INFINITY;
-                for (int w = 0; w < kWarps; ++w) v = fmaxf(v, warp_top[w * kHeads + (tid & 3)]);
-                st_cluster(in_block(smem_u32(top_s + slice * kHeads + (tid & 3)), tid >> 2), v);
-            }
-            cluster_barrier();
-            float sum[kHeads];
+            // weights relative to this block's maximum, which every block puts right when it has all maxima
+            float top[kHeads], sum[kHeads];
 #pragma unroll
             for (int r = 0; r < kHeads; ++r) {
-                float top = -INFINITY;
-                for (int k = 0; k < kSlices; ++k) top = fmaxf(top, top_s[k * kHeads + r]);
-                const float p = mine ? __expf(sc[r] - top) : 0.0f;
-                sum[r] = p;
+                top[r] = warp_top[r];
+#pragma unroll 5
+                for (int w = 1; w < kWarps; ++w) top[r] = fmaxf(top[r], warp_top[w * kHeads + r]);
+                sum[r] = mine ? __expf(sc[r] - top[r]) : 0.0f;
             }
             if (mine)
                 for (int k = 0; k < kSlices; ++k) st_cluster4(in_block(area_u32 + t * 16, k), make_float4(sum[0], sum[1], sum[2], sum[3]));
@@ -343,12 +351,21 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                 if (lane == 0) warp_sum[warp * kHeads + r] = sum[r];
             }
             __syncthreads();
-            if (tid < kSlices * kHeads) {
+            if (tid < kSlices * kHeads) {  // of head tid % 4, to block tid / 4
+                const int r = tid & 3;
                 float v = 0.0f;
-                for (int w = 0; w < kWarps; ++w) v += warp_sum[w * kHeads + (tid & 3)];
-                st_cluster(in_block(smem_u32(sum_s + slice * kHeads + (tid & 3)), tid >> 2), v);
+                for (int w = 0; w < kWarps; ++w) v += warp_sum[w * kHeads + r];
+                const float own = r == 0 ? top[0] : r == 1 ? top[1] : r == 2 ? top[2] : top[3];
+                st_cluster(in_block(smem_u32(sum_s + slice * kHeads + r), tid >> 2), v);
+                st_cluster(in_block(smem_u32(top_s + slice * kHeads + r), tid >> 2), own);
             }
             cluster_barrier();
+            if (tid < kSlices * kHeads) {
+                float most = -INFINITY;
+                for (int k = 0; k < kSlices; ++k) most = fmaxf(most, top_s[k * kHeads + (tid & 3)]);
+                factor_s[tid] = top_s[tid] == -INFINITY ? 0.0f : __expf(top_s[tid] - most);  // no token there, or none of a finite score
+            }
+            __syncthreads();
         }
 
         // ---- weights by code, stages `slice` and `slice` + 8 ----------------------------------------------------------------
@@ -356,7 +373,9 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
         for (int i = 0; i < kChunk / kThreads; ++i) {
             const int t = tid + i * kThreads;
             if (t >= n) break;
-            const float4 p4 = *reinterpret_cast<const float4 *>(area + t * 16);
+            float4 p4 = *reinterpret_cast<const float4 *>(area + t * 16);
+            const float4 f4 = *reinterpret_cast<const float4 *>(factor_s + t / share * kHeads);
+            p4 = make_float4(p4.x * f4.x, p4.y * f4.y, p4.z * f4.z, p4.w * f4.w);
             // lane l takes the heads in the order l, l + 1, ..: the 32 adds of an instruction spread over all banks
             float p[kHeads] = {p4.x, p4.y, p4.z, p4.w};
             if (lane & 1) {
@@ -437,7 +456,7 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
             float a = 0.0f, l = 0.0f, top = -INFINITY;
             for (int k = 0; k < kSlices; ++k) {
                 a += out_s[k * 64 + tid];
-                l += sum_s[k * kHeads + r];
+                l += sum_s[k * kHeads + r] * factor_s[k * kHeads + r];
                 top = fmaxf(top, top_s[k * kHeads + r]);
             }
             if (l != l) a = l;
