@@ -312,6 +312,7 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
 
     // A decode step's new codes and ranges come from the kernel before this one; the tables and the query do not.
     wait_for_previous_kernel();
+    launch_dependents();
     const int lo_all = max(seq_start ? seq_start[b] : 0, 0);
     const int hi_all = min(seq_end ? seq_end[b] : (int)T_cap, (int)T_cap);
     const int n_all = hi_all > lo_all ? hi_all - lo_all : 0;

@@ -157,6 +157,12 @@ struct LadderStep {
 // memory that nobody changes while the kernel runs, which the compiler may move above the wait.
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The first statement of a kernel that follows as a dependent only to be scheduled early: from here on everything older is there.  As the next
+// kernel may start only now, it may read what is older than this grid before its own wait.
+__device__ __forceinline__ void start_after_previous_kernel() {
+    wait_for_previous_kernel();
+    launch_dependents();
+}
 
 template <typename... Params, typename... Args>
 inline cudaError_t launch_dependent(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

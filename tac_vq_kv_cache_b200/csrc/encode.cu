@@ -173,8 +173,8 @@ encode_small_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t 
 // above, so the codes are too.
 
 template <int DSUB, typename XT>
-__device__ __forceinline__ void encode_row_unit(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t sxt,
-                                                const __half *__restrict__ tables, const float *__restrict__ sqnorm_in,
+__device__ __forceinline__ void encode_row_unit(const XT *x, int64_t sxb, int64_t sxh, int64_t sxt,
+                                                const __half *tables, const float *sqnorm_in,
                                                 uint8_t *__restrict__ codes, void *__restrict__ recon, int recon_dtype, int H,
                                                 int T, int G, int S, int K, int64_t t0, int64_t T_cap, int64_t unit, int lane) {
     const int g = (int)(unit % G);
@@ -221,16 +221,16 @@ encode_rows_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t s
 }
 
 // One decode step's bookkeeping in a single launch: the new rows of K and of V are encoded in place (a
-// warp per (row, head, group) and side, as above) and every row's visible range is set.  The kernel lets
-// its successor start at once (programmatic dependent launch): a successor that needs these outputs
-// waits for this grid by itself.
+// warp per (row, head, group) and side, as above) and every row's visible range is set.  It is scheduled while the launch in front of it
+// runs, waits for that, and lets its successor start (programmatic dependent launches): a successor that needs these outputs waits for
+// this grid by itself.  (As an ordinary launch a step began 2 to 3 us later: 2 x 128, 16 rows x 16384 tokens 33.5 / 31.4 us.)
 template <int DSUB, typename XT>
 __global__ void __launch_bounds__(256)
-decode_prologue_kernel(const XT *__restrict__ k_rows, const XT *__restrict__ v_rows, int64_t sxb, int64_t sxh, int64_t sxt,
-                       const __half *__restrict__ ktab, const __half *__restrict__ vtab, uint8_t *__restrict__ kcodes,
+decode_prologue_kernel(const XT *k_rows, const XT *v_rows, int64_t sxb, int64_t sxh, int64_t sxt,
+                       const __half *ktab, const __half *vtab, uint8_t *__restrict__ kcodes,
                        uint8_t *__restrict__ vcodes, int32_t *__restrict__ seq_start, int32_t *__restrict__ seq_end, int start,
                        int end, int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap) {
-    launch_dependents();
+    start_after_previous_kernel();
     if (blockIdx.x == 0) {
         for (int b = threadIdx.x; b < B; b += blockDim.x) {
             seq_start[b] = start;
@@ -253,10 +253,10 @@ static int launch_prologue(const void *k_rows, const void *v_rows, int64_t sxb, 
                            int start, int end, int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap,
                            cudaStream_t stream) {
     const int64_t units = (int64_t)B * T * H * G;
-    decode_prologue_kernel<DSUB, XT><<<(unsigned)((2 * units + 7) / 8), 256, 0, stream>>>(
-        (const XT *)k_rows, (const XT *)v_rows, sxb, sxh, sxt, ktab, vtab, kcodes, vcodes, seq_start, seq_end, start, end, B, H,
-        T, G, S, K, t0, T_cap);
-    return launch_status();
+    const cudaError_t e = launch_dependent(true, decode_prologue_kernel<DSUB, XT>, dim3((unsigned)((2 * units + 7) / 8)), dim3(256), 0, stream,
+                                           (const XT *)k_rows, (const XT *)v_rows, sxb, sxh, sxt, ktab, vtab, kcodes, vcodes, seq_start, seq_end,
+                                           start, end, B, H, T, G, S, K, t0, T_cap);
+    return e == cudaSuccess ? launch_status() : (int)e;
 }
 
 template <int DSUB, typename XT>

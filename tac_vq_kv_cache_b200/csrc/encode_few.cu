@@ -195,7 +195,7 @@ encode_few_wide_kernel(FewSide first, FewSide second, int64_t sxb, int64_t sxh, 
                          : "=r"(ok) : "r"(bar0 + slot * 8), "r"((uint32_t)phase) : "memory");
         return ok != 0;
     };
-    if (seq_start != nullptr) launch_dependents();  // a decode step: its attention is next, and waits for this grid where it has to
+    if (seq_start != nullptr) start_after_previous_kernel();  // a decode step: its attention is next, and waits for this grid where it has to
     if (tid == 0) {
         for (int i = 0; i < ring; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + i * 8) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -426,9 +426,10 @@ static int launch_few(const FewSide &first, const FewSide &second, int sides, in
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         dim3 grid((unsigned)((rows + per_block - 1) / per_block), (unsigned)(H * G), (unsigned)sides);
-        kernel<<<grid, 2 * kThreads, smem, stream>>>(first, second, sxb, sxh, sxt, recon_dtype, ring, seq_start, seq_end, start, end, B,
-                                                 H, T, G, S, K, t0, T_cap, spins < 0 ? kSpins : spins, first_map, second_map);
-        return launch_status();
+        const cudaError_t launched = launch_dependent(seq_start != nullptr, kernel, grid, dim3(2 * kThreads), smem, stream, first, second, sxb, sxh, sxt,
+                                                      recon_dtype, ring, seq_start, seq_end, start, end, B, H, T, G, S, K, t0, T_cap,
+                                                      spins < 0 ? kSpins : spins, first_map, second_map);
+        return launched == cudaSuccess ? launch_status() : (int)launched;
     };
     // the fewest rows per block that keep the launch to about one block per SM
     const int64_t units = (int64_t)H * G * sides;

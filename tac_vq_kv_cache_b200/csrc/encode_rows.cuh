@@ -49,8 +49,7 @@ __device__ __forceinline__ void unpack8(const uint4 &w, float (&c)[8]) {
 }
 
 template <int DSUB>
-__device__ __forceinline__ int nearest_word_in_warp(const float (&res)[DSUB], const __half *__restrict__ words,
-                                                    const float *__restrict__ sqnorm_in, int K, int lane) {
+__device__ __forceinline__ int nearest_word_in_warp(const float (&res)[DSUB], const __half *words, const float *sqnorm_in, int K, int lane) {
     const float xx = sqnorm_ordered<DSUB>([&](int i) { return res[i]; });
     float best = __int_as_float(0x7f800000);
     int arg = 0x7fffffff;
@@ -59,7 +58,7 @@ __device__ __forceinline__ int nearest_word_in_warp(const float (&res)[DSUB], co
         float c[DSUB];
         if constexpr (DSUB == 8) {
             if (aligned) {  // one 16-byte load per word: the same values
-                unpack8(__ldg(reinterpret_cast<const uint4 *>(words + (int64_t)k * DSUB)), c);
+                unpack8(*reinterpret_cast<const uint4 *>(words + (int64_t)k * DSUB), c);
             } else {
 #pragma unroll
                 for (int i = 0; i < DSUB; ++i) c[i] = __half2float(words[(int64_t)k * DSUB + i]);

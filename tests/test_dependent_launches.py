@@ -68,3 +68,23 @@ def test_the_table_preparation_lets_the_scan_start_only_after_its_own_wait():
     ((_, scan, _),) = [found[1:] for found in _kernels() if found[0] == "attn_gsrq_scan_kernel"]
     before = scan[scan.index("while (cursor < my_end)") : scan.index("wait_once();\n        uint4 k0")]
     assert not {"lut_g", "scale_g", "part", "marks", "out"} & set(re.findall(r"\w+", before))
+
+
+def test_no_kernel_lets_the_next_one_start_before_its_own_wait():
+    """The next kernel reads what is older than the one in front of it (tables, old codes, ranges) before it waits itself."""
+    triggers = {name: body for name, _, body, _ in _kernels() if "launch_dependents()" in body or "start_after_previous_kernel()" in body}
+    assert {"decode_prologue_kernel", "encode_few_wide_kernel", "attn_slots_kernel", "attn_combine_kernel"} <= set(triggers)
+    for name, body in triggers.items():
+        if "launch_dependents()" in body:
+            assert body.index("wait_for_previous_kernel()") < body.index("launch_dependents()"), name
+
+
+def test_the_rows_and_tables_of_a_step_are_not_constant_memory_to_its_first_kernel():
+    """It may be scheduled while the launch that computes them runs."""
+    found = {name: (params, body) for name, params, body, _ in _kernels()}
+    params, body = found["decode_prologue_kernel"]
+    assert body.split(";")[0].strip() == "start_after_previous_kernel()"
+    for param in params.split(","):
+        if re.findall(r"\w+", param)[-1] in {"k_rows", "v_rows", "ktab", "vtab"}:
+            assert "__restrict__" not in param, param.strip()
+    assert "__ldg" not in (CSRC / "encode_rows.cuh").read_text() and "__ldg" not in found["encode_few_wide_kernel"][1]
