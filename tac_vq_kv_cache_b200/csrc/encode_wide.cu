@@ -505,7 +505,9 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             // previous use, which is then not refilled either, so that all warps end up this way.
             if (!fail && !bounded_wait(full_bar + 8 * buf, (u >> 1) & 1u, a.spins)) fail = true;
             fail = __any_sync(0xffffffffu, fail);
-            if ((warp & 15) == 0) {
+            // by a warp that refills no tables where four do: a thread is held up by the products that it asks for nearly until they are done (1300
+            // clocks), a refill takes 1450.  By warp 0, one after the other, 16 stages x 2048 rows took 105 us, so 102; x 16384 rows 525 / 507.
+            if ((warp & 15) == 15) {
                 if (lane == 0 && !fail) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t d0 = tmem_base + (uint32_t)grp * kMaxWords, a0 = smem_u32(A), b0 = smem_u32(tab);
