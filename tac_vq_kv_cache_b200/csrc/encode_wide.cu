@@ -8,8 +8,8 @@
 //      first step of 16 columns (A: ones, B: -|c|^2/2 in three fp16 parts) makes every sum the score
 //      t = r.c - |c|^2/2, the distance being |r|^2 - 2t,
 //   2. reads its scores twice: once for the row's maximum, once for the mask of words within a margin of it,
-//   3. takes the only word of the mask; two words are scored in fp32, and where that leaves them too close, or where
-//      there are more, the row goes to shared memory and the library's exact chains decide,
+//   3. takes the only word of the mask; two or three words are scored in fp32, and where that leaves the best too close to
+//      another, or where there are more, the row goes to shared memory and the library's exact chains decide,
 //   4. subtracts the chosen word and writes the new fp16 row.
 // The two groups share the word tables: resident for the block's life up to two stages, otherwise a ring of two
 // that the group which leaves a stage last refills (words by TMA, norms by its warps).  While one group waits for its product the other one reads
@@ -591,19 +591,21 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             }
             sync_quad();
             // ---- the choice ----
-            int n_words = 0, wa = 0, wb = 0;  // the last two listed, of the first two of every thread
+            int n_words = 0, wa = 0, wb = 0, wc = 0;  // the last three listed, of the first two of every thread
+            bool hidden = false;  // a thread lists more words than it tells
 #pragma unroll
             for (int i = 0; i < kShare; ++i) {
                 const int info = infos[i * kRows], n = info >> 12;
                 n_words += n;
-                if (n >= 1) wb = wa, wa = i * 64 + (info & 63);
-                if (n >= 2) wb = wa, wa = i * 64 + ((info >> 6) & 63);
+                hidden |= n > 2;
+                if (n >= 1) wc = wb, wb = wa, wa = i * 64 + (info & 63);
+                if (n >= 2) wc = wb, wb = wa, wa = i * 64 + ((info >> 6) & 63);
             }
             int pick = min(wa, K - 1);  // (a row past the end may have listed padding words)
             // (rows past the end are all alike: one that is undecided would be 32 in a row)
             bool undecided = live && n_words != 1;
             if (__any_sync(0xffffffffu, undecided)) {  // the same in the four warps
-                // Two words (nearly always all there are): their dot products once more in fp32, each thread over its part of the
+                // Two words (mostly all there are): their dot products once more in fp32, each thread over its part of the
                 // row.  E is then 2^-17 u for the chain that it stands for, 2^-18 u of its own and 2^-23 (|r|^2 + cc), which
                 // settles about 49 rows in 50.
                 if (undecided) {
@@ -633,11 +635,44 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                     xxs[q * kRows] = dots[2] + dots[3];
                 }
                 sync_quad();
-                if (undecided && n_words == 2 && max(wa, wb) < K) {
+                const bool three = undecided && n_words == 3 && !hidden && max(max(wa, wb), wc) < K;
+                float better = 0.0f;  // of the first two
+                if ((undecided && n_words == 2 && max(wa, wb) < K) || three) {
                     const float ta = ((tops[0] + tops[kRows]) + (tops[2 * kRows] + tops[3 * kRows])) - 0.5f * nrm[wa];
                     const float tb = ((xxs[0] + xxs[kRows]) + (xxs[2 * kRows] + xxs[3 * kRows])) - 0.5f * nrm[wb];
                     pick = tb > ta ? wb : wa;
+                    better = fmaxf(ta, tb);
                     undecided = !(fabsf(ta - tb) > 3.2e-5f * u_top + 4.8e-7f * (xx + cc_top) + 1.0e-30f);
+                }
+                // The third word of a row, in a quarter of the stages of 32 whitened rows.  Left to the chains, which hold up the whole group, us:
+                // 16 stages x 2048 rows 102 / 96, whitened 207 / 185, whitened 4 x 4096 rows 1144 / 1025.
+                if (__any_sync(0xffffffffu, three)) {  // the same in the four warps
+                    sync_quad();
+                    if (three) {
+                        float dots[2] = {0.0f, 0.0f};
+#pragma unroll
+                        for (int m = 0; m < kOwn; ++m) {
+                            const int e = 8 * (4 * m + q);
+                            float c0[8];
+                            if constexpr (EXACT32) {
+#pragma unroll
+                                for (int i = 0; i < 2; ++i)
+                                    *reinterpret_cast<float4 *>(c0 + 4 * i) = __ldg(reinterpret_cast<const float4 *>(a.words32 + (first + wc) * DSUB + e) + i);
+                            } else {
+                                unpack8(*reinterpret_cast<const uint4 *>(tab + L::template at<kMaxWords>(wc, e)), c0);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 8; j += 2) fma2(dots[0], dots[1], r[8 * m + j], r[8 * m + j + 1], c0[j], c0[j + 1]);
+                        }
+                        tops[q * kRows] = dots[0] + dots[1];
+                    }
+                    sync_quad();
+                    if (three) {
+                        const float tc = ((tops[0] + tops[kRows]) + (tops[2 * kRows] + tops[3 * kRows])) - 0.5f * nrm[wc];
+                        const float close = 3.2e-5f * u_top + 4.8e-7f * (xx + cc_top) + 1.0e-30f;
+                        if (tc > better + close) pick = wc, undecided = false;  // however close the other two are
+                        else if (!(better > tc + close)) undecided = true;
+                    }
                 }
                 sync_quad();  // all of it is read
                 // ---- the exact chains of every listed word, one row after the other through shared memory ----
@@ -683,7 +718,9 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                         if ((((half ? listed[1] : listed[0]) >> lane) & 1u) != 0u && k < K) {
                             float dot = 0.0f;
                             auto chain = [&](auto fetch) {
-#pragma unroll 2
+// (words from L2, 16 whitened stages x 2048 rows: 181 us, two pieces at a time 185; two groups a block would spill)
+                                // words from L2, 16 whitened stages x 2048 rows: 181 us, two pieces at a time 185; with two groups a block four spill
+#pragma unroll (EXACT32 && GROUPS == 1 ? 4 : 2)
                                 for (int p = 0; p < kPieces; ++p) {
                                     const float *from = piece_at(p & 3, p >> 2);
                                     float e[8], w[8];

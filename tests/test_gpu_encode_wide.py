@@ -101,3 +101,27 @@ def test_rows_between_words_take_the_exact_chains(device):
     want, want_recon = C.encode(states, tables)
     codes, recon = ops.encode(states.to(device), tables.to(device))
     assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
+
+
+@pytest.mark.parametrize("sub,groups,tokens,dtype,whitened", [(128, 1, 300, torch.float16, False), (64, 2, 129, torch.float32, False), (128, 1, 260, torch.float16, True), (128, 1, 9500, torch.float32, False)])
+@pytest.mark.parametrize("alike", [(3, 70, 200), (5, 6, 200), (8, 9, 10), (3, 70, 140, 250)])
+def test_rows_near_three_words(device, sub, groups, tokens, dtype, whitened, alike):
+    """Words that differ by a few units of their last place: in three shares of the table, in two, in one (which tells of two), and four of them."""
+    from tac_vq_kv_cache_b200 import ops
+
+    gen = torch.Generator().manual_seed(tokens + len(alike))
+    tables = make_tables(gen, 2, 2, groups, sub, [0.1, 0.1])
+    for i, k in enumerate(alike):
+        apart = (1e-4, 4e-4, 4e-5, 2e-4)[i] * torch.randn(2, groups, sub, generator=gen)
+        tables[:, 0, :, k] = (tables[:, 0, :, alike[0]].float() + apart).half()
+    states = 10.0 * tables[:, 0, :, alike[0]].float().reshape(1, 2, 1, groups * sub) + 0.5 * torch.randn(1, 2, tokens, groups * sub, generator=gen)
+    states[:, :, ::3] = torch.randn(1, 2, (tokens + 2) // 3, groups * sub, generator=gen)
+    states = states.to(dtype)
+    if whitened:
+        w = torch.eye(sub).expand(2, groups, sub, sub) + 0.05 * torch.randn(2, groups, sub, sub, generator=gen) / sub**0.5
+        want, want_recon = C.encode_whitened(states, tables, w)
+        codes, recon = ops.encode(states.to(device), tables.to(device), whitener=w.to(device))
+    else:
+        want, want_recon = C.encode(states, tables)
+        codes, recon = ops.encode(states.to(device), tables.to(device))
+    assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
