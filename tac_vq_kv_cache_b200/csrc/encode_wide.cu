@@ -26,7 +26,7 @@
 // Rows or words outside fp16's range, and a product that never arrived, list every word.
 //
 // What bounds it: latency between the phases of a stage more than the tensor core (1152 cycles a tile and stage) or the
-// issue slots, hence two tiles a block and four threads a row.  262144 fp16 rows x 8 heads, 128 wide, 2 stages: 837 us,
+// issue slots, hence two tiles a block and four threads a row.  262144 fp16 rows x 8 heads, 128 wide, 2 stages: 815 us,
 // against 1675 us for one tile of 128 rows a block with the residual in tensor memory.
 //
 // Reference statements: src/jointkv/closed_loop_vq.py:52-76 (search), :343-395 (stage recursion), :312-320, 384-390
@@ -229,6 +229,11 @@ __global__ void __launch_bounds__(GROUPS * kGroupThreads, 1)
 encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) {
     using L = Layout<DSUB>;
     constexpr int kPieces = DSUB / 8, kOwn = kPieces / kShare;
+    // Fp32 scores further apart than this many u tell which of two words the exact distances prefer.  Each word's share, in units of 2^-24 u: DSUB
+    // roundings of the exact chain, DSUB / 8 + 3 of the score's sums, one where the norm is subtracted and one in the distance; a hundredth
+    // is left for the bound u itself.  (3.2e-5, twice what is needed at 128, sent 1.8 times as many rows to the chains:
+    // 849 us where it is 815, 16 whitened stages x 2048 rows 181 / 177.)
+    constexpr float kClose = 1.01f * 2.0f * (DSUB + DSUB / 8 + 5) * 5.9604645e-8f;
     extern __shared__ __align__(1024) unsigned char smem[];
     __half *tabs = reinterpret_cast<__half *>(smem + L::kTab);
     float *nrms = reinterpret_cast<float *>(smem + L::kNrm);
@@ -606,8 +611,8 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
             bool undecided = live && n_words != 1;
             if (__any_sync(0xffffffffu, undecided)) {  // the same in the four warps
                 // Two words (mostly all there are): their dot products once more in fp32, each thread over its part of the
-                // row.  E is then 2^-17 u for the chain that it stands for, 2^-18 u of its own and 2^-23 (|r|^2 + cc), which
-                // settles about 49 rows in 50.
+                // row.  Further apart than kClose u and 2^-22 (|r|^2 + cc), for the roundings of the norms' and distances' sums, they
+                // settle about 99 rows in 100.
                 if (undecided) {
                     const int ka = min(wa, K - 1), kb = min(wb, K - 1);
                     float dots[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -642,7 +647,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                     const float tb = ((xxs[0] + xxs[kRows]) + (xxs[2 * kRows] + xxs[3 * kRows])) - 0.5f * nrm[wb];
                     pick = tb > ta ? wb : wa;
                     better = fmaxf(ta, tb);
-                    undecided = !(fabsf(ta - tb) > 3.2e-5f * u_top + 4.8e-7f * (xx + cc_top) + 1.0e-30f);
+                    undecided = !(fabsf(ta - tb) > kClose * u_top + 2.4e-7f * (xx + cc_top) + 1.0e-30f);
                 }
                 // The third word of a row, in a quarter of the stages of 32 whitened rows.  Left to the chains, which hold up the whole group, us:
                 // 16 stages x 2048 rows 102 / 96, whitened 207 / 185, whitened 4 x 4096 rows 1144 / 1025.
@@ -669,7 +674,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                     sync_quad();
                     if (three) {
                         const float tc = ((tops[0] + tops[kRows]) + (tops[2 * kRows] + tops[3 * kRows])) - 0.5f * nrm[wc];
-                        const float close = 3.2e-5f * u_top + 4.8e-7f * (xx + cc_top) + 1.0e-30f;
+                        const float close = kClose * u_top + 2.4e-7f * (xx + cc_top) + 1.0e-30f;
                         if (tc > better + close) pick = wc, undecided = false;  // however close the other two are
                         else if (!(better > tc + close)) undecided = true;
                     }
