@@ -20,7 +20,7 @@
 // first stage of fp16 rows); the exact chain, 2^-17 u; the tensor core's sums, at most nine steps that each lose
 // 17 units of 2^-24 of a magnitude below u + cc / 2, so 2^-16.7 (u + cc / 2); the roundings of the distance,
 // 2^-23 (|r|^2 + cc); the three fp16 parts of -|c|^2/2, 2^-25; rows that are subnormal in fp16, 2^-25 sqrt(d) max|c|.
-// The kernel allows  (1.0625 * 2^-10, or 2^-13) u  +  2^-20 |r|^2  +  2^-15 cc  +  2^-18 max|c|  +  2^-23.
+// The kernel allows  (1.0625 * 2^-10, or 2^-14) u  +  2^-20 |r|^2  +  2^-15 cc  +  2^-18 max|c|  +  2^-23.
 // With EXACT32 the words are fp32 (transformed by a whitener) and their fp16 rounding is scored: 2^-10 u more, and
 // 2^-20 |r| for words that are subnormal in fp16; everything that decides reads the fp32 words.
 // Rows or words outside fp16's range, and a product that never arrived, list every word.
@@ -542,7 +542,7 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
 #pragma unroll 1
                 for (int i = 4; i < shares; ++i) cc_top = fmaxf(cc_top, share_tops[i]);
             const float u_top = rough_sqrt(xx * cc_top);
-            const float margin = (sizeof(XT) == 2 && s == 0 ? 1.220703125e-04f : EXACT32 ? 2.01416015625e-03f : 1.03759765625e-03f) * u_top +
+            const float margin = (sizeof(XT) == 2 && s == 0 ? 6.103515625e-05f : EXACT32 ? 2.01416015625e-03f : 1.03759765625e-03f) * u_top +
                                  9.5367431640625e-07f * xx + 3.0517578125e-05f * cc_top + 3.814697265625e-06f * rough_sqrt(cc_top) +
                                  (EXACT32 ? 9.5367431640625e-07f * rough_sqrt(xx) : 0.0f) + 1.1920929e-07f;
             if (!fail && !bounded_wait(my_mma, mma_phase, a.spins)) fail = true;
