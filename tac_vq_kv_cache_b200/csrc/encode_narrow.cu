@@ -11,11 +11,11 @@
 // 2^-18 sqrt(cc_max) in units of t; the three fp16 parts of -|c|^2/2 add 2^-25, the kernel 2^-23).  Rows or words outside
 // fp16's range, and a product that never arrived, re-evaluate every word.
 //
-// Blocks split the tiles of all (head, group) pairs evenly, span by span of 8192 rows, and bring a pair's tables in when they
+// Blocks split the tiles of all (head, group) pairs evenly, span by span of 16384 rows, and bring a pair's tables in when they
 // enter it, so the chip stays full whatever the number of pairs; a table costs about one tile's time.
 //
 // Bound by latency between the phases of a stage at 16 warps an SM.  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
-// stages, rows wanted: 344 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.  Whitened (fp32 words, a third product a
+// stages, rows wanted: 325 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.  Whitened (fp32 words, a third product a
 // half): 3001 fp32 rows x 8 heads, 32 x 4, one stage 51 us against 125 for the fp32 scan of all words.
 // (Words as fp32 pairs in copies without bank conflicts, two exact chains an instruction: 372 us where this takes 344, as look-ups are scarcer than
 // issue slots.)
@@ -30,7 +30,7 @@ namespace tacvq {
 namespace narrow {
 
 constexpr int kRows = 128, kGroups = 4, kThreads = kRows * kGroups, kHalf = kMaxWords / 2;
-constexpr uint32_t kSpan = 64;  // tiles
+constexpr uint32_t kSpan = 128;  // tiles
 constexpr size_t kWordBytes = kMaxWords * 32, kSeedBytes = kMaxWords * 32, kNormBytes = kMaxWords * 4;
 constexpr size_t kStageBytes = kWordBytes + kSeedBytes + kNormBytes;  // (word | word), seeds, |word|^2
 // fp32 words: their fp16 rounding takes the place of the words above; what it leaves follows, (low | 0), and the words themselves
@@ -202,13 +202,16 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
 #pragma unroll 1
     for (uint32_t span = 0; span < tiles; span += kSpan) {
     const uint32_t wide = min(kSpan, tiles - span);
-    const int64_t work = (int64_t)pairs * wide, end = work * (blockIdx.x + 1) / gridDim.x;
+    // Blocks get turns, a tile for every group of threads: where a block's part of a pair was any number of tiles, groups idled at its end.  With that
+    // and spans of 64 tiles, us, 16 x 2 x 8 with rows, 32768 rows x 8 heads 344 / 325 (fp32 rows 359 / 318), 16384 rows 157 / 149, 700 rows
+    // 23.6 / 22; 32 x 4, 32768 rows 362 / 316.  From 9 to 31 tiles a pair the coarser parts cost what they save: 3333 rows 47.6 / 50.1.
+    const uint32_t unit = wide > 2 * kGroups && wide < 8 * kGroups ? 1u : (uint32_t)kGroups, units = (wide + unit - 1) / unit;
+    const int64_t work = (int64_t)pairs * units, end = work * (blockIdx.x + 1) / gridDim.x;
 #pragma unroll 1
     for (int64_t at = work * blockIdx.x / gridDim.x; at < end;) {
-        const int hg = (int)(at / wide), h = hg / G, g = hg % G;
-        const uint32_t offset0 = (uint32_t)(at - (int64_t)hg * wide);
-        const uint32_t tile0 = span + offset0;
-        const uint32_t tile1 = span + (uint32_t)min((int64_t)wide, (int64_t)offset0 + (end - at));  // tiles of this pair that are this block's
+        const int hg = (int)(at / units), h = hg / G, g = hg % G;
+        const uint32_t unit0 = (uint32_t)(at - (int64_t)hg * units), mine = (uint32_t)min((int64_t)(units - unit0), end - at);
+        const uint32_t tile0 = span + unit0 * unit, tile1 = span + min(wide, (unit0 + mine) * unit);  // of this pair, for this block
         // ---- the pair's tables ----
         __syncthreads();  // the previous pair's are no longer read
         if (tid < S) cc_tops[tid] = 0;
@@ -458,7 +461,7 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
                 }
             }
         }
-        at += tile1 - tile0;
+        at += mine;
     }
     }
     if (__syncthreads_or(fail)) {  // each group's last product ends before the block's memory goes

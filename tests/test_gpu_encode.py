@@ -464,6 +464,20 @@ def test_both_kernels_of_narrow_groups_where_one_takes_over_from_the_other(devic
     assert ops.encode_tensor_memory_timeouts(device) == 0
 
 
+@pytest.mark.parametrize("heads,tokens,sub,groups,stages", [(3, 1024, 8, 16, 2), (3, 1025, 4, 32, 1), (1, 3968, 8, 16, 2), (1, 3969, 8, 16, 1), (1, 16513, 8, 4, 2), (3, 33000, 4, 3, 1)])
+def test_narrow_groups_where_the_parts_of_a_block_change(device, heads, tokens, sub, groups, stages):
+    """8 and 9, 31 and 32 tiles a pair, which are dealt out singly or by fours; spans of 128 tiles with a short one behind; whitened words too."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(tokens)
+    tables = make_tables(gen, heads, stages, groups, sub, [0.5 * 0.8**s for s in range(stages)])
+    states = make_states(gen, (1, heads, tokens, sub * groups), torch.float32)
+    w = torch.eye(sub).expand(heads, groups, sub, sub) + 0.3 * torch.randn(heads, groups, sub, sub, generator=gen) / sub**0.5
+    for want, arguments in ((C.encode(states, tables), {}), (C.encode_whitened(states, tables, w), {"whitener": w.to(device)})):
+        codes, recon = ops.encode(states.to(device), tables.to(device), **arguments)
+        assert torch.equal(codes.cpu(), want[0]) and torch.equal(recon.cpu(), want[1])
+    assert ops.encode_tensor_memory_timeouts(device) == 0
+
+
 @pytest.mark.parametrize(
     "batch,tokens,sub,groups,stages,words,depth,dtype",
     [
