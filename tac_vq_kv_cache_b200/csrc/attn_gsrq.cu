@@ -824,6 +824,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
         // the blocks that hold a partial state of this pair (this block among them)
         const int c_lo = block_of_unit(pair_first + kItemCost, total_tiles, blocks);
         const int n_parts = block_of_unit(pair_end - 1, total_tiles, blocks) - c_lo + 1;
+        __half *result = reinterpret_cast<__half *>(stage_s);  // [4][128]; the value codes are used up
         __syncthreads();
         for (int o = tid; o < kRep * kDim; o += kThreads) {
             // output o <-> (product mm, register j, lane of visiting-order class 0); its class-1 twin is
@@ -843,7 +844,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             }
             if (n_parts == 1) {  // the whole pair was scanned here: this is the result
                 const size_t row = (size_t)b * Hq + h * kRep + r;
-                if (out) out[row * kDim + dim] = __float2half_rn(lsum == 0.0f ? 0.0f : asum / lsum);
+                result[r * kDim + dim] = __float2half_rn(lsum == 0.0f ? 0.0f : asum / lsum);
                 if (state_out) {
                     float *dst = state_out + row * kStateWidth;
                     if (dim == 0) {
@@ -861,7 +862,12 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
                 dst[2 + dim] = asum;
             }
         }
-        if (n_parts > 1) {
+        if (n_parts == 1) {
+            // in whole lines, as the result may lie in the host's memory
+            __syncthreads();
+            if (out)
+                for (int o = tid; o < kRep * kDim; o += kThreads) out[((size_t)b * Hq + h * kRep) * kDim + o] = result[o];
+        } else {
             // Mark this partial with the call's epoch; whoever then finds every partial of the pair marked
             // merges them.  The fences order (partial, mark) and (mark, reading the other marks), so the block
             // whose mark lands last always sees all of them; two blocks may both see them and then write the same
