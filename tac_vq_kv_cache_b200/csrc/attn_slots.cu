@@ -312,7 +312,10 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
 
     // A decode step's new codes and ranges come from the kernel before this one; the tables and the query do not.
     wait_for_previous_kernel();
-    launch_dependents();
+    // The next kernel's blocks stay on the SMs that are free when they may start, so they may early only where a third of the SMs is.  us a step,
+    // always / never / so: 2 x 128, 8 rows x 16384 tokens 27.5 / 26.2 / 26.2; 16 x 2 x 8 with one head a KV head, 16 x 396 29.6 / 27.7 / 27.7,
+    // 4 x 466 19.7 / 24.0 / 19.7.
+    if (gridDim.x * gridDim.y * gridDim.z <= 98u) launch_dependents();
     const int lo_all = max(seq_start ? seq_start[b] : 0, 0);
     const int hi_all = min(seq_end ? seq_end[b] : (int)T_cap, (int)T_cap);
     const int n_all = hi_all > lo_all ? hi_all - lo_all : 0;
