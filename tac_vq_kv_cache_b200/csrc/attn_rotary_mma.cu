@@ -20,7 +20,7 @@
 //
 // What bounds it: wavefronts of the L1/shared pipe and the latency between them at 16 warps.  A block of 4856 tokens, in clocks: copies
 // and softmax 16 k (25 k when scattered 16-byte cp.async filled the tables), pass K 44 k (9.2 a token, 6.2 of them wavefronts), pass V 25 k (5.2, of
-// which 4.4 are look-ups).  us a decode step with 8 KV heads, 8 rows x 32768: 165 (180 with those copies).  Against a row and at most 4096 tokens a
+// which 4.4 are look-ups).  us a decode step with 8 KV heads, 8 rows x 32768: 163 (180 with those copies).  Against a row and at most 4096 tokens a
 // block, before: 8 rows x 32768 183 / 205, a window of 4096 of them 45 / 91, 2 x 65536 115 / 148.
 //
 // Every shared-memory gather is conflict-free for arbitrary codes: a code's 32 codewords lie in one

@@ -26,7 +26,7 @@
 // Rows or words outside fp16's range, and a product that never arrived, list every word.
 //
 // What bounds it: latency between the phases of a stage more than the tensor core (1152 cycles a tile and stage) or the
-// issue slots, hence two tiles a block and four threads a row.  262144 fp16 rows x 8 heads, 128 wide, 2 stages: 815 us,
+// issue slots, hence two tiles a block and four threads a row.  262144 fp16 rows x 8 heads, 128 wide, 2 stages: 807 us,
 // against 1675 us for one tile of 128 rows a block with the residual in tensor memory.
 //
 // Reference statements: src/jointkv/closed_loop_vq.py:52-76 (search), :343-395 (stage recursion), :312-320, 384-390
