@@ -28,8 +28,8 @@
 // are exact.
 //
 // Where a cluster's time goes, us after its start, one row with 4096 tokens: tables there 5.9, scores of 64 SMs 27.8, parts exchanged 31.6, weights
-// exchanged 36.9, histograms 40.5, end 44.7.  The weights are relative to the maximum of the block that has their share of the tokens and put right by the
-// reader, which saves one of four exchanges (2 us); sums in two chains of products and rotary rows in whole channel pairs take 1 us off the scores.
+// exchanged 36.9, histograms 40.5, end 44.7.  Scores travel in one exchange with the blocks' maxima, and every block takes the weights of all tokens
+// itself, which saves one of four exchanges (2 us); sums in two chains of products and rotary rows in whole channel pairs take 1 us off the scores.
 //
 // A sum of 16 words by the tensor core is no further from the exact one than fp32 adds in order: over 2^20 sums of 4, 8, 12 and 16 normal values,
 // of equal spread and falling by 0.9 and 0.6 a stage, 3.5e-10 to 9.3e-9 in the 2-norm against 3.5e-10 to 1.3e-8, and the same fp16
@@ -57,10 +57,10 @@ constexpr int kThreads = 512, kWarps = kThreads / 32;
 constexpr int kDim = 128, kWords = 256, kStages = 16, kSlices = 8, kHeads = 4;
 constexpr int kRowBytes = kStages * 2 * 16;           // a code's words of all stages, this block's 16 channels
 constexpr int kTabBytes = kWords * kRowBytes;         // 131072
-constexpr int kScoreBytes = kChunk * kHeads * 4;      // parts of the scores, then weights, then per-warp sums
+constexpr int kScoreBytes = kChunk * kHeads * 4;      // parts of the scores, then scores, then per-warp sums
 constexpr int kHistBytes = 2 * 2 * kWords * kHeads * 4;  // [multiples | rest][stage j or j + 8][word][head]
 constexpr int kOutBytes = kSlices * 64 * 4;           // [source block][64 of the 512 outputs]
-constexpr int kSmallFloats = 3 * kSlices * kHeads + 2 * kWarps * kHeads;  // maxima, sums and factors of the blocks, maxima and sums of the warps
+constexpr int kSmallFloats = kSlices * kHeads + 2 * kWarps * kHeads;  // maxima of the blocks, maxima and sums of the warps
 constexpr int kSmemBytes = kTabBytes + kScoreBytes + kHistBytes + kOutBytes + kSmallFloats * 4;
 static_assert(kWarps * kHeads * kDim * 4 <= kScoreBytes, "per-warp sums reuse the score area");
 static_assert(kSmemBytes <= 227 * 1024, "");
@@ -141,9 +141,8 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
     unsigned char *area = smem + kTabBytes;                              // scores, then weights, then sums
     uint32_t *hist = reinterpret_cast<uint32_t *>(area + kScoreBytes);
     float *out_s = reinterpret_cast<float *>(area + kScoreBytes + kHistBytes);
-    float *top_s = out_s + kSlices * 64, *sum_s = top_s + kSlices * kHeads;  // [block][head]
-    float *warp_top = sum_s + kSlices * kHeads, *warp_sum = warp_top + kWarps * kHeads;
-    float *factor_s = warp_sum + kWarps * kHeads;  // [block][head]: from weights relative to a block's maximum to the largest of all
+    float *top_s = out_s + kSlices * 64;  // [block][head]
+    float *warp_top = top_s + kSlices * kHeads, *warp_sum = warp_top + kWarps * kHeads;
     const uint32_t tab_u32 = smem_u32(smem), area_u32 = smem_u32(area);
 
     const int slice = blockIdx.x % kSlices, cluster = blockIdx.x / kSlices, clusters = gridDim.x / kSlices;
@@ -310,13 +309,12 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                 v_words[k] = ldg_in_place(vtab + (((int64_t)h * S + slice + 8 * (k >> 3)) * kWords + (k & 7) * 32 + (tid >> 4)) * kDim + piece * 8);
         cluster_barrier();
 
-        // ---- block j adds up the parts of its share of the tokens; weights go to every block ------------------------------
-        const int share = (n + kSlices - 1) / kSlices;  // at most kThreads
+        // ---- block j adds up the parts of its share of the tokens; scores and the share's maxima go to every block --------------
         {
+            const int share = (n + kSlices - 1) / kSlices;  // at most kThreads
             const int t = slice * share + tid;
-            const bool mine = tid < share && t < n;
             float sc[kHeads] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            if (mine) {
+            if (tid < share && t < n) {
                 float4 v[kSlices];
 #pragma unroll
                 for (int k = 0; k < kSlices; ++k) v[k] = ld_cluster4(in_block(area_u32 + t * 16, k));
@@ -324,6 +322,8 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
 #pragma unroll
                 for (int k = 1; k < kSlices; ++k) s.x += v[k].x, s.y += v[k].y, s.z += v[k].z, s.w += v[k].w;
                 sc[0] = s.x, sc[1] = s.y, sc[2] = s.z, sc[3] = s.w;
+#pragma unroll
+                for (int k = 0; k < kSlices; ++k) st_cluster4(in_block(area_u32 + t * 16, k), s);
             }
 #pragma unroll
             for (int r = 0; r < kHeads; ++r) {
@@ -333,51 +333,33 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                 if (lane == 0) warp_top[warp * kHeads + r] = v;
             }
             __syncthreads();
-            // weights relative to this block's maximum, which every block puts right when it has all maxima
-            float top[kHeads], sum[kHeads];
-#pragma unroll
-            for (int r = 0; r < kHeads; ++r) {
-                top[r] = warp_top[r];
-#pragma unroll 5
-                for (int w = 1; w < kWarps; ++w) top[r] = fmaxf(top[r], warp_top[w * kHeads + r]);
-                sum[r] = mine ? __expf(sc[r] - top[r]) : 0.0f;
-            }
-            if (mine)
-                for (int k = 0; k < kSlices; ++k) st_cluster4(in_block(area_u32 + t * 16, k), make_float4(sum[0], sum[1], sum[2], sum[3]));
-#pragma unroll
-            for (int r = 0; r < kHeads; ++r) {
-#pragma unroll
-                for (int off = 16; off >= 1; off >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], off);
-                if (lane == 0) warp_sum[warp * kHeads + r] = sum[r];
-            }
-            __syncthreads();
-            if (tid < kSlices * kHeads) {  // of head tid % 4, to block tid / 4
-                const int r = tid & 3;
-                float v = 0.0f;
-                for (int w = 0; w < kWarps; ++w) v += warp_sum[w * kHeads + r];
-                const float own = r == 0 ? top[0] : r == 1 ? top[1] : r == 2 ? top[2] : top[3];
-                st_cluster(in_block(smem_u32(sum_s + slice * kHeads + r), tid >> 2), v);
-                st_cluster(in_block(smem_u32(top_s + slice * kHeads + r), tid >> 2), own);
+            if (tid < kSlices * kHeads) {  // this block's maximum of head tid % 4, to block tid / 4
+                float v = warp_top[tid & 3];
+                for (int w = 1; w < kWarps; ++w) v = fmaxf(v, warp_top[w * kHeads + (tid & 3)]);
+                st_cluster(in_block(smem_u32(top_s + slice * kHeads + (tid & 3)), tid >> 2), v);
             }
             cluster_barrier();
-            if (tid < kSlices * kHeads) {
-                float most = -INFINITY;
-                for (int k = 0; k < kSlices; ++k) most = fmaxf(most, top_s[k * kHeads + (tid & 3)]);
-                factor_s[tid] = top_s[tid] == -INFINITY ? 0.0f : __expf(top_s[tid] - most);  // no token there, or none of a finite score
-            }
-            __syncthreads();
         }
 
-        // ---- weights by code, stages `slice` and `slice` + 8 ----------------------------------------------------------------
+        // ---- weights by code, stages `slice` and `slice` + 8; every block takes the weights of all tokens, relative to the largest score of all --------
+        float ref[kHeads], weight_sum[kHeads];
+#pragma unroll
+        for (int r = 0; r < kHeads; ++r) {
+            float top = top_s[r];
+#pragma unroll
+            for (int k = 1; k < kSlices; ++k) top = fmaxf(top, top_s[k * kHeads + r]);
+            ref[r] = top == -INFINITY ? 0.0f : top;  // a score of -inf weighs nothing, also where there is no other; NaN stays NaN
+            weight_sum[r] = 0.0f;
+        }
 #pragma unroll
         for (int i = 0; i < kChunk / kThreads; ++i) {
             const int t = tid + i * kThreads;
             if (t >= n) break;
-            float4 p4 = *reinterpret_cast<const float4 *>(area + t * 16);
-            const float4 f4 = *reinterpret_cast<const float4 *>(factor_s + t / share * kHeads);
-            p4 = make_float4(p4.x * f4.x, p4.y * f4.y, p4.z * f4.z, p4.w * f4.w);
+            const float4 s4 = *reinterpret_cast<const float4 *>(area + t * 16);
+            float p[kHeads] = {__expf(s4.x - ref[0]), __expf(s4.y - ref[1]), __expf(s4.z - ref[2]), __expf(s4.w - ref[3])};
+#pragma unroll
+            for (int r = 0; r < kHeads; ++r) weight_sum[r] += p[r];
             // lane l takes the heads in the order l, l + 1, ..: the 32 adds of an instruction spread over all banks
-            float p[kHeads] = {p4.x, p4.y, p4.z, p4.w};
             if (lane & 1) {
                 const float x = p[0];
                 p[0] = p[1], p[1] = p[2], p[2] = p[3], p[3] = x;
@@ -390,7 +372,7 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
             }
             uint32_t w[kHeads], rest[kHeads];
 #pragma unroll
-            for (int r = 0; r < kHeads; ++r) {  // a NaN leaves some integer here; its sum above spoils the result
+            for (int r = 0; r < kHeads; ++r) {  // a NaN leaves some integer here; the sum of the weights spoils the result
                 const float near = fmaf(p[r], kFine, kRound);
                 w[r] = __float_as_uint(near) & 0x7fffffu;
                 rest[r] = __float_as_uint(fmaf(fmaf(p[r], kFine, kRound - near), kFine, kRoundSigned)) - __float_as_uint(kRoundSigned);
@@ -403,6 +385,12 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
                     atomicAdd(bin + 2 * kWords * kHeads + ((r + lane) & 3), rest[r]);
                 }
             }
+        }
+#pragma unroll
+        for (int r = 0; r < kHeads; ++r) {
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) weight_sum[r] += __shfl_xor_sync(0xffffffffu, weight_sum[r], off);
+            if (lane == 0) warp_sum[warp * kHeads + r] = weight_sum[r];
         }
         __syncthreads();
 
@@ -456,10 +444,12 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
             float a = 0.0f, l = 0.0f, top = -INFINITY;
             for (int k = 0; k < kSlices; ++k) {
                 a += out_s[k * 64 + tid];
-                l += sum_s[k * kHeads + r] * factor_s[k * kHeads + r];
                 top = fmaxf(top, top_s[k * kHeads + r]);
             }
+            for (int w = 0; w < kWarps; ++w) l += warp_sum[w * kHeads + r];
             if (l != l) a = l;
+            // Scores of -inf alone: not the neutral state (a sum of 0).  The merge gives it no weight beside others and makes NaN of it alone.
+            if (top == -INFINITY && l == 0.0f) l = 1.0f;
             if (r < rep) {
                 dst[r * (kDim + 2) + 2 + channel] = a;
                 if (channel == 0) {

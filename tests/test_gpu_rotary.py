@@ -184,6 +184,33 @@ def test_an_infinite_key_word_of_a_ladder_stays_with_its_token(device, stages, w
     out, _ = ops.attn_decode(*(x.to(device) for x in (q, kcodes, vcodes, ktab, vtab)), rope=ops.rope_table(100, 128, 1e6, device))
     _check(out.float().cpu(), want)
 
+@pytest.mark.parametrize("stages", [4, 16])
+@pytest.mark.parametrize("tokens,first,last", [(2, 1, 2), (3, 1, 2), (8, 7, 8), (9, 8, 9), (57, 56, 57), (800, 100, 200), (800, 95, 205), (4500, 1, 4500), (9000, 1, 9000)])
+def test_infinite_scores_of_a_whole_share_of_a_ladder_weigh_nothing(device, stages, tokens, first, last):
+    """Tokens first..last score -inf: all that one of eight blocks adds up the scores of, or a whole split.  That is so for one head of
+    four; the others score +inf there, which is NaN, and no other head's result is."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(stages + tokens)
+    kcodes, vcodes = (torch.randint(0, 255, (1, 1, tokens, stages, 1), generator=gen, dtype=torch.uint8) for _ in range(2))
+    ktab, vtab = (make_tables(gen, 1, stages, 1, 128, [0.3 * 0.85**s for s in range(stages)]) for _ in range(2))
+    q = (torch.randn(1, 4, 128, generator=gen) / 128**0.5).half()
+    q[:, :, [63, 127]] = 0.1
+    q[:, 2, [63, 127]] = -0.1  # from position 1 on channel 63 and its partner both get words of the same sign
+    ktab[:, 1, 0, 255, 63] = float("inf")
+    kcodes[:, :, first:last, 1, 0] = 255
+    arguments = [x.to(device) for x in (q, kcodes, vcodes, ktab, vtab)]
+    rope = ops.rope_table(tokens, 128, 1e6, device)
+    want, *_ = O.attention_over_codes(q, kcodes, vcodes, ktab, vtab, rope_theta=1e6)
+    assert bool(want[:, 2].isfinite().all()) and bool(want[:, [0, 1, 3]].isnan().all())
+    out, state = ops.attn_decode(*arguments, rope=rope, want_state=True)
+    _check(out[:, 2].float().cpu(), want[:, 2])
+    assert bool(out[:, [0, 1, 3]].isnan().all()) and bool(state[:, 2].isfinite().all())
+    # a range of nothing but such tokens has no result, as it has none in softmax
+    start, end = (torch.tensor([x], dtype=torch.int32, device=device) for x in (first, last))
+    out, _ = ops.attn_decode(*arguments, seq_start=start, seq_end=end, rope=rope)
+    assert bool(out.isnan().all())
+
+
 @pytest.mark.parametrize("b,hq,hkv,stages,t", [(1, 4, 1, 16, 4096), (2, 8, 4, 16, 700), (1, 2, 2, 8, 3000), (2, 8, 2, 4, 9000)])
 def test_ladder_weights_have_the_precision_of_fp32(device, b, hq, hkv, stages, t):
     """The state against 64 bits, for logits over a range of about 30 and a rotary table that turns nothing: keys are the sums of their
