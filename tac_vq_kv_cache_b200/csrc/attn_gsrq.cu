@@ -107,7 +107,7 @@ constexpr int kVCodeBytes = kTile * 32;                     // one tile of V cod
 constexpr int kProbStride = 72;                             // bytes per head of the fp16 probabilities: 64 + 8, so the four heads' reads hit different banks
 constexpr int kStagePerWarp = kVCodeBytes + 4 * kProbStride + 32;  // + fp16 probabilities [4 heads][32 tokens], 64-byte multiple
 constexpr int kStageBytes = kWarps * kStagePerWarp;         // 20480 at 16 warps (also scratch of the table build)
-constexpr int kPrefixBytes = (kMaxBatch + 8) * 4 + (12 + 2 * kWarps * kRep) * 4;  // the work prefix; steps and offset; the warps' references and weights
+constexpr int kPrefixBytes = (kMaxBatch + 8) * 4 + (12 + 3 * kWarps * kRep) * 4;  // the work prefix; steps and offset; the warps' references, weights and factors
 constexpr int kSmemBytes = kLutBytes + kVtabBytes + kStageBytes + kPrefixBytes;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -789,7 +789,8 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             l_warp[r] = t;
         }
         // a warp's sums are relative to its own reference, which is within the rescale gap of its maximum
-        float *wm = scale_s + 12, *wl = wm + kWarps * kRep;  // [warps][4] each
+        float *wm = scale_s + 12;                                     // [warps][4]
+        float2 *wfl = reinterpret_cast<float2 *>(wm + kWarps * kRep);  // [warps][4]: factor of the warp's sums, its sum of weights
         if (lane == 0) *reinterpret_cast<float4 *>(wm + warp * kRep) = make_float4(m_ref[0], m_ref[1], m_ref[2], m_ref[3]);
         __syncthreads();  // every warp is done with the tables' score part and the staging area
         static_assert(kWarps * 32 * 32 * 4 <= kLutBytes, "merge scratch must fit in the score table");
@@ -807,20 +808,22 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             for (int r = 0; r < kRep; ++r) {
                 // a warp without a token has nothing to add; a sum that is NaN spoils the others
                 factor[r] = l_warp[r] == 0.0f ? 0.0f : fast_exp2(m_ref[r] - top[r]);
-                l_warp[r] *= factor[r];
             }
         }
-        if (lane == 0) *reinterpret_cast<float4 *>(wl + warp * kRep) = make_float4(l_warp[0], l_warp[1], l_warp[2], l_warp[3]);
+        if (lane == 0) {
+            float4 *to = reinterpret_cast<float4 *>(wfl + warp * kRep);
+            to[0] = make_float4(factor[0], l_warp[0], factor[1], l_warp[1]);
+            to[1] = make_float4(factor[2], l_warp[2], factor[3], l_warp[3]);
+        }
         {
             // accumulator register j of product mm: column 2kq + (j&1) -> head, row half j>>1; stored lane-major
-            const float f0 = (kq & 1) ? factor[2] : factor[0], f1 = (kq & 1) ? factor[3] : factor[1];
             float *base = wacc + (size_t)warp * 1024 + lane;
 #pragma unroll
             for (int mm = 0; mm < 8; ++mm) {
-                base[(mm * 4 + 0) * 32] = acc[mm][0] * f0;
-                base[(mm * 4 + 1) * 32] = acc[mm][1] * f1;
-                base[(mm * 4 + 2) * 32] = acc[mm][2] * f0;
-                base[(mm * 4 + 3) * 32] = acc[mm][3] * f1;
+                base[(mm * 4 + 0) * 32] = acc[mm][0];
+                base[(mm * 4 + 1) * 32] = acc[mm][1];
+                base[(mm * 4 + 2) * 32] = acc[mm][2];
+                base[(mm * 4 + 3) * 32] = acc[mm][3];
             }
         }
         // the blocks that hold a partial state of this pair (this block among them)
@@ -841,8 +844,9 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
 #pragma unroll 4
             for (int w = 0; w < kWarps; ++w) {
                 const float *src = wacc + (size_t)w * 1024;
-                lsum += wl[w * kRep + r];
-                asum += src[(mm * 4 + j) * 32 + lane0] + src[(mm * 4 + (j ^ 2)) * 32 + (lane0 ^ 2)];
+                const float2 fl = wfl[w * kRep + r];
+                lsum = fmaf(fl.x, fl.y, lsum);
+                asum = fmaf(fl.x, src[(mm * 4 + j) * 32 + lane0] + src[(mm * 4 + (j ^ 2)) * 32 + (lane0 ^ 2)], asum);
             }
             if (n_parts == 1) {  // the whole pair was scanned here: this is the result
                 const size_t row = (size_t)b * Hq + h * kRep + r;
