@@ -571,20 +571,26 @@ def test_rebuilt_fp16_rows_equal_the_oracle_bit_for_bit(device, sub, groups, sta
     assert torch.equal(got.view(torch.int16), C.decode(codes, tables, torch.float16, depth=depth).view(torch.int16))
 
 
-@pytest.mark.parametrize("shape", [(8, 128, 128), (1, 1, 1), (3, 7, 7), (2, 2, 33, 33), (5, 64, 64)])
+@pytest.mark.parametrize("shape", [(8, 128, 128), (1, 1, 1), (3, 7, 7), (2, 2, 33, 33), (5, 64, 64), (300, 4, 4), (2, 260, 260), (65, 128, 128), (40, 63, 63)])
 def test_the_identity_is_told_from_its_neighbours(device, shape):
-    """Every corner, the element after the diagonal, another sign of zero, a NaN; the question goes out before the answer is waited for."""
+    """Corners, the element after the diagonal, places of every block's share, another sign of zero, a NaN, a start that is not 16-byte aligned; the
+    question goes out before the answer is waited for."""
     ops = _ops()
     eye = torch.eye(shape[-1], device=device).expand(shape).contiguous()
     assert ops.ask_identity(eye)()
     assert ops.ask_identity(torch.where(eye == 0, -eye, eye))()
     asked = []
-    for at in {0, 1 % eye.numel(), shape[-1] - 1, shape[-1] + 1, eye.numel() // 2, eye.numel() - 1} - {eye.numel()}:
+    somewhere = torch.randint(0, eye.numel(), (12,), generator=torch.Generator().manual_seed(eye.numel())).tolist()
+    for at in {0, 1 % eye.numel(), shape[-1] - 1, shape[-1] + 1, eye.numel() // 2, eye.numel() - 1, *somewhere} - {eye.numel()}:
         if at < eye.numel():
             for value in (2.0, float("nan")):
                 other = eye.clone()
                 other.view(-1)[at] = value
                 asked.append(ops.ask_identity(other))
     assert asked and not any(wait() for wait in asked)
+    aside = torch.empty(eye.numel() + 1, device=device)[1:].view(shape).copy_(eye)
+    assert ops.ask_identity(aside)()
+    aside.view(-1)[-1] = 0.0
+    assert not ops.ask_identity(aside)()
     with pytest.raises(ValueError):
         ops.ask_identity(eye.double())
