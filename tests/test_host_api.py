@@ -141,3 +141,18 @@ def test_host_validation_and_no_cpu_fallback():
     assert set(cq.state_dict()) == {"key_tables.0", "value_tables.0", "key_selector_whitener_00"}
     with pytest.raises(ValueError, match="uniform"):
         cq(0, x, x, mode="mixed")
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+def test_a_layer_that_is_not_there_is_an_index_error(grouped):
+    from tac_vq_kv_cache_b200.jointkv.cq_tac import ClosedLoopGroupedCQ
+    from tac_vq_kv_cache_b200.jointkv.uniform_depth_tac import ClosedLoopUniformResidualVQ
+
+    tables, states = [torch.randn(2, 2, 256, 8)], torch.randn(1, 2, 3, 16 if grouped else 8)
+    if grouped:
+        codec = ClosedLoopGroupedCQ(tables, tables, [torch.eye(8).expand(2, 2, 8, 8)], dynamic_bpa=1.0)
+    else:
+        codec = ClosedLoopUniformResidualVQ(tables, tables, [torch.eye(8).expand(2, 8, 8)], depth=2, dynamic_bpa=1.0)
+    for layer, error in ((1, IndexError), (-2, IndexError), ("0", TypeError)):
+        with pytest.raises(error):
+            codec(layer, states, states)
