@@ -149,6 +149,53 @@ def test_a_step_equals_append_and_attend_bit_for_bit(device, batch, heads, q_hea
 
 
 @pytest.mark.parametrize("rope", [None, 1e6])
+@pytest.mark.parametrize("groups,stages,sub,q_heads", [(16, 2, 8, 8), (16, 2, 8, 2), (1, 2, 128, 8), (1, 16, 128, 8), (16, 1, 8, 8), (32, 1, 4, 8), (2, 3, 64, 8)])
+def test_three_steps_in_one_graph_equal_three_steps(device, groups, stages, sub, q_heads, rope):
+    """A step's first launch may start before what computes its rows has ended, in a graph too: there behind a copy on another
+    stream, a product and the step before.  The graph is replayed on other inputs, over codes that are not the new ones."""
+    from tac_vq_kv_cache_b200.code_cache import VQCodeCache
+
+    gen = torch.Generator().manual_seed(groups + stages)
+    batch, heads, tokens = 3, 2, 500
+    tables = [make_tables(gen, heads, stages, groups, sub, [0.3 * 0.8**s for s in range(stages)] if sub >= 16 else None) for _ in range(2)]
+    plain, captured = (VQCodeCache(*tables, batch=batch, max_tokens=tokens, window=300, device=device, rope_theta=rope) for _ in range(2))
+    codes = [torch.randint(0, 256, plain.key.shape, generator=gen, dtype=torch.uint8).to(device) for _ in range(2)]
+    turn = (torch.randn(128, 128, generator=gen) / 128**0.5).half().to(device)
+    source = [torch.zeros(3, batch, n, 128, dtype=torch.float16, device=device) for n in (q_heads, heads, heads)]
+    landed = [torch.zeros_like(x) for x in source]
+
+    def three(cache):
+        cache.key.copy_(codes[0]), cache.value.copy_(codes[1])
+        cache.length = 400
+        here, aside = torch.cuda.current_stream(), torch.cuda.Stream()
+        aside.wait_stream(here)
+        with torch.cuda.stream(aside):
+            for to, x in zip(landed, source):
+                to.copy_(x)
+        here.wait_stream(aside)
+        return [cache.decode_step(*(x[i] @ turn if j == 0 else (x[i] @ turn)[:, :, None] for j, x in enumerate(landed))) for i in range(3)]
+
+    def renew():
+        for x in source:
+            x.copy_(torch.randn(x.shape, generator=gen) * (0.2 if x is source[0] else 1.0))
+
+    renew()
+    three(captured)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = three(captured)
+    for _ in range(3):
+        renew()
+        want = three(plain)
+        graph.replay()
+        for i, (out, expected) in enumerate(zip(got, want)):
+            assert torch.equal(out, expected), (i, rel_l2(out, expected))
+        assert torch.equal(captured.key, plain.key) and torch.equal(captured.value, plain.value) and captured.length == plain.length == 403
+        assert not torch.equal(plain.key[:, :, 400:403], codes[0][:, :, 400:403])
+
+
+@pytest.mark.parametrize("rope", [None, 1e6])
 @pytest.mark.parametrize("groups,stages,sub", [(16, 2, 8), (1, 2, 128)])
 def test_a_step_uses_the_buffers_tables_and_window_that_the_cache_has_now(device, groups, stages, sub, rope):
     gen = torch.Generator().manual_seed(8611)
