@@ -176,10 +176,7 @@ attn_rotary_ladder_kernel(const __half *__restrict__ q, const uint8_t *kcodes, c
     // A decode step's new codes come from the kernel before this one, and nothing else that is read here; without one, all may.
     bool waited = false;
     auto wait_once = [&]() {
-        if (!waited) {
-            wait_for_previous_kernel();
-            launch_dependents();
-        }
+        if (!waited) wait_for_previous_kernel();
         waited = true;
     };
     if (step.fresh == 0) wait_once();

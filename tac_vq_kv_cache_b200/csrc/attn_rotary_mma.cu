@@ -132,7 +132,6 @@ attn_rotary_mma_kernel(const __half *__restrict__ q, const uint8_t *kcodes, cons
     // A decode step's new codes and ranges come from the kernel before this one; the tables and the query do not.
     copy_table_rows<kWarps>(tab_u32, ktab + (size_t)h * 2 * 16 * kWords * 8, warp, lane);
     wait_for_previous_kernel();
-    if (gridDim.x * gridDim.y * gridDim.z <= 98u) launch_dependents();
     // positions that some row of the block sees, and this split's share of them
     int lo_all = 0x7fffffff, hi_all = 0;
     for (int r = 0; r < n_rows; ++r) {

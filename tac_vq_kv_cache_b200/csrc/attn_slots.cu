@@ -47,6 +47,7 @@ namespace slots {
 
 constexpr int kThreads = 512, kWarps = kThreads / 32;
 constexpr int kDim = 128, kWords = 256, kRowBytes = 256;
+constexpr unsigned kEarlyBlocks = 98;  // two thirds of a B200's 148 SMs: a third is free for a merge that starts early
 constexpr int kAreaBytes = kWords * kRowBytes;  // score table; histogram of large weights; of small weights
 // 4096 weights of at most 1 x kLarge, or of less than 2^-10 x kSmall, add up below 2^32
 constexpr float kLarge = 1048575.0f, kSmall = 1073740800.0f, kBorder = 0.0009765625f;
@@ -312,10 +313,9 @@ attn_slots_kernel(const __half *__restrict__ q, const uint8_t *kcodes, const uin
 
     // A decode step's new codes and ranges come from the kernel before this one; the tables and the query do not.
     wait_for_previous_kernel();
-    // The next kernel's blocks stay on the SMs that are free when they may start, so they may early only where a third of the SMs is.  us a step,
-    // always / never / so: 2 x 128, 8 rows x 16384 tokens 27.5 / 26.2 / 26.2; 16 x 2 x 8 with one head a KV head, 16 x 396 29.6 / 27.7 / 27.7,
-    // 4 x 466 19.7 / 24.0 / 19.7.
-    if (gridDim.x * gridDim.y * gridDim.z <= 98u) launch_dependents();
+    // us a step, always / never / so: 2 x 128, 8 rows x 16384 tokens 27.4 / 26.1 / 26.1; 16 x 2 x 8 with one head a KV head, 16 x 396 29.6 / 27.7 / 27.7,
+    // 4 x 466 20.1 / 23.9 / 20.1.
+    if (gridDim.x * gridDim.y * gridDim.z <= kEarlyBlocks) launch_dependents();
     const int lo_all = max(seq_start ? seq_start[b] : 0, 0);
     const int hi_all = min(seq_end ? seq_end[b] : (int)T_cap, (int)T_cap);
     const int n_all = hi_all > lo_all ? hi_all - lo_all : 0;
@@ -652,7 +652,7 @@ int attn_slots_splits(int B, int Hq, int Hkv, int G, int S, int64_t visible, int
     return best;
 }
 
-// `after_prologue`: the launch before this one is the prologue of the same decode step, itself launched after everything before it.
+// `after_prologue`: the launch before this one is the prologue of the same decode step, which lets this one start when everything before it has ended.
 int attn_slots_dispatch(const __half *q, const uint8_t *kcodes, const uint8_t *vcodes, const __half *ktab, const __half *vtab,
                         const int32_t *seq_start, const int32_t *seq_end, float *part, __half *out, float *state_out, int B, int Hq,
                         int Hkv, int G, int S, int64_t T_cap, int splits, bool after_prologue, cudaStream_t stream) {

@@ -157,6 +157,13 @@ struct LadderStep {
 // memory that nobody changes while the kernel runs, which the compiler may move above the wait.
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Which kernels let the next one start early, and what that gives (us a step where steps follow one another, with / without):
+//   the first kernel of a step, always: the attention brings its tables in meanwhile;
+//   the scan of the benchmark layout, unless a state is wanted (attn_gsrq.cu), and the merge: the next step begins behind them.  In the merge, ladder of 16 stages, 2 rows
+//   x 4000 tokens 86.7 / 88.2, 1 x 6144 47.5 / 47.8; rotary benchmark layout, 8 x 4000 36.0 / 35.8;
+//   attention over slots with at most kEarlyBlocks blocks (attn_slots.cu): the blocks of a merge stay on the SMs that are free when they may start;
+//   rotary attention never, for the same reason: benchmark layout, 8 x 32768 165.8 / 162.8, 8 x 4000 38.5 / 35.9, 1 x 300 18.0 / 17.9; ladder, 2 x 4000 87.9 / 86.5,
+//   8 x 2000 155.5 / 154.3, 1 x 6144 47.5 / 47.4.
 // The first statement of a kernel that follows as a dependent only to be scheduled early: from here on everything older is there.  As the next
 // kernel may start only now, it may read what is older than this grid before its own wait.
 __device__ __forceinline__ void start_after_previous_kernel() {
