@@ -869,7 +869,7 @@ attn_gsrq_scan_kernel(const uint8_t *kcodes, const uint8_t *vcodes, const uint2 
             }
         }
         if (n_parts == 1) {
-            // in whole lines, as the result may lie in the host's memory
+            // 64 bytes a warp, as the result may lie in the host's memory
             __syncthreads();
             if (out)
                 for (int o = tid; o < kRep * kDim; o += kThreads) out[((size_t)b * Hq + h * kRep) * kDim + o] = result[o];

@@ -27,16 +27,16 @@
 // 2^-19 goes to one bin and what that leaves, in units of 2^-38, to another, which keeps all 24 bits of a weight down to 2^-15.  The sums
 // are exact.
 //
-// Where a cluster's time goes, us after its start, one row with 4096 tokens: tables there 5.9, scores of 64 SMs 27.8, parts exchanged 31.6, weights
-// exchanged 36.9, histograms 40.5, end 44.7.  Scores travel in one exchange with the blocks' maxima, and every block takes the weights of all tokens
+// Where a cluster's time goes, us after its start, one row with 4096 tokens: tables there 5.5, scores of 64 SMs 27.5, parts exchanged 31.5, scores
+// exchanged 36.0, histograms 40.2, end 44.1.  Scores travel in one exchange with the blocks' maxima, and every block takes the weights of all tokens
 // itself, which saves one of four exchanges (2 us); sums in two chains of products and rotary rows in whole channel pairs take 1 us off the scores.
 //
 // A sum of 16 words by the tensor core is no further from the exact one than fp32 adds in order: over 2^20 sums of 4, 8, 12 and 16 normal values,
 // of equal spread and falling by 0.9 and 0.6 a stage, 3.5e-10 to 9.3e-9 in the 2-norm against 3.5e-10 to 1.3e-8, and the same fp16
 // value in every case.
 //
-// us a decode step of 16 stages and 8 KV heads, against attn_rotary_kernel: one row of 6144 tokens with a window of 4096 48 / 107, 600
-// tokens 39 / 103 (27 are the new token's encode), 16384 tokens 120 / 232, 8 x 2000 159 / 225, 16 x 1000 193 / 228; ladder_plan.cuh has the sizes that
+// us a decode step of 16 stages and 8 KV heads, against attn_rotary_kernel: one row of 6144 tokens with a window of 4096 47 / 107, 600
+// tokens 39 / 103 (27 are the new token's encode), 16384 tokens 117 / 232, 8 x 2000 154 / 225, 16 x 1000 184 / 228; ladder_plan.cuh has the sizes that
 // are left to that kernel.  Tables, gathers and products are 16 stages wide for fewer stages too.
 //
 // Semantics replaced: experiments_followup_mistral/evaluate_mistral_longbench.py:112-122 including the rotary step

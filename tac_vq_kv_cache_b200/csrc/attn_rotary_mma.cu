@@ -18,8 +18,8 @@
 // times a token's codes): a warp keeps those of its 8 positions in registers and goes through the block's rows.  A chunk is as
 // long as the score area allows, because each one copies both tables (2 x 128 KB).
 //
-// What bounds it: wavefronts of the L1/shared pipe and the latency between them at 16 warps.  A block of 4856 tokens, in clocks: copies
-// and softmax 16 k (25 k when scattered 16-byte cp.async filled the tables), pass K 44 k (9.2 a token, 6.2 of them wavefronts), pass V 25 k (5.2, of
+// What bounds it: wavefronts of the L1/shared pipe and the latency between them at 16 warps.  A block of 4856 tokens, in clocks: tables,
+// softmax and sums 20 k (29 k when scattered 16-byte cp.async filled the tables), pass K 50 k (10.3 a token, 6.2 of them wavefronts), pass V 25 k (5.2, of
 // which 4.4 are look-ups).  us a decode step with 8 KV heads, 8 rows x 32768: 163 (180 with those copies).  Against a row and at most 4096 tokens a
 // block, before: 8 rows x 32768 183 / 205, a window of 4096 of them 45 / 91, 2 x 65536 115 / 148.
 //

@@ -16,7 +16,7 @@
 //
 // Bound by latency between the phases of a stage at 16 warps an SM.  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
 // stages, rows wanted: 325 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.  Whitened (fp32 words, a third product a
-// half): 3001 fp32 rows x 8 heads, 32 x 4, one stage 51 us against 125 for the fp32 scan of all words.
+// half): 3001 fp32 rows x 8 heads, 32 x 4, one stage 47 us against 125 for the fp32 scan of all words.
 // (Words as fp32 pairs in copies without bank conflicts, two exact chains an instruction: 372 us where this takes 344, as look-ups are scarcer than
 // issue slots.)
 //
@@ -137,7 +137,7 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
     extern __shared__ __align__(1024) unsigned char smem[];
     // Columns of a load from tensor memory.  What is decided by them is registers: 32 at a time made the kernels keep part of a row's state in
     // local memory in every stage.  us, 32 / 16 columns, 32768 rows x 8 heads with rows: 16 x 2 x 8 fp16 441 / 344, 16 x 8 286 / 207, 32 x 4
-    // 436 / 363; whitened 32 x 4, 3001 fp32 rows 106 / 85.  fp32 rows of 8-wide words fit either way: 360 / 383, whitened 73 / 74.  (8 columns: 364
+    // 436 / 363; whitened 32 x 4, 3001 fp32 rows, with the whitening, 106 / 85.  fp32 rows of 8-wide words fit either way: 360 / 383, whitened 73 / 74.  (8 columns: 364
     // where 16 take 344; the next 16 asked for before these are looked at: 368.)
     constexpr int kColumns = DSUB == 8 && sizeof(XT) == 4 ? 32 : 16;
     constexpr size_t kStageBytes = kStage<DSUB, EXACT32>, kExactAt = narrow::kStageBytes + kWordBytes;

@@ -230,8 +230,8 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
     using L = Layout<DSUB>;
     constexpr int kPieces = DSUB / 8, kOwn = kPieces / kShare;
     // Fp32 scores further apart than this many u tell which of two words the exact distances prefer.  Each word's share, in units of 2^-24 u: DSUB
-    // roundings of the exact chain, DSUB / 8 + 3 of the score's sums, one where the norm is subtracted and one in the distance; a hundredth
-    // is left for the bound u itself.  (3.2e-5, twice what is needed at 128, sent 1.8 times as many rows to the chains:
+    // roundings of the exact chain, DSUB / 8 + 3 of the score's sums, one where the norm is subtracted and one in the distance (twice u, but a score is half a
+    // distance); a hundredth is left for the bound u itself, and the term of the norms is twice what it needs.  (3.2e-5, twice what is needed at 128, sent 1.8 times as many rows to the chains:
     // 849 us where it is 815, 16 whitened stages x 2048 rows 181 / 177.)
     constexpr float kClose = 1.01f * 2.0f * (DSUB + DSUB / 8 + 5) * 5.9604645e-8f;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -723,7 +723,6 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                         if ((((half ? listed[1] : listed[0]) >> lane) & 1u) != 0u && k < K) {
                             float dot = 0.0f;
                             auto chain = [&](auto fetch) {
-// (words from L2, 16 whitened stages x 2048 rows: 181 us, two pieces at a time 185; two groups a block would spill)
                                 // words from L2, 16 whitened stages x 2048 rows: 181 us, two pieces at a time 185; with two groups a block four spill
 #pragma unroll (EXACT32 && GROUPS == 1 ? 4 : 2)
                                 for (int p = 0; p < kPieces; ++p) {
