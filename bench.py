@@ -56,9 +56,9 @@ METRIC = "vq_kv_decode_attention_tokens_per_s_at_32k_ctx"
 UNIT = "decode tokens/s (per layer; batch 8, 32768-token context, GQA 32/8, 2x16 code bytes per token and side)"
 WORKLOAD = ("packed-code decode attention, one layer per GPU: batch 8, 32 query / 8 KV heads, head_dim 128, 32768-token context, "
             "K and V as GSRQ 2-stage x 16-group uint8 codes, fp16 tables, fp16 query scaled 1/sqrt(128)")
-# dram__bytes_read.sum + dram__bytes_write.sum of one full-size launch of the scan kernel (one ncu capture of
+# dram__bytes_read.sum + dram__bytes_write.sum of one full-size launch of the scan kernel (mean of two in one ncu capture of
 # this workload): the codes once, the score tables written by the prepare grid and read back, partial states
-SCAN_TRAFFIC_BYTES = 144_018_176
+SCAN_TRAFFIC_BYTES = 146_568_704
 FP32_FMA_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12  # 148 SMs x 128 lanes x 2 flop at the maximum SM clock
 
 
