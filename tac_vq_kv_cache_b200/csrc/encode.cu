@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "encode_rows.cuh"
+#include "narrow_plan.cuh"
 
 #ifndef TACVQ_ENCODE_TC
 #define TACVQ_ENCODE_TC 1  // 0: the kernels of this file alone, without the tensor-core filtered ones
@@ -471,17 +472,6 @@ static int launch_large(const EncodeArgs &a) {
 
 constexpr int kFewRows = 32;  // at or below this many rows a warp per (row, head, group) wins
 
-// Whether 8- and 4-wide groups go to the tcgen05 kernel, whose 148 blocks take four tiles of 128 rows at a time, or to the mma.sync
-// kernel of many small blocks.  The former takes a round's time however few rows its tiles hold, the latter goes by rows: 33000 rows of a
-// (head, group) cost as much as a round.  us of the mma.sync / tcgen05 kernel, rows not wanted; n = rows x heads x groups:
-//   16 x 8, two stages  8 heads x 250 rows (n 32000) 9.7/8.6, 400 15.8/10.3, 640 21.3/14.9, 1000 30.1/18.5; one head x 1500 (24000) 8.6/10.2, 3000 14.7/10.3
-//   16 x 8, one stage   8 x 250 6.6/6.6, 400 10.8/7.8, 640 14.4/10.6; 1 x 1500 6.1/7.5, 3000 10.1/7.4
-//   32 x 4, one stage   8 x 130 (33280) 10.2/9.9, 250 11.4/10.1, 400 18.6/14.1, 1000 31.3/20.0; 1 x 1000 (32000) 6.7/7.7, 1500 10.0/7.9
-static bool narrow_pays(int64_t rows, int64_t pairs) {
-    const int64_t rounds = ((rows + 127) / 128 * pairs + 4 * 148 - 1) / (4 * 148);
-    return rows * pairs >= 33000 * rounds;
-}
-
 // 32-, 64- and 128-wide groups: a block per (head, group) and four rows while that is at most two blocks per SM, or one and a half
 // for one stage of 32-wide words.  Measured against a launch of 128-row tiles: 256 blocks of 16 x 128 77 us against 107, of 2 x 128 16.5
 // against 19.8, of 2 x 64 12.7 against 14.0, of two stages of 32 11.2 against 12.8, of one 8.4 against 7.6 (192 blocks 7.4 against
@@ -502,7 +492,7 @@ static int dispatch_d(const EncodeArgs &a) {
             }
         }
         if (TACVQ_ENCODE_TC && (a.D / a.G == 8 || a.D / a.G == 4)) {
-            if (narrow_pays((int64_t)a.B * a.T, (int64_t)a.H * a.G)) {
+            if (narrow::pays((int64_t)a.B * a.T, (int64_t)a.H * a.G, a.S, 148)) {
                 const int st = encode_narrow_launch(a);
                 if (st != TACVQ_ERR_UNSUPPORTED) return st;
             }

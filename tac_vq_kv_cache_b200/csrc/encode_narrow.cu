@@ -24,13 +24,13 @@
 // src/jointkv/cq_tac.py:86-105.
 
 #include "common.cuh"
+#include "narrow_plan.cuh"
 
 namespace tacvq {
 
 namespace narrow {
 
-constexpr int kRows = 128, kGroups = 4, kThreads = kRows * kGroups, kHalf = kMaxWords / 2;
-constexpr uint32_t kSpan = 128;  // tiles
+constexpr int kThreads = kRows * kGroups, kHalf = kMaxWords / 2;
 constexpr size_t kWordBytes = kMaxWords * 32, kSeedBytes = kMaxWords * 32, kNormBytes = kMaxWords * 4;
 constexpr size_t kStageBytes = kWordBytes + kSeedBytes + kNormBytes;  // (word | word), seeds, |word|^2
 // fp32 words: their fp16 rounding takes the place of the words above; what it leaves follows, (low | 0), and the words themselves
@@ -133,7 +133,7 @@ template <int DSUB, typename XT, bool EXACT32>
 __global__ void __launch_bounds__(kThreads, 1)
 encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t sxt, const void *__restrict__ tables_in,
                      const __half *__restrict__ plain, const float *__restrict__ sqnorm_in, uint8_t *__restrict__ codes, void *__restrict__ recon, int recon_dtype,
-                     int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap, int vec_ok, int spins) {
+                     int B, int H, int T, int G, int S, int K, int64_t t0, int64_t T_cap, int vec_ok, int last_shift, int spins) {
     extern __shared__ __align__(1024) unsigned char smem[];
     // Columns of a load from tensor memory.  What is decided by them is registers: 32 at a time made the kernels keep part of a row's state in
     // local memory in every stage.  us, 32 / 16 columns, 32768 rows x 8 heads with rows: 16 x 2 x 8 fp16 441 / 344, 16 x 8 286 / 207, 32 x 4
@@ -201,17 +201,17 @@ encode_narrow_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t
     // sectors, are then read and written while the row is in L2.
 #pragma unroll 1
     for (uint32_t span = 0; span < tiles; span += kSpan) {
-    const uint32_t wide = min(kSpan, tiles - span);
+    const uint32_t wide = min((uint32_t)kSpan, tiles - span);
     // Blocks get turns, a tile for every group of threads: where a block's part of a pair was any number of tiles, groups idled at its end.  With that
-    // and spans of 64 tiles, us, 16 x 2 x 8 with rows, 32768 rows x 8 heads 344 / 325 (fp32 rows 359 / 318), 16384 rows 157 / 149, 700 rows
-    // 23.6 / 22; 32 x 4, 32768 rows 362 / 316.  From 9 to 31 tiles a pair the coarser parts cost what they save: 3333 rows 47.6 / 50.1.
-    const uint32_t unit = wide > 2 * kGroups && wide < 8 * kGroups ? 1u : (uint32_t)kGroups, units = (wide + unit - 1) / unit;
+    // and spans of 64 tiles, us, 16 x 2 x 8 with rows, 32768 rows x 8 heads 344 / 325 (fp32 rows 359 / 318), 16384 rows 157 / 149; 32 x 4, 32768
+    // rows 362 / 316.  Smaller units, and fewer blocks, for a call (or the end of one) of less than a span: narrow_plan.cuh.
+    const uint32_t shift = wide == kSpan ? 2u : (uint32_t)last_shift, units = (wide + (1u << shift) - 1) >> shift;
     const int64_t work = (int64_t)pairs * units, end = work * (blockIdx.x + 1) / gridDim.x;
 #pragma unroll 1
     for (int64_t at = work * blockIdx.x / gridDim.x; at < end;) {
         const int hg = (int)(at / units), h = hg / G, g = hg % G;
         const uint32_t unit0 = (uint32_t)(at - (int64_t)hg * units), mine = (uint32_t)min((int64_t)(units - unit0), end - at);
-        const uint32_t tile0 = span + unit0 * unit, tile1 = span + min(wide, (unit0 + mine) * unit);  // of this pair, for this block
+        const uint32_t tile0 = span + (unit0 << shift), tile1 = span + min(wide, (unit0 + mine) << shift);  // of this pair, for this block
         // ---- the pair's tables ----
         __syncthreads();  // the previous pair's are no longer read
         if (tid < S) cc_tops[tid] = 0;
@@ -488,26 +488,18 @@ int encode_narrow_launch(const EncodeArgs &a) {
     if (a.recon != nullptr && (reinterpret_cast<uintptr_t>(a.recon) & 15u) != 0) return TACVQ_ERR_UNSUPPORTED;
     const int64_t rows = (int64_t)a.B * a.T;
     if (rows >= (int64_t)1 << 31) return TACVQ_ERR_UNSUPPORTED;
-    const int64_t tiles = (rows + kRows - 1) / kRows, all_tiles = tiles * a.H * a.G;
+    const int64_t tiles = (rows + kRows - 1) / kRows;
     const int elem = a.x_dtype == TACVQ_F16 ? 2 : 4, vec = sub * elem < 16 ? sub * elem : 16, per_vec = vec / elem;
     const int vec_ok = (reinterpret_cast<uintptr_t>(a.x) % vec) == 0 && a.sxb % per_vec == 0 && a.sxh % per_vec == 0 && a.sxt % per_vec == 0;
     const size_t stage = a.tables_f32 ? (sub == 8 ? kStage<8, true> : kStage<4, true>) : kStageBytes;
     const size_t smem = (size_t)a.S * stage + kFixedBytes + (size_t)a.S * 4;
     if (smem > 227 * 1024) return TACVQ_ERR_UNSUPPORTED;
-    // one block an SM; fewer where that would leave less than a tile for every group
-    int64_t blocks = (all_tiles + kGroups - 1) / kGroups;
-    // Few rows: whole pairs, as copying another pair's words costs more than idle threads.  Whitened 16 x 8, two stages, us with tiles / 4
-    // blocks and so: one head x 33 rows 28.9 / 12.9, eight 32.5 / 16.6.
-    if (tiles < kGroups) {
-        const int64_t pairs = (int64_t)a.H * a.G, turns = (pairs + 147) / 148;
-        blocks = (pairs + turns - 1) / turns;
-    }
-    if (blocks > 148) blocks = 148;
+    const Deal dealt = deal(tiles, (int64_t)a.H * a.G, 148);
     auto launch = [&](auto kernel, auto *xp) -> int {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        kernel<<<(unsigned)blocks, kThreads, smem, a.stream>>>(xp, a.sxb, a.sxh, a.sxt, a.tables, a.recon_tables, a.sqnorm, a.codes, a.recon,
-                                                               a.recon_dtype, a.B, a.H, a.T, a.G, a.S, a.K, a.t0, a.T_cap, vec_ok,
+        kernel<<<(unsigned)dealt.blocks, kThreads, smem, a.stream>>>(xp, a.sxb, a.sxh, a.sxt, a.tables, a.recon_tables, a.sqnorm, a.codes, a.recon,
+                                                               a.recon_dtype, a.B, a.H, a.T, a.G, a.S, a.K, a.t0, a.T_cap, vec_ok, dealt.shift,
                                                                a.wait_spins < 0 ? kSpins : a.wait_spins);
         return launch_status();
     };

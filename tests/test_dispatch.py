@@ -21,6 +21,7 @@ STAND_INS = r"""
 #include <string>
 #include "common.cuh"
 #include "ladder_plan.cuh"
+#include "narrow_plan.cuh"
 namespace {
 std::string calls;
 std::map<std::string, int> told;  // status, or number of splits
@@ -36,6 +37,11 @@ extern "C" __attribute__((visibility("default"))) void stand_in_reset() { calls.
 extern "C" __attribute__((visibility("default"))) void stand_in_tell(const char *name, int value) { told[name] = value; }
 extern "C" __attribute__((visibility("default"))) int ladder_splits(int B, int Hq, int Hkv, int S, int64_t T_cap, int64_t visible) {
     return tacvq::ladder::plan(B, Hq, Hkv, S, T_cap, visible, 148, 15).splits;
+}
+extern "C" __attribute__((visibility("default"))) int narrow_pays(int64_t rows, int64_t pairs, int stages) { return tacvq::narrow::pays(rows, pairs, stages, 148); }
+extern "C" __attribute__((visibility("default"))) void narrow_deal(int64_t tiles, int64_t pairs, int *out) {
+    const tacvq::narrow::Deal dealt = tacvq::narrow::deal(tiles, pairs, 148);
+    out[0] = dealt.blocks, out[1] = 1 << dealt.shift, out[2] = dealt.rounds, out[3] = dealt.visits;
 }
 namespace tacvq {
 int encode_dispatch(const EncodeArgs &) { return called("encode"); }
@@ -176,3 +182,51 @@ def test_ladders_go_to_the_kernel_that_is_quicker_for_them(library):
     for visible in (1, 4096, 4097):
         splits = library.ladder_splits(1, 32, 8, 16, 262144, visible)
         assert splits >= 1 and -(-visible // splits) <= 4096
+
+
+# us a call of fp16 rows with rows wanted, through the mma.sync / the tcgen05 kernel of 8- and 4-wide groups; groups, stages, heads, rows
+NARROW_TIMES = """
+16 1 1 1500 6.2 7.1; 16 1 1 2250 7.2 7.4; 16 1 4 520 7.0 7.8; 16 1 8 256 7.0 7.2; 16 1 8 300 10.0 7.9; 16 1 8 520 12.0 10.0; 16 1 32 128 11.8 16.6
+32 1 2 520 7.3 7.4; 32 1 4 300 10.1 7.4; 32 1 16 130 16.4 16.8; 16 1 16 700 27.5 17.9; 16 2 1 1500 8.7 9.3; 16 2 1 2250 10.3 9.5; 16 2 2 700 8.7 9.2
+16 2 4 520 10.1 10.2; 16 2 8 300 14.1 10.2; 16 2 8 1030 31.9 19.8; 16 2 32 90 17.6 23.0; 16 2 32 130 24.0 25.8; 16 3 4 450 13.2 11.5; 16 3 8 190 11.2 11.5
+16 4 2 520 11.8 13.6; 16 4 4 300 13.9 13.6; 16 4 4 450 23.0 13.5; 16 4 16 128 22.6 20.3; 16 8 2 512 19.9 22.4; 16 8 4 300 36.4 22.0
+"""
+
+
+def test_narrow_groups_go_to_the_kernel_that_is_quicker_for_them(library):
+    """Or is no more than an eighth behind it."""
+    library.narrow_pays.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int]
+    for line in NARROW_TIMES.replace("\n", ";").split(";"):
+        if line.strip():
+            groups, stages, heads, rows, small, tiled = map(float, line.split())
+            taken = library.narrow_pays(int(rows), int(groups * heads), int(stages))
+            assert (tiled if taken else small) <= 1.125 * min(small, tiled), line
+
+
+@pytest.mark.parametrize("pairs", [1, 3, 16, 17, 64, 100, 128, 256, 512, 777])
+def test_narrow_tiles_are_dealt_out_once_each(library, pairs):
+    """As the kernel walks its part: span by span, pair by pair.  No block has more rounds and tables than the plan counts with."""
+    library.narrow_deal.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p]
+    plan = (ctypes.c_int * 4)()
+    for tiles in (*range(1, 34), 47, 63, 94, 127, 128, 129, 140, 256, 260):
+        library.narrow_deal(tiles, pairs, plan)
+        blocks, last_unit, rounds, visits = plan
+        assert 1 <= blocks <= 148 and last_unit in (1, 2, 4)
+        for span in range(0, tiles, 128):
+            wide = min(128, tiles - span)
+            unit = 4 if wide == 128 else last_unit
+            units = -(-wide // unit)
+            seen = [0] * (pairs * wide)
+            for block in range(blocks):
+                at, end, own = pairs * units * block // blocks, pairs * units * (block + 1) // blocks, []
+                while at < end:
+                    pair, first = divmod(at, units)
+                    mine = min(units - first, end - at)
+                    begin, stop = first * unit, min(wide, (first + mine) * unit)
+                    for tile in range(begin, stop):
+                        seen[pair * wide + tile] += 1
+                    own.append(stop - begin)
+                    at += mine
+                if wide < 128 or tiles == 128:
+                    assert len(own) <= visits and sum(-(-n // 4) for n in own) <= rounds, (tiles, block)
+            assert set(seen) == {1}, tiles

@@ -479,6 +479,24 @@ def test_narrow_groups_where_the_parts_of_a_block_change(device, heads, tokens, 
 
 
 @pytest.mark.parametrize(
+    "heads,tokens,sub,groups,stages",
+    [(4, 520, 8, 16, 2), (1, 2250, 8, 16, 1), (1, 17000, 8, 16, 2), (9, 385, 4, 32, 1), (3, 1300, 8, 16, 4), (2, 700, 4, 32, 3), (37, 128, 8, 8, 2), (19, 640, 4, 16, 1)],
+)
+def test_narrow_tiles_dealt_out_by_one_two_or_four(device, heads, tokens, sub, groups, stages):
+    """Fewer blocks than SMs and as many; parts that end inside a pair; a short last unit; whitened words, which always go to this kernel."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(heads * tokens)
+    tables = make_tables(gen, heads, stages, groups, sub, [0.5 * 0.8**s for s in range(stages)])
+    w = torch.eye(sub).expand(heads, groups, sub, sub) + 0.3 * torch.randn(heads, groups, sub, sub, generator=gen) / sub**0.5
+    for dtype in (torch.float16, torch.float32):
+        states = make_states(gen, (1, heads, tokens, sub * groups), dtype)
+        for want, arguments in ((C.encode(states, tables), {}), (C.encode_whitened(states, tables, w), {"whitener": w.to(device)})):
+            codes, recon = ops.encode(states.to(device), tables.to(device), **arguments)
+            assert torch.equal(codes.cpu(), want[0]) and torch.equal(recon.cpu(), want[1])
+    assert ops.encode_tensor_memory_timeouts(device) == 0
+
+
+@pytest.mark.parametrize(
     "batch,tokens,sub,groups,stages,words,depth,dtype",
     [
         (1, 1025, 8, 16, 2, 256, None, torch.float16),
