@@ -173,7 +173,7 @@ encode_small_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t 
 // the same first-minimum as a sequential scan.  Arithmetic per distance is identical to the kernels
 // above, so the codes are too.
 
-template <int DSUB, typename XT>
+template <int DSUB, typename XT, bool CONSTANT>
 __device__ __forceinline__ void encode_row_unit(const XT *x, int64_t sxb, int64_t sxh, int64_t sxt,
                                                 const __half *tables, const float *sqnorm_in,
                                                 uint8_t *__restrict__ codes, void *__restrict__ recon, int recon_dtype, int H,
@@ -191,7 +191,7 @@ __device__ __forceinline__ void encode_row_unit(const XT *x, int64_t sxb, int64_
     }
     for (int s = 0; s < S; ++s) {
         const int64_t base = (((int64_t)h * S + s) * G + g) * K;
-        const int arg = nearest_word_in_warp<DSUB>(res, tables + base * DSUB, sqnorm_in ? sqnorm_in + base : nullptr, K, lane);
+        const int arg = nearest_word_in_warp<DSUB, CONSTANT>(res, tables + base * DSUB, sqnorm_in ? sqnorm_in + base : nullptr, K, lane);
 #pragma unroll
         for (int i = 0; i < DSUB; ++i) {
             const float w = __half2float(tables[(base + arg) * DSUB + i]);
@@ -218,7 +218,7 @@ encode_rows_kernel(const XT *__restrict__ x, int64_t sxb, int64_t sxh, int64_t s
     const int lane = threadIdx.x & 31;
     const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (unit >= (int64_t)B * T * H * G) return;
-    encode_row_unit<DSUB, XT>(x, sxb, sxh, sxt, tables, sqnorm_in, codes, recon, recon_dtype, H, T, G, S, K, t0, T_cap, unit, lane);
+    encode_row_unit<DSUB, XT, true>(x, sxb, sxh, sxt, tables, sqnorm_in, codes, recon, recon_dtype, H, T, G, S, K, t0, T_cap, unit, lane);
 }
 
 // One decode step's bookkeeping in a single launch: the new rows of K and of V are encoded in place (a
@@ -244,7 +244,7 @@ decode_prologue_kernel(const XT *k_rows, const XT *v_rows, int64_t sxb, int64_t 
     const bool value_side = unit >= units;
     if (value_side) unit -= units;
     if (unit >= units) return;
-    encode_row_unit<DSUB, XT>(value_side ? v_rows : k_rows, sxb, sxh, sxt, value_side ? vtab : ktab, nullptr,
+    encode_row_unit<DSUB, XT, false>(value_side ? v_rows : k_rows, sxb, sxh, sxt, value_side ? vtab : ktab, nullptr,
                               value_side ? vcodes : kcodes, nullptr, TACVQ_F16, H, T, G, S, K, t0, T_cap, unit, lane);
 }
 

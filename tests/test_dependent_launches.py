@@ -96,4 +96,7 @@ def test_the_rows_and_tables_of_a_step_are_not_constant_memory_to_its_first_kern
     assert READ_THROUGH[name] <= set(declared)
     for word in READ_THROUGH[name]:
         assert "__restrict__" not in declared[word], declared[word].strip()
+    body = re.sub(r"if constexpr \(CONSTANT\)[^;]*;", "", body)
     assert "__ldg" not in body and ".nc" not in body
+    ((_, prologue, _),) = [found[1:] for found in _kernels() if found[0] == "decode_prologue_kernel"]
+    assert re.findall(r"encode_row_unit<[^>]*>", prologue) == ["encode_row_unit<DSUB, XT, false>"]
