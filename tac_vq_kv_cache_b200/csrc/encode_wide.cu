@@ -789,8 +789,20 @@ encode_wide_kernel(const Args a, const __grid_constant__ CUtensorMap table_map) 
                 if constexpr (EXACT32 && DSUB == 128 && GROUPS == 1) {
                     // 16 bytes of 32 words a load are 32 lines; the words of 32 rows together are 4 lines a load.  Whole calls, us, 16 stages x 2048
                     // fp16 rows x 8 heads with rows 217 / 206.  (With two groups a block another one hides it: 1154 / 1157 for 4 x 4096 rows.)
+                    // A few rows have few lines, and the exchange costs more: one row, one head, 16 stages 69 / 77, nine rows 75 / 81.
                     float words[kOwn * 8];
-                    fetch_fp32((unsigned long long)(a.words32 + (first + pick) * DSUB), words);
+                    const float *word = a.words32 + (first + pick) * DSUB;
+                    if (__popc(__ballot_sync(0xffffffffu, live)) > 8) {  // the same in the four warps
+                        fetch_fp32((unsigned long long)word, words);
+                    } else if (live) {
+#pragma unroll
+                        for (int m = 0; m < kOwn; ++m)
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(words + 8 * m + 4 * i) = __ldg(reinterpret_cast<const float4 *>(word + 8 * (4 * m + q)) + i);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < kOwn * 8; ++i) words[i] = 0.0f;
+                    }
 #pragma unroll
                     for (int m = 0; m < kOwn; ++m) {
 #pragma unroll

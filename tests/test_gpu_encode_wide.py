@@ -125,3 +125,18 @@ def test_rows_near_three_words(device, sub, groups, tokens, dtype, whitened, ali
         want, want_recon = C.encode(states, tables)
         codes, recon = ops.encode(states.to(device), tables.to(device))
     assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
+
+
+@pytest.mark.parametrize("tokens", [1, 8, 9, 40, 41, 136, 137, 300])
+def test_whitened_words_of_few_and_of_many_rows(device, tokens):
+    """Chosen words are fetched row by row where at most eight of 32 neighbouring rows exist, by whole lines otherwise."""
+    from tac_vq_kv_cache_b200 import ops
+
+    gen = torch.Generator().manual_seed(tokens)
+    tables = make_tables(gen, 3, 4, 1, 128, [0.1 * 0.9**s for s in range(4)])
+    w = torch.eye(128).expand(3, 1, 128, 128) + 0.3 * torch.randn(3, 1, 128, 128, generator=gen) / 128**0.5
+    for dtype in (torch.float16, torch.float32):
+        states = torch.randn(1, 3, tokens, 128, generator=gen).to(dtype)
+        want, want_recon = C.encode_whitened(states, tables, w)
+        codes, recon = ops.encode(states.to(device), tables.to(device), whitener=w.to(device))
+        assert torch.equal(codes.cpu(), want) and torch.equal(recon.cpu(), want_recon)
