@@ -15,7 +15,7 @@
 // enter it, so the chip stays full whatever the number of pairs; a table costs about one tile's time.
 //
 // Bound by latency between the phases of a stage at 16 warps an SM.  4 x 8192 fp16 rows x 8 heads, 16 x 8, two
-// stages, rows wanted: 325 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.  Whitened (fp32 words, a third product a
+// stages, rows wanted: 320 us a side, against 572 us for the mma.sync kernel of encode_tc.cu.  Whitened (fp32 words, a third product a
 // half): 3001 fp32 rows x 8 heads, 32 x 4, one stage 47 us against 125 for the fp32 scan of all words.
 // (Words as fp32 pairs in copies without bank conflicts, two exact chains an instruction: 372 us where this takes 344, as look-ups are scarcer than
 // issue slots.)
